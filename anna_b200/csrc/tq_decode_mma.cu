@@ -5,10 +5,11 @@
 //
 //   packed bytes of the tile --bulk copy (cp.async.bulk, mbarrier)--> shared (2 stages per warp); a tile of a 16-token
 //              page is one linear copy issued by one lane, larger pages take six
-//   K codes -> fp16 A fragments in registers: byte-permute (PRMT) table lookups turn 4-bit / 2-bit fields into
-//              centroid values and +-1 signs, two tokens x D/4 coordinates per lane, no shared-memory round trip
-//   S1[16 tok x 8 heads] = centroid(K) . Q1^T      S2 = sign(K) . Q2^T        (2 x D/16 mma.sync m16n8k16, fp16)
-//   score = norm * (S1 + rnorm * S2)   with Q1 = fwht(s1*q) * scaling / sqrt(D)  (times c0 for 1-bit indices)
+//   K codes -> 8-bit A fragments in registers, two tokens x D/4 coordinates per lane, no shared-memory round trip:
+//              4-bit codes through byte-permute (PRMT) table lookups (centroids and signs as bytes), 2- and 3-bit codes
+//              as the bit planes they are made of (a mask leaves one bit in each of four bytes)
+//   S1[16 tok x 8 heads] = centroid(K) . Q1^T      S2 = sign(K) . Q2^T        (mma.sync m16n8k32, 8-bit integers)
+//   score = norm * (S1 + rnorm * S2)   with Q1 = fwht(s1*q) * scaling / D
 //                                           Q2 = fwht(s2*fwht(s1*q)) * scaling * sqrt(pi/2) / D^1.5
 //   online softmax in fp32 on the C fragments; P packed to fp16 and transposed with movmatrix
 //   V codes -> fp16 (magic-number trick) -> (code * scale + zero) in fp16 pairs -> A fragments of V^T
@@ -31,12 +32,6 @@ __device__ int32_t g_tq_mma_faults;  // bumped when a bounded wait on a tile cop
 // Byte permute and logic helpers are plain intrinsics / C so that the compiler can fold the constant selectors and
 // masks into immediates; the packed fp16 arithmetic goes through PTX on raw registers.
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) { return __byte_perm(a, b, sel); }
-__device__ __forceinline__ uint32_t lop3_and_or(uint32_t x, uint32_t mask, uint32_t bits) { return (x & mask) | bits; }
-__device__ __forceinline__ uint32_t hsub2_u32(uint32_t a, uint32_t b) {
-  uint32_t r;
-  asm("sub.rn.f16x2 %0, %1, %2;\n" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
 // Packed fp16 fused multiply-add on raw registers.  (Going through __half2 objects costs a logic operation per call to
 // put the two halves back together.)
 __device__ __forceinline__ uint32_t hfma2_u32(uint32_t a, uint32_t b, uint32_t c) {
@@ -62,13 +57,6 @@ __device__ __forceinline__ uint32_t and_or_regs(uint32_t x, uint32_t mask, uint3
   return r;
 }
 
-// fp16 pair (+-1, +-1) from bits b and b + 16 of x (0 <= b <= 15): a set bit gives +1.  One shift and one logic op,
-// ((x << (15 - b)) & 0x80008000) ^ 0xBC00BC00 with both constants in registers (`sign_bits`, `minus_one`).
-__device__ __forceinline__ uint32_t pm_one_pair(uint32_t x, int b, uint32_t sign_bits, uint32_t minus_one) {
-  uint32_t r;
-  asm("lop3.b32 %0, %1, %2, %3, 0x6A;\n" : "=r"(r) : "r"(x << (15 - b)), "r"(sign_bits), "r"(minus_one));
-  return r;
-}
 // mma.sync m16n8k16 (fp16 in, fp32 accumulate) without the volatile qualifier: a pure function of its operands, so
 // the compiler may interleave the independent accumulation chains of this kernel
 __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -80,6 +68,12 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], u
 // mma.sync m16n8k32 (signed 8-bit in, 32-bit integer accumulate); same C fragment layout as the fp16 shape above
 __device__ __forceinline__ void mma_s8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// the same with unsigned A bytes (one bit of a code plane each)
+__device__ __forceinline__ void mma_u8s8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
       : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
@@ -114,6 +108,13 @@ __device__ __forceinline__ void lds_words(const uint8_t* ptr, uint32_t (&dst)[N]
 // it exits, so "the packed kernel is done" implies "the window kernel is done" for whatever comes next in the stream.
 __device__ __forceinline__ void wait_for_prior_grids() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
+// Larger of two values, NaN if either is: a NaN query must reach the scores although its bytes cannot hold it.
+__device__ __forceinline__ float fmax_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;\n" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -143,15 +144,20 @@ constexpr float kLazyRescale = 8.0f;  // log2 units: probabilities stay below 2^
 template <typename T, int D, int BITS>
 struct TqMmaCfg {
   static constexpr int kSteps = D / 16;
-  // 4-bit key codes are scored as 8-bit integers: one byte permute turns four codes into four centroid bytes, another
-  // into four sign bytes, and the rotated queries are rounded to 8 bits per head (127 steps up to their largest
-  // coordinate) -- about a third of the instructions of the fp16 expansion the 2- and 3-bit formats use
-  static constexpr bool kInt8Keys = BITS == 4;
+  // Keys are scored as 8-bit integers against rotated queries that are split into a coarse and a fine byte.  4-bit
+  // codes: one byte permute turns four codes into four centroid bytes, another into four sign bytes.  2- and 3-bit
+  // codes: their centroids are linear in the code's bits (+-c0; +-c0 and +-c1 by symmetry), so each bit plane is
+  // multiplied by the query bytes as it is -- a mask leaves one bit in each of four bytes, which is four coordinates of
+  // a fragment for one logic operation -- and the planes are weighted with the exact centroids afterwards.  Against the
+  // fp16 fragments of +-1 (a shift and a logic operation per two coordinates) and 11-bit queries this was: 64 ragged rows
+  // of 4-32 K tokens, 2 bits, head_dim 256: 247 -> 212 us; 128 rows of 0.5-16 K, 3 bits, head_dim 128: 261 -> 253 us.
+  static constexpr bool kPlanes = BITS != 4;
   static constexpr int kSteps8 = D / 32;                       // k-steps of the 8-bit score products
-  static constexpr int kFragBytes = kInt8Keys ? 32 * kSteps8 * 16 : 32 * kSteps * 16;  // query fragments of one unit
-  static constexpr int kFragLoBytes = kInt8Keys ? 32 * kSteps8 * 8 : 0;  // second (fine) byte of the rotated queries
-  static constexpr int kConstOffset = kFragBytes + kFragLoBytes;         // per-head factors and the centroid bytes
-  static_assert(!kInt8Keys || kConstOffset + 128 <= 32 * D, "the query scratch of a unit is 32 * D bytes");
+  // query fragments of one unit, then a second array: the fine bytes of Q1 (4-bit codes) or all of Q2 (planes)
+  static constexpr int kFragBytes = 32 * kSteps8 * 16;
+  static constexpr int kFrag2Bytes = 32 * kSteps8 * (kPlanes ? 16 : 8);
+  static constexpr int kConstOffset = kFragBytes + kFrag2Bytes;  // per-head factors (and centroid bytes) behind them
+  static_assert(kConstOffset + kTqQueryConstBytes <= tq_query_unit_bytes(D), "the query scratch of a unit is too small");
   static constexpr int kGroups = D / 32;                       // value group size is 32 on this path
   static constexpr int kKeyBytes = D * BITS / 8;               // packed key bytes per token
   static constexpr int kIdxBytes = BITS == 3 ? D / 4 : kKeyBytes;  // first plane (all of it unless BITS == 3)
@@ -177,9 +183,8 @@ struct TqMmaCfg {
   // behind the working area (which the epilogue reuses): one mbarrier per warp and stage, one valid-token count per tile
   static constexpr int kBarrierBytes = kMmaWarps * kStages * 8;
   static constexpr int kQueryOffset = (kWorkSmem + kBarrierBytes + kMmaWarps * kStages * kTilesPerStep * 4 + 15) / 16 * 16;
-  // 8-bit scoring keeps the query fragments of the CTA in shared memory (a 16-byte and an 8-byte load per k-step
-  // and step) instead of 24 registers per lane
-  static constexpr int kSmemBytes = kQueryOffset + (kInt8Keys ? kFragBytes + kFragLoBytes : 0);
+  // the query fragments of the CTA live in shared memory (two loads per k-step and step) instead of registers
+  static constexpr int kSmemBytes = kQueryOffset + kFragBytes + kFrag2Bytes;
   // bytes of one 16-token tile in the stage (= in a 16-token page chunk, padding excluded)
   static constexpr int kTileDataBytes = kOffZero + 16 * kGroups * 2;
   // per-lane key code words per token (this lane's D/4 coordinates)
@@ -189,32 +194,26 @@ struct TqMmaCfg {
   static_assert(D == 128 || D == 256, "tensor-core TurboQuant decode is built for head_dim 128 and 256");
 };
 
-// Coordinate that lane `tig` feeds into slot k (0..3 = 2tig, 2tig+1, 2tig+8, 2tig+9) of k-step s.
-template <int D, int BITS>
-__device__ __forceinline__ int idx_coord(int tig, int s, int k) {
-  constexpr int kRun = D / 4;
-  if constexpr (BITS == 4) return tig * kRun + 4 * s + k;
-  if constexpr (BITS == 3) return tig * kRun + 8 * (s / 2) + 2 * k + (s % 2);
-  // 1-bit indices: bits 2c of a 16-coordinate word; a register pairs coordinates c and c + 8
-  return tig * kRun + 16 * (s / 4) + 2 * (s % 4) + (k >> 1) + 8 * (k & 1);
+// Bit planes of 2- and 3-bit codes.  A lane holds the codes of its D/4 coordinates (tig * D/4 ...) of a token as words:
+// 16 two-bit fields (2-bit codes; the indices of 3-bit codes) or 32 sign bits (3-bit codes).  Shifted left so that the
+// wanted bits sit at the top of each byte, one mask leaves the bits of the four fields / signs that share a position
+// inside their byte.  Coordinate behind byte `i` of register `r` (0: k 4tig.., 1: k 16 + 4tig..) of k-step `s`:
+template <int D>
+__device__ __forceinline__ int field_plane_coord(int tig, int s, int r, int i) {
+  constexpr int kPairs = D / 128;  // word pairs per lane; s = position * kPairs + pair
+  return tig * (D / 4) + 16 * (2 * (s % kPairs) + r) + 4 * i + s / kPairs;
 }
-template <int D, int BITS>
-__device__ __forceinline__ int sign_coord(int tig, int s, int k) {
-  constexpr int kRun = D / 4;
-  // the two halves of a register take sign bits 16 apart in their word: 4 coordinates (4-bit codes), 8 (2-bit codes)
-  // or 16 (the separate sign plane of 3-bit codes) apart
-  if constexpr (BITS == 4) return tig * kRun + 8 * (s / 2) + 2 * (s % 2) + (k >> 1) + 4 * (k & 1);
-  if constexpr (BITS == 3) return tig * kRun + 32 * (s / 8) + 2 * (s % 8) + (k >> 1) + 16 * (k & 1);
-  return idx_coord<D, BITS>(tig, s, k);
+template <int D>
+__device__ __forceinline__ int sign_plane_coord(int tig, int s, int r, int i) {
+  return tig * (D / 4) + 32 * (s / 4) + 8 * i + 2 * (s % 4) + r;  // s = word * 4 + pair of positions
 }
 
-// Rotates the queries of one (row, kv-head group) and stores them as fp16 B fragments in the register order of the
-// split kernel: [row][group][lane][step][q1 b0, q1 b1, q2 b0, q2 b1].  Q1 = fwht(s1*q) / sqrt(D), Q2 = fwht(s2*fwht(s1*q)) / D.
+// Rotates the queries of one (row, kv-head group), rounds them to a coarse and a fine byte and stores them as B fragments
+// in the register order of the split kernel, with the per-head factors behind them.
 template <typename T, int D, int BITS>
 __global__ void __launch_bounds__(kMmaThreads) tq_prepare_queries_kernel(const TqDecodeParams p) {
   using Cfg = TqMmaCfg<T, D, BITS>;
   constexpr int E = D / 32;
-  constexpr int kSteps = D / 16;
   __shared__ float q_rot[2][8][D];
   __shared__ float q_amax[2][8];
   const int group_tiles = (p.groups + 7) / 8;
@@ -240,19 +239,19 @@ __global__ void __launch_bounds__(kMmaThreads) tq_prepare_queries_kernel(const T
     for (int j = 0; j < E; ++j) {
       const int d = lane * E + j;
       q_rot[0][g][d] = w[j];
-      amax1 = fmaxf(amax1, fabsf(w[j]));
+      amax1 = fmax_nan(amax1, fabsf(w[j]));
       if (p.signs2[d] < 0.0f) w[j] = -w[j];
     }
     warp_fwht<E>(w, lane);
 #pragma unroll
     for (int j = 0; j < E; ++j) {
       q_rot[1][g][lane * E + j] = w[j];
-      amax2 = fmaxf(amax2, fabsf(w[j]));
+      amax2 = fmax_nan(amax2, fabsf(w[j]));
     }
 #pragma unroll
     for (int dl = 1; dl < 32; dl <<= 1) {
-      amax1 = fmaxf(amax1, __shfl_xor_sync(0xffffffffu, amax1, dl));
-      amax2 = fmaxf(amax2, __shfl_xor_sync(0xffffffffu, amax2, dl));
+      amax1 = fmax_nan(amax1, __shfl_xor_sync(0xffffffffu, amax1, dl));
+      amax2 = fmax_nan(amax2, __shfl_xor_sync(0xffffffffu, amax2, dl));
     }
     if (lane == 0) {
       q_amax[0][g] = amax1;
@@ -262,14 +261,14 @@ __global__ void __launch_bounds__(kMmaThreads) tq_prepare_queries_kernel(const T
   __syncthreads();
   // score (log2 units) = norm * (S1 + rnorm * S2) with every constant folded into the fragments:
   //   q.k_hat = norm/D * [Q1.c + sqrt(pi/2)/sqrt(D) * rnorm * Q2.sign],  Q1 = fwht(s1*q), Q2 = fwht(s2*Q1)
-  //   (1-bit indices: the centroids are +-c0 and the fragments carry +-1, so c0 goes into the factor)
   const float inv_sqrt_d = rsqrt_dim_const<D>();
   const float log2e = 1.4426950408889634f;
-  const float f1 = (BITS == 2 ? __ldg(p.centroids + 1) : 1.0f) * p.scaling * log2e * inv_sqrt_d * inv_sqrt_d;
+  const float f1 = p.scaling * log2e * inv_sqrt_d * inv_sqrt_d;
   const float f2 = p.scaling * log2e * 1.2533141373155001f * inv_sqrt_d * inv_sqrt_d * inv_sqrt_d;
-  // every unit owns 32 * D bytes of the scratch
-  uint8_t* unit = reinterpret_cast<uint8_t*>(p.query_frags) + ((int64_t)b * gridDim.x + blockIdx.x) * (32 * D);
-  if constexpr (Cfg::kInt8Keys) {
+  uint8_t* unit = reinterpret_cast<uint8_t*>(p.query_frags) + ((int64_t)b * gridDim.x + blockIdx.x) * tq_query_unit_bytes(D);
+  auto coarse = [](float v, float k) { return max(-127, min(127, __float2int_rn(v * k))); };
+  auto fine = [](float v, float k, int c) { return max(-127, min(127, __float2int_rn((v * k - (float)c) * 254.0f))); };
+  if constexpr (!Cfg::kPlanes) {
     // 8-bit B fragments of m16n8k32: lane (gid, tig) feeds head gid with the coordinates of its code word s,
     // tig * D/4 + 8s + {0..3} in the first register and + {4..7} in the second.  The rotated query is split into a
     // coarse byte (127 steps up to the head's largest coordinate) and a fine byte (the rounding remainder in 1/254
@@ -321,8 +320,6 @@ __global__ void __launch_bounds__(kMmaThreads) tq_prepare_queries_kernel(const T
       }
     }
     __syncthreads();
-    auto coarse = [](float v, float k) { return max(-127, min(127, __float2int_rn(v * k))); };
-    auto fine = [](float v, float k, int c) { return max(-127, min(127, __float2int_rn((v * k - (float)c) * 254.0f))); };
     uint4* out = reinterpret_cast<uint4*>(unit);
     uint2* out_lo = reinterpret_cast<uint2*>(unit + Cfg::kFragBytes);
     for (int item = threadIdx.x; item < 32 * kSteps8; item += kMmaThreads) {
@@ -358,19 +355,66 @@ __global__ void __launch_bounds__(kMmaThreads) tq_prepare_queries_kernel(const T
       reinterpret_cast<int*>(consts)[16 + g] = -total;
     }
   } else {
+    // [s][lane][Q1 coarse b0, b1, Q1 fine b0, b1]   then   [s][lane][Q2 coarse b0, b1, Q2 fine b0, b1]
+    constexpr int kSteps8 = Cfg::kSteps8;
     uint4* out = reinterpret_cast<uint4*>(unit);
-    for (int item = threadIdx.x; item < 32 * kSteps; item += kMmaThreads) {
-      const int ln = item / kSteps;
-      const int s = item % kSteps;
+    uint4* out2 = reinterpret_cast<uint4*>(unit + Cfg::kFragBytes);
+    for (int item = threadIdx.x; item < 32 * kSteps8; item += kMmaThreads) {
+      const int ln = item & 31;
+      const int s = item >> 5;
       const int gid = ln >> 2, tig = ln & 3;
-      const float* r1 = q_rot[0][gid];
-      const float* r2 = q_rot[1][gid];
-      uint4 v;
-      v.x = pack2<__half>(r1[idx_coord<D, BITS>(tig, s, 0)] * f1, r1[idx_coord<D, BITS>(tig, s, 1)] * f1);
-      v.y = pack2<__half>(r1[idx_coord<D, BITS>(tig, s, 2)] * f1, r1[idx_coord<D, BITS>(tig, s, 3)] * f1);
-      v.z = pack2<__half>(r2[sign_coord<D, BITS>(tig, s, 0)] * f2, r2[sign_coord<D, BITS>(tig, s, 1)] * f2);
-      v.w = pack2<__half>(r2[sign_coord<D, BITS>(tig, s, 2)] * f2, r2[sign_coord<D, BITS>(tig, s, 3)] * f2);
-      out[item] = v;
+#pragma unroll
+      for (int which = 0; which < 2; ++which) {
+        const float k = q_amax[which][gid] > 0.0f ? 127.0f / q_amax[which][gid] : 0.0f;
+        uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int d = (BITS == 3 && which == 1) ? sign_plane_coord<D>(tig, s, r, i) : field_plane_coord<D>(tig, s, r, i);
+            const float v = q_rot[which][gid][d];
+            const int c = coarse(v, k);
+            w[r] |= ((uint32_t)c & 0xffu) << (8 * i);
+            w[2 + r] |= ((uint32_t)fine(v, k, c) & 0xffu) << (8 * i);
+          }
+        (which == 0 ? out : out2)[s * 32 + ln] = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    }
+    // Per head, with u = the value of one step of the fine byte and Q the 254 * coarse + fine integers: a plane with
+    // its bits at weight 2^j of a byte gives T = 2^j * sum over set bits of Q.
+    //   sign plane (+1 set, -1 clear, weight 128):  S2 = T * 2u / 128 - u * sum(Q)
+    //   index planes: centroid = z0 + z1 * bit0 + z2 * bit1 (+ z3 * bit0 * bit1, zero for the symmetric codebooks):
+    //   S1 = T0 * z1 * u / 64 (+ T1 * z2 * u / 128 + T01 * z3 * u / 64) + z0 * u * sum(Q)
+    // [0] factor of bit plane 0, [8] of bit plane 1, [16] of both, [24] constant of S1, [32] factor and [40] constant of S2
+    float* consts = reinterpret_cast<float*>(unit + Cfg::kConstOffset);
+    for (int g = warp; g < 8; g += kMmaWarps) {
+      int total[2] = {0, 0};
+#pragma unroll
+      for (int which = 0; which < 2; ++which) {
+        const float k = q_amax[which][g] > 0.0f ? 127.0f / q_amax[which][g] : 0.0f;
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+          const float v = q_rot[which][g][lane + 32 * j];
+          const int c = coarse(v, k);
+          total[which] += 254 * c + fine(v, k, c);
+        }
+        total[which] = __reduce_add_sync(0xffffffffu, total[which]);
+      }
+      if (lane == 0) {
+        const float u1 = q_amax[0][g] * f1 / (127.0f * 254.0f), u2 = q_amax[1][g] * f2 / (127.0f * 254.0f);
+        const float z0 = __ldg(p.centroids), z1 = __ldg(p.centroids + 1) - z0;
+        float z2 = 0.0f, z3 = 0.0f;
+        if constexpr (BITS == 3) {
+          z2 = __ldg(p.centroids + 2) - z0;
+          z3 = (__ldg(p.centroids + 3) - __ldg(p.centroids + 2)) - z1;
+        }
+        consts[g] = z1 * u1 / 64.0f;
+        consts[8 + g] = z2 * u1 / 128.0f;
+        consts[16 + g] = z3 * u1 / 64.0f;
+        consts[24 + g] = z0 * u1 * (float)total[0];
+        consts[32 + g] = u2 / 64.0f;
+        consts[40 + g] = -u2 * (float)total[1];
+      }
     }
   }
 }
@@ -476,63 +520,48 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
   const int lane = threadIdx.x & 31;
   const int gid = lane >> 2;
   const int tig = lane & 3;
-  // Q fragments (softmax scale and log2(e) folded in) were prepared by tq_prepare_queries_kernel in exactly this
-  // lane's register order: [row b][blockIdx.y][lane][step][q1 b0, q1 b1, q2 b0, q2 b1]; fp16 pairs, or bytes with the
-  // per-head factors behind them when the key codes are scored as 8-bit integers
-  constexpr int kQSteps = Cfg::kInt8Keys ? 1 : Cfg::kSteps;
-  uint32_t q1f[kQSteps][2], q2f[kQSteps][2];
+  // Q fragments (softmax scale and log2(e) folded into the factors) were prepared by tq_prepare_queries_kernel in exactly
+  // this lane's register order, with the per-head factors behind them; they go to shared memory once per CTA
+  const uint4* q_frag = reinterpret_cast<const uint4*>(smem_raw + Cfg::kQueryOffset) + lane;                     // [s][lane]
+  const uint2* q_fine = reinterpret_cast<const uint2*>(smem_raw + Cfg::kQueryOffset + Cfg::kFragBytes) + lane;   // 4-bit
+  const uint4* q_frag2 = reinterpret_cast<const uint4*>(smem_raw + Cfg::kQueryOffset + Cfg::kFragBytes) + lane;  // planes
+  (void)q_fine; (void)q_frag2;
   float beta1[2] = {0.0f, 0.0f}, beta2[2] = {0.0f, 0.0f};  // this lane's two heads (columns 2tig, 2tig + 1)
-  int s2_start[2] = {0, 0};
-  uint32_t cent_bytes[2] = {0u, 0u};
-  const uint4* q_coarse = reinterpret_cast<const uint4*>(smem_raw + Cfg::kQueryOffset) + lane;          // [s][lane]
-  const uint2* q_fine = reinterpret_cast<const uint2*>(smem_raw + Cfg::kQueryOffset + Cfg::kFragBytes) + lane;
+  float k_bit1[2] = {0.0f, 0.0f}, k_both[2] = {0.0f, 0.0f}, c_idx[2] = {0.0f, 0.0f}, c_sign[2] = {0.0f, 0.0f};  // planes
+  int s2_start[2] = {0, 0};                                                                                      // 4-bit
+  uint32_t lut[2] = {0u, 0u};  // 4-bit: the centroids as signed bytes, as the query preparation rounded them
+  (void)k_bit1; (void)k_both; (void)c_idx; (void)c_sign; (void)s2_start; (void)lut;
   {
-    const uint8_t* unit = reinterpret_cast<const uint8_t*>(p.query_frags) + ((int64_t)b * gridDim.y + blockIdx.y) * (32 * D);
-    if constexpr (Cfg::kInt8Keys) {
-      // the CTA's query fragments go to shared memory once; every warp reads them after the barrier below
-      const uint4* src = reinterpret_cast<const uint4*>(unit);
-      uint4* dst = reinterpret_cast<uint4*>(smem_raw + Cfg::kQueryOffset);
-      for (int i = threadIdx.x; i < (Cfg::kFragBytes + Cfg::kFragLoBytes) / 16; i += kMmaThreads) dst[i] = __ldg(src + i);
-      const float* consts = reinterpret_cast<const float*>(unit + Cfg::kConstOffset);
+    const uint8_t* unit = reinterpret_cast<const uint8_t*>(p.query_frags) + ((int64_t)b * gridDim.y + blockIdx.y) * tq_query_unit_bytes(D);
+    const uint4* src = reinterpret_cast<const uint4*>(unit);
+    uint4* dst = reinterpret_cast<uint4*>(smem_raw + Cfg::kQueryOffset);
+    for (int i = threadIdx.x; i < (Cfg::kFragBytes + Cfg::kFrag2Bytes) / 16; i += kMmaThreads) dst[i] = __ldg(src + i);
+    const float* consts = reinterpret_cast<const float*>(unit + Cfg::kConstOffset);
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        beta1[c] = __ldg(consts + 2 * tig + c);
+    for (int c = 0; c < 2; ++c) {
+      beta1[c] = __ldg(consts + 2 * tig + c);
+      if constexpr (Cfg::kPlanes) {
+        if constexpr (BITS == 3) {
+          k_bit1[c] = __ldg(consts + 8 + 2 * tig + c);
+          k_both[c] = __ldg(consts + 16 + 2 * tig + c);
+        }
+        c_idx[c] = __ldg(consts + 24 + 2 * tig + c);
+        beta2[c] = __ldg(consts + 32 + 2 * tig + c);
+        c_sign[c] = __ldg(consts + 40 + 2 * tig + c);
+      } else {
         beta2[c] = __ldg(consts + 8 + 2 * tig + c);
         s2_start[c] = __ldg(reinterpret_cast<const int*>(consts) + 16 + 2 * tig + c);
       }
-      cent_bytes[0] = __ldg(reinterpret_cast<const uint32_t*>(consts) + 24);
-      cent_bytes[1] = __ldg(reinterpret_cast<const uint32_t*>(consts) + 25);
-      __syncthreads();
-    } else {
-      const uint4* frag = reinterpret_cast<const uint4*>(unit) + lane * kQSteps;
-#pragma unroll
-      for (int s = 0; s < kQSteps; ++s) {
-        const uint4 v = __ldg(frag + s);
-        q1f[s][0] = v.x; q1f[s][1] = v.y; q2f[s][0] = v.z; q2f[s][1] = v.w;
-      }
     }
+    if constexpr (!Cfg::kPlanes) {
+      lut[0] = pinned_u32(__ldg(reinterpret_cast<const uint32_t*>(consts) + 24), lane);
+      lut[1] = pinned_u32(__ldg(reinterpret_cast<const uint32_t*>(consts) + 25), lane);
+    }
+    __syncthreads();
   }
 
-  // centroid lookup tables for PRMT (up to 8 entries): low bytes and high bytes of the fp16 centroids, or -- 4-bit
-  // codes -- the centroids as signed bytes in lut_lo, as the query preparation rounded them
-  uint32_t lut_lo[2] = {0u, 0u}, lut_hi[2] = {0u, 0u};
-  if constexpr (Cfg::kInt8Keys) {
-    lut_lo[0] = pinned_u32(cent_bytes[0], lane);
-    lut_lo[1] = pinned_u32(cent_bytes[1], lane);
-  } else if constexpr (BITS != 2) {
-    constexpr int kEntries = 1 << (BITS - 1);
-#pragma unroll
-    for (int e = 0; e < kEntries; ++e) {
-      const __half h = __float2half_rn(__ldg(p.centroids + e));
-      const uint32_t bits = (uint32_t)__half_as_ushort(h);
-      lut_lo[e / 4] |= (bits & 0xffu) << (8 * (e % 4));
-      lut_hi[e / 4] |= (bits >> 8) << (8 * (e % 4));
-    }
-    if constexpr (BITS == 3) {  // 4 entries: mirror them so that PRMT may pick from either operand
-      lut_lo[1] = lut_lo[0];
-      lut_hi[1] = lut_hi[0];
-    }
-  }
+  const bool skewed = BITS == 3 && __any_sync(0xffffffffu, k_both[0] != 0.0f || k_both[1] != 0.0f);
+  (void)skewed;
 
   // loop constants held in registers
   // (only the ones this instantiation uses are created)
@@ -540,11 +569,11 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
   const uint32_t magic16 = BITS != 2 ? pinned_u32(0x4C004C00u, lane) : 0u;
   const uint32_t kTwo = BITS == 4 ? pinned_u32(0x02020202u, lane) : 0u;        // 4-bit key codes
   const uint32_t kIdxMask = BITS == 4 ? pinned_u32(0x77777777u, lane) : 0u;
-  const uint32_t kSignBits = BITS != 4 ? pinned_u32(0x80008000u, lane) : 0u;   // +-1 fragments of 2- and 3-bit key codes
-  const uint32_t kMinusOne = BITS != 4 ? pinned_u32(0xBC00BC00u, lane) : 0u;
+  const uint32_t kTop = BITS != 4 ? pinned_u32(0x80808080u, lane) : 0u;        // bit planes of 2- and 3-bit key codes
+  const uint32_t kNext = BITS != 4 ? pinned_u32(0x40404040u, lane) : 0u;
   const uint32_t kTwoBitMask = BITS == 2 ? pinned_u32(0x03000300u, lane) : 0u;  // 2-bit value codes
   const uint32_t kMagic4 = BITS == 2 ? pinned_u32(0x44004400u, lane) : 0u;
-  (void)nib_mask; (void)magic16; (void)kTwo; (void)kIdxMask; (void)kSignBits; (void)kMinusOne; (void)kTwoBitMask;
+  (void)nib_mask; (void)magic16; (void)kTwo; (void)kIdxMask; (void)kTop; (void)kNext; (void)kTwoBitMask;
   (void)kMagic4;
 
   const uint32_t warp_smem_u32 = smem_u32(smem_raw + warp * Cfg::kWarpSmem);
@@ -656,10 +685,6 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
 
     // ---- scores: U independent pairs of accumulation chains ------------------------------------------------------------
     float s1[U][4], s2[U][4];
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) s1[u][r] = s2[u][r] = 0.0f;
     {
       uint32_t iw_lo[U][Cfg::kIdxWords], iw_hi[U][Cfg::kIdxWords];
 #pragma unroll
@@ -682,15 +707,15 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
         }
 #pragma unroll
         for (int s = 0; s < Cfg::kSteps8; ++s) {
-          const uint4 qc = q_coarse[s * 32];  // q1 b0, q1 b1, q2 b0, q2 b1
+          const uint4 qc = q_frag[s * 32];  // q1 b0, q1 b1, q2 b0, q2 b1
           const uint2 qf = q_fine[s * 32];
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             const uint32_t xl = iw_lo[u][s], xh = iw_hi[u][s];
             const uint32_t ml = xl & kIdxMask, mh = xh & kIdxMask;
-            const uint32_t a[4] = {prmt_ptx(lut_lo[0], lut_lo[1], ml), prmt_ptx(lut_lo[0], lut_lo[1], mh),
-                                   prmt_ptx(lut_lo[0], lut_lo[1], ml >> 16),
-                                   prmt_ptx(lut_lo[0], lut_lo[1], mh >> 16)};
+            const uint32_t a[4] = {prmt_ptx(lut[0], lut[1], ml), prmt_ptx(lut[0], lut[1], mh),
+                                   prmt_ptx(lut[0], lut[1], ml >> 16),
+                                   prmt_ptx(lut[0], lut[1], mh >> 16)};
             mma_s8(i1[u], a, qc.x, qc.y);
             if (ANNA_TQ_FINE_QUERY) mma_s8(i1l[u], a, qf.x, qf.y);
           }
@@ -710,56 +735,93 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
             s1[u][r] = (float)(ANNA_TQ_FINE_QUERY ? i1[u][r] * 254 + i1l[u][r] : i1[u][r]) * beta1[r & 1];
             s2[u][r] = (float)i2[u][r] * beta2[r & 1];
           }
-      } else if constexpr (BITS == 2) {
-#pragma unroll
-        for (int s = 0; s < Cfg::kSteps; ++s) {
-          const int h = s % 4;
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const uint32_t xl = iw_lo[u][s / 4], xh = iw_hi[u][s / 4];
-            const uint32_t a[4] = {pm_one_pair(xl, 4 * h, kSignBits, kMinusOne), pm_one_pair(xh, 4 * h, kSignBits, kMinusOne), pm_one_pair(xl, 4 * h + 2, kSignBits, kMinusOne),
-                                   pm_one_pair(xh, 4 * h + 2, kSignBits, kMinusOne)};
-            mma_f16(s1[u], a, q1f[s][0], q1f[s][1]);
-          }
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const uint32_t xl = iw_lo[u][s / 4], xh = iw_hi[u][s / 4];
-            const uint32_t a[4] = {pm_one_pair(xl, 4 * h + 1, kSignBits, kMinusOne), pm_one_pair(xh, 4 * h + 1, kSignBits, kMinusOne), pm_one_pair(xl, 4 * h + 3, kSignBits, kMinusOne),
-                                   pm_one_pair(xh, 4 * h + 3, kSignBits, kMinusOne)};
-            mma_f16(s2[u], a, q2f[s][0], q2f[s][1]);
-          }
-        }
       } else {
-        uint32_t sw_lo[U][Cfg::kSignWords], sw_hi[U][Cfg::kSignWords];
+        // fields: bit 1 of a 2-bit field (the sign, or the index's upper bit) at the top of its byte, bit 0 next to it
+        constexpr int kPairs = Cfg::kIdxWords / 2;
+        int lo_c[U][4], lo_f[U][4], hi_c[U][4], hi_f[U][4];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const uint8_t* signs = st0 + u * Cfg::kStageBytes + Cfg::kOffKey + Cfg::kIdxBytes + tig * (Cfg::kSignWords * 4);
-          lds_words<Cfg::kSignWords>(signs + tok_lo * Cfg::kKeyBytes, sw_lo[u]);
-          lds_words<Cfg::kSignWords>(signs + tok_hi * Cfg::kKeyBytes, sw_hi[u]);
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) lo_c[u][r] = lo_f[u][r] = hi_c[u][r] = hi_f[u][r] = 0;
+#pragma unroll
+        for (int s = 0; s < Cfg::kSteps8; ++s) {
+          const int up = 6 - 2 * (s / kPairs), w = 2 * (s % kPairs);
+          const uint4 q1 = q_frag[s * 32];  // coarse b0, b1, fine b0, b1
+          const uint4 qh = BITS == 2 ? q_frag2[s * 32] : q1;
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const uint32_t x[4] = {iw_lo[u][w] << up, iw_hi[u][w] << up, iw_lo[u][w + 1] << up, iw_hi[u][w + 1] << up};
+            const uint32_t a_lo[4] = {x[0] & kNext, x[1] & kNext, x[2] & kNext, x[3] & kNext};
+            mma_u8s8(lo_c[u], a_lo, q1.x, q1.y);
+            mma_u8s8(lo_f[u], a_lo, q1.z, q1.w);
+            const uint32_t a_hi[4] = {x[0] & kTop, x[1] & kTop, x[2] & kTop, x[3] & kTop};
+            mma_u8s8(hi_c[u], a_hi, qh.x, qh.y);
+            mma_u8s8(hi_f[u], a_hi, qh.z, qh.w);
+          }
         }
+        // 254 * coarse + fine stays below 2^31: |T| <= 128 * 127 * D * 255
 #pragma unroll
-        for (int s = 0; s < Cfg::kSteps; ++s) {
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            s1[u][r] = fmaf((float)(lo_c[u][r] * 254 + lo_f[u][r]), beta1[r & 1], c_idx[r & 1]);
+            const float t = (float)(hi_c[u][r] * 254 + hi_f[u][r]);
+            if constexpr (BITS == 2) s2[u][r] = fmaf(t, beta2[r & 1], c_sign[r & 1]);
+            else s1[u][r] = fmaf(t, k_bit1[r & 1], s1[u][r]);
+          }
+        if constexpr (BITS == 3) {
+          if (skewed) {  // the codebook is not symmetric: a third plane, where both bits are set
+            asm volatile("" ::: "memory");
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+              for (int r = 0; r < 4; ++r) lo_c[u][r] = lo_f[u][r] = 0;
+#pragma unroll
+            for (int s = 0; s < Cfg::kSteps8; ++s) {
+              const int up = 6 - 2 * (s / kPairs), w = 2 * (s % kPairs);
+              const uint4 q1 = q_frag[s * 32];
+#pragma unroll
+              for (int u = 0; u < U; ++u) {
+                const uint32_t x[4] = {iw_lo[u][w] << up, iw_hi[u][w] << up, iw_lo[u][w + 1] << up, iw_hi[u][w + 1] << up};
+                uint32_t a[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) a[i] = x[i] & (x[i] >> 1) & kNext;
+                mma_u8s8(lo_c[u], a, q1.x, q1.y);
+                mma_u8s8(lo_f[u], a, q1.z, q1.w);
+              }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+              for (int r = 0; r < 4; ++r)
+                s1[u][r] = fmaf((float)(lo_c[u][r] * 254 + lo_f[u][r]), k_both[r & 1], s1[u][r]);
+          }
+          uint32_t sw_lo[U][Cfg::kSignWords], sw_hi[U][Cfg::kSignWords];
 #pragma unroll
           for (int u = 0; u < U; ++u) {
-            // 2-bit indices: half-word s / 2 of the lane's run, even (s % 2 == 0) or odd fields
-            const uint32_t wl = iw_lo[u][s / 4] >> (16 * ((s / 2) % 2) + 2 * (s % 2));
-            const uint32_t wh = iw_hi[u][s / 4] >> (16 * ((s / 2) % 2) + 2 * (s % 2));
-            const uint32_t sl = wl & 0x3333u, sh = wh & 0x3333u;
-            const uint32_t lo_l = prmt(lut_lo[0], lut_lo[1], sl), hi_l = prmt(lut_hi[0], lut_hi[1], sl);
-            const uint32_t lo_h = prmt(lut_lo[0], lut_lo[1], sh), hi_h = prmt(lut_hi[0], lut_hi[1], sh);
-            const uint32_t a[4] = {prmt(lo_l, hi_l, 0x5140u), prmt(lo_h, hi_h, 0x5140u), prmt(lo_l, hi_l, 0x7362u),
-                                   prmt(lo_h, hi_h, 0x7362u)};
-            mma_f16(s1[u], a, q1f[s][0], q1f[s][1]);
+            const uint8_t* signs = st0 + u * Cfg::kStageBytes + Cfg::kOffKey + Cfg::kIdxBytes + tig * (Cfg::kSignWords * 4);
+            lds_words<Cfg::kSignWords>(signs + tok_lo * Cfg::kKeyBytes, sw_lo[u]);
+            lds_words<Cfg::kSignWords>(signs + tok_hi * Cfg::kKeyBytes, sw_hi[u]);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) hi_c[u][r] = hi_f[u][r] = 0;
           }
 #pragma unroll
-          for (int u = 0; u < U; ++u) {
-            // sign plane: bits 2h, 2h + 1 (and + 16) of word s / 8, h = s % 8
-            const uint32_t xl = sw_lo[u][s / 8], xh = sw_hi[u][s / 8];
-            const int h = s % 8;
-            const uint32_t a[4] = {pm_one_pair(xl, 2 * h, kSignBits, kMinusOne), pm_one_pair(xh, 2 * h, kSignBits, kMinusOne), pm_one_pair(xl, 2 * h + 1, kSignBits, kMinusOne),
-                                   pm_one_pair(xh, 2 * h + 1, kSignBits, kMinusOne)};
-            mma_f16(s2[u], a, q2f[s][0], q2f[s][1]);
+          for (int s = 0; s < Cfg::kSteps8; ++s) {
+            const int up = 7 - 2 * (s % 4), w = s / 4;
+            const uint4 q2 = q_frag2[s * 32];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              const uint32_t a[4] = {(sw_lo[u][w] << up) & kTop, (sw_hi[u][w] << up) & kTop,
+                                     (sw_lo[u][w] << (up - 1)) & kTop, (sw_hi[u][w] << (up - 1)) & kTop};
+              mma_u8s8(hi_c[u], a, q2.x, q2.y);
+              mma_u8s8(hi_f[u], a, q2.z, q2.w);
+            }
           }
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+              s2[u][r] = fmaf((float)(hi_c[u][r] * 254 + hi_f[u][r]), beta2[r & 1], c_sign[r & 1]);
         }
       }
     }

@@ -29,7 +29,7 @@ struct TqDecodeParams {
   float scaling;
   anna_tq_layout layout;
   FusedCombine fused;
-  void* query_frags;  // scratch for the rotated fp16 query fragments (tensor-core path), or nullptr
+  void* query_frags;  // scratch for the rotated query fragments (tensor-core path), or nullptr
 };
 
 // Tensor-memory split pass (tq_decode_umma.cu): 16-bit cache dtypes, head_dim 128, 3- / 4-bit codes, 16-token pages,
@@ -41,11 +41,16 @@ size_t tq_umma_query_bytes();  // query operand image per (row, kv head) of that
 // the window-ring launch of the tensor-core paths (tq_decode_mma.cu)
 int launch_tq_window_split(const TqDecodeParams& p, int batch, int head_dim, int dtype, cudaStream_t stream);
 
-// Bytes of query scratch the tensor-core paths need per call: 32 * head_dim fragment bytes per (row, kv head, group of
-// 8 query heads) for the mma.sync path, one query operand image per (row, kv head) for the tensor-memory path.
+// Query scratch of one (row, kv head, group of 8 query heads) of the mma.sync path: up to 32 * head_dim fragment bytes (two
+// rotations of 8 heads, a coarse and a fine byte each), then the per-head factors.
+constexpr int kTqQueryConstBytes = 256;
+constexpr __host__ __device__ int tq_query_unit_bytes(int head_dim) { return 32 * head_dim + kTqQueryConstBytes; }
+
+// Bytes of query scratch the tensor-core paths need per call: one unit per (row, kv head, group of 8 query heads) for the
+// mma.sync path, one query operand image per (row, kv head) for the tensor-memory path.
 inline size_t tq_query_scratch_bytes(int batch, int q_heads, int kv_heads, int head_dim) {
   const size_t units = (size_t)batch * kv_heads * ((q_heads / kv_heads + 7) / 8);
-  const size_t frag = (size_t)32 * head_dim;
+  const size_t frag = (size_t)tq_query_unit_bytes(head_dim);
   const size_t image = tq_umma_query_bytes();
   return units * (frag > image ? frag : image);
 }

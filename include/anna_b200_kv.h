@@ -268,7 +268,7 @@ int anna_tq_append(const void* k_new, const void* v_new, int64_t kn_stride_b, in
  * turboquant.py:290-332) instead of from a dense de-quantized copy.
  *   lengths   int64 [B]: total tokens per row (quantized = max(0, L - R), window = min(L, R)); L == 0 gives zeros
  *   query_scratch: optional 16-byte aligned device scratch of at least anna_tq_query_scratch_bytes(B, Hq, Hkv, D)
- *   bytes; the tensor-core path stores the rotated queries there (as fp16 MMA fragments)
+ *   bytes; the tensor-core path stores the rotated queries there (as MMA fragments)
  *   before the split pass.  Without it, or for fp32 caches, head_dim 64, value groups other than 32 or page sizes that
  *   are not a multiple of 16, the CUDA-core path runs.
  *   split-K slots: anna_tq_decode_plan gives the chunk length and the slot count (window chunks first, then the
