@@ -19,10 +19,10 @@ constexpr int kBalancedTileTokens = 16;
 
 // Block-wide exclusive scan of the tiles per row: s_prefix[b] = tiles (over all streams) of the rows before row b,
 // s_prefix[batch] = all tiles.  Returns the largest number of tiles of any single stream.  Ends with a barrier.
-// THREADS = blockDim.x (a multiple of 32); batch <= kBalancedMaxRows.
+// THREADS = blockDim.x (a multiple of 32); batch <= kBalancedMaxRows.  The newest `tail` tokens of a row have no tile here.
 template <int THREADS>
 __device__ __forceinline__ int balanced_scan(const int64_t* visible_lengths, int64_t max_len, int batch,
-                                             int streams_per_row, int* s_prefix) {
+                                             int streams_per_row, int* s_prefix, int tail) {
   constexpr int kWarps = THREADS / 32;
   constexpr int kRowsPerThread = (kBalancedMaxRows + THREADS - 1) / THREADS;
   __shared__ int s_warp_sum[kWarps];
@@ -38,7 +38,7 @@ __device__ __forceinline__ int balanced_scan(const int64_t* visible_lengths, int
     int tiles = 0;
     if (i < rpt && b < batch) {
       int64_t len = visible_lengths ? visible_lengths[b] : max_len;
-      len = max((int64_t)0, min(len, max_len));
+      len = max((int64_t)0, min(len, max_len) - tail);
       tiles = (int)((len + kBalancedTileTokens - 1) / kBalancedTileTokens);
     }
     local[i] = tiles;
@@ -82,58 +82,22 @@ __device__ __forceinline__ int balanced_share(int total, int units, int max_tile
   return max(share, (max_tiles + chunk_capacity - 2) / (chunk_capacity - 1));
 }
 
-// Position in the tile line, resolved to (row, stream of the row, tile of the stream).  All fields are warp-uniform.
-struct TileCursor {
-  int pos;        // index in the line
-  int b;          // row
-  int row_first;  // s_prefix[b]
-  int n;          // tiles of every stream of row b
-  int stream;     // stream inside the row
-  int tile;       // tile inside the stream
-
-  // Point at tile `at` (0 <= at < s_prefix[batch]).
-  __device__ __forceinline__ void seek(const int* s_prefix, int batch, int streams_per_row, int at) {
-    int lo = 0, hi = batch;  // invariant: s_prefix[lo] <= at < s_prefix[hi]
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (s_prefix[mid] <= at) lo = mid; else hi = mid;
-    }
-    pos = at;
-    b = lo;
-    row_first = s_prefix[b];
-    n = (s_prefix[b + 1] - row_first) / streams_per_row;
-    stream = (at - row_first) / n;
-    tile = (at - row_first) - stream * n;
-  }
-  // Step to the next tile of the line; the caller guarantees pos + 1 < s_prefix[batch] before using the fields.
-  __device__ __forceinline__ void advance(const int* s_prefix, int streams_per_row, int line_end) {
-    ++pos;
-    if (++tile < n) return;
-    tile = 0;
-    if (++stream < streams_per_row) return;
-    stream = 0;
-    if (pos >= line_end) return;  // past the end: fields are not used any more
-    do { ++b; } while (s_prefix[b + 1] <= pos);
-    row_first = s_prefix[b];
-    n = (s_prefix[b + 1] - row_first) / streams_per_row;
-  }
-  __device__ __forceinline__ int stream_first() const { return row_first + stream * n; }
-};
-
 // Calls zero_row(b) for this CTA's share of the rows without any visible key, then
 // segment(b, stream, t0, t1, slot, partials_of_stream) for each piece of this CTA's tile range, in order.
 // THREADS = blockDim.x (a multiple of 32, at most 1024 / 8 rows per thread); all threads of the CTA must call it and
-// `segment` may synchronise the CTA.
+// `segment` may synchronise the CTA.  `tail`: the newest tokens of every row that the line leaves out; `min_tiles`: the
+// smallest share of a CTA.
 template <int THREADS, typename ZeroFn, typename SegmentFn>
 __device__ __forceinline__ void balanced_for_each_segment(const int64_t* visible_lengths, int64_t max_len, int batch,
                                                           int streams_per_row, int chunk_capacity, ZeroFn&& zero_row,
-                                                          SegmentFn&& segment) {
+                                                          SegmentFn&& segment, int tail = 0,
+                                                          int min_tiles = kBalancedMinTiles) {
   __shared__ int s_prefix[kBalancedMaxRows + 1];
-  const int max_tiles = balanced_scan<THREADS>(visible_lengths, max_len, batch, streams_per_row, s_prefix);
+  const int max_tiles = balanced_scan<THREADS>(visible_lengths, max_len, batch, streams_per_row, s_prefix, tail);
   const int total = s_prefix[batch];
   auto row_len = [&](int b) -> int {
     int64_t len = visible_lengths ? visible_lengths[b] : max_len;
-    return (int)max((int64_t)0, min(len, max_len));
+    return (int)max((int64_t)0, min(len, max_len) - tail);
   };
 
   // rows without a visible key have no tile: their zero outputs are dealt round-robin
@@ -141,7 +105,7 @@ __device__ __forceinline__ void balanced_for_each_segment(const int64_t* visible
     if (s_prefix[b + 1] == s_prefix[b]) zero_row(b);
   if (total == 0) return;
 
-  const int tpc = balanced_share(total, (int)gridDim.x, max_tiles, chunk_capacity, kBalancedMinTiles);
+  const int tpc = balanced_share(total, (int)gridDim.x, max_tiles, chunk_capacity, min_tiles);
   int pos = (int)min((int64_t)blockIdx.x * tpc, (int64_t)total);
   const int end = (int)min((int64_t)pos + tpc, (int64_t)total);
   if (pos >= end) return;

@@ -338,6 +338,7 @@ static int tq_paged_decode_impl(const void* q, int64_t q_stride_b, int64_t q_str
     return set_error(ANNA_ERR_WORKSPACE, "split-K scratch holds %d chunks per head, %d needed", chunk_capacity, num_chunks);
   SplitWorkspace ws{partial_stats, partial_values, chunk_capacity};
   p.stats = ws.stats; p.values = ws.values;
+  p.given_chunks = chunk_tokens_in > 0;
   p.chunk_tokens = chunk_tokens; p.num_chunks = num_chunks; p.chunk_capacity = chunk_capacity;
   p.num_window_chunks = (residual_len + chunk_tokens - 1) / chunk_tokens;
   {
@@ -348,6 +349,7 @@ static int tq_paged_decode_impl(const void* q, int64_t q_stride_b, int64_t q_str
   }
   if (tq_split_mma_applicable(p, head_dim, dtype)) {
     const bool umma = tq_split_umma_applicable(p, head_dim, bits, dtype);
+    p.window_arrives = umma;
     if (split_counters != nullptr && num_chunks <= kFusedMaxChunks) {
       p.fused = FusedCombine{split_counters, out, out_stride_b, out_stride_h, gate, gate_stride_b, gate_stride_h};
       for (int i = 0; i < num_peers; ++i) p.fused.peers[i] = peer_outputs[i];
@@ -438,7 +440,7 @@ extern "C" int anna_tq_decode_plan(int batch, int kv_heads, int64_t max_blocks, 
   // (measured: 64 x 32768-token rows run 4.5 % faster with 4096-token chunks than with 1024-token ones, and every
   // problem that is short of CTAs gets slower when the chunks shrink further).
   const int64_t streams = (int64_t)batch * kv_heads;
-  int64_t ct = 4096;
+  int64_t ct = kTqLongestChunk;
   while (ct > 64 && streams * ((max_q + residual_len + ct - 1) / ct) < 148 * 8) ct >>= 1;
   *chunk_tokens = (int)ct;
   *num_chunks = (int)((residual_len + ct - 1) / ct + (max_q + ct - 1) / ct);

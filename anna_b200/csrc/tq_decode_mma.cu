@@ -17,6 +17,7 @@
 //
 // The K-dimension slots of the two score products are free to permute, so each lane takes the coordinates whose
 // codes it can unpack with the fewest instructions; Q1 / Q2 fragments are gathered with the same permutation.
+#include "balanced_schedule.cuh"
 #include "dense_mma_body.cuh"
 #include "mbarrier_utils.cuh"
 #include "tq_common.cuh"
@@ -135,9 +136,6 @@ __device__ __forceinline__ float fast_exp2(float x) {
 #endif
 #ifndef ANNA_TQ_FINE_QUERY
 #define ANNA_TQ_FINE_QUERY 1
-#endif
-#ifndef ANNA_TQ_OVERLAP_WINDOW
-#define ANNA_TQ_OVERLAP_WINDOW 1
 #endif
 constexpr float kLazyRescale = 8.0f;  // log2 units: probabilities stay below 2^8, well inside fp16
 
@@ -424,12 +422,10 @@ __global__ void __launch_bounds__(kMmaThreads) tq_prepare_queries_kernel(const T
 template <typename T, int D>
 __global__ void __launch_bounds__(kMmaThreads, MmaCfg<D>::kMinBlocks) tq_window_split_mma_kernel(const TqDecodeParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-#if ANNA_TQ_OVERLAP_WINDOW
   // The packed-chunk kernel that follows in the stream reads nothing this kernel writes before the arrival counters
   // say so, and each of its CTAs waits for this grid to complete before it counts itself in or exits, so it may start
   // as soon as every CTA here has been scheduled.
   asm volatile("griddepcontrol.launch_dependents;\n" ::);
-#endif
   const int slot = blockIdx.x;
   const int group_tiles = (p.groups + 7) / 8;
   const int kvh = blockIdx.y / group_tiles;
@@ -464,57 +460,35 @@ __global__ void __launch_bounds__(kMmaThreads, MmaCfg<D>::kMinBlocks) tq_window_
   dp.chunk_tokens = p.chunk_tokens; dp.num_chunks = p.num_chunks; dp.chunk_capacity = p.chunk_capacity;
   dp.scaling = p.scaling;
   dp.fused = p.fused;
+  if (!p.window_arrives && Lq > 0) dp.fused.counters = nullptr;  // the packed CTAs wait for this grid before they count
   const int t0 = Lq + slot * p.chunk_tokens;
   const int t1 = min(len, t0 + p.chunk_tokens);
   dense_split_mma_body<T, D>(dp, smem_raw, b, kvh, g0, g_count, t0, t1, slot, active_chunks,
                              (int64_t)b * gridDim.y + blockIdx.y);
 }
 
+// Copy ring of one warp of a packed-prefix CTA; it runs on from one segment to the next.
+struct PackedRing {
+  int stage;       // stage of the next step
+  uint32_t phase;  // parity of the mbarrier phase that step completes
+  bool dead;       // a bounded wait expired: this warp consumes nothing any more
+};
+
+// One packed segment: tokens [t0, t1) of the quantized prefix of (row b, unit = kv head and group of 8 query heads).  The
+// partial goes to split-K slot `out_slot` and counts as one of `arrivals`; the CTA that counts last merges `slots` partials.
+// All threads of the CTA call it; it ends with the CTA synchronised against reuse of the ring.
 template <typename T, int D, int BITS>
-__global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
-    tq_decode_split_mma_kernel(const TqDecodeParams p) {
+__device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8_t* smem_raw, PackedRing& ring, int b,
+                                                  int unit, int units, int t0, int t1, int out_slot, int slots,
+                                                  int arrivals) {
   using Cfg = TqMmaCfg<T, D, BITS>;
   constexpr int U = Cfg::kTilesPerStep;
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-
-  const int slot = blockIdx.x;
   const int group_tiles = (p.groups + 7) / 8;
-  const int kvh = blockIdx.y / group_tiles;
-  const int g0 = (blockIdx.y % group_tiles) * 8;
+  const int kvh = unit / group_tiles;
+  const int g0 = (unit % group_tiles) * 8;
   const int g_count = min(8, p.groups - g0);
-  const int b = blockIdx.z;
   const int hq0 = kvh * p.groups + g0;
-
-  int64_t len64 = p.lengths[b];
-  len64 = max((int64_t)0, min(len64, p.max_len));
-  const int len = (int)len64;
-  const int R = p.residual_len;
-  const int Lq = len > R ? len - R : 0;
-  const int win = len - Lq;
-  const int active_window = (win + p.chunk_tokens - 1) / p.chunk_tokens;
-  const int active_packed = (Lq + p.chunk_tokens - 1) / p.chunk_tokens;
-  const int active_chunks = active_window + active_packed;
-  if (len == 0 || slot < p.num_window_chunks) {  // window chunks run in tq_window_split_mma_kernel
-    wait_for_prior_grids();
-    return;
-  }
-
-  // ---- packed chunks ------------------------------------------------------------------------------------------------------
-  const int chunk = slot - p.num_window_chunks;
-  const int t0 = chunk * p.chunk_tokens;
-  if (t0 >= Lq) {
-    wait_for_prior_grids();
-    return;
-  }
-  const int t1 = min(Lq, t0 + p.chunk_tokens);
-  const int out_slot = active_window + chunk;  // active slots stay contiguous: [window | packed]
   const int num_tiles = (t1 - t0 + kTileTokens - 1) / kTileTokens;
-  if (threadIdx.x == 0) {
-    const uint32_t bars = smem_u32(smem_raw + Cfg::kWorkSmem);
-    for (int i = 0; i < kMmaWarps * Cfg::kStages; ++i) mbar_init(bars + i * 8, 1);
-    mbar_init_fence();
-  }
-  __syncthreads();
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -532,11 +506,11 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
   uint32_t lut[2] = {0u, 0u};  // 4-bit: the centroids as signed bytes, as the query preparation rounded them
   (void)k_bit1; (void)k_both; (void)c_idx; (void)c_sign; (void)s2_start; (void)lut;
   {
-    const uint8_t* unit = reinterpret_cast<const uint8_t*>(p.query_frags) + ((int64_t)b * gridDim.y + blockIdx.y) * tq_query_unit_bytes(D);
-    const uint4* src = reinterpret_cast<const uint4*>(unit);
+    const uint8_t* unit_frags = reinterpret_cast<const uint8_t*>(p.query_frags) + ((int64_t)b * units + unit) * tq_query_unit_bytes(D);
+    const uint4* src = reinterpret_cast<const uint4*>(unit_frags);
     uint4* dst = reinterpret_cast<uint4*>(smem_raw + Cfg::kQueryOffset);
     for (int i = threadIdx.x; i < (Cfg::kFragBytes + Cfg::kFrag2Bytes) / 16; i += kMmaThreads) dst[i] = __ldg(src + i);
-    const float* consts = reinterpret_cast<const float*>(unit + Cfg::kConstOffset);
+    const float* consts = reinterpret_cast<const float*>(unit_frags + Cfg::kConstOffset);
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       beta1[c] = __ldg(consts + 2 * tig + c);
@@ -639,10 +613,10 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
     for (int r = 0; r < 4; ++r) o_acc[j][r] = 0.0f;
 
   const int num_steps = (num_tiles + U - 1) / U;
-  const int my_steps = num_steps > warp ? (num_steps - warp + kMmaWarps - 1) / kMmaWarps : 0;
+  const int my_steps = num_steps > warp && !ring.dead ? (num_steps - warp + kMmaWarps - 1) / kMmaWarps : 0;
 #pragma unroll
   for (int i = 0; i < Cfg::kStages - 1; ++i)
-    if (i < my_steps) issue_step(i, i);
+    if (i < my_steps) issue_step(i, (ring.stage + i) % Cfg::kStages);
 
   // MMA row r of a tile holds token r ^ ((r >> 1) & 1): neighbouring token rows sit in different halves of the
   // shared-memory banks, and with this order the four token rows one value load touches fall into both halves.
@@ -653,8 +627,8 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
   // this lane's value dims: D/8 consecutive dims starting at gid * D/8, all inside value group (gid * D/8) / 32
   const int v_group = (gid * (D / 8)) / 32;
 
-  int stage = 0;        // stage of step n
-  uint32_t phase = 0;   // parity of the mbarrier phase that step n completes
+  int stage = ring.stage;
+  uint32_t phase = ring.phase;
   for (int n = 0; n < my_steps; ++n) {
     __syncwarp();  // every lane is done with the stage that is re-armed next (the one step n - 1 used)
     {
@@ -666,8 +640,9 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
       // wait (bounded) for the copies still in flight before the epilogue reuses the stages
       for (int k = 1; k < Cfg::kStages && n + k < my_steps; ++k) {
         const int st_k = (stage + k) % Cfg::kStages;
-        (void)mbar_wait(bars_u32 + st_k * 8, (uint32_t)((n + k) / Cfg::kStages) & 1u);
+        (void)mbar_wait(bars_u32 + st_k * 8, stage + k >= Cfg::kStages ? phase ^ 1u : phase);
       }
+      ring.dead = true;
       break;  // give up on this chunk: the fault counter tells the host that the output is not valid
     }
     const int cur = stage;
@@ -982,6 +957,8 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
       }
     }
   }
+  ring.stage = stage;
+  ring.phase = phase;
   // ---- merge the four warps; m-tile j holds dims gid*D/8 + 2j (row gid) and + 2j + 1 (row gid + 8) --------------------------
 #pragma unroll
   for (int d = 4; d <= 16; d <<= 1) {
@@ -1038,10 +1015,87 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
   if (p.fused.counters != nullptr) {
     const int64_t head0 = ((int64_t)b * p.q_heads + hq0) * p.chunk_capacity;
     __syncthreads();
-    fused_combine_tail<T, D, kMmaThreads>(p.fused, b, hq0, g_count, active_chunks, p.chunk_capacity,
-                                          p.stats + head0 * 2, p.values + head0 * D,
-                                          reinterpret_cast<float*>(smem_raw), (int64_t)b * gridDim.y + blockIdx.y);
+    fused_combine_tail<T, D, kMmaThreads>(p.fused, b, hq0, g_count, slots, p.chunk_capacity, p.stats + head0 * 2,
+                                          p.values + head0 * D, reinterpret_cast<float*>(smem_raw),
+                                          (int64_t)b * units + unit, arrivals);
   }
+  // the merge buffers lie where the next segment's copies land: order those writes before the copy engine's
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  __syncthreads();
+}
+
+template <typename T, int D, int BITS>
+__device__ __forceinline__ void init_packed_barriers(uint8_t* smem_raw) {
+  using Cfg = TqMmaCfg<T, D, BITS>;
+  if (threadIdx.x == 0) {
+    const uint32_t bars = smem_u32(smem_raw + Cfg::kWorkSmem);
+    for (int i = 0; i < kMmaWarps * Cfg::kStages; ++i) mbar_init(bars + i * 8, 1);
+    mbar_init_fence();
+  }
+  __syncthreads();
+}
+
+// Fixed chunks of the context, handed out by the block scheduler: grid (window chunks + packed chunks, units, batch).
+template <typename T, int D, int BITS>
+__global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
+    tq_decode_split_mma_kernel(const TqDecodeParams p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const int b = blockIdx.z;
+  int64_t len64 = p.lengths[b];
+  len64 = max((int64_t)0, min(len64, p.max_len));
+  const int len = (int)len64;
+  const int R = p.residual_len;
+  const int Lq = len > R ? len - R : 0;
+  const int active_window = (len - Lq + p.chunk_tokens - 1) / p.chunk_tokens;
+  const int active_packed = (Lq + p.chunk_tokens - 1) / p.chunk_tokens;
+  const int chunk = (int)blockIdx.x - p.num_window_chunks;  // window chunks run in tq_window_split_mma_kernel
+  if (chunk < 0 || chunk >= active_packed) {
+    wait_for_prior_grids();
+    return;
+  }
+  const int t0 = chunk * p.chunk_tokens;
+  init_packed_barriers<T, D, BITS>(smem_raw);
+  PackedRing ring{0, 0u, false};
+  // active slots stay contiguous: [window | packed]
+  tq_packed_segment<T, D, BITS>(p, smem_raw, ring, b, (int)blockIdx.y, (int)gridDim.y, t0, min(Lq, t0 + p.chunk_tokens),
+                                active_window + chunk, active_window + active_packed, active_packed);
+}
+
+// Persistent variant: one resident wave, every CTA takes an even share of the packed tiles (balanced_schedule.cuh).
+template <typename T, int D, int BITS>
+__global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
+    tq_decode_balanced_mma_kernel(const TqDecodeParams p, const int batch) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const int units = p.kv_heads * ((p.groups + 7) / 8);
+  init_packed_barriers<T, D, BITS>(smem_raw);
+  PackedRing ring{0, 0u, false};
+  balanced_for_each_segment<kMmaThreads>(
+      p.lengths, p.max_len, batch, units, min(p.chunk_capacity, kFusedMaxChunks) - p.num_window_chunks,
+      [](int) {},  // rows without packed tokens belong to the window kernel
+      [&](int b, int unit, int t0, int t1, int slot, int partials) {
+        const int active_window = (p.residual_len + p.chunk_tokens - 1) / p.chunk_tokens;  // the window of this row is full
+        tq_packed_segment<T, D, BITS>(p, smem_raw, ring, b, unit, units, t0, t1, active_window + slot,
+                                      active_window + partials, partials);
+      },
+      p.residual_len, kMmaWarps * TqMmaCfg<T, D, BITS>::kTilesPerStep);
+  wait_for_prior_grids();
+}
+
+// Which schedule the packed prefix takes.
+static bool tq_use_balanced(const TqDecodeParams& p, int batch) {
+  static const bool disabled = [] {
+    const char* flag = std::getenv("ANNA_B200_DISABLE_BALANCED");
+    return flag != nullptr && flag[0] != '\0' && flag[0] != '0';
+  }();
+  const int64_t units = (int64_t)p.kv_heads * ((p.groups + 7) / 8);
+  const int packed_slots = min(p.chunk_capacity, kFusedMaxChunks) - p.num_window_chunks;
+  if (disabled || p.given_chunks || p.fused.counters == nullptr || !balanced_schedule_fits(batch, units, p.max_len, packed_slots)) return false;
+  // The plan's longest chunks mean that there are enough of them for a few waves, which the block scheduler hands out as SMs
+  // get free (64 rows of 32 K tokens: 669 us, even shares 684; 128 ragged rows of 0.5-16 K: 253 and 261).  With less work
+  // the chunks shrink, down to 64 tokens, and every CTA's fixed cost and the number of partials grow (16 rows of 0.4-4 K
+  // tokens, head_dim 256: 115 us, even shares 74; 64 rows of 4-32 K with two KV heads: 212 and 199; one row of 4 K: 36.8
+  // and 35.3).
+  return p.chunk_tokens < kTqLongestChunk;
 }
 
 template <typename T, int D, int BITS>
@@ -1073,28 +1127,37 @@ static int launch_tq_mma(const TqDecodeParams& p, int batch, cudaStream_t stream
   tq_window_split_mma_kernel<T, D><<<window_grid, kMmaThreads, MmaCfg<D>::kSmemBytes, stream>>>(p);
   rc = check_launch("tq_window_split_mma_kernel");
   if (rc != ANNA_OK) return rc;
-  if (p.num_chunks > p.num_window_chunks) {
-    dim3 grid((unsigned)p.num_chunks, (unsigned)(p.kv_heads * group_tiles), (unsigned)batch);
-#if ANNA_TQ_OVERLAP_WINDOW
-    // programmatic dependent launch: the packed chunks run beside the (small) window launch instead of after it; the
-    // query fragments they read come from the launch before that one, which has completed by then
-    cudaLaunchConfig_t config = {};
-    config.gridDim = grid;
-    config.blockDim = dim3(kMmaThreads);
-    config.dynamicSmemBytes = Cfg::kSmemBytes;
-    config.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = attr;
-    config.numAttrs = 1;
-    ANNA_CUDA_CHECK(cudaLaunchKernelEx(&config, kernel, p));
-#else
-    kernel<<<grid, kMmaThreads, Cfg::kSmemBytes, stream>>>(p);
-#endif
-    rc = check_launch("tq_decode_split_mma_kernel");
+  if (p.num_chunks <= p.num_window_chunks) return rc;
+  // Programmatic dependent launch: the packed chunks run beside the (small) window launch instead of after it; the query
+  // fragments they read come from the launch before that one, which has completed by then.
+  cudaLaunchConfig_t config = {};
+  config.blockDim = dim3(kMmaThreads);
+  config.dynamicSmemBytes = Cfg::kSmemBytes;
+  config.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attr;
+  config.numAttrs = 1;
+  if (tq_use_balanced(p, batch)) {
+    static int resident[64] = {};  // per device: CTAs of this kernel that fit the whole GPU at once
+    auto balanced = tq_decode_balanced_mma_kernel<T, D, BITS>;
+    int ctas = (device >= 0 && device < 64) ? resident[device] : 0;
+    if (ctas == 0) {
+      ANNA_CUDA_CHECK(cudaFuncSetAttribute(balanced, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
+      int sms = 0, per_sm = 0;
+      ANNA_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+      ANNA_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, balanced, kMmaThreads, Cfg::kSmemBytes));
+      ctas = sms * (per_sm > 0 ? per_sm : 1);
+      if (device >= 0 && device < 64) resident[device] = ctas;
+    }
+    config.gridDim = dim3((unsigned)ctas);
+    ANNA_CUDA_CHECK(cudaLaunchKernelEx(&config, balanced, p, batch));
+    return check_launch("tq_decode_balanced_mma_kernel");
   }
-  return rc;
+  config.gridDim = dim3((unsigned)p.num_chunks, (unsigned)(p.kv_heads * group_tiles), (unsigned)batch);
+  ANNA_CUDA_CHECK(cudaLaunchKernelEx(&config, kernel, p));
+  return check_launch("tq_decode_split_mma_kernel");
 }
 
 template <typename T, int D>

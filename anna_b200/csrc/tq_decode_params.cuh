@@ -6,6 +6,8 @@
 
 namespace anna {
 
+constexpr int kTqLongestChunk = 4096;  // tokens; see anna_tq_decode_plan
+
 struct TqDecodeParams {
   const void* q;
   int64_t q_stride_b, q_stride_h;
@@ -25,11 +27,13 @@ struct TqDecodeParams {
   int block_shift;  // log2(block_size) when it is a power of two, else -1
   int64_t num_pages, max_blocks, max_len;
   int chunk_tokens, num_chunks, chunk_capacity;
+  bool given_chunks;      // chunk_tokens is the caller's choice, not the plan's
+  bool window_arrives;    // the window CTAs of a row with packed tokens count on the merge counter, too
   int num_window_chunks;  // split-K slots [0, num_window_chunks) cover the window ring, the rest the packed prefix
   float scaling;
   anna_tq_layout layout;
   FusedCombine fused;
-  void* query_frags;  // scratch for the rotated query fragments (tensor-core path), or nullptr
+  void* query_frags;  // scratch for the rotated fp16 query fragments (tensor-core path), or nullptr
 };
 
 // Tensor-memory split pass (tq_decode_umma.cu): 16-bit cache dtypes, head_dim 128, 3- / 4-bit codes, 16-token pages,
