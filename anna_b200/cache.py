@@ -143,7 +143,7 @@ class _DeviceLengths:
     def __init__(self, batch: int, device: torch.device) -> None:
         self.rows = list(torch.zeros((self.DEPTH, batch), dtype=torch.int64, device=device).unbind(0))
         self.pos = 0
-        self.host: list[int] | None = None
+        self.host: list[int] | None = [0] * batch
         self.slots_dev: torch.Tensor | None = None
         self.slots_host: list[int] | None = None
         self.device = device
@@ -168,6 +168,27 @@ class _DeviceLengths:
             self.slots_dev = MetadataUploader.for_device(self.device).upload([slots])[0]
             self.slots_host = list(slots)
         return self.slots_dev
+
+
+class _QuantizedStep:
+    """What one decode step of a TurboQuant layer needs and the next one can go on from: the rows with their device block
+    table, lengths and ring slots, and how many tokens every row still takes without a new page.
+
+    It holds while the layer has the same row objects and nothing about any row of the pool has changed since
+    (``TurboQuantLayerPool.version``); otherwise the step is derived from the rows again."""
+
+    __slots__ = ("pool", "version", "rows", "table", "lengths", "lengths_dev", "slots", "slots_dev", "headroom", "longest")
+
+    def __init__(self, pool: TurboQuantLayerPool, rows: list, table: torch.Tensor | None, lengths: list[int],
+                 lengths_dev: torch.Tensor, slots: list[int], slots_dev: torch.Tensor, headroom: int) -> None:
+        self.pool, self.version, self.rows = pool, pool.version, list(rows)
+        self.table, self.lengths, self.lengths_dev = table, lengths, lengths_dev
+        self.slots, self.slots_dev = slots, slots_dev
+        self.headroom, self.longest = headroom, max(lengths)
+
+    def holds(self, pool: TurboQuantLayerPool, rows: list, device: torch.device) -> bool:
+        return (self.pool is pool and self.version == pool.version and self.slots_dev.device == device
+                and self.rows == rows)
 
 
 class Qwen3DynamicCache:
@@ -205,6 +226,7 @@ class Qwen3DynamicCache:
         # returned by the last sync (valid while no table has changed)
         self._page_headroom: list[int | None] = [None] * layers
         self._table_view: list[torch.Tensor | None] = [None] * layers
+        self._tq_step: list[_QuantizedStep | None] = [None] * layers
         self.seen_tokens = 0
         self.rope_deltas: torch.Tensor | None = None
         self.reserved_seq_capacity = 0
@@ -604,20 +626,40 @@ class Qwen3DynamicCache:
         self._ensure_batch_size(batch_size)
         device = key_states.device
         pool = self._tq_pool(layer_idx)
+        step = self._tq_step[layer_idx]
+        if step is not None and 0 < append_length <= step.headroom:
+            past_lengths = self._append_quantized_step(step, pool, key_states, value_states, layer_idx)
+            if past_lengths is not None:
+                if not require_dense_cache:
+                    return None, None, past_lengths
+                keys, values, _ = self._gather_quantized(layer_idx)
+                return keys, values, past_lengths
         pool.configure(kv_heads=kv_heads, head_dim=head_dim, bits=self.kv_cache_quant_bits,
                        residual_len=self.kv_cache_residual_len, dtype=key_states.dtype, device=device)
         rows = self.turboquant_rows[layer_idx]
         past = list(self.layer_lengths[layer_idx])
-        missing = sum(1 for row in rows if row is None)
+        missing = rows.count(None)
         if missing:
             pool.ensure_slot_capacity(pool.slot_capacity() - len(pool.free_slots) + missing)
         use_prefix_share = self._prefix_kv_share and batch_size == 1 and self._prompt_token_ids is not None
         shared_blocks: list[int] = []
+        if missing == batch_size and not use_prefix_share and append_length > 0:
+            # new sequences: when the free list holds their pages, one take hands them out in the order of a take per row
+            blocks = (max(0, append_length - self.kv_cache_residual_len) + self.block_size - 1) // self.block_size
+            if 0 < blocks * batch_size <= len(pool.free_pages):
+                pages = pool.allocate(blocks * batch_size)
+            else:
+                blocks, pages = 0, []
+            for batch_idx in range(batch_size):
+                row = TurboQuantKVRow(bits=self.kv_cache_quant_bits, residual_len=self.kv_cache_residual_len)
+                row._attach(pool)
+                row._blocks = pages[batch_idx * blocks:(batch_idx + 1) * blocks]
+                rows[batch_idx] = row
         for batch_idx in range(batch_size):
             row = rows[batch_idx]
             if row is None:
                 row = TurboQuantKVRow(bits=self.kv_cache_quant_bits, residual_len=self.kv_cache_residual_len)
-                row._bind(pool, kv_heads=kv_heads, head_dim=head_dim, dtype=key_states.dtype, device=device)
+                row._attach(pool)
                 rows[batch_idx] = row
             if use_prefix_share:
                 shared_blocks = self._reserve_shared_packed_blocks(row, pool, layer_idx, row.length + append_length)
@@ -629,8 +671,9 @@ class Qwen3DynamicCache:
         slots = [row.slot for row in rows]
         lengths = self.layer_lengths[layer_idx]
         for batch_idx, row in enumerate(rows):
-            row._length += append_length
-            lengths[batch_idx] = row._length
+            row._tokens += append_length
+            lengths[batch_idx] = row._tokens
+        pool.version += 1
         if device.type == "cuda":
             state = self._device_lengths_of(layer_idx, batch_size, device)
             past_lengths, new_lengths = state.before_append(past)
@@ -653,11 +696,46 @@ class Qwen3DynamicCache:
                 state.after_append(lengths)
             if use_prefix_share:
                 self._register_packed_blocks(rows[0], pool, layer_idx)
+            if state is not None:
+                # with pages that have several owners the next append has to look for blocks to copy first
+                room = -1
+                if not use_prefix_share and not pool.has_shared_pages:
+                    room = min(len(row._blocks) * pool.block_size + row.residual_len - row._tokens for row in rows)
+                self._tq_step[layer_idx] = _QuantizedStep(pool, rows, table_dev, list(lengths), new_lengths, slots,
+                                                          slots_dev, room)
         self.seen_tokens = max(self.seen_tokens, max(lengths, default=0))
         if not require_dense_cache:
             return None, None, past_lengths
-        keys, values, _ = self._gather_layer_cache(layer_idx)
+        keys, values, _ = self._gather_quantized(layer_idx)
         return keys, values, past_lengths
+
+    def _append_quantized_step(self, step: _QuantizedStep, pool: TurboQuantLayerPool, key_states, value_states,
+                               layer_idx: int) -> torch.Tensor | None:
+        """Append to rows that all have room in their last page: no page, ring slot or table entry changes, so the launch
+        goes on from the previous step's device tensors.  Returns the lengths before, or None when the step is stale."""
+        rows = self.turboquant_rows[layer_idx]
+        batch, kv_heads, tokens, dim = key_states.shape
+        state = self._dev_lengths[layer_idx]
+        if (state is None or not step.holds(pool, rows, key_states.device) or batch != len(rows)
+                or kv_heads != pool.kv_heads or dim != pool.head_dim or key_states.dtype != pool.dtype
+                or self.layer_lengths[layer_idx] != step.lengths or state.current(step.lengths) is not step.lengths_dev
+                or (batch == 1 and self._prefix_kv_share and self._prompt_token_ids is not None)):
+            return None
+        past_lengths, new_lengths = state.before_append(step.lengths)
+        lengths = [n + tokens for n in step.lengths]
+        for row in rows:
+            row._tokens += tokens
+        self.layer_lengths[layer_idx][:] = lengths
+        pool.version += 1
+        launch_tq_append(pool, key_states, value_states, step.table, step.slots, step.lengths, slots_dev=step.slots_dev,
+                         past_dev=past_lengths, new_lengths_dev=new_lengths)
+        state.after_append(lengths)
+        step.version, step.lengths, step.lengths_dev = pool.version, lengths, new_lengths
+        step.headroom -= tokens
+        step.longest += tokens
+        if step.longest > self.seen_tokens:
+            self.seen_tokens = step.longest
+        return past_lengths
 
     def turboquant_single_token_decode_attention(self, layer_idx: int, query_states: torch.Tensor, *, scaling: float,
                                                  num_key_value_groups: int, gate: torch.Tensor | None = None,
@@ -677,6 +755,12 @@ class Qwen3DynamicCache:
         if batch != len(rows):
             raise ValueError(f"Cache batch size mismatch: expected {len(rows)}, got {batch}")
         pool = self._tq_pool(layer_idx)
+        step = self._tq_step[layer_idx]
+        if (step is not None and query_states.shape[1] == pool.kv_heads * num_key_value_groups
+                and step.holds(pool, rows, query_states.device)):
+            return launch_tq_decode(pool, query_states, step.table, step.slots, step.lengths, scaling, gate,
+                                    slots_dev=step.slots_dev, lengths_dev=step.lengths_dev, output=output,
+                                    peer_outputs=peer_outputs)
         if not pool.configured or all(row is None or row.length <= 0 for row in rows):
             if output is not None or peer_outputs:
                 raise RuntimeError("an empty TurboQuant cache cannot decode into caller-provided outputs")
@@ -693,6 +777,13 @@ class Qwen3DynamicCache:
         if state is not None and state.device == device:
             lengths_dev = state.current(lengths)
             slots_dev = state.slots(slots)
+        if device.type == "cuda" and (lengths_dev is None or slots_dev is None):
+            meta = MetadataUploader.for_device(device).upload([lengths, slots])
+            lengths_dev = meta[0] if lengths_dev is None else lengths_dev
+            slots_dev = meta[1] if slots_dev is None else slots_dev
+        if lengths_dev is not None and None not in rows:
+            # no headroom: the next append derives its step from the rows
+            self._tq_step[layer_idx] = _QuantizedStep(pool, rows, table_dev, lengths, lengths_dev, slots, slots_dev, -1)
         return launch_tq_decode(pool, query_states, table_dev, slots, lengths, scaling, gate, slots_dev=slots_dev,
                                 lengths_dev=lengths_dev, output=output, peer_outputs=peer_outputs)
 
@@ -734,17 +825,11 @@ class Qwen3DynamicCache:
         lengths = self.layer_lengths[layer_idx]
         max_length = max(lengths, default=0)
         if self.uses_turboquant_for_layer(layer_idx):
-            if max_length <= 0:
-                return None, None, torch.tensor(lengths, dtype=torch.long)
-            rows = self.turboquant_rows[layer_idx]
-            if any(row is None for row in rows):
-                raise RuntimeError(f"TurboQuant cache row for layer {layer_idx} is missing.")
-            pool = self._tq_pool(layer_idx)
-            device = pool.device
-            assert device is not None
-            table_dev = self._sync_page_table_layer_buffer(layer_idx, batch_size=batch_size, device=device)
-            # the lengths come back as the device tensor the launch read them from (no second host-to-device copy)
-            return launch_tq_gather_dense(pool, table_dev, [row.slot for row in rows], list(lengths), max_length)
+            keys, values, visible = self._gather_quantized(layer_idx)
+            state = self._dev_lengths[layer_idx]
+            if state is not None and any(visible is row for row in state.rows):
+                visible = visible.clone()  # the ring's row is written again by later appends
+            return keys, values, visible
         layer = self.allocator.layers[layer_idx]
         if layer.key_pages is None or layer.value_pages is None or max_length <= 0:
             return None, None, torch.tensor(lengths, dtype=torch.long)
@@ -763,6 +848,29 @@ class Qwen3DynamicCache:
                 int(keys.shape[3]), self.block_size, layer.capacity(), int(table.shape[1]), max_length,
                 dtype_code(keys.dtype), stream_ptr(device)), "anna_paged_kv_gather")
         return keys, values, visible
+
+    def _gather_quantized(self, layer_idx: int):
+        """Dense view of a TurboQuant layer in one launch.  The lengths come back as the device tensor the launch read
+        them from: the row the last append left in the ring of ``_DeviceLengths`` when it still holds."""
+        batch_size = self.get_batch_size()
+        lengths = list(self.layer_lengths[layer_idx])
+        max_length = max(lengths, default=0)
+        if max_length <= 0:
+            return None, None, torch.tensor(lengths, dtype=torch.long)
+        rows = self.turboquant_rows[layer_idx]
+        if None in rows:
+            raise RuntimeError(f"TurboQuant cache row for layer {layer_idx} is missing.")
+        pool = self._tq_pool(layer_idx)
+        device = pool.device
+        assert device is not None
+        table_dev = self._sync_page_table_layer_buffer(layer_idx, batch_size=batch_size, device=device)
+        slots = [row.slot for row in rows]
+        state = self._dev_lengths[layer_idx]
+        lengths_dev = slots_dev = None
+        if state is not None and state.device == device and state.slots_host == slots:
+            lengths_dev, slots_dev = state.current(lengths), state.slots_dev
+        return launch_tq_gather_dense(pool, table_dev, slots, lengths, max_length, slots_dev=slots_dev,
+                                      lengths_dev=lengths_dev)
 
     def visible_key_cache(self, layer_idx: int):
         return self._gather_layer_cache(layer_idx)[0]
@@ -903,6 +1011,7 @@ class Qwen3DynamicCache:
             self._dev_lengths[layer_idx] = None
             self._page_headroom[layer_idx] = None
             self._table_view[layer_idx] = None
+            self._tq_step[layer_idx] = None
         self.seen_tokens = 0
         self.rope_deltas = None
         self.reserved_seq_capacity = 0
@@ -946,9 +1055,7 @@ class Qwen3DynamicCache:
             return
         for layer_idx in range(self.config.num_hidden_layers):
             if self.uses_turboquant_for_layer(layer_idx):
-                for row in self.turboquant_rows[layer_idx]:
-                    if row is not None:
-                        row.release()
+                TurboQuantKVRow.release_all(row for row in self.turboquant_rows[layer_idx] if row is not None)
             else:
                 for page_ids in self.page_tables[layer_idx]:
                     self.allocator.release_pages(layer_idx, page_ids)

@@ -178,12 +178,14 @@ def _require_cuda(name: str, **tensors: torch.Tensor | None) -> torch.device:
     for label, tensor in tensors.items():
         if tensor is None:
             continue
-        if not tensor.is_cuda:
+        where = tensor.device
+        if where == device:  # the same CUDA device as the first tensor
+            continue
+        if where.type != "cuda":
             raise RuntimeError(f"{name}: {label} must be a CUDA tensor (there is no CPU implementation of this op)")
-        if device is None:
-            device = tensor.device
-        elif tensor.device != device:
+        if device is not None:
             raise RuntimeError(f"{name}: {label} must be on the same device as query")
+        device = where
     assert device is not None
     return device
 
@@ -270,10 +272,16 @@ _SCRATCH = _Scratch()
 
 def query_scratch(device: torch.device, batch: int, heads: int, kv_heads: int, head_dim: int) -> torch.Tensor:
     """Scratch for the rotated query fragments of the packed tensor-core decode."""
-    need = int(_lib.lib().anna_tq_query_scratch_bytes(batch, heads, kv_heads, head_dim))
+    key = (batch, heads, kv_heads, head_dim)
+    need = _QUERY_SCRATCH_BYTES.get(key)
+    if need is None:
+        if len(_QUERY_SCRATCH_BYTES) > 4096:
+            _QUERY_SCRATCH_BYTES.clear()
+        need = _QUERY_SCRATCH_BYTES[key] = int(_lib.lib().anna_tq_query_scratch_bytes(*key))
     return _SCRATCH.bytes(device, need)
 
 
+_QUERY_SCRATCH_BYTES: dict[tuple, int] = {}
 _PLAN_CACHE: dict[tuple, int] = {}
 
 
@@ -488,21 +496,25 @@ def _op_gqa_decode_splitkv_turboquant_fused_out(query, quantized_key, value_data
 def _op_paged_gqa_decode_fused(query, key_pages, value_pages, page_table, visible_lengths, scaling, gate=None):
     name = "paged_gqa_decode_fused"
     query = _check_query(name, query)
-    if key_pages.dim() != 4 or value_pages.dim() != 4:
+    page_shape, table_shape, length_shape = tuple(key_pages.shape), tuple(page_table.shape), tuple(visible_lengths.shape)
+    if len(page_shape) != 4 or value_pages.dim() != 4:
         raise RuntimeError("key_pages and value_pages must be [pages, kv_heads, block_size, head_dim]")
-    if key_pages.shape != value_pages.shape:
+    if page_shape != tuple(value_pages.shape):
         raise RuntimeError("key_pages and value_pages must share the same shape")
-    if page_table.dim() != 2 or page_table.shape[0] != query.shape[0]:
+    batch, heads, _, dim = query.shape
+    if len(table_shape) != 2 or table_shape[0] != batch:
         raise RuntimeError("page_table must be [batch, max_blocks]")
-    if visible_lengths.dim() != 1 or visible_lengths.shape[0] != query.shape[0]:
+    if length_shape != (batch,):
         raise RuntimeError("visible_lengths must be [batch]")
-    if key_pages.shape[0] < 1 or key_pages.shape[1] < 1 or key_pages.shape[2] < 1:
+    pages, kv_heads, block, page_dim = page_shape
+    if pages < 1 or kv_heads < 1 or block < 1:
         raise RuntimeError("pages, kv_heads and block_size must be positive")
-    if query.shape[1] % key_pages.shape[1] != 0:
+    if heads % kv_heads != 0:
         raise RuntimeError("query heads must be divisible by kv_heads")
-    if query.shape[3] != key_pages.shape[3]:
+    if dim != page_dim:
         raise RuntimeError("query/key_pages head_dim mismatch")
-    if not (query.dtype == key_pages.dtype == value_pages.dtype):
+    dtype = query.dtype
+    if not (dtype == key_pages.dtype == value_pages.dtype):
         raise RuntimeError("query, key_pages, and value_pages must share the same dtype")
     if page_table.dtype != torch.int32:
         raise RuntimeError("page_table must be int32")
@@ -519,19 +531,18 @@ def _op_paged_gqa_decode_fused(query, key_pages, value_pages, page_table, visibl
     if visible_lengths.stride(0) != 1:
         visible_lengths = visible_lengths.contiguous()
     gate, gate_sb, gate_sh = _check_gate(name, query, gate)
-    batch, heads, _, dim = (int(v) for v in query.shape)
-    pages, kv_heads, block = int(key_pages.shape[0]), int(key_pages.shape[1]), int(key_pages.shape[2])
-    max_blocks = int(page_table.shape[1])
-    out = torch.empty((batch, heads, 1, dim), dtype=query.dtype, device=device)
+    max_blocks = table_shape[1]
+    out = torch.empty((batch, heads, 1, dim), dtype=dtype, device=device)
     if max_blocks == 0:
         return out.zero_()
     stats, values, capacity, counters = split_scratch(device, batch, heads, dim, kv_heads, max_blocks * block)
+    q_sb, q_sh, _, _ = query.stride()
     with on_device(device):
         _lib.check(_lib.lib().anna_paged_gqa_decode(
-            ptr(query), query.stride(0), query.stride(1), ptr(key_pages), ptr(value_pages), ptr(page_table),
-            page_table.stride(0), ptr(visible_lengths), ptr(gate), gate_sb, gate_sh, ptr(out), out.stride(0),
-            out.stride(1), ptr(stats), ptr(values), capacity, 0, ptr(counters), batch, heads, kv_heads, dim, block,
-            pages, max_blocks, float(scaling), dtype_code(query.dtype), stream_ptr(device)), name)
+            ptr(query), q_sb, q_sh, ptr(key_pages), ptr(value_pages), ptr(page_table), page_table.stride(0),
+            ptr(visible_lengths), ptr(gate), gate_sb, gate_sh, ptr(out), heads * dim, dim, ptr(stats), ptr(values),
+            capacity, 0, ptr(counters), batch, heads, kv_heads, dim, block, pages, max_blocks, float(scaling),
+            dtype_code(dtype), stream_ptr(device)), name)
     return out
 
 

@@ -6,11 +6,13 @@ The bookkeeping (LIFO free list, growth by ``max(n, capacity or 16)``, reversed 
 from __future__ import annotations
 
 from collections.abc import Callable
+from itertools import repeat
 
 import torch
 
 from . import _lib
 from .fused_ops import dtype_code
+from .tq_tables import KeyQuantizerTables, key_tables
 
 
 def resolve_value_group_size(head_dim: int) -> int:
@@ -39,8 +41,8 @@ class _PageBook:
             out = self.free_pages[-count:]
             out.reverse()
             del self.free_pages[-count:]
-            stale = self.refcount.keys() & out
-            if stale:
+            if not self.refcount.keys().isdisjoint(out):
+                stale = self.refcount.keys() & out
                 raise RuntimeError(f"Invariant violated: free list page {min(stale)} has non-zero refcount.")
             self.refcount.update(dict.fromkeys(out, 1))
         missing = num_pages - len(out)
@@ -91,12 +93,16 @@ class _PageBook:
         callback (for callers that know nobody listens, e.g. an empty prefix registry)."""
         refcount = self.refcount
         ids = page_ids if isinstance(page_ids, list) else list(page_ids)
-        if self._shared == 0 and refcount.keys() >= set(ids) and len(set(ids)) == len(ids):
-            # nothing is shared and every id is held exactly once: all of them become free, at C speed
-            for _ in map(refcount.__delitem__, ids):
-                pass
+        counts: list[int] = []
+        if self._shared == 0:
+            # normally every id is held exactly once: one pass at C speed takes all of them out
+            counts = list(map(refcount.pop, ids, repeat(0)))
+        if counts and counts.count(1) == len(ids):
             freed = ids
         else:
+            for page_id, rc in zip(ids, counts):  # a free or repeated id among them: put back, then one by one
+                if rc:
+                    refcount[page_id] = rc
             freed = []
             for page_id in ids:
                 rc = refcount.get(page_id, 0)
@@ -221,7 +227,11 @@ class TurboQuantLayerPool:
         self.kv_heads = self.head_dim = self.bits = self.residual_len = self.value_group = 0
         self.dtype: torch.dtype | None = None
         self.device: torch.device | None = None
+        self._tables: KeyQuantizerTables | None = None
         self.status: torch.Tensor | None = None        # int32 [1] device status word
+        # counts every change of a row of this pool (length, pages, ring slot), so that a cache can tell whether what it
+        # derived from its rows still holds
+        self.version = 0
 
     @property
     def free_pages(self) -> list[int]:
@@ -246,6 +256,14 @@ class TurboQuantLayerPool:
         self.dtype, self.device = dtype, device
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
 
+    @property
+    def tables(self) -> KeyQuantizerTables:
+        """Constants of the key quantizer on the pool's device."""
+        if self._tables is None:
+            assert self.device is not None
+            self._tables = key_tables(head_dim=self.head_dim, bits=self.bits, device=self.device)
+        return self._tables
+
     def capacity(self) -> int:
         return 0 if self.packed_pages is None else int(self.packed_pages.shape[0])
 
@@ -264,6 +282,7 @@ class TurboQuantLayerPool:
         self.packed_pages = new
 
     def allocate(self, num_pages: int) -> list[int]:
+        self.version += 1
         page_ids, new_capacity, _ = self._book.take(num_pages, self.capacity())
         self._resize(new_capacity)
         return page_ids
@@ -273,7 +292,13 @@ class TurboQuantLayerPool:
         return self.capacity()
 
     def release_pages(self, page_ids: list[int]) -> None:
-        self._book.release_many(reversed(page_ids))
+        self.version += 1
+        self._book.release_many(page_ids[::-1])
+
+    @property
+    def has_shared_pages(self) -> bool:
+        """Whether any packed page has more than one owner."""
+        return self._book._shared > 0
 
     def page_owners(self, page_id: int) -> int:
         """How many rows map this packed page (0 for a free page)."""
@@ -283,12 +308,14 @@ class TurboQuantLayerPool:
         """One more owner of a packed page (a sequence that maps it for a shared prompt prefix, or a clone)."""
         if page_id < 0 or page_id >= self.capacity() or self._book.refcount.get(page_id, 0) <= 0:
             raise ValueError(f"retain_page: page {page_id} is not a live packed page (capacity {self.capacity()}).")
+        self.version += 1
         self._book.retain(page_id)
 
     def slot_capacity(self) -> int:
         return 0 if self.window is None else int(self.window.shape[0])
 
     def allocate_slot(self) -> int:
+        self.version += 1
         if not self.free_slots:
             old = self.slot_capacity()
             new_capacity = old + max(1, old or 16)
@@ -314,12 +341,14 @@ class TurboQuantLayerPool:
             self.free_slots.extend(reversed(range(old, new_capacity)))
 
     def release_slot(self, slot: int) -> None:
+        self.version += 1
         self.free_slots.append(int(slot))
 
     def trim(self) -> int:
         capacity = self.capacity()
         if self.used_pages() > 0 or len(self.free_slots) != self.slot_capacity():
             return 0
+        self.version += 1
         self._book.clear()
         self.packed_pages = None
         self.window = None
@@ -328,6 +357,7 @@ class TurboQuantLayerPool:
 
     def clear(self) -> int:
         capacity = self.capacity()
+        self.version += 1
         self._book.clear()
         self.packed_pages = None
         self.window = None

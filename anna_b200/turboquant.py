@@ -8,6 +8,8 @@ whole batch of rows is appended or decoded by one launch.
 """
 from __future__ import annotations
 
+from array import array
+
 import torch
 
 from . import _lib
@@ -57,7 +59,7 @@ def launch_tq_append(pool: TurboQuantLayerPool, key_states: torch.Tensor, value_
         key_states, value_states = key_states.contiguous(), value_states.contiguous()
     device = key_states.device
     batch, kv_heads, tokens, dim = (int(v) for v in key_states.shape)
-    tables = key_tables(head_dim=dim, bits=pool.bits, device=device)
+    tables = pool.tables if dim == pool.head_dim else key_tables(head_dim=dim, bits=pool.bits, device=device)
     if slots_dev is None or past_dev is None:
         meta = MetadataUploader.for_device(device).upload([past, slots])
         past_dev = meta[0] if past_dev is None else past_dev
@@ -90,16 +92,17 @@ def launch_tq_decode(pool: TurboQuantLayerPool, query_states: torch.Tensor, tabl
     if gate is not None and gate.stride(3) != 1:
         gate = gate.contiguous()
     device = query.device
-    batch, heads, _, dim = (int(v) for v in query.shape)
-    if query.dtype != pool.dtype:
-        raise RuntimeError(f"query dtype {query.dtype} must match the cache dtype {pool.dtype}")
-    tables = key_tables(head_dim=dim, bits=pool.bits, device=device)
+    batch, heads, _, dim = query.shape
+    dtype = query.dtype
+    if dtype != pool.dtype:
+        raise RuntimeError(f"query dtype {dtype} must match the cache dtype {pool.dtype}")
+    tables = pool.tables if dim == pool.head_dim else key_tables(head_dim=dim, bits=pool.bits, device=device)
     if slots_dev is None or lengths_dev is None:
         meta = MetadataUploader.for_device(device).upload([lengths, slots])
         lengths_dev = meta[0] if lengths_dev is None else lengths_dev
         slots_dev = meta[1] if slots_dev is None else slots_dev
     if output is None:
-        out = torch.empty((batch, heads, 1, dim), dtype=query.dtype, device=device)
+        out = torch.empty((batch, heads, 1, dim), dtype=dtype, device=device)
     else:
         if tuple(output.shape) != (batch, heads, 1, dim) or output.dtype != query.dtype or output.device != device \
                 or output.stride(3) != 1:
@@ -112,14 +115,16 @@ def launch_tq_decode(pool: TurboQuantLayerPool, query_states: torch.Tensor, tabl
     stats, values, capacity, counters = split_scratch(device, batch, heads, dim, pool.kv_heads, max_len,
                                                       turboquant=(max_blocks, pool.block_size, pool.residual_len))
     frags = query_scratch(device, batch, heads, pool.kv_heads, dim)
+    q_sb, q_sh, _, _ = query.stride()
+    out_sb, out_sh, _, _ = out.stride()
     common = (
-        ptr(query), query.stride(0), query.stride(1), ptr(pool.packed_pages), ptr(table_dev), table_stride,
+        ptr(query), q_sb, q_sh, ptr(pool.packed_pages), ptr(table_dev), table_stride,
         ptr(pool.window), ptr(slots_dev), ptr(lengths_dev), ptr(tables.signs1), ptr(tables.signs2),
         ptr(tables.centroids), ptr(gate), 0 if gate is None else gate.stride(0),
-        0 if gate is None else gate.stride(1), ptr(out), out.stride(0), out.stride(1), ptr(stats), ptr(values),
-        capacity, 0, ptr(counters), ptr(frags), frags.numel(), batch, heads, pool.kv_heads, dim, pool.block_size,
+        0 if gate is None else gate.stride(1), ptr(out), out_sb, out_sh, ptr(stats), ptr(values), capacity, 0,
+        ptr(counters), ptr(frags), frags.numel(), batch, heads, pool.kv_heads, dim, pool.block_size,
         pool.residual_len, pool.bits, pool.value_group, pool.capacity(), max_blocks, float(scaling),
-        dtype_code(query.dtype))
+        dtype_code(dtype))
     with on_device(device):
         if peer_outputs:
             import ctypes
@@ -140,7 +145,7 @@ def launch_tq_materialize(pool: TurboQuantLayerPool, table_dev: torch.Tensor, qu
     if key_out.stride() != value_out.stride() or key_out.stride(3) != 1:
         raise ValueError("materialize outputs must share strides and be contiguous in the last dimension")
     batch, kv_heads, max_lq, dim = (int(v) for v in key_out.shape)
-    tables = key_tables(head_dim=dim, bits=pool.bits, device=device)
+    tables = pool.tables if dim == pool.head_dim else key_tables(head_dim=dim, bits=pool.bits, device=device)
     lq_dev = _i64(quantized_lengths, device)
     with on_device(device):
         _lib.check(_lib.lib().anna_tq_materialize(
@@ -152,26 +157,31 @@ def launch_tq_materialize(pool: TurboQuantLayerPool, table_dev: torch.Tensor, qu
 
 
 def launch_tq_gather_dense(pool: TurboQuantLayerPool, table_dev: torch.Tensor | None, slots: list[int], lengths: list[int],
-                           max_len: int) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+                           max_len: int, *, slots_dev: torch.Tensor | None = None,
+                           lengths_dev: torch.Tensor | None = None) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """Dense ``[B, Hkv, max_len, D]`` keys and values of B rows of one layer in one launch: de-quantized prefix, window
-    tokens, zero padding; and the rows' lengths as the int64 device tensor the launch read them from."""
+    tokens, zero padding; and the rows' lengths as the int64 device tensor the launch read them from.
+    ``slots_dev`` / ``lengths_dev``: as for ``launch_tq_decode``."""
     assert pool.window is not None and pool.device is not None and pool.dtype is not None
     device = pool.device
     batch = len(lengths)
-    tables = key_tables(head_dim=pool.head_dim, bits=pool.bits, device=device)
-    meta = MetadataUploader.for_device(device).upload([lengths, slots])
+    tables = pool.tables
+    if slots_dev is None or lengths_dev is None:
+        meta = MetadataUploader.for_device(device).upload([lengths, slots])
+        lengths_dev = meta[0] if lengths_dev is None else lengths_dev
+        slots_dev = meta[1] if slots_dev is None else slots_dev
     keys = torch.empty((batch, pool.kv_heads, max_len, pool.head_dim), dtype=pool.dtype, device=device)
     values = torch.empty_like(keys)
     table_stride = 0 if table_dev is None else table_dev.stride(0)
     max_blocks = 0 if table_dev is None else int(table_dev.shape[1])
     with on_device(device):
         _lib.check(_lib.lib().anna_tq_gather_dense(
-            ptr(pool.packed_pages), ptr(table_dev), table_stride, ptr(pool.window), ptr(meta[1]), ptr(meta[0]),
+            ptr(pool.packed_pages), ptr(table_dev), table_stride, ptr(pool.window), ptr(slots_dev), ptr(lengths_dev),
             ptr(tables.signs1), ptr(tables.signs2), ptr(tables.centroids), ptr(keys), ptr(values), keys.stride(0),
             keys.stride(1), keys.stride(2), batch, pool.kv_heads, pool.head_dim, pool.block_size, pool.residual_len,
             pool.bits, pool.value_group, pool.capacity(), max_blocks, int(max_len), dtype_code(pool.dtype),
             stream_ptr(device)), "anna_tq_gather_dense")
-    return keys, values, meta[0]
+    return keys, values, lengths_dev
 
 
 class TurboQuantTensorRow:
@@ -330,13 +340,34 @@ class TurboQuantKVRow:
         self.num_heads: int | None = None
         self.pool: TurboQuantLayerPool | None = None
         self.slot = -1
-        self.block_table: list[int] = []
+        self._blocks: list[int] = []
         self._table_np = None   # int32 mirror of block_table (see table_array)
         self._table_np_valid = 0
-        self._length = 0
+        self._tokens = 0
         self._privatized_block: int | None = None  # block whose page id changed by copy on write (see _reserve_blocks)
 
     # -- state ----------------------------------------------------------------------------------------------------------
+    # Assigning the block table or the length counts as a change of the pool (see TurboQuantLayerPool.version).
+
+    @property
+    def block_table(self) -> list[int]:
+        return self._blocks
+
+    @block_table.setter
+    def block_table(self, pages: list[int]) -> None:
+        self._blocks = pages
+        if self.pool is not None:
+            self.pool.version += 1
+
+    @property
+    def _length(self) -> int:
+        return self._tokens
+
+    @_length.setter
+    def _length(self, tokens: int) -> None:
+        self._tokens = tokens
+        if self.pool is not None:
+            self.pool.version += 1
 
     @property
     def initialized(self) -> bool:
@@ -344,23 +375,27 @@ class TurboQuantKVRow:
 
     @property
     def length(self) -> int:
-        return self._length
+        return self._tokens
 
     @property
     def quantized_length(self) -> int:
-        return max(0, self._length - self.residual_len)
+        return max(0, self._tokens - self.residual_len)
 
     @property
     def residual_length(self) -> int:
-        return min(self._length, self.residual_len)
+        return min(self._tokens, self.residual_len)
 
     def _bind(self, pool: TurboQuantLayerPool, *, kv_heads: int, head_dim: int, dtype: torch.dtype,
               device: torch.device) -> None:
         pool.configure(kv_heads=kv_heads, head_dim=head_dim, bits=self.bits, residual_len=self.residual_len,
                        dtype=dtype, device=device, value_group=self.value_group_size)
+        self._attach(pool)
+
+    def _attach(self, pool: TurboQuantLayerPool) -> None:
+        """Become a row of a pool that is configured for it."""
         self.pool = pool
-        self.device, self.dtype = device, dtype
-        self.head_dim, self.num_heads = int(head_dim), int(kv_heads)
+        self.device, self.dtype = pool.device, pool.dtype
+        self.head_dim, self.num_heads = pool.head_dim, pool.kv_heads
         self.value_group_size = pool.value_group
         self.slot = pool.allocate_slot()
 
@@ -410,7 +445,7 @@ class TurboQuantKVRow:
                 grown[:valid] = arr[:valid]
             arr = self._table_np = grown
         if valid < n:
-            arr[valid:n] = self.block_table[valid:n]
+            arr[valid:n] = array("i", self._blocks[valid:n])
         self._table_np_valid = n
         return arr[:n]
 
@@ -517,6 +552,25 @@ class TurboQuantKVRow:
         self._table_np_valid = 0
         self.slot = -1
         self._length = 0
+
+    @staticmethod
+    def release_all(rows) -> None:
+        """``release`` of several rows: the pages of rows of one pool go back in one pass, in the same order."""
+        rows = [row for row in rows if row.pool is not None and row.slot >= 0]
+        pools = {id(row.pool): row.pool for row in rows}
+        for pool in pools.values():
+            pages: list[int] = []
+            for row in rows:
+                if row.pool is pool:
+                    pages += row._blocks[::-1]
+            pages.reverse()
+            pool.release_pages(pages)  # which gives back the last one first
+        for row in rows:
+            row.pool.release_slot(row.slot)
+            row._blocks = []
+            row._table_np_valid = 0
+            row.slot = -1
+            row._tokens = 0
 
     def to(self, *, device: torch.device | None = None, dtype: torch.dtype | None = None) -> "TurboQuantKVRow":
         if device is not None and self.device is not None and torch.device(device) != self.device:
