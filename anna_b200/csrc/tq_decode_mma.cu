@@ -154,8 +154,7 @@ struct TqMmaCfg {
   // query fragments of one unit, then a second array: the fine bytes of Q1 (4-bit codes) or all of Q2 (planes)
   static constexpr int kFragBytes = 32 * kSteps8 * 16;
   static constexpr int kFrag2Bytes = 32 * kSteps8 * (kPlanes ? 16 : 8);
-  static constexpr int kConstOffset = kFragBytes + kFrag2Bytes;  // per-head factors (and centroid bytes) behind them
-  static_assert(kConstOffset + kTqQueryConstBytes <= tq_query_unit_bytes(D), "the query scratch of a unit is too small");
+  static constexpr int kConstOffset = kFragBytes + kFrag2Bytes;  // per-head factors behind them: [6][8] floats
   static constexpr int kGroups = D / 32;                       // value group size is 32 on this path
   static constexpr int kKeyBytes = D * BITS / 8;               // packed key bytes per token
   static constexpr int kIdxBytes = BITS == 3 ? D / 4 : kKeyBytes;  // first plane (all of it unless BITS == 3)
@@ -182,7 +181,13 @@ struct TqMmaCfg {
   static constexpr int kBarrierBytes = kMmaWarps * kStages * 8;
   static constexpr int kQueryOffset = (kWorkSmem + kBarrierBytes + kMmaWarps * kStages * kTilesPerStep * 4 + 15) / 16 * 16;
   // the query fragments of the CTA live in shared memory (two loads per k-step and step) instead of registers
-  static constexpr int kSmemBytes = kQueryOffset + kFragBytes + kFrag2Bytes;
+  static constexpr int kSmemBytes = kQueryOffset + kConstOffset + 6 * 8 * 4;
+  // While they are made, the rotated queries (two vectors of two heads per warp) lie in the ring stage that the warp's
+  // first copies leave free: with room of their own, four CTAs fill the shared memory and leave the L1 cache nothing.
+  // A vector's quarters are 4 floats further apart than their length and odd heads start 16 floats in, so that the eight
+  // lanes that load together (two heads x four quarters) find their 16 bytes in different banks.
+  static constexpr int kRotFloats = D + 32;
+  static_assert(kStages >= 2 && kTilesPerStep * kStageBytes >= 2 * 2 * kRotFloats * 4, "the rotated queries need a free stage");
   // bytes of one 16-token tile in the stage (= in a 16-token page chunk, padding excluded)
   static constexpr int kTileDataBytes = kOffZero + 16 * kGroups * 2;
   // per-lane key code words per token (this lane's D/4 coordinates)
@@ -195,139 +200,259 @@ struct TqMmaCfg {
 // Bit planes of 2- and 3-bit codes.  A lane holds the codes of its D/4 coordinates (tig * D/4 ...) of a token as words:
 // 16 two-bit fields (2-bit codes; the indices of 3-bit codes) or 32 sign bits (3-bit codes).  Shifted left so that the
 // wanted bits sit at the top of each byte, one mask leaves the bits of the four fields / signs that share a position
-// inside their byte.  Coordinate behind byte `i` of register `r` (0: k 4tig.., 1: k 16 + 4tig..) of k-step `s`:
-template <int D>
-__device__ __forceinline__ int field_plane_coord(int tig, int s, int r, int i) {
-  constexpr int kPairs = D / 128;  // word pairs per lane; s = position * kPairs + pair
-  return tig * (D / 4) + 16 * (2 * (s % kPairs) + r) + 4 * i + s / kPairs;
-}
-template <int D>
-__device__ __forceinline__ int sign_plane_coord(int tig, int s, int r, int i) {
-  return tig * (D / 4) + 32 * (s / 4) + 8 * i + 2 * (s % 4) + r;  // s = word * 4 + pair of positions
-}
+// inside their byte: byte i of register r (0: k 4tig.., 1: k 16 + 4tig..) of k-step s is
+//   fields: coordinate 16 * (2 * (s % kPairs) + r) + 4i + s / kPairs of the lane's run, kPairs = D/128 word pairs
+//   signs:  coordinate 32 * (s / 4) + 8i + 2 * (s % 4) + r
 
-// Rotates the queries of one (row, kv-head group), rounds them to a coarse and a fine byte and stores them as B fragments
-// in the register order of the split kernel, with the per-head factors behind them.
-template <typename T, int D, int BITS>
-__global__ void __launch_bounds__(kMmaThreads) tq_prepare_queries_kernel(const TqDecodeParams p) {
-  using Cfg = TqMmaCfg<T, D, BITS>;
+// What the query preparation needs besides the queries: the same for every segment of a CTA.
+struct TqQueryConsts {
+  uint32_t flips;    // bit j: coordinate lane * E + j is negated by the first rotation (low byte) / by the second
+  uint32_t lut[2];   // 4-bit: the centroids as signed bytes
+  float cent_step;   // 4-bit: the value of one step of those bytes
+};
+
+template <int D, int BITS>
+__device__ __forceinline__ TqQueryConsts load_query_consts(const TqDecodeParams& p) {
   constexpr int E = D / 32;
-  __shared__ float q_rot[2][8][D];
-  __shared__ float q_amax[2][8];
-  const int group_tiles = (p.groups + 7) / 8;
-  const int kvh = blockIdx.x / group_tiles;
-  const int g0 = (blockIdx.x % group_tiles) * 8;
-  const int g_count = min(8, p.groups - g0);
-  const int b = blockIdx.y;
-  const int hq0 = kvh * p.groups + g0;
+  constexpr int kEntries = 1 << (BITS - 1);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const T* q_ptr = reinterpret_cast<const T*>(p.q) + (int64_t)b * p.q_stride_b;
-  for (int g = warp; g < 8; g += kMmaWarps) {
-    float w[E];
+  TqQueryConsts qc{0u, {0u, 0u}, 0.0f};
 #pragma unroll
-    for (int j = 0; j < E; ++j) {
-      const int d = lane * E + j;
-      w[j] = g < g_count ? ElemTraits<T>::to_float(q_ptr[(int64_t)(hq0 + g) * p.q_stride_h + d]) : 0.0f;
-      if (p.signs1[d] < 0.0f) w[j] = -w[j];
-    }
-    warp_fwht<E>(w, lane);
-    float amax1 = 0.0f, amax2 = 0.0f;
+  for (int j = 0; j < E; ++j) {
+    qc.flips |= (__ldg(p.signs1 + lane * E + j) < 0.0f ? 1u : 0u) << j;
+    qc.flips |= (__ldg(p.signs2 + lane * E + j) < 0.0f ? 1u : 0u) << (8 + j);
+  }
+  if constexpr (BITS == 4) {
+    // The byte scale of the centroids is the one, among 256 candidates from 127 down to 63 steps for the largest
+    // centroid, that leaves the smallest squared rounding error over the codebook.
+    __shared__ float best_err_of[kMmaWarps], best_k_of[kMmaWarps];
+    float cent[kEntries], cmax = 0.0f;
 #pragma unroll
-    for (int j = 0; j < E; ++j) {
-      const int d = lane * E + j;
-      q_rot[0][g][d] = w[j];
-      amax1 = fmax_nan(amax1, fabsf(w[j]));
-      if (p.signs2[d] < 0.0f) w[j] = -w[j];
+    for (int e = 0; e < kEntries; ++e) {
+      cent[e] = __ldg(p.centroids + e);
+      cmax = fmaxf(cmax, fabsf(cent[e]));
     }
-    warp_fwht<E>(w, lane);
+    float best_err = INFINITY, best_k = 0.0f;
+    if (cmax > 0.0f) {
+      for (int j = threadIdx.x; j < 256; j += kMmaThreads) {
+        const float k = (127.0f - 0.25f * (float)j) / cmax;
+        float err = 0.0f;
 #pragma unroll
-    for (int j = 0; j < E; ++j) {
-      q_rot[1][g][lane * E + j] = w[j];
-      amax2 = fmax_nan(amax2, fabsf(w[j]));
+        for (int e = 0; e < kEntries; ++e) {
+          const float d = cent[e] * k - rintf(cent[e] * k);
+          err = fmaf(d, d, err);
+        }
+        err /= k * k;
+        if (err < best_err) { best_err = err; best_k = k; }
+      }
     }
+    auto take = [&](float other_err, float other_k) {
+      if (other_err < best_err || (other_err == best_err && other_k > best_k)) { best_err = other_err; best_k = other_k; }
+    };
 #pragma unroll
     for (int dl = 1; dl < 32; dl <<= 1) {
-      amax1 = fmax_nan(amax1, __shfl_xor_sync(0xffffffffu, amax1, dl));
-      amax2 = fmax_nan(amax2, __shfl_xor_sync(0xffffffffu, amax2, dl));
+      const float other_err = __shfl_xor_sync(0xffffffffu, best_err, dl);
+      const float other_k = __shfl_xor_sync(0xffffffffu, best_k, dl);
+      take(other_err, other_k);
     }
-    if (lane == 0) {
-      q_amax[0][g] = amax1;
-      q_amax[1][g] = amax2;
-    }
+    if (lane == 0) { best_err_of[warp] = best_err; best_k_of[warp] = best_k; }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kMmaWarps; ++w) take(best_err_of[w], best_k_of[w]);
+#pragma unroll
+    for (int e = 0; e < kEntries; ++e)
+      qc.lut[e / 4] |= ((uint32_t)__float2int_rn(cent[e] * best_k) & 0xffu) << (8 * (e % 4));
+    qc.lut[0] = pinned_u32(qc.lut[0], lane);
+    qc.lut[1] = pinned_u32(qc.lut[1], lane);
+    qc.cent_step = best_k > 0.0f ? 1.0f / best_k : 0.0f;
   }
-  __syncthreads();
-  // score (log2 units) = norm * (S1 + rnorm * S2) with every constant folded into the fragments:
+  return qc;
+}
+
+// Rotates the queries of one (row, kv-head group), rounds them to a coarse and a fine byte and leaves them at `query` in
+// shared memory as the B fragments of m16n8k32 in the register order of the score products, with the per-head factors
+// behind them (offsets of TqMmaCfg).  Every CTA does this for itself, once per segment, while its first tiles are on
+// their way: 2-3 us of a CTA, against 5-14 us of a kernel in front of the whole call (which read the rotated vectors with
+// 32 lanes in one bank): one row of 4 K tokens 35 -> 27 us, 16 rows of 0.4-4 K at head_dim 256 74 -> 60 us, 128 rows of
+// 0.5-16 K 253 -> 247 us, 64 rows of 32 K 630 -> 636 us.  The caller synchronises afterwards.
+template <typename T, int D, int BITS>
+__device__ __forceinline__ void prepare_query_fragments(const TqDecodeParams& p, uint8_t* smem_raw, uint8_t* query,
+                                                        int free_stage, int b, int hq0, int g_count,
+                                                        const TqQueryConsts& qc) {
+  using Cfg = TqMmaCfg<T, D, BITS>;
+  constexpr int E = D / 32;
+  constexpr int kSteps8 = Cfg::kSteps8;
+  __shared__ float q_scale[2][8];    // 127 / largest coordinate
+  __shared__ int rot_at[kMmaWarps];  // where the heads g, g + 4 of warp g are: the free stage differs from warp to warp
+  float* consts = reinterpret_cast<float*>(query + Cfg::kConstOffset);
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) rot_at[warp] = warp * Cfg::kWarpSmem + free_stage * Cfg::kTilesPerStep * Cfg::kStageBytes;
+  __syncwarp();
+  // quarter `tig` of rotation `which` of head g
+  auto rotated = [&](int which, int g, int tig) {
+    return reinterpret_cast<float*>(smem_raw + rot_at[g % kMmaWarps]) + (2 * (g / kMmaWarps) + which) * Cfg::kRotFloats +
+           16 * (g & 1) + tig * (D / 4 + 4);
+  };
+  // heads that do not exist: scale and factors zero, which makes bytes of zero of whatever their vectors hold
+  if (threadIdx.x < 8 && (int)threadIdx.x >= g_count) {
+    q_scale[0][threadIdx.x] = q_scale[1][threadIdx.x] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) consts[8 * i + threadIdx.x] = 0.0f;
+  }
+  auto coarse = [](float v, float k) { return max(-127, min(127, __float2int_rn(v * k))); };
+  auto fine = [](float v, float k, int c) { return max(-127, min(127, __float2int_rn((v * k - (float)c) * 254.0f))); };
+  const uint32_t flips = qc.flips;
+  // score (log2 units) = norm * (S1 + rnorm * S2) with every constant folded into the factors:
   //   q.k_hat = norm/D * [Q1.c + sqrt(pi/2)/sqrt(D) * rnorm * Q2.sign],  Q1 = fwht(s1*q), Q2 = fwht(s2*Q1)
   const float inv_sqrt_d = rsqrt_dim_const<D>();
   const float log2e = 1.4426950408889634f;
   const float f1 = p.scaling * log2e * inv_sqrt_d * inv_sqrt_d;
   const float f2 = p.scaling * log2e * 1.2533141373155001f * inv_sqrt_d * inv_sqrt_d * inv_sqrt_d;
-  uint8_t* unit = reinterpret_cast<uint8_t*>(p.query_frags) + ((int64_t)b * gridDim.x + blockIdx.x) * tq_query_unit_bytes(D);
-  auto coarse = [](float v, float k) { return max(-127, min(127, __float2int_rn(v * k))); };
-  auto fine = [](float v, float k, int c) { return max(-127, min(127, __float2int_rn((v * k - (float)c) * 254.0f))); };
-  if constexpr (!Cfg::kPlanes) {
-    // 8-bit B fragments of m16n8k32: lane (gid, tig) feeds head gid with the coordinates of its code word s,
-    // tig * D/4 + 8s + {0..3} in the first register and + {4..7} in the second.  The rotated query is split into a
-    // coarse byte (127 steps up to the head's largest coordinate) and a fine byte (the rounding remainder in 1/254
-    // steps), so the centroid product sees about 15 bits of it; the sign product uses a coarse byte only.
-    //   [s][lane][q1 b0, q1 b1, q2 b0, q2 b1]   then   [s][lane][q1 fine b0, q1 fine b1]
-    // Behind them, per head: the factor of the centroid product, the factor of the sign product and the integer the
-    // sign accumulators start from (sign bytes are 2 for a clear bit and 0 for a set one: 2 * sum over clear bits
-    // minus the sum over all coordinates is minus the +-1 product); then the centroids as signed bytes.
-    constexpr int kSteps8 = Cfg::kSteps8;
-    constexpr int kEntries = 1 << (BITS - 1);
-    __shared__ float cent_scale;
-    if (warp == 0) {
-      // The byte scale of the centroids is the one, among 256 candidates from 127 down to 63 steps for the largest
-      // centroid, that leaves the smallest squared rounding error over the codebook.
-      float cent[kEntries], cmax = 0.0f;
+  const T* q_ptr = reinterpret_cast<const T*>(p.q) + (int64_t)b * p.q_stride_b + (int64_t)hq0 * p.q_stride_h;
+  for (int g = warp; g < g_count; g += kMmaWarps) {
+    float w[E], w1[E];
 #pragma unroll
-      for (int e = 0; e < kEntries; ++e) {
-        cent[e] = __ldg(p.centroids + e);
-        cmax = fmaxf(cmax, fabsf(cent[e]));
-      }
-      float best_err = INFINITY, best_k = 0.0f;
-      if (cmax > 0.0f) {
-        for (int j = lane; j < 256; j += 32) {
-          const float k = (127.0f - 0.25f * (float)j) / cmax;
-          float err = 0.0f;
+    for (int j = 0; j < E; ++j) {
+      w[j] = ElemTraits<T>::to_float(q_ptr[(int64_t)g * p.q_stride_h + lane * E + j]);
+      if ((flips >> j) & 1u) w[j] = -w[j];
+    }
+    warp_fwht<E>(w, lane);
+    float amax1 = 0.0f, amax2 = 0.0f;
 #pragma unroll
-          for (int e = 0; e < kEntries; ++e) {
-            const float d = (cent[e] * k - rintf(cent[e] * k)) / k;
-            err += d * d;
-          }
-          if (err < best_err) { best_err = err; best_k = k; }
-        }
-      }
+    for (int j = 0; j < E; ++j) {
+      w1[j] = w[j];
+      rotated(0, g, lane / 8)[lane % 8 * E + j] = w[j];
+      amax1 = fmax_nan(amax1, fabsf(w[j]));
+      if ((flips >> (8 + j)) & 1u) w[j] = -w[j];
+    }
+    warp_fwht<E>(w, lane);
 #pragma unroll
-      for (int dl = 1; dl < 32; dl <<= 1) {
-        const float other_err = __shfl_xor_sync(0xffffffffu, best_err, dl);
-        const float other_k = __shfl_xor_sync(0xffffffffu, best_k, dl);
-        if (other_err < best_err || (other_err == best_err && other_k > best_k)) { best_err = other_err; best_k = other_k; }
-      }
-      if (lane == 0) {
-        cent_scale = best_k;
-        uint32_t lut[2] = {0u, 0u};
+    for (int j = 0; j < E; ++j) {
+      rotated(1, g, lane / 8)[lane % 8 * E + j] = w[j];
+      amax2 = fmax_nan(amax2, fabsf(w[j]));
+    }
+    // as integers, non-negative floats keep their order and a NaN is above all of them
+    amax1 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax1)));
+    amax2 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax2)));
+    const float k1 = amax1 > 0.0f ? 127.0f / amax1 : 0.0f, k2 = amax2 > 0.0f ? 127.0f / amax2 : 0.0f;
+    int total1 = 0, total2 = 0;
 #pragma unroll
-        for (int e = 0; e < kEntries; ++e)
-          lut[e / 4] |= ((uint32_t)__float2int_rn(cent[e] * best_k) & 0xffu) << (8 * (e % 4));
-        uint32_t* consts = reinterpret_cast<uint32_t*>(unit + Cfg::kConstOffset);
-        consts[24] = lut[0];
-        consts[25] = lut[1];
+    for (int j = 0; j < E; ++j) {
+      const int c2 = coarse(w[j], k2);
+      if constexpr (Cfg::kPlanes) {
+        const int c1 = coarse(w1[j], k1);
+        total1 += 254 * c1 + fine(w1[j], k1, c1);
+        total2 += 254 * c2 + fine(w[j], k2, c2);
+      } else {
+        total2 += c2;
       }
     }
-    __syncthreads();
-    uint4* out = reinterpret_cast<uint4*>(unit);
-    uint2* out_lo = reinterpret_cast<uint2*>(unit + Cfg::kFragBytes);
-    for (int item = threadIdx.x; item < 32 * kSteps8; item += kMmaThreads) {
-      const int ln = item / kSteps8;
-      const int s = item % kSteps8;
-      const int gid = ln >> 2, tig = ln & 3;
-      const float k1 = q_amax[0][gid] > 0.0f ? 127.0f / q_amax[0][gid] : 0.0f;
-      const float k2 = q_amax[1][gid] > 0.0f ? 127.0f / q_amax[1][gid] : 0.0f;
-      const float* r1 = q_rot[0][gid] + tig * (D / 4) + 8 * s;
-      const float* r2 = q_rot[1][gid] + tig * (D / 4) + 8 * s;
+    if constexpr (Cfg::kPlanes) total1 = __reduce_add_sync(0xffffffffu, total1);
+    total2 = __reduce_add_sync(0xffffffffu, total2);
+    if (lane == 0) {
+      q_scale[0][g] = k1;
+      q_scale[1][g] = k2;
+      if constexpr (Cfg::kPlanes) {
+        // With u = the value of one step of the fine byte and Q the 254 * coarse + fine integers: a plane with its bits
+        // at weight 2^j of a byte gives T = 2^j * sum over set bits of Q.
+        //   sign plane (+1 set, -1 clear, weight 128):  S2 = T * 2u / 128 - u * sum(Q)
+        //   index planes: centroid = z0 + z1 * bit0 + z2 * bit1 (+ z3 * bit0 * bit1, zero for the symmetric codebooks):
+        //   S1 = T0 * z1 * u / 64 (+ T1 * z2 * u / 128 + T01 * z3 * u / 64) + z0 * u * sum(Q)
+        // [0] factor of bit plane 0, [1] of bit plane 1, [2] of both, [3] constant of S1, [4] factor, [5] constant of S2
+        const float u1 = amax1 * f1 / (127.0f * 254.0f), u2 = amax2 * f2 / (127.0f * 254.0f);
+        const float* cent = p.centroids;
+        const float z1 = __ldg(cent + 1) - __ldg(cent);
+        consts[g] = z1 * u1 / 64.0f;
+        if constexpr (BITS == 3) {
+          consts[8 + g] = (__ldg(cent + 2) - __ldg(cent)) * u1 / 128.0f;
+          consts[16 + g] = ((__ldg(cent + 3) - __ldg(cent + 2)) - z1) * u1 / 64.0f;
+        }
+        consts[24 + g] = __ldg(cent) * u1 * (float)total1;
+        consts[32 + g] = u2 / 64.0f;
+        consts[40 + g] = -u2 * (float)total2;
+      } else {
+        // factor of the centroid product, factor of the sign product and the
+        // integer the sign accumulators start from: sign bytes are 2 for a clear bit and 0 for a set one, and 2 * sum
+        // over clear bits minus the sum over all coordinates is minus the +-1 product
+        consts[g] = amax1 * f1 / (127.0f * 254.0f) * qc.cent_step;
+        consts[8 + g] = -(amax2 * f2 / 127.0f);
+        reinterpret_cast<int*>(consts)[16 + g] = -total2;
+      }
+    }
+  }
+  __syncthreads();
+  const int gid = lane >> 2, tig = lane & 3;
+  if constexpr (Cfg::kPlanes) {
+    // [s][lane][Q1 coarse b0, b1, Q1 fine b0, b1]   then   [s][lane][Q2 coarse b0, b1, Q2 fine b0, b1]: a warp makes one
+    // register of one rotation
+    const int which = warp >> 1, r = warp & 1;
+    const float k = q_scale[which][gid];
+    const float* v = rotated(which, gid, tig);
+    uint32_t* out = reinterpret_cast<uint32_t*>(query) + which * 32 * kSteps8 * 4 + lane * 4 + r;
+    auto put = [&](int s, float v0, float v1, float v2, float v3) {
+      const float x[4] = {v0, v1, v2, v3};
+      uint32_t hi = 0u, lo = 0u;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int c = coarse(x[i], k);
+        hi |= ((uint32_t)c & 0xffu) << (8 * i);
+        lo |= ((uint32_t)fine(x[i], k, c) & 0xffu) << (8 * i);
+      }
+      out[s * 128] = hi;
+      out[s * 128 + 2] = lo;
+    };
+    auto four = [&](int d) { return *reinterpret_cast<const float4*>(v + d); };
+    if (BITS == 3 && which == 1) {
+      // sign plane: k-step s takes, of each group of 8 coordinates of word s / 4, number 2 * (s % 4) + r
+#pragma unroll
+      for (int w = 0; w < D / 128; ++w) {
+        float4 a[4], b4[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          a[i] = four(32 * w + 8 * i);
+          b4[i] = four(32 * w + 8 * i + 4);
+        }
+        if (r == 0) {
+          put(4 * w + 0, a[0].x, a[1].x, a[2].x, a[3].x);
+          put(4 * w + 1, a[0].z, a[1].z, a[2].z, a[3].z);
+          put(4 * w + 2, b4[0].x, b4[1].x, b4[2].x, b4[3].x);
+          put(4 * w + 3, b4[0].z, b4[1].z, b4[2].z, b4[3].z);
+        } else {
+          put(4 * w + 0, a[0].y, a[1].y, a[2].y, a[3].y);
+          put(4 * w + 1, a[0].w, a[1].w, a[2].w, a[3].w);
+          put(4 * w + 2, b4[0].y, b4[1].y, b4[2].y, b4[3].y);
+          put(4 * w + 3, b4[0].w, b4[1].w, b4[2].w, b4[3].w);
+        }
+      }
+    } else {
+      // fields: k-step s takes, of each group of 4 coordinates of word 2 * (s % kPairs) + r, number s / kPairs
+      constexpr int kPairs = D / 128;
+#pragma unroll
+      for (int pair = 0; pair < kPairs; ++pair) {
+        float4 a[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = four(16 * (2 * pair + r) + 4 * i);
+        put(0 * kPairs + pair, a[0].x, a[1].x, a[2].x, a[3].x);
+        put(1 * kPairs + pair, a[0].y, a[1].y, a[2].y, a[3].y);
+        put(2 * kPairs + pair, a[0].z, a[1].z, a[2].z, a[3].z);
+        put(3 * kPairs + pair, a[0].w, a[1].w, a[2].w, a[3].w);
+      }
+    }
+  } else {
+    // lane (gid, tig) feeds head gid with the coordinates of its code word s, tig * D/4 + 8s + {0..3} in the first
+    // register and + {4..7} in the second; the sign product uses a coarse byte only
+    //   [s][lane][Q1 coarse b0, b1, Q2 coarse b0, b1]   then   [s][lane][Q1 fine b0, b1]
+    const float k1 = q_scale[0][gid], k2 = q_scale[1][gid];
+#pragma unroll
+    for (int s = warp; s < kSteps8; s += kMmaWarps) {
+      float r1[8], r2[8];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        *reinterpret_cast<float4*>(r1 + 4 * h) = *reinterpret_cast<const float4*>(rotated(0, gid, tig) + 8 * s + 4 * h);
+        *reinterpret_cast<float4*>(r2 + 4 * h) = *reinterpret_cast<const float4*>(rotated(1, gid, tig) + 8 * s + 4 * h);
+      }
       uint32_t w[4] = {0u, 0u, 0u, 0u}, wl[2] = {0u, 0u};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -339,80 +464,8 @@ __global__ void __launch_bounds__(kMmaThreads) tq_prepare_queries_kernel(const T
         w[2] |= ((uint32_t)coarse(r2[i], k2) & 0xffu) << (8 * i);
         w[3] |= ((uint32_t)coarse(r2[4 + i], k2) & 0xffu) << (8 * i);
       }
-      out[s * 32 + ln] = make_uint4(w[0], w[1], w[2], w[3]);
-      out_lo[s * 32 + ln] = make_uint2(wl[0], wl[1]);
-    }
-    if (threadIdx.x < 8) {
-      const int g = threadIdx.x;
-      const float k2 = q_amax[1][g] > 0.0f ? 127.0f / q_amax[1][g] : 0.0f;
-      int total = 0;
-      for (int d = 0; d < D; ++d) total += coarse(q_rot[1][g][d], k2);
-      float* consts = reinterpret_cast<float*>(unit + Cfg::kConstOffset);
-      consts[g] = cent_scale > 0.0f ? (q_amax[0][g] * f1 / 127.0f) / cent_scale / (ANNA_TQ_FINE_QUERY ? 254.0f : 1.0f) : 0.0f;
-      consts[8 + g] = -(q_amax[1][g] * f2 / 127.0f);
-      reinterpret_cast<int*>(consts)[16 + g] = -total;
-    }
-  } else {
-    // [s][lane][Q1 coarse b0, b1, Q1 fine b0, b1]   then   [s][lane][Q2 coarse b0, b1, Q2 fine b0, b1]
-    constexpr int kSteps8 = Cfg::kSteps8;
-    uint4* out = reinterpret_cast<uint4*>(unit);
-    uint4* out2 = reinterpret_cast<uint4*>(unit + Cfg::kFragBytes);
-    for (int item = threadIdx.x; item < 32 * kSteps8; item += kMmaThreads) {
-      const int ln = item & 31;
-      const int s = item >> 5;
-      const int gid = ln >> 2, tig = ln & 3;
-#pragma unroll
-      for (int which = 0; which < 2; ++which) {
-        const float k = q_amax[which][gid] > 0.0f ? 127.0f / q_amax[which][gid] : 0.0f;
-        uint32_t w[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-        for (int r = 0; r < 2; ++r)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int d = (BITS == 3 && which == 1) ? sign_plane_coord<D>(tig, s, r, i) : field_plane_coord<D>(tig, s, r, i);
-            const float v = q_rot[which][gid][d];
-            const int c = coarse(v, k);
-            w[r] |= ((uint32_t)c & 0xffu) << (8 * i);
-            w[2 + r] |= ((uint32_t)fine(v, k, c) & 0xffu) << (8 * i);
-          }
-        (which == 0 ? out : out2)[s * 32 + ln] = make_uint4(w[0], w[1], w[2], w[3]);
-      }
-    }
-    // Per head, with u = the value of one step of the fine byte and Q the 254 * coarse + fine integers: a plane with
-    // its bits at weight 2^j of a byte gives T = 2^j * sum over set bits of Q.
-    //   sign plane (+1 set, -1 clear, weight 128):  S2 = T * 2u / 128 - u * sum(Q)
-    //   index planes: centroid = z0 + z1 * bit0 + z2 * bit1 (+ z3 * bit0 * bit1, zero for the symmetric codebooks):
-    //   S1 = T0 * z1 * u / 64 (+ T1 * z2 * u / 128 + T01 * z3 * u / 64) + z0 * u * sum(Q)
-    // [0] factor of bit plane 0, [8] of bit plane 1, [16] of both, [24] constant of S1, [32] factor and [40] constant of S2
-    float* consts = reinterpret_cast<float*>(unit + Cfg::kConstOffset);
-    for (int g = warp; g < 8; g += kMmaWarps) {
-      int total[2] = {0, 0};
-#pragma unroll
-      for (int which = 0; which < 2; ++which) {
-        const float k = q_amax[which][g] > 0.0f ? 127.0f / q_amax[which][g] : 0.0f;
-#pragma unroll
-        for (int j = 0; j < E; ++j) {
-          const float v = q_rot[which][g][lane + 32 * j];
-          const int c = coarse(v, k);
-          total[which] += 254 * c + fine(v, k, c);
-        }
-        total[which] = __reduce_add_sync(0xffffffffu, total[which]);
-      }
-      if (lane == 0) {
-        const float u1 = q_amax[0][g] * f1 / (127.0f * 254.0f), u2 = q_amax[1][g] * f2 / (127.0f * 254.0f);
-        const float z0 = __ldg(p.centroids), z1 = __ldg(p.centroids + 1) - z0;
-        float z2 = 0.0f, z3 = 0.0f;
-        if constexpr (BITS == 3) {
-          z2 = __ldg(p.centroids + 2) - z0;
-          z3 = (__ldg(p.centroids + 3) - __ldg(p.centroids + 2)) - z1;
-        }
-        consts[g] = z1 * u1 / 64.0f;
-        consts[8 + g] = z2 * u1 / 128.0f;
-        consts[16 + g] = z3 * u1 / 64.0f;
-        consts[24 + g] = z0 * u1 * (float)total[0];
-        consts[32 + g] = u2 / 64.0f;
-        consts[40 + g] = -u2 * (float)total[1];
-      }
+      reinterpret_cast<uint4*>(query)[s * 32 + lane] = make_uint4(w[0], w[1], w[2], w[3]);
+      reinterpret_cast<uint2*>(query + Cfg::kFragBytes)[s * 32 + lane] = make_uint2(wl[0], wl[1]);
     }
   }
 }
@@ -478,9 +531,9 @@ struct PackedRing {
 // partial goes to split-K slot `out_slot` and counts as one of `arrivals`; the CTA that counts last merges `slots` partials.
 // All threads of the CTA call it; it ends with the CTA synchronised against reuse of the ring.
 template <typename T, int D, int BITS>
-__device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8_t* smem_raw, PackedRing& ring, int b,
-                                                  int unit, int units, int t0, int t1, int out_slot, int slots,
-                                                  int arrivals) {
+__device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8_t* smem_raw,
+                                                  const TqQueryConsts& qc, PackedRing& ring, int b, int unit,
+                                                  int units, int t0, int t1, int out_slot, int slots, int arrivals) {
   using Cfg = TqMmaCfg<T, D, BITS>;
   constexpr int U = Cfg::kTilesPerStep;
   const int group_tiles = (p.groups + 7) / 8;
@@ -494,49 +547,6 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
   const int lane = threadIdx.x & 31;
   const int gid = lane >> 2;
   const int tig = lane & 3;
-  // Q fragments (softmax scale and log2(e) folded into the factors) were prepared by tq_prepare_queries_kernel in exactly
-  // this lane's register order, with the per-head factors behind them; they go to shared memory once per CTA
-  const uint4* q_frag = reinterpret_cast<const uint4*>(smem_raw + Cfg::kQueryOffset) + lane;                     // [s][lane]
-  const uint2* q_fine = reinterpret_cast<const uint2*>(smem_raw + Cfg::kQueryOffset + Cfg::kFragBytes) + lane;   // 4-bit
-  const uint4* q_frag2 = reinterpret_cast<const uint4*>(smem_raw + Cfg::kQueryOffset + Cfg::kFragBytes) + lane;  // planes
-  (void)q_fine; (void)q_frag2;
-  float beta1[2] = {0.0f, 0.0f}, beta2[2] = {0.0f, 0.0f};  // this lane's two heads (columns 2tig, 2tig + 1)
-  float k_bit1[2] = {0.0f, 0.0f}, k_both[2] = {0.0f, 0.0f}, c_idx[2] = {0.0f, 0.0f}, c_sign[2] = {0.0f, 0.0f};  // planes
-  int s2_start[2] = {0, 0};                                                                                      // 4-bit
-  uint32_t lut[2] = {0u, 0u};  // 4-bit: the centroids as signed bytes, as the query preparation rounded them
-  (void)k_bit1; (void)k_both; (void)c_idx; (void)c_sign; (void)s2_start; (void)lut;
-  {
-    const uint8_t* unit_frags = reinterpret_cast<const uint8_t*>(p.query_frags) + ((int64_t)b * units + unit) * tq_query_unit_bytes(D);
-    const uint4* src = reinterpret_cast<const uint4*>(unit_frags);
-    uint4* dst = reinterpret_cast<uint4*>(smem_raw + Cfg::kQueryOffset);
-    for (int i = threadIdx.x; i < (Cfg::kFragBytes + Cfg::kFrag2Bytes) / 16; i += kMmaThreads) dst[i] = __ldg(src + i);
-    const float* consts = reinterpret_cast<const float*>(unit_frags + Cfg::kConstOffset);
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      beta1[c] = __ldg(consts + 2 * tig + c);
-      if constexpr (Cfg::kPlanes) {
-        if constexpr (BITS == 3) {
-          k_bit1[c] = __ldg(consts + 8 + 2 * tig + c);
-          k_both[c] = __ldg(consts + 16 + 2 * tig + c);
-        }
-        c_idx[c] = __ldg(consts + 24 + 2 * tig + c);
-        beta2[c] = __ldg(consts + 32 + 2 * tig + c);
-        c_sign[c] = __ldg(consts + 40 + 2 * tig + c);
-      } else {
-        beta2[c] = __ldg(consts + 8 + 2 * tig + c);
-        s2_start[c] = __ldg(reinterpret_cast<const int*>(consts) + 16 + 2 * tig + c);
-      }
-    }
-    if constexpr (!Cfg::kPlanes) {
-      lut[0] = pinned_u32(__ldg(reinterpret_cast<const uint32_t*>(consts) + 24), lane);
-      lut[1] = pinned_u32(__ldg(reinterpret_cast<const uint32_t*>(consts) + 25), lane);
-    }
-    __syncthreads();
-  }
-
-  const bool skewed = BITS == 3 && __any_sync(0xffffffffu, k_both[0] != 0.0f || k_both[1] != 0.0f);
-  (void)skewed;
-
   // loop constants held in registers
   // (only the ones this instantiation uses are created)
   const uint32_t nib_mask = BITS != 2 ? pinned_u32(0x03C003C0u, lane) : 0u;    // 4-bit value codes
@@ -617,6 +627,41 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
 #pragma unroll
   for (int i = 0; i < Cfg::kStages - 1; ++i)
     if (i < my_steps) issue_step(i, (ring.stage + i) % Cfg::kStages);
+
+  // Q fragments and their factors for this lane's two heads (columns 2tig, 2tig + 1); the softmax scale and log2(e) are
+  // folded into the factors
+  uint8_t* query = smem_raw + Cfg::kQueryOffset;
+  const uint32_t lut[2] = {qc.lut[0], qc.lut[1]};
+  prepare_query_fragments<T, D, BITS>(p, smem_raw, query, (ring.stage + 1) % Cfg::kStages, b, hq0, g_count, qc);
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // the loop's first copy lands where the rotations were
+  __syncthreads();
+  const uint4* q_frag = reinterpret_cast<const uint4*>(query) + lane;                     // [s][lane]
+  const uint2* q_fine = reinterpret_cast<const uint2*>(query + Cfg::kFragBytes) + lane;   // 4-bit
+  const uint4* q_frag2 = reinterpret_cast<const uint4*>(query + Cfg::kFragBytes) + lane;  // planes
+  float beta1[2], beta2[2];                                              // factors of the two products
+  float k_bit1[2] = {0.0f, 0.0f}, k_both[2] = {0.0f, 0.0f}, c_idx[2] = {0.0f, 0.0f}, c_sign[2] = {0.0f, 0.0f};  // planes
+  int s2_start[2] = {0, 0};                                                                                      // 4-bit
+  {
+    const float* consts = reinterpret_cast<const float*>(query + Cfg::kConstOffset) + 2 * tig;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      beta1[c] = consts[c];
+      if constexpr (Cfg::kPlanes) {
+        if constexpr (BITS == 3) {
+          k_bit1[c] = consts[8 + c];
+          k_both[c] = consts[16 + c];
+        }
+        c_idx[c] = consts[24 + c];
+        beta2[c] = consts[32 + c];
+        c_sign[c] = consts[40 + c];
+      } else {
+        beta2[c] = consts[8 + c];
+        s2_start[c] = reinterpret_cast<const int*>(consts)[16 + c];
+      }
+    }
+  }
+  const bool skewed = BITS == 3 && __any_sync(0xffffffffu, k_both[0] != 0.0f || k_both[1] != 0.0f);
+  (void)q_fine; (void)q_frag2; (void)k_bit1; (void)k_both; (void)c_idx; (void)c_sign; (void)s2_start; (void)lut; (void)skewed;
 
   // MMA row r of a tile holds token r ^ ((r >> 1) & 1): neighbouring token rows sit in different halves of the
   // shared-memory banks, and with this order the four token rows one value load touches fall into both halves.
@@ -1056,8 +1101,9 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
   const int t0 = chunk * p.chunk_tokens;
   init_packed_barriers<T, D, BITS>(smem_raw);
   PackedRing ring{0, 0u, false};
+  const TqQueryConsts qc = load_query_consts<D, BITS>(p);
   // active slots stay contiguous: [window | packed]
-  tq_packed_segment<T, D, BITS>(p, smem_raw, ring, b, (int)blockIdx.y, (int)gridDim.y, t0, min(Lq, t0 + p.chunk_tokens),
+  tq_packed_segment<T, D, BITS>(p, smem_raw, qc, ring, b, (int)blockIdx.y, (int)gridDim.y, t0, min(Lq, t0 + p.chunk_tokens),
                                 active_window + chunk, active_window + active_packed, active_packed);
 }
 
@@ -1069,12 +1115,13 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
   const int units = p.kv_heads * ((p.groups + 7) / 8);
   init_packed_barriers<T, D, BITS>(smem_raw);
   PackedRing ring{0, 0u, false};
+  const TqQueryConsts qc = load_query_consts<D, BITS>(p);
   balanced_for_each_segment<kMmaThreads>(
       p.lengths, p.max_len, batch, units, min(p.chunk_capacity, kFusedMaxChunks) - p.num_window_chunks,
       [](int) {},  // rows without packed tokens belong to the window kernel
       [&](int b, int unit, int t0, int t1, int slot, int partials) {
         const int active_window = (p.residual_len + p.chunk_tokens - 1) / p.chunk_tokens;  // the window of this row is full
-        tq_packed_segment<T, D, BITS>(p, smem_raw, ring, b, unit, units, t0, t1, active_window + slot,
+        tq_packed_segment<T, D, BITS>(p, smem_raw, qc, ring, b, unit, units, t0, t1, active_window + slot,
                                       active_window + partials, partials);
       },
       p.residual_len, kMmaWarps * TqMmaCfg<T, D, BITS>::kTilesPerStep);
@@ -1119,17 +1166,12 @@ static int launch_tq_mma(const TqDecodeParams& p, int batch, cudaStream_t stream
        p.layout.chunk_bytes < Cfg::kTileDataBytes))
     return set_error(ANNA_ERR_INVALID, "packed page layout does not match the decode kernel's tile layout");
   const int group_tiles = (p.groups + 7) / 8;
-  dim3 prep_grid((unsigned)(p.kv_heads * group_tiles), (unsigned)batch);
-  tq_prepare_queries_kernel<T, D, BITS><<<prep_grid, kMmaThreads, 0, stream>>>(p);
-  int rc = check_launch("tq_prepare_queries_kernel");
-  if (rc != ANNA_OK) return rc;
   dim3 window_grid((unsigned)p.num_window_chunks, (unsigned)(p.kv_heads * group_tiles), (unsigned)batch);
   tq_window_split_mma_kernel<T, D><<<window_grid, kMmaThreads, MmaCfg<D>::kSmemBytes, stream>>>(p);
-  rc = check_launch("tq_window_split_mma_kernel");
+  const int rc = check_launch("tq_window_split_mma_kernel");
   if (rc != ANNA_OK) return rc;
   if (p.num_chunks <= p.num_window_chunks) return rc;
-  // Programmatic dependent launch: the packed chunks run beside the (small) window launch instead of after it; the query
-  // fragments they read come from the launch before that one, which has completed by then.
+  // programmatic dependent launch: the packed chunks run beside the (small) window launch instead of after it
   cudaLaunchConfig_t config = {};
   config.blockDim = dim3(kMmaThreads);
   config.dynamicSmemBytes = Cfg::kSmemBytes;

@@ -45,16 +45,11 @@ size_t tq_umma_query_bytes();  // query operand image per (row, kv head) of that
 // the window-ring launch of the tensor-core paths (tq_decode_mma.cu)
 int launch_tq_window_split(const TqDecodeParams& p, int batch, int head_dim, int dtype, cudaStream_t stream);
 
-// Query scratch of one (row, kv head, group of 8 query heads) of the mma.sync path: up to 32 * head_dim fragment bytes (two
-// rotations of 8 heads, a coarse and a fine byte each), then the per-head factors.
-constexpr int kTqQueryConstBytes = 256;
-constexpr __host__ __device__ int tq_query_unit_bytes(int head_dim) { return 32 * head_dim + kTqQueryConstBytes; }
-
-// Bytes of query scratch the tensor-core paths need per call: one unit per (row, kv head, group of 8 query heads) for the
-// mma.sync path, one query operand image per (row, kv head) for the tensor-memory path.
+// Bytes of query scratch of a call: one query operand image per (row, kv head) for the tensor-memory path; the mma.sync
+// path needs none, but callers keep handing in what it used to need.
 inline size_t tq_query_scratch_bytes(int batch, int q_heads, int kv_heads, int head_dim) {
   const size_t units = (size_t)batch * kv_heads * ((q_heads / kv_heads + 7) / 8);
-  const size_t frag = (size_t)tq_query_unit_bytes(head_dim);
+  const size_t frag = (size_t)32 * head_dim;
   const size_t image = tq_umma_query_bytes();
   return units * (frag > image ? frag : image);
 }
