@@ -134,9 +134,6 @@ __device__ __forceinline__ float fast_exp2(float x) {
 #ifndef ANNA_TQ_RING_TILES
 #define ANNA_TQ_RING_TILES 4
 #endif
-#ifndef ANNA_TQ_FINE_QUERY
-#define ANNA_TQ_FINE_QUERY 1
-#endif
 constexpr float kLazyRescale = 8.0f;  // log2 units: probabilities stay below 2^8, well inside fp16
 
 template <typename T, int D, int BITS>
@@ -530,12 +527,19 @@ struct PackedRing {
 // One packed segment: tokens [t0, t1) of the quantized prefix of (row b, unit = kv head and group of 8 query heads).  The
 // partial goes to split-K slot `out_slot` and counts as one of `arrivals`; the CTA that counts last merges `slots` partials.
 // All threads of the CTA call it; it ends with the CTA synchronised against reuse of the ring.
-template <typename T, int D, int BITS>
+//
+// kPair (at most 4 query heads): the eight columns of the products are 4 heads x the two tiles of a step.  The query
+// operand of a tile is zero in the other tile's columns, so both tiles add into one set of accumulators, and the score
+// arithmetic, the softmax and the registers behind it are spent once per two tiles instead of once per tile with half of
+// the columns empty; columns j and j + 4 are two partials of head j, merged with those of the other warps.
+template <typename T, int D, int BITS, bool kPair>
 __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8_t* smem_raw,
                                                   const TqQueryConsts& qc, PackedRing& ring, int b, int unit,
                                                   int units, int t0, int t1, int out_slot, int slots, int arrivals) {
   using Cfg = TqMmaCfg<T, D, BITS>;
   constexpr int U = Cfg::kTilesPerStep;
+  constexpr int A = kPair ? 1 : U;  // sets of score accumulators
+  static_assert(!kPair || U == 2, "a pair is the two tiles of a step");
   const int group_tiles = (p.groups + 7) / 8;
   const int kvh = unit / group_tiles;
   const int g0 = (unit % group_tiles) * 8;
@@ -638,11 +642,15 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
   const uint4* q_frag = reinterpret_cast<const uint4*>(query) + lane;                     // [s][lane]
   const uint2* q_fine = reinterpret_cast<const uint2*>(query + Cfg::kFragBytes) + lane;   // 4-bit
   const uint4* q_frag2 = reinterpret_cast<const uint4*>(query + Cfg::kFragBytes) + lane;  // planes
+  // the fragments of the second tile of a pair: heads 0-3 in columns 4-7 and (from the empty heads 4-7) zeros in 0-3
+  const int flip = (lane ^ 16) - lane;
+  const int my_tile = kPair ? tig >> 1 : 0;  // tile whose scores this lane's two columns hold
+  const int my_head = kPair ? (2 * tig) & 3 : 2 * tig;
   float beta1[2], beta2[2];                                              // factors of the two products
   float k_bit1[2] = {0.0f, 0.0f}, k_both[2] = {0.0f, 0.0f}, c_idx[2] = {0.0f, 0.0f}, c_sign[2] = {0.0f, 0.0f};  // planes
   int s2_start[2] = {0, 0};                                                                                      // 4-bit
   {
-    const float* consts = reinterpret_cast<const float*>(query + Cfg::kConstOffset) + 2 * tig;
+    const float* consts = reinterpret_cast<const float*>(query + Cfg::kConstOffset) + my_head;
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       beta1[c] = consts[c];
@@ -661,7 +669,7 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
     }
   }
   const bool skewed = BITS == 3 && __any_sync(0xffffffffu, k_both[0] != 0.0f || k_both[1] != 0.0f);
-  (void)q_fine; (void)q_frag2; (void)k_bit1; (void)k_both; (void)c_idx; (void)c_sign; (void)s2_start; (void)lut; (void)skewed;
+  (void)q_fine; (void)q_frag2; (void)k_bit1; (void)k_both; (void)c_idx; (void)c_sign; (void)s2_start; (void)lut; (void)skewed; (void)flip;
 
   // MMA row r of a tile holds token r ^ ((r >> 1) & 1): neighbouring token rows sit in different halves of the
   // shared-memory banks, and with this order the four token rows one value load touches fall into both halves.
@@ -704,7 +712,7 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
     const uint8_t* st0 = warp_smem + cur * U * Cfg::kStageBytes;
 
     // ---- scores: U independent pairs of accumulation chains ------------------------------------------------------------
-    float s1[U][4], s2[U][4];
+    float s1[A][4], s2[A][4];
     {
       uint32_t iw_lo[U][Cfg::kIdxWords], iw_hi[U][Cfg::kIdxWords];
 #pragma unroll
@@ -717,9 +725,9 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
         // one code word = 8 coordinates of a token = one k-step: its low half-word selects four centroid bytes (and,
         // unmasked, four sign bytes: bit 3 of a selector nibble asks for the top bit of the byte 0x02, i.e. 0), its high
         // half-word the next four
-        int i1[U][4], i1l[U][4], i2[U][4];
+        int i1[A][4], i1l[A][4], i2[A][4];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
+        for (int u = 0; u < A; ++u) {
           i1[u][0] = i1[u][1] = i1[u][2] = i1[u][3] = 0;
           i1l[u][0] = i1l[u][1] = i1l[u][2] = i1l[u][3] = 0;
           i2[u][0] = i2[u][2] = s2_start[0];
@@ -727,8 +735,13 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
         }
 #pragma unroll
         for (int s = 0; s < Cfg::kSteps8; ++s) {
-          const uint4 qc = q_frag[s * 32];  // q1 b0, q1 b1, q2 b0, q2 b1
-          const uint2 qf = q_fine[s * 32];
+          uint4 qc[U];  // q1 b0, q1 b1, q2 b0, q2 b1
+          uint2 qf[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            qc[u] = u == 0 || !kPair ? q_frag[s * 32] : q_frag[s * 32 + flip];
+            qf[u] = u == 0 || !kPair ? q_fine[s * 32] : q_fine[s * 32 + flip];
+          }
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             const uint32_t xl = iw_lo[u][s], xh = iw_hi[u][s];
@@ -736,52 +749,57 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
             const uint32_t a[4] = {prmt_ptx(lut[0], lut[1], ml), prmt_ptx(lut[0], lut[1], mh),
                                    prmt_ptx(lut[0], lut[1], ml >> 16),
                                    prmt_ptx(lut[0], lut[1], mh >> 16)};
-            mma_s8(i1[u], a, qc.x, qc.y);
-            if (ANNA_TQ_FINE_QUERY) mma_s8(i1l[u], a, qf.x, qf.y);
+            mma_s8(i1[u % A], a, qc[u].x, qc[u].y);
+            mma_s8(i1l[u % A], a, qf[u].x, qf[u].y);
           }
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             const uint32_t xl = iw_lo[u][s], xh = iw_hi[u][s];
             const uint32_t a[4] = {prmt_ptx(kTwo, kTwo, xl), prmt_ptx(kTwo, kTwo, xh),
                                    prmt_ptx(kTwo, kTwo, xl >> 16), prmt_ptx(kTwo, kTwo, xh >> 16)};
-            mma_s8(i2[u], a, qc.z, qc.w);
+            mma_s8(i2[u % A], a, qc[u].z, qc[u].w);
           }
         }
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+        for (int u = 0; u < A; ++u)
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
             // 254 * coarse + fine stays below 2^31 (|coarse| <= 127 * 127 * D); beta1 carries the 1 / 254
-            s1[u][r] = (float)(ANNA_TQ_FINE_QUERY ? i1[u][r] * 254 + i1l[u][r] : i1[u][r]) * beta1[r & 1];
+            s1[u][r] = (float)(i1[u][r] * 254 + i1l[u][r]) * beta1[r & 1];
             s2[u][r] = (float)i2[u][r] * beta2[r & 1];
           }
       } else {
         // fields: bit 1 of a 2-bit field (the sign, or the index's upper bit) at the top of its byte, bit 0 next to it
         constexpr int kPairs = Cfg::kIdxWords / 2;
-        int lo_c[U][4], lo_f[U][4], hi_c[U][4], hi_f[U][4];
+        int lo_c[A][4], lo_f[A][4], hi_c[A][4], hi_f[A][4];
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+        for (int u = 0; u < A; ++u)
 #pragma unroll
           for (int r = 0; r < 4; ++r) lo_c[u][r] = lo_f[u][r] = hi_c[u][r] = hi_f[u][r] = 0;
 #pragma unroll
         for (int s = 0; s < Cfg::kSteps8; ++s) {
           const int up = 6 - 2 * (s / kPairs), w = 2 * (s % kPairs);
-          const uint4 q1 = q_frag[s * 32];  // coarse b0, b1, fine b0, b1
-          const uint4 qh = BITS == 2 ? q_frag2[s * 32] : q1;
+          uint4 q1[U], qh[U];  // coarse b0, b1, fine b0, b1
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int at = s * 32 + (u == 0 || !kPair ? 0 : flip);
+            q1[u] = q_frag[at];
+            qh[u] = BITS == 2 ? q_frag2[at] : q1[u];
+          }
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             const uint32_t x[4] = {iw_lo[u][w] << up, iw_hi[u][w] << up, iw_lo[u][w + 1] << up, iw_hi[u][w + 1] << up};
             const uint32_t a_lo[4] = {x[0] & kNext, x[1] & kNext, x[2] & kNext, x[3] & kNext};
-            mma_u8s8(lo_c[u], a_lo, q1.x, q1.y);
-            mma_u8s8(lo_f[u], a_lo, q1.z, q1.w);
+            mma_u8s8(lo_c[u % A], a_lo, q1[u].x, q1[u].y);
+            mma_u8s8(lo_f[u % A], a_lo, q1[u].z, q1[u].w);
             const uint32_t a_hi[4] = {x[0] & kTop, x[1] & kTop, x[2] & kTop, x[3] & kTop};
-            mma_u8s8(hi_c[u], a_hi, qh.x, qh.y);
-            mma_u8s8(hi_f[u], a_hi, qh.z, qh.w);
+            mma_u8s8(hi_c[u % A], a_hi, qh[u].x, qh[u].y);
+            mma_u8s8(hi_f[u % A], a_hi, qh[u].z, qh[u].w);
           }
         }
         // 254 * coarse + fine stays below 2^31: |T| <= 128 * 127 * D * 255
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+        for (int u = 0; u < A; ++u)
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
             s1[u][r] = fmaf((float)(lo_c[u][r] * 254 + lo_f[u][r]), beta1[r & 1], c_idx[r & 1]);
@@ -793,25 +811,25 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
           if (skewed) {  // the codebook is not symmetric: a third plane, where both bits are set
             asm volatile("" ::: "memory");
 #pragma unroll
-            for (int u = 0; u < U; ++u)
+            for (int u = 0; u < A; ++u)
 #pragma unroll
               for (int r = 0; r < 4; ++r) lo_c[u][r] = lo_f[u][r] = 0;
 #pragma unroll
             for (int s = 0; s < Cfg::kSteps8; ++s) {
               const int up = 6 - 2 * (s / kPairs), w = 2 * (s % kPairs);
-              const uint4 q1 = q_frag[s * 32];
 #pragma unroll
               for (int u = 0; u < U; ++u) {
+                const uint4 q1 = q_frag[s * 32 + (u == 0 || !kPair ? 0 : flip)];
                 const uint32_t x[4] = {iw_lo[u][w] << up, iw_hi[u][w] << up, iw_lo[u][w + 1] << up, iw_hi[u][w + 1] << up};
                 uint32_t a[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) a[i] = x[i] & (x[i] >> 1) & kNext;
-                mma_u8s8(lo_c[u], a, q1.x, q1.y);
-                mma_u8s8(lo_f[u], a, q1.z, q1.w);
+                mma_u8s8(lo_c[u % A], a, q1.x, q1.y);
+                mma_u8s8(lo_f[u % A], a, q1.z, q1.w);
               }
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u)
+            for (int u = 0; u < A; ++u)
 #pragma unroll
               for (int r = 0; r < 4; ++r)
                 s1[u][r] = fmaf((float)(lo_c[u][r] * 254 + lo_f[u][r]), k_both[r & 1], s1[u][r]);
@@ -823,22 +841,22 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
             lds_words<Cfg::kSignWords>(signs + tok_lo * Cfg::kKeyBytes, sw_lo[u]);
             lds_words<Cfg::kSignWords>(signs + tok_hi * Cfg::kKeyBytes, sw_hi[u]);
 #pragma unroll
-            for (int r = 0; r < 4; ++r) hi_c[u][r] = hi_f[u][r] = 0;
+            for (int r = 0; r < 4; ++r) hi_c[u % A][r] = hi_f[u % A][r] = 0;
           }
 #pragma unroll
           for (int s = 0; s < Cfg::kSteps8; ++s) {
             const int up = 7 - 2 * (s % 4), w = s / 4;
-            const uint4 q2 = q_frag2[s * 32];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
+              const uint4 q2 = q_frag2[s * 32 + (u == 0 || !kPair ? 0 : flip)];
               const uint32_t a[4] = {(sw_lo[u][w] << up) & kTop, (sw_hi[u][w] << up) & kTop,
                                      (sw_lo[u][w] << (up - 1)) & kTop, (sw_hi[u][w] << (up - 1)) & kTop};
-              mma_u8s8(hi_c[u], a, q2.x, q2.y);
-              mma_u8s8(hi_f[u], a, q2.z, q2.w);
+              mma_u8s8(hi_c[u % A], a, q2.x, q2.y);
+              mma_u8s8(hi_f[u % A], a, q2.z, q2.w);
             }
           }
 #pragma unroll
-          for (int u = 0; u < U; ++u)
+          for (int u = 0; u < A; ++u)
 #pragma unroll
             for (int r = 0; r < 4; ++r)
               s2[u][r] = fmaf((float)(hi_c[u][r] * 254 + hi_f[u][r]), beta2[r & 1], c_sign[r & 1]);
@@ -846,11 +864,12 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
       }
     }
     // score (log2 units) = norm * (S1 + rnorm * S2); the constant factors are folded into the query fragments
-    float sc[U][4];
+    float sc[A][4];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const float* norms = reinterpret_cast<const float*>(st0 + u * Cfg::kStageBytes + Cfg::kOffNorm);
-      const float* rnorms = reinterpret_cast<const float*>(st0 + u * Cfg::kStageBytes + Cfg::kOffRnorm);
+    for (int u = 0; u < A; ++u) {
+      const uint8_t* st = st0 + (kPair ? my_tile : u) * Cfg::kStageBytes;
+      const float* norms = reinterpret_cast<const float*>(st + Cfg::kOffNorm);
+      const float* rnorms = reinterpret_cast<const float*>(st + Cfg::kOffRnorm);
       const float n_lo = norms[tok_lo], r_lo = rnorms[tok_lo], n_hi = norms[tok_hi], r_hi = rnorms[tok_hi];
       sc[u][0] = n_lo * fmaf(r_lo, s2[u][0], s1[u][0]);
       sc[u][1] = n_lo * fmaf(r_lo, s2[u][1], s1[u][1]);
@@ -858,15 +877,16 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
       sc[u][3] = n_hi * fmaf(r_hi, s2[u][3], s1[u][3]);
       if (!full) {  // rows past the end of the prefix (their bytes may be anything)
         asm volatile("" ::: "memory");  // a real (warp-uniform) branch: full steps pay nothing for the masking
-        if (tok_lo >= valid[u]) sc[u][0] = sc[u][1] = -INFINITY;
-        if (tok_hi >= valid[u]) sc[u][2] = sc[u][3] = -INFINITY;
+        const int tokens = kPair && my_tile != 0 ? valid[U - 1] : valid[u];
+        if (tok_lo >= tokens) sc[u][0] = sc[u][1] = -INFINITY;
+        if (tok_hi >= tokens) sc[u][2] = sc[u][3] = -INFINITY;
       }
     }
 
     // ---- online softmax over the U * 16 tokens; the running maximum moves only when it would grow by more than 2^8 ----
     float mx[2] = {fmaxf(sc[0][0], sc[0][2]), fmaxf(sc[0][1], sc[0][3])};
 #pragma unroll
-    for (int u = 1; u < U; ++u) {
+    for (int u = 1; u < A; ++u) {
       mx[0] = fmaxf(mx[0], fmaxf(sc[u][0], sc[u][2]));
       mx[1] = fmaxf(mx[1], fmaxf(sc[u][1], sc[u][3]));
     }
@@ -895,7 +915,7 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
     const float m_ref[2] = {m_run[0] == -INFINITY ? 0.0f : m_run[0], m_run[1] == -INFINITY ? 0.0f : m_run[1]};
     uint32_t pb[U][2];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
+    for (int u = 0; u < A; ++u) {
       const float p0 = fast_exp2(sc[u][0] - m_ref[0]);
       const float p1 = fast_exp2(sc[u][1] - m_ref[1]);
       const float p2 = fast_exp2(sc[u][2] - m_ref[0]);
@@ -904,6 +924,14 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
       l_run[1] += p1 + p3;
       pb[u][0] = movmatrix_trans(pack2<__half>(p0, p1));  // rows 2tig, 2tig+1 of head gid
       pb[u][1] = movmatrix_trans(pack2<__half>(p2, p3));  // rows 2tig+8, 2tig+9
+    }
+
+    if constexpr (kPair) {  // each tile's probabilities in its own columns, zeros in the other's
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        pb[1][i] = gid >= 4 ? pb[0][i] : 0u;
+        pb[0][i] = gid >= 4 ? 0u : pb[0][i];
+      }
     }
 
     // ---- values: lane holds rows {2tig, 2tig+1} and {2tig+8, 2tig+9}, dims gid*D/8 .. +D/8 -----------------------------------
@@ -1037,16 +1065,18 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
   for (int item = threadIdx.x; item < g_count * D; item += kMmaThreads) {
     const int g = item / D;
     const int d = item % D;
+    constexpr int kParts = kPair ? 2 * kMmaWarps : kMmaWarps;  // columns g (and g + 4) of every warp
+    constexpr int kPartStep = kPair ? 4 : 8;
     float m_all = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < kMmaWarps; ++w) m_all = fmaxf(m_all, sm_m[w * 8 + g]);
+    for (int w = 0; w < kParts; ++w) m_all = fmaxf(m_all, sm_m[w * kPartStep + g]);
     const float m_ref = m_all == -INFINITY ? 0.0f : m_all;
     float l_all = 0.0f, o_all = 0.0f;
 #pragma unroll
-    for (int w = 0; w < kMmaWarps; ++w) {
-      const float wgt = exp2f(sm_m[w * 8 + g] - m_ref);
-      l_all += sm_l[w * 8 + g] * wgt;
-      o_all += sm_o[(w * 8 + g) * kPad + d] * wgt;
+    for (int w = 0; w < kParts; ++w) {
+      const float wgt = exp2f(sm_m[w * kPartStep + g] - m_ref);
+      l_all += sm_l[w * kPartStep + g] * wgt;
+      o_all += sm_o[(w * kPartStep + g) * kPad + d] * wgt;
     }
     values_out[(int64_t)g * p.chunk_capacity * D + d] = o_all;
     if (d == 0) {
@@ -1081,7 +1111,7 @@ __device__ __forceinline__ void init_packed_barriers(uint8_t* smem_raw) {
 }
 
 // Fixed chunks of the context, handed out by the block scheduler: grid (window chunks + packed chunks, units, batch).
-template <typename T, int D, int BITS>
+template <typename T, int D, int BITS, bool kPair>
 __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
     tq_decode_split_mma_kernel(const TqDecodeParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -1103,12 +1133,12 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
   PackedRing ring{0, 0u, false};
   const TqQueryConsts qc = load_query_consts<D, BITS>(p);
   // active slots stay contiguous: [window | packed]
-  tq_packed_segment<T, D, BITS>(p, smem_raw, qc, ring, b, (int)blockIdx.y, (int)gridDim.y, t0, min(Lq, t0 + p.chunk_tokens),
+  tq_packed_segment<T, D, BITS, kPair>(p, smem_raw, qc, ring, b, (int)blockIdx.y, (int)gridDim.y, t0, min(Lq, t0 + p.chunk_tokens),
                                 active_window + chunk, active_window + active_packed, active_packed);
 }
 
 // Persistent variant: one resident wave, every CTA takes an even share of the packed tiles (balanced_schedule.cuh).
-template <typename T, int D, int BITS>
+template <typename T, int D, int BITS, bool kPair>
 __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
     tq_decode_balanced_mma_kernel(const TqDecodeParams p, const int batch) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -1121,7 +1151,7 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
       [](int) {},  // rows without packed tokens belong to the window kernel
       [&](int b, int unit, int t0, int t1, int slot, int partials) {
         const int active_window = (p.residual_len + p.chunk_tokens - 1) / p.chunk_tokens;  // the window of this row is full
-        tq_packed_segment<T, D, BITS>(p, smem_raw, qc, ring, b, unit, units, t0, t1, active_window + slot,
+        tq_packed_segment<T, D, BITS, kPair>(p, smem_raw, qc, ring, b, unit, units, t0, t1, active_window + slot,
                                       active_window + partials, partials);
       },
       p.residual_len, kMmaWarps * TqMmaCfg<T, D, BITS>::kTilesPerStep);
@@ -1145,10 +1175,10 @@ static bool tq_use_balanced(const TqDecodeParams& p, int batch) {
   return p.chunk_tokens < kTqLongestChunk;
 }
 
-template <typename T, int D, int BITS>
+template <typename T, int D, int BITS, bool kPair>
 static int launch_tq_mma(const TqDecodeParams& p, int batch, cudaStream_t stream) {
   using Cfg = TqMmaCfg<T, D, BITS>;
-  auto kernel = tq_decode_split_mma_kernel<T, D, BITS>;
+  auto kernel = tq_decode_split_mma_kernel<T, D, BITS, kPair>;
   static bool configured[64] = {};
   int device = 0;
   ANNA_CUDA_CHECK(cudaGetDevice(&device));
@@ -1183,7 +1213,7 @@ static int launch_tq_mma(const TqDecodeParams& p, int batch, cudaStream_t stream
   config.numAttrs = 1;
   if (tq_use_balanced(p, batch)) {
     static int resident[64] = {};  // per device: CTAs of this kernel that fit the whole GPU at once
-    auto balanced = tq_decode_balanced_mma_kernel<T, D, BITS>;
+    auto balanced = tq_decode_balanced_mma_kernel<T, D, BITS, kPair>;
     int ctas = (device >= 0 && device < 64) ? resident[device] : 0;
     if (ctas == 0) {
       ANNA_CUDA_CHECK(cudaFuncSetAttribute(balanced, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
@@ -1260,7 +1290,9 @@ bool tq_split_mma_applicable(const TqDecodeParams& p, int head_dim, int dtype) {
 
 int launch_tq_split_mma(const TqDecodeParams& p, int batch, int head_dim, int bits, int dtype, cudaStream_t stream) {
 #define ANNA_TQ_MMA_CASE(TYPE, DIM, BITS_) \
-  if (head_dim == DIM && bits == BITS_) return launch_tq_mma<TYPE, DIM, BITS_>(p, batch, stream);
+  if (head_dim == DIM && bits == BITS_)          \
+    return p.groups <= 4 ? launch_tq_mma<TYPE, DIM, BITS_, true>(p, batch, stream) \
+                         : launch_tq_mma<TYPE, DIM, BITS_, false>(p, batch, stream);
   if (dtype == ANNA_DTYPE_BF16) {
     ANNA_TQ_MMA_CASE(__nv_bfloat16, 128, 2) ANNA_TQ_MMA_CASE(__nv_bfloat16, 128, 3) ANNA_TQ_MMA_CASE(__nv_bfloat16, 128, 4)
     ANNA_TQ_MMA_CASE(__nv_bfloat16, 256, 2) ANNA_TQ_MMA_CASE(__nv_bfloat16, 256, 3) ANNA_TQ_MMA_CASE(__nv_bfloat16, 256, 4)
