@@ -20,18 +20,21 @@ constexpr int kBalancedTileTokens = 16;
 // Block-wide exclusive scan of the tiles per row: s_prefix[b] = tiles (over all streams) of the rows before row b,
 // s_prefix[batch] = all tiles.  Returns the largest number of tiles of any single stream.  Ends with a barrier.
 // THREADS = blockDim.x (a multiple of 32); batch <= kBalancedMaxRows.  The newest `tail` tokens of a row have no tile here.
+// tiles_per_piece > 0 counts pieces of at most that many tiles instead of tiles.  *streams = streams with a tile.
 template <int THREADS>
 __device__ __forceinline__ int balanced_scan(const int64_t* visible_lengths, int64_t max_len, int batch,
-                                             int streams_per_row, int* s_prefix, int tail) {
+                                             int streams_per_row, int* s_prefix, int tail, int tiles_per_piece,
+                                             int* streams) {
   constexpr int kWarps = THREADS / 32;
   constexpr int kRowsPerThread = (kBalancedMaxRows + THREADS - 1) / THREADS;
   __shared__ int s_warp_sum[kWarps];
   __shared__ int s_warp_max[kWarps];
+  __shared__ int s_warp_rows[kWarps];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int rpt = (batch + THREADS - 1) / THREADS;
   int local[kRowsPerThread];
-  int sum = 0, mx = 0;
+  int sum = 0, mx = 0, rows = 0;
 #pragma unroll
   for (int i = 0; i < kRowsPerThread; ++i) {
     const int b = threadIdx.x * rpt + i;
@@ -41,9 +44,11 @@ __device__ __forceinline__ int balanced_scan(const int64_t* visible_lengths, int
       len = max((int64_t)0, min(len, max_len) - tail);
       tiles = (int)((len + kBalancedTileTokens - 1) / kBalancedTileTokens);
     }
+    mx = max(mx, tiles);
+    rows += tiles > 0 ? 1 : 0;
+    if (tiles_per_piece > 0) tiles = (tiles + tiles_per_piece - 1) / tiles_per_piece;
     local[i] = tiles;
     sum += tiles;
-    mx = max(mx, tiles);
   }
   int incl = sum;
 #pragma unroll
@@ -52,17 +57,23 @@ __device__ __forceinline__ int balanced_scan(const int64_t* visible_lengths, int
     if (lane >= d) incl += v;
     mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, d));
   }
+  rows = __reduce_add_sync(0xffffffffu, rows);
   if (lane == 31) s_warp_sum[warp] = incl;
-  if (lane == 0) s_warp_max[warp] = mx;
+  if (lane == 0) {
+    s_warp_max[warp] = mx;
+    s_warp_rows[warp] = rows;
+  }
   __syncthreads();
   int excl = incl - sum;
-  int total = 0, max_tiles = 0;
+  int total = 0, max_tiles = 0, filled = 0;
 #pragma unroll
   for (int w = 0; w < kWarps; ++w) {
     if (w < warp) excl += s_warp_sum[w];
     total += s_warp_sum[w];
     max_tiles = max(max_tiles, s_warp_max[w]);
+    filled += s_warp_rows[w];
   }
+  *streams = filled * streams_per_row;
 #pragma unroll
   for (int i = 0; i < kRowsPerThread; ++i) {
     const int b = threadIdx.x * rpt + i;
@@ -86,14 +97,15 @@ __device__ __forceinline__ int balanced_share(int total, int units, int max_tile
 // segment(b, stream, t0, t1, slot, partials_of_stream) for each piece of this CTA's tile range, in order.
 // THREADS = blockDim.x (a multiple of 32, at most 1024 / 8 rows per thread); all threads of the CTA must call it and
 // `segment` may synchronise the CTA.  `tail`: the newest tokens of every row that the line leaves out; `min_tiles`: the
-// smallest share of a CTA.
+// smallest share of a CTA; `segment_tiles`: the cost of a segment beyond its tiles, in tiles (0: shares always cross).
 template <int THREADS, typename ZeroFn, typename SegmentFn>
 __device__ __forceinline__ void balanced_for_each_segment(const int64_t* visible_lengths, int64_t max_len, int batch,
                                                           int streams_per_row, int chunk_capacity, ZeroFn&& zero_row,
                                                           SegmentFn&& segment, int tail = 0,
-                                                          int min_tiles = kBalancedMinTiles) {
+                                                          int min_tiles = kBalancedMinTiles, int segment_tiles = 0) {
   __shared__ int s_prefix[kBalancedMaxRows + 1];
-  const int max_tiles = balanced_scan<THREADS>(visible_lengths, max_len, batch, streams_per_row, s_prefix, tail);
+  int streams = 0;
+  const int max_tiles = balanced_scan<THREADS>(visible_lengths, max_len, batch, streams_per_row, s_prefix, tail, 0, &streams);
   const int total = s_prefix[batch];
   auto row_len = [&](int b) -> int {
     int64_t len = visible_lengths ? visible_lengths[b] : max_len;
@@ -106,11 +118,27 @@ __device__ __forceinline__ void balanced_for_each_segment(const int64_t* visible
   if (total == 0) return;
 
   const int tpc = balanced_share(total, (int)gridDim.x, max_tiles, chunk_capacity, min_tiles);
+  // Short shares: a CTA whose share crosses from one stream into the next pays for two segments, which is most of its
+  // time.  Pieces of single streams, one per CTA: with t = total / (CTAs - streams) tiles at most in each, the streams
+  // have no more than total / t + streams = CTAs pieces.  Taken when such a piece is less than a segment's cost longer
+  // than the even share.
+  int piece_tiles = 0;
+  if (segment_tiles > 0 && streams < (int)gridDim.x) {
+    const int spare = (int)gridDim.x - streams;
+    const int t = max(max((total + spare - 1) / spare, min_tiles), (max_tiles + chunk_capacity - 1) / chunk_capacity);
+    if (t - tpc < segment_tiles) piece_tiles = t;
+  }
   int pos = (int)min((int64_t)blockIdx.x * tpc, (int64_t)total);
-  const int end = (int)min((int64_t)pos + tpc, (int64_t)total);
+  int end = (int)min((int64_t)pos + tpc, (int64_t)total);
+  if (piece_tiles > 0) {
+    __syncthreads();  // s_prefix is written again: pieces instead of tiles
+    balanced_scan<THREADS>(visible_lengths, max_len, batch, streams_per_row, s_prefix, tail, piece_tiles, &streams);
+    pos = (int)blockIdx.x;
+    end = min(pos + 1, s_prefix[batch]);
+  }
   if (pos >= end) return;
 
-  // row that holds tile `pos`: the last b with s_prefix[b] <= pos (rows without tiles are skipped by construction)
+  // row that holds position `pos`: the last b with s_prefix[b] <= pos (rows without tiles are skipped by construction)
   int lo = 0, hi = batch;  // invariant: s_prefix[lo] <= pos < s_prefix[hi]
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -120,15 +148,26 @@ __device__ __forceinline__ void balanced_for_each_segment(const int64_t* visible
   while (pos < end) {
     while (s_prefix[b + 1] <= pos) ++b;
     const int row_first = s_prefix[b];
-    const int n = (s_prefix[b + 1] - row_first) / streams_per_row;  // tiles of each stream of this row
+    const int n = (s_prefix[b + 1] - row_first) / streams_per_row;  // tiles (or pieces) of each stream of this row
     const int stream = (pos - row_first) / n;
-    const int tile = (pos - row_first) - stream * n;
-    const int seg = min(n - tile, end - pos);
-    const int stream_first = row_first + stream * n;
-    const int first_cta = stream_first / tpc;
-    const int slot = (int)blockIdx.x - first_cta;
-    const int partials = (stream_first + n - 1) / tpc - first_cta + 1;
-    segment(b, stream, tile * kBalancedTileTokens, min(row_len(b), (tile + seg) * kBalancedTileTokens), slot, partials);
+    int first = (pos - row_first) - stream * n;  // tile (or piece) of the stream
+    const int seg = min(n - first, end - pos);
+    const int len = row_len(b);
+    int slot, partials, last;
+    if (piece_tiles > 0) {
+      const int tiles = (len + kBalancedTileTokens - 1) / kBalancedTileTokens;
+      slot = first;
+      partials = n;
+      last = (int)((int64_t)tiles * (slot + 1) / n);
+      first = (int)((int64_t)tiles * slot / n);
+    } else {
+      const int stream_first = row_first + stream * n;
+      const int first_cta = stream_first / tpc;
+      slot = (int)blockIdx.x - first_cta;
+      partials = (stream_first + n - 1) / tpc - first_cta + 1;
+      last = first + seg;
+    }
+    segment(b, stream, first * kBalancedTileTokens, min(len, last * kBalancedTileTokens), slot, partials);
     pos += seg;
   }
 }

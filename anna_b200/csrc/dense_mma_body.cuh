@@ -26,6 +26,52 @@ struct MmaCfg {
   static constexpr int kMinBlocks = D >= 256 ? 1 : (D == 128 ? 3 : 4);
 };
 
+// Merges the partials that the warps of a CTA left in shared memory (parts w = 0 .. PARTS - 1 of head g at index
+// w * STEP + g of sm_m (log2 units, overwritten), sm_l and sm_o, whose rows are D + 4 floats apart) into one split-K partial
+// per head.  One thread per head works out the weights, then every thread sums four dims at a time: with the weights
+// recomputed for each of a thread's single dims this part of a CTA took longer than a tile.  Called by all threads, after
+// a barrier.
+template <int D, int PARTS, int STEP>
+__device__ __forceinline__ void merge_parts_and_store(float* sm_m, const float* sm_l, const float* sm_o, int g_count,
+                                                      float* stats_out, float* values_out, int chunk_capacity) {
+  if ((int)threadIdx.x < g_count) {
+    const int g = threadIdx.x;
+    float m_all = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < PARTS; ++w) m_all = fmaxf(m_all, sm_m[w * STEP + g]);
+    const float m_ref = m_all == -INFINITY ? 0.0f : m_all;
+    float l_all = 0.0f;
+#pragma unroll
+    for (int w = 0; w < PARTS; ++w) {
+      const float wgt = exp2f(sm_m[w * STEP + g] - m_ref);
+      l_all += sm_l[w * STEP + g] * wgt;
+      sm_m[w * STEP + g] = wgt;
+    }
+    // the combine pass works in natural-log units
+    stats_out[(int64_t)g * chunk_capacity * 2 + 0] = m_all * 0.6931471805599453f;
+    stats_out[(int64_t)g * chunk_capacity * 2 + 1] = l_all;
+  }
+  __syncthreads();
+  const bool aligned = (reinterpret_cast<uintptr_t>(values_out) & 15u) == 0;  // rows are multiples of 16 bytes apart
+  for (int item = threadIdx.x; item < g_count * (D / 4); item += kMmaThreads) {
+    const int g = item / (D / 4);
+    const int d = 4 * (item % (D / 4));
+    float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int w = 0; w < PARTS; ++w) {
+      const float wgt = sm_m[w * STEP + g];
+      const float4 v = *reinterpret_cast<const float4*>(sm_o + (w * STEP + g) * (D + 4) + d);
+      o.x += v.x * wgt; o.y += v.y * wgt; o.z += v.z * wgt; o.w += v.w * wgt;
+    }
+    float* dst = values_out + (int64_t)g * chunk_capacity * D + d;
+    if (aligned) {
+      *reinterpret_cast<float4*>(dst) = o;
+    } else {
+      dst[0] = o.x; dst[1] = o.y; dst[2] = o.z; dst[3] = o.w;
+    }
+  }
+}
+
 // Split pass over tokens [t0, t1) of (row b, kv head kvh, query heads g0 .. g0 + g_count) for one CTA of kMmaThreads
 // threads; the partial goes to split-K slot `slot`, and with a fused merge it counts as one of the `active_chunks`
 // arrivals on counters[counter_index].
@@ -271,29 +317,8 @@ __device__ __forceinline__ void dense_split_mma_body(const DenseDecodeParams& p,
   }
   __syncthreads();
   const int64_t part = ((int64_t)b * p.q_heads + hq0) * p.chunk_capacity + slot;
-  float* stats_out = p.stats + part * 2;
-  float* values_out = p.values + part * D;
-  for (int item = threadIdx.x; item < g_count * D; item += kMmaThreads) {
-    const int g = item / D;
-    const int d = item % D;
-    float m_all = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < kMmaWarps; ++w) m_all = fmaxf(m_all, sm_m[w * 8 + g]);
-    const float m_ref = m_all == -INFINITY ? 0.0f : m_all;
-    float l_all = 0.0f, o_all = 0.0f;
-#pragma unroll
-    for (int w = 0; w < kMmaWarps; ++w) {
-      const float wgt = exp2f(sm_m[w * 8 + g] - m_ref);
-      l_all += sm_l[w * 8 + g] * wgt;
-      o_all += sm_o[(w * 8 + g) * kPad + d] * wgt;
-    }
-    values_out[(int64_t)g * p.chunk_capacity * D + d] = o_all;
-    if (d == 0) {
-      // the combine pass works in natural-log units
-      stats_out[(int64_t)g * p.chunk_capacity * 2 + 0] = m_all * 0.6931471805599453f;
-      stats_out[(int64_t)g * p.chunk_capacity * 2 + 1] = l_all;
-    }
-  }
+  merge_parts_and_store<D, kMmaWarps, 8>(sm_m, sm_l, sm_o, g_count, p.stats + part * 2, p.values + part * D,
+                                         p.chunk_capacity);
   if (p.fused.counters != nullptr) {
     const int64_t head0 = ((int64_t)b * p.q_heads + hq0) * p.chunk_capacity;
     __syncthreads();  // the epilogue buffers above are dead; reuse shared memory for the merge weights

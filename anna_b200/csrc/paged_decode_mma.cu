@@ -42,6 +42,9 @@ dense_decode_split_mma_kernel(const DenseDecodeParams p) {
                              (int64_t)b * gridDim.y + blockIdx.y);
 }
 
+// What a segment costs beyond its tiles (first copies, merge: about 3 us), in tiles.
+constexpr int kDenseSegmentTiles = 12;
+
 // ---------------------------------------------------------------------------------------------------------------------
 // Persistent variant: one resident wave, every CTA takes an even share of the tiles (balanced_schedule.cuh).
 template <typename T, int D>
@@ -65,7 +68,8 @@ dense_decode_balanced_mma_kernel(const DenseDecodeParams p, const int batch) {
         dense_split_mma_body<T, D>(p, smem_raw, b, stream / group_tiles, g0, min(8, p.groups - g0), t0, t1, slot,
                                    partials, (int64_t)b * streams_per_row + stream);
         __syncthreads();  // the next segment reuses the pipeline and merge buffers
-      });
+      },
+      0, kBalancedMinTiles, kDenseSegmentTiles);
 }
 
 template <typename T, int D>

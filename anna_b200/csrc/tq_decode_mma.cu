@@ -1060,30 +1060,9 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
   }
   __syncthreads();
   const int64_t part = ((int64_t)b * p.q_heads + hq0) * p.chunk_capacity + out_slot;
-  float* stats_out = p.stats + part * 2;
-  float* values_out = p.values + part * D;
-  for (int item = threadIdx.x; item < g_count * D; item += kMmaThreads) {
-    const int g = item / D;
-    const int d = item % D;
-    constexpr int kParts = kPair ? 2 * kMmaWarps : kMmaWarps;  // columns g (and g + 4) of every warp
-    constexpr int kPartStep = kPair ? 4 : 8;
-    float m_all = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < kParts; ++w) m_all = fmaxf(m_all, sm_m[w * kPartStep + g]);
-    const float m_ref = m_all == -INFINITY ? 0.0f : m_all;
-    float l_all = 0.0f, o_all = 0.0f;
-#pragma unroll
-    for (int w = 0; w < kParts; ++w) {
-      const float wgt = exp2f(sm_m[w * kPartStep + g] - m_ref);
-      l_all += sm_l[w * kPartStep + g] * wgt;
-      o_all += sm_o[(w * kPartStep + g) * kPad + d] * wgt;
-    }
-    values_out[(int64_t)g * p.chunk_capacity * D + d] = o_all;
-    if (d == 0) {
-      stats_out[(int64_t)g * p.chunk_capacity * 2 + 0] = m_all * 0.6931471805599453f;
-      stats_out[(int64_t)g * p.chunk_capacity * 2 + 1] = l_all;
-    }
-  }
+  // kPair: columns g and g + 4 of every warp
+  merge_parts_and_store<D, kPair ? 2 * kMmaWarps : kMmaWarps, kPair ? 4 : 8>(sm_m, sm_l, sm_o, g_count, p.stats + part * 2,
+                                                                             p.values + part * D, p.chunk_capacity);
   // The window kernel's partials and, when it arrives last, its merged output must be complete before this CTA
   // counts itself in (fused merge) or the kernel ends (two-pass merge).
   wait_for_prior_grids();
@@ -1137,6 +1116,9 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
                                 active_window + chunk, active_window + active_packed, active_packed);
 }
 
+// What a segment costs beyond its tiles (query preparation, first copy, merge: about 6 us), in tiles.
+constexpr int kTqSegmentTiles = 20;
+
 // Persistent variant: one resident wave, every CTA takes an even share of the packed tiles (balanced_schedule.cuh).
 template <typename T, int D, int BITS, bool kPair>
 __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
@@ -1154,7 +1136,7 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
         tq_packed_segment<T, D, BITS, kPair>(p, smem_raw, qc, ring, b, unit, units, t0, t1, active_window + slot,
                                       active_window + partials, partials);
       },
-      p.residual_len, kMmaWarps * TqMmaCfg<T, D, BITS>::kTilesPerStep);
+      p.residual_len, kMmaWarps * TqMmaCfg<T, D, BITS>::kTilesPerStep, kTqSegmentTiles);
   wait_for_prior_grids();
 }
 
@@ -1168,10 +1150,9 @@ static bool tq_use_balanced(const TqDecodeParams& p, int batch) {
   const int packed_slots = min(p.chunk_capacity, kFusedMaxChunks) - p.num_window_chunks;
   if (disabled || p.given_chunks || p.fused.counters == nullptr || !balanced_schedule_fits(batch, units, p.max_len, packed_slots)) return false;
   // The plan's longest chunks mean that there are enough of them for a few waves, which the block scheduler hands out as SMs
-  // get free (64 rows of 32 K tokens: 669 us, even shares 684; 128 ragged rows of 0.5-16 K: 253 and 261).  With less work
+  // get free (64 rows of 32 K tokens: 609 us, even shares 617; 128 ragged rows of 0.5-16 K: 226 and 234).  With less work
   // the chunks shrink, down to 64 tokens, and every CTA's fixed cost and the number of partials grow (16 rows of 0.4-4 K
-  // tokens, head_dim 256: 115 us, even shares 74; 64 rows of 4-32 K with two KV heads: 212 and 199; one row of 4 K: 36.8
-  // and 35.3).
+  // tokens, head_dim 256: 69 us, even shares 36; 64 rows of 4-32 K with two KV heads: 196 and 175).
   return p.chunk_tokens < kTqLongestChunk;
 }
 
