@@ -19,7 +19,11 @@ dense_decode_split_kernel(const DenseDecodeParams p) {
   int64_t len = p.visible_lengths ? p.visible_lengths[b] : p.max_len;
   len = max((int64_t)0, min(len, p.max_len));
   const int64_t t0 = (int64_t)chunk * p.chunk_tokens;
-  if (t0 >= len) return;
+  if (t0 >= len) {
+    if (p.fused.counters != nullptr && chunk == 0)  // nobody else will write the output of an empty row
+      fused_write_zero_row<T, D, kDecodeThreads>(p.fused, b, kvh * p.groups + g0, g_count);
+    return;
+  }
   const int64_t t1 = min(len, t0 + p.chunk_tokens);
 
   const int warp = threadIdx.x >> 5;
@@ -79,6 +83,12 @@ dense_decode_split_kernel(const DenseDecodeParams p) {
   const int64_t part = ((int64_t)b * p.q_heads + hq0) * p.chunk_capacity + chunk;
   cta_merge_store<T, D, G>(st, smem, warp, sub, dl, g_count, p.stats + part * 2, p.values + part * D,
                            (int64_t)p.chunk_capacity * 2, (int64_t)p.chunk_capacity * D);
+  if (p.fused.counters != nullptr) {
+    const int64_t head0 = ((int64_t)b * p.q_heads + hq0) * p.chunk_capacity;
+    const int chunks = (int)((len + p.chunk_tokens - 1) / p.chunk_tokens);
+    fused_combine_tail<T, D, kDecodeThreads>(p.fused, b, hq0, g_count, chunks, p.chunk_capacity, p.stats + head0 * 2,
+                                             p.values + head0 * D, smem, (int64_t)b * gridDim.y + blockIdx.y);
+  }
 }
 
 template <typename T, int D, int G>
@@ -86,7 +96,9 @@ static int launch_dense_split(const DenseDecodeParams& p, int batch, cudaStream_
   using Cfg = DecodeCfg<T, D, G>;
   const size_t smem_merge = sizeof(float) * (size_t)Cfg::kTeams * G * (D + 2);
   const size_t smem_q = sizeof(float) * (size_t)G * D;
-  const size_t smem = smem_merge > smem_q ? smem_merge : smem_q;
+  const size_t smem_tail = p.fused.counters != nullptr ? sizeof(float) * (size_t)G * kFusedMaxChunks : 0;
+  size_t smem = smem_merge > smem_q ? smem_merge : smem_q;
+  if (smem < smem_tail) smem = smem_tail;
   auto kernel = dense_decode_split_kernel<T, D, G>;
   if (smem > 48 * 1024) {
     ANNA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -127,12 +139,15 @@ static int run_dense_decode(DenseDecodeParams p, const void* gate, int64_t gate_
     }
     rc = launch_dense_split_mma(p, batch, head_dim, dtype, stream);
   } else {
+    const bool merged = split_counters != nullptr && num_chunks <= kFusedMaxChunks;
+    if (merged) p.fused = FusedCombine{split_counters, out, out_stride_b, out_stride_h, gate, gate_stride_b, gate_stride_h};
     const int gpad = padded_group(p.groups);
     rc = ANNA_DISPATCH_DTYPE(dtype, T, [&]() -> int {
       return ANNA_DISPATCH_DIM(head_dim, D, [&]() -> int {
         return ANNA_DISPATCH_GROUP(gpad, G, [&]() -> int { return launch_dense_split<T, D, G>(p, batch, stream); });
       });
     });
+    if (merged) return rc;
   }
   if (rc != ANNA_OK) return rc;
   return launch_split_combine(ws, nullptr, p.visible_lengths, p.visible_lengths ? -1 : p.max_len, p.max_len, 0, gate,

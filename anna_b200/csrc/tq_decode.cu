@@ -49,7 +49,11 @@ __global__ void __launch_bounds__(kDecodeThreads) tq_decode_split_kernel(const T
 
   int64_t len = p.lengths[b];
   len = max((int64_t)0, min(len, p.max_len));
-  if (len == 0) return;
+  if (len == 0) {
+    if (p.fused.counters != nullptr && chunk == 0)  // nobody else will write the output of an empty row
+      fused_write_zero_row<T, D, kDecodeThreads>(p.fused, b, kvh * p.groups + g0, g_count);
+    return;
+  }
   const int64_t R = p.residual_len;
   const int64_t Lq = len > R ? len - R : 0;
   const int active_window = (int)((len - Lq + p.chunk_tokens - 1) / p.chunk_tokens);
@@ -259,6 +263,12 @@ __global__ void __launch_bounds__(kDecodeThreads) tq_decode_split_kernel(const T
   const int64_t part = ((int64_t)b * p.q_heads + hq0) * p.chunk_capacity + out_slot;
   cta_merge_store<T, D, G>(st, smem, warp, sub, dl, g_count, p.stats + part * 2, p.values + part * D,
                            (int64_t)p.chunk_capacity * 2, (int64_t)p.chunk_capacity * D);
+  if (p.fused.counters != nullptr) {
+    const int64_t head0 = ((int64_t)b * p.q_heads + hq0) * p.chunk_capacity;
+    const int chunks = active_window + (int)((Lq + p.chunk_tokens - 1) / p.chunk_tokens);
+    fused_combine_tail<T, D, kDecodeThreads>(p.fused, b, hq0, g_count, chunks, p.chunk_capacity, p.stats + head0 * 2,
+                                             p.values + head0 * D, smem, (int64_t)b * gridDim.y + blockIdx.y);
+  }
 }
 
 template <typename T, int D, int G, int BITS>
@@ -266,7 +276,9 @@ static int launch_tq_split(const TqDecodeParams& p, int batch, cudaStream_t stre
   using Cfg = DecodeCfg<T, D, G>;
   const size_t smem_merge = sizeof(float) * (size_t)Cfg::kTeams * G * (D + 2);
   const size_t smem_q = sizeof(float) * (size_t)3 * G * D;
-  const size_t smem = smem_merge > smem_q ? smem_merge : smem_q;
+  const size_t smem_tail = p.fused.counters != nullptr ? sizeof(float) * (size_t)G * kFusedMaxChunks : 0;
+  size_t smem = smem_merge > smem_q ? smem_merge : smem_q;
+  if (smem < smem_tail) smem = smem_tail;
   auto kernel = tq_decode_split_kernel<T, D, G, BITS>;
   if (smem > 48 * 1024) {
     ANNA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -369,6 +381,9 @@ static int tq_paged_decode_impl(const void* q, int64_t q_stride_b, int64_t q_str
   }
   if (num_peers > 0)
     return set_error(ANNA_ERR_UNSUPPORTED, "peer outputs need the tensor-core decode path (16-bit cache, head_dim 128/256)");
+  // the last CTA of a (row, head group) merges here, too, which saves the second launch whenever there are counters
+  const bool merged = split_counters != nullptr && num_chunks <= kFusedMaxChunks;
+  if (merged) p.fused = FusedCombine{split_counters, out, out_stride_b, out_stride_h, gate, gate_stride_b, gate_stride_h};
   const int gpad = padded_group(p.groups);
   rc = ANNA_DISPATCH_DTYPE(dtype, T, [&]() -> int {
     return ANNA_DISPATCH_TQ_DIM(head_dim, D, [&]() -> int {
@@ -379,7 +394,7 @@ static int tq_paged_decode_impl(const void* q, int64_t q_stride_b, int64_t q_str
       });
     });
   });
-  if (rc != ANNA_OK) return rc;
+  if (rc != ANNA_OK || merged) return rc;
   return launch_split_combine(ws, nullptr, p.lengths, -1, p.max_len, residual_len, gate, gate_stride_b, gate_stride_h,
                               out, out_stride_b, out_stride_h, batch, q_heads, head_dim, chunk_tokens, num_chunks,
                               dtype, (cudaStream_t)stream);
