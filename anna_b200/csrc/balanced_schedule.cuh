@@ -121,7 +121,8 @@ __device__ __forceinline__ void balanced_for_each_segment(const int64_t* visible
   // Short shares: a CTA whose share crosses from one stream into the next pays for two segments, which is most of its
   // time.  Pieces of single streams, one per CTA: with t = total / (CTAs - streams) tiles at most in each, the streams
   // have no more than total / t + streams = CTAs pieces.  Taken when such a piece is less than a segment's cost longer
-  // than the even share.
+  // than the even share: 16 quantized rows of 0.4-4 K tokens 49 -> 36 us, 4 un-quantized rows of 60-900 tokens
+  // 14.4 -> 12.4 us.
   int piece_tiles = 0;
   if (segment_tiles > 0 && streams < (int)gridDim.x) {
     const int spare = (int)gridDim.x - streams;

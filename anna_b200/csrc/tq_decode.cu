@@ -381,7 +381,8 @@ static int tq_paged_decode_impl(const void* q, int64_t q_stride_b, int64_t q_str
   }
   if (num_peers > 0)
     return set_error(ANNA_ERR_UNSUPPORTED, "peer outputs need the tensor-core decode path (16-bit cache, head_dim 128/256)");
-  // the last CTA of a (row, head group) merges here, too, which saves the second launch whenever there are counters
+  // the last CTA of a (row, head group) merges here, too, which saves the second launch whenever there are counters (two
+  // fp32 rows of 576 tokens: 21.6 -> 18.5 us)
   const bool merged = split_counters != nullptr && num_chunks <= kFusedMaxChunks;
   if (merged) p.fused = FusedCombine{split_counters, out, out_stride_b, out_stride_h, gate, gate_stride_b, gate_stride_h};
   const int gpad = padded_group(p.groups);

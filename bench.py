@@ -440,15 +440,15 @@ def run_cfg5_gpu(args, dist: Dist, device) -> dict:
                 "serial_value": total * args.steps / m["e2e_serial_s"],
                 "note": "value: results return asynchronously into two pinned buffers, the host waits for a buffer "
                         "only before reusing it; serial_value: the host waits for every step's result before the next"},
-        # per step: tq_append_kernel, tq_prepare_queries_kernel, tq_window_split_mma_kernel, tq_decode_split_mma_kernel
-        # (the merge of the split-K partials is fused into the tail of the last one)
-        "gpu_launches": 4 * args.steps,
+        # per step: tq_append_kernel, tq_window_split_mma_kernel, tq_decode_split_mma_kernel (which prepares its queries and
+        # merges the split-K partials itself)
+        "gpu_launches": 3 * args.steps,
         "clocks": m["clocks"],
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": int(m["algo_bytes"] * NCU_TRAFFIC_RATIO["packed"]),
                      "traffic_source": NCU_TRAFFIC_SOURCE["packed"], "peak_kind": peak_kind,
-                     "kernel": "tq_decode_split_mma_kernel (timed with the query-preparation and window launches of "
-                               "the same decode call; the split-K merge runs in its tail)",
+                     "kernel": "tq_decode_split_mma_kernel (timed with the window launch of the same decode call; the "
+                               "query preparation runs in its head, the split-K merge in its tail)",
                      "algorithmic_bytes_per_launch": m["algo_bytes"], "launch_ms": m["decode_ms"],
                      "frac_of_8TBps_nominal": achieved / 8000.0},
     }
@@ -557,9 +557,9 @@ def run_kvhead_variant(args, dist: Dist, device) -> dict:
                        "(peer stores over NVLink) and one flag exchange per step" if peer is not None else
                        "one all-gather of [B, Hq/N, D] per step"),
                    "l2_policy": f"{per_rank_bytes / 1e6:.0f} MB of packed KV per rank and step exceed the 126 MB L2"},
-        # per step: tq_append, tq_prepare_queries, tq_window_split_mma, tq_decode_split_mma, and either the flag
-        # exchange kernel or NCCL's all-gather with one strided copy (library kernels, not counted)
-        "gpu_launches": (5 if peer is not None else 4) * args.steps, "clocks": clocks,
+        # per step: tq_append, tq_window_split_mma, the packed decode, and either the flag exchange kernel or NCCL's
+        # all-gather with one strided copy (library kernels, not counted)
+        "gpu_launches": (4 if peer is not None else 3) * args.steps, "clocks": clocks,
         "self_check": {"max_abs_vs_unsharded": check_err, "rows": check_rows, "context": check_tokens},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": None, "peak_kind": peak_kind,

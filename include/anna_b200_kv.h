@@ -95,7 +95,7 @@ int anna_kv_selftest_umma_ts(const void* a, const void* b, float* d, int* status
  * library will use and the number of chunks the scratch must hold.
  *
  * split_counters (optional, may be NULL): int32 [2, B, Hkv * ceil(G / 8)] that is all-zero on entry (arrival counters,
- * then tile cursors).  When given (and the plan has at most 512 chunks) the 16-bit tensor-core path merges the
+ * then tile cursors).  When given (and the plan has at most 512 chunks) the split kernel merges the
  * partials inside the split kernel: whoever finishes a (row, kv-head group) last does the merge and puts the counters
  * back to zero, so the buffer can be reused by the next call on the same stream without clearing.  Without it a second
  * small kernel does the merge.
@@ -268,7 +268,7 @@ int anna_tq_append(const void* k_new, const void* v_new, int64_t kn_stride_b, in
  * turboquant.py:290-332) instead of from a dense de-quantized copy.
  *   lengths   int64 [B]: total tokens per row (quantized = max(0, L - R), window = min(L, R)); L == 0 gives zeros
  *   query_scratch: optional 16-byte aligned device scratch of at least anna_tq_query_scratch_bytes(B, Hq, Hkv, D)
- *   bytes; the tensor-core path stores the rotated queries there (as MMA fragments)
+ *   bytes; the tensor-memory path stores the rotated queries there
  *   before the split pass.  Without it, or for fp32 caches, head_dim 64, value groups other than 32 or page sizes that
  *   are not a multiple of 16, the CUDA-core path runs.
  *   split-K slots: anna_tq_decode_plan gives the chunk length and the slot count (window chunks first, then the
