@@ -6,8 +6,8 @@
 //   packed bytes of the tile --bulk copy (cp.async.bulk, mbarrier)--> shared (2 stages per warp); a tile of a 16-token
 //              page is one linear copy issued by one lane, larger pages take six
 //   K codes -> 8-bit A fragments in registers, two tokens x D/4 coordinates per lane, no shared-memory round trip:
-//              4-bit codes through byte-permute (PRMT) table lookups (centroids and signs as bytes), 2- and 3-bit codes
-//              as the bit planes they are made of (a mask leaves one bit in each of four bytes)
+//              centroids of 4-bit codes through byte-permute (PRMT) table lookups; signs, and the indices of 2- and 3-bit
+//              codes, as the bit planes they are made of (a mask leaves one bit in each of four bytes)
 //   S1[16 tok x 8 heads] = centroid(K) . Q1^T      S2 = sign(K) . Q2^T        (mma.sync m16n8k32, 8-bit integers)
 //   score = norm * (S1 + rnorm * S2)   with Q1 = fwht(s1*q) * scaling / D
 //                                           Q2 = fwht(s2*fwht(s1*q)) * scaling * sqrt(pi/2) / D^1.5
@@ -140,7 +140,7 @@ template <typename T, int D, int BITS>
 struct TqMmaCfg {
   static constexpr int kSteps = D / 16;
   // Keys are scored as 8-bit integers against rotated queries that are split into a coarse and a fine byte.  4-bit
-  // codes: one byte permute turns four codes into four centroid bytes, another into four sign bytes.  2- and 3-bit
+  // codes: one byte permute turns four codes into four centroid bytes, a mask leaves four signs.  2- and 3-bit
   // codes: their centroids are linear in the code's bits (+-c0; +-c0 and +-c1 by symmetry), so each bit plane is
   // multiplied by the query bytes as it is -- a mask leaves one bit in each of four bytes, which is four coordinates of
   // a fragment for one logic operation -- and the planes are weighted with the exact centroids afterwards.  Against the
@@ -370,12 +370,11 @@ __device__ __forceinline__ void prepare_query_fragments(const TqDecodeParams& p,
         consts[32 + g] = u2 / 64.0f;
         consts[40 + g] = -u2 * (float)total2;
       } else {
-        // factor of the centroid product, factor of the sign product and the
-        // integer the sign accumulators start from: sign bytes are 2 for a clear bit and 0 for a set one, and 2 * sum
-        // over clear bits minus the sum over all coordinates is minus the +-1 product
+        // factor of the centroid product; factor and constant of the sign product: the sign plane has its bits at weight
+        // 128, and twice the sum over set bits minus the sum over all coordinates is the +-1 product
         consts[g] = amax1 * f1 / (127.0f * 254.0f) * qc.cent_step;
-        consts[8 + g] = -(amax2 * f2 / 127.0f);
-        reinterpret_cast<int*>(consts)[16 + g] = -total2;
+        consts[32 + g] = amax2 * f2 / (127.0f * 64.0f);
+        consts[40 + g] = -(amax2 * f2 / 127.0f) * (float)total2;
       }
     }
   }
@@ -439,7 +438,8 @@ __device__ __forceinline__ void prepare_query_fragments(const TqDecodeParams& p,
     }
   } else {
     // lane (gid, tig) feeds head gid with the coordinates of its code word s, tig * D/4 + 8s + {0..3} in the first
-    // register and + {4..7} in the second; the sign product uses a coarse byte only
+    // register and + {4..7} in the second; for the sign product, which uses a coarse byte only, + {0, 2, 4, 6} and
+    // + {1, 3, 5, 7} (the low and the high nibbles of the word's bytes)
     //   [s][lane][Q1 coarse b0, b1, Q2 coarse b0, b1]   then   [s][lane][Q1 fine b0, b1]
     const float k1 = q_scale[0][gid], k2 = q_scale[1][gid];
 #pragma unroll
@@ -458,8 +458,8 @@ __device__ __forceinline__ void prepare_query_fragments(const TqDecodeParams& p,
         w[1] |= ((uint32_t)c1 & 0xffu) << (8 * i);
         wl[0] |= ((uint32_t)fine(r1[i], k1, c0) & 0xffu) << (8 * i);
         wl[1] |= ((uint32_t)fine(r1[4 + i], k1, c1) & 0xffu) << (8 * i);
-        w[2] |= ((uint32_t)coarse(r2[i], k2) & 0xffu) << (8 * i);
-        w[3] |= ((uint32_t)coarse(r2[4 + i], k2) & 0xffu) << (8 * i);
+        w[2] |= ((uint32_t)coarse(r2[2 * i], k2) & 0xffu) << (8 * i);
+        w[3] |= ((uint32_t)coarse(r2[2 * i + 1], k2) & 0xffu) << (8 * i);
       }
       reinterpret_cast<uint4*>(query)[s * 32 + lane] = make_uint4(w[0], w[1], w[2], w[3]);
       reinterpret_cast<uint2*>(query + Cfg::kFragBytes)[s * 32 + lane] = make_uint2(wl[0], wl[1]);
@@ -556,13 +556,12 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
   // (only the ones this instantiation uses are created)
   const uint32_t nib_mask = BITS != 2 ? pinned_u32(0x03C003C0u, lane) : 0u;    // 4-bit value codes
   const uint32_t magic16 = BITS != 2 ? pinned_u32(0x4C004C00u, lane) : 0u;
-  const uint32_t kTwo = BITS == 4 ? pinned_u32(0x02020202u, lane) : 0u;        // 4-bit key codes
-  const uint32_t kIdxMask = BITS == 4 ? pinned_u32(0x77777777u, lane) : 0u;
-  const uint32_t kTop = BITS != 4 ? pinned_u32(0x80808080u, lane) : 0u;        // bit planes of 2- and 3-bit key codes
+  const uint32_t kIdxMask = BITS == 4 ? pinned_u32(0x77777777u, lane) : 0u;    // 4-bit key codes
+  const uint32_t kTop = pinned_u32(0x80808080u, lane);                         // bit planes of key codes
   const uint32_t kNext = BITS != 4 ? pinned_u32(0x40404040u, lane) : 0u;
   const uint32_t kTwoBitMask = BITS == 2 ? pinned_u32(0x03000300u, lane) : 0u;  // 2-bit value codes
   const uint32_t kMagic4 = BITS == 2 ? pinned_u32(0x44004400u, lane) : 0u;
-  (void)nib_mask; (void)magic16; (void)kTwo; (void)kIdxMask; (void)kTop; (void)kNext; (void)kTwoBitMask;
+  (void)nib_mask; (void)magic16; (void)kIdxMask; (void)kTop; (void)kNext; (void)kTwoBitMask;
   (void)kMagic4;
 
   const uint32_t warp_smem_u32 = smem_u32(smem_raw + warp * Cfg::kWarpSmem);
@@ -649,7 +648,6 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
   const int my_head = kPair ? (2 * tig) & 3 : 2 * tig;
   float beta1[2], beta2[2];                                              // factors of the two products
   float k_bit1[2] = {0.0f, 0.0f}, k_both[2] = {0.0f, 0.0f}, c_idx[2] = {0.0f, 0.0f}, c_sign[2] = {0.0f, 0.0f};  // planes
-  int s2_start[2] = {0, 0};                                                                                      // 4-bit
   {
     const float* consts = reinterpret_cast<const float*>(query + Cfg::kConstOffset) + my_head;
 #pragma unroll
@@ -661,16 +659,13 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
           k_both[c] = consts[16 + c];
         }
         c_idx[c] = consts[24 + c];
-        beta2[c] = consts[32 + c];
-        c_sign[c] = consts[40 + c];
-      } else {
-        beta2[c] = consts[8 + c];
-        s2_start[c] = reinterpret_cast<const int*>(consts)[16 + c];
       }
+      beta2[c] = consts[32 + c];
+      c_sign[c] = consts[40 + c];
     }
   }
   const bool skewed = BITS == 3 && __any_sync(0xffffffffu, k_both[0] != 0.0f || k_both[1] != 0.0f);
-  (void)q_fine; (void)q_frag2; (void)k_bit1; (void)k_both; (void)c_idx; (void)c_sign; (void)s2_start; (void)lut; (void)skewed; (void)flip;
+  (void)q_fine; (void)q_frag2; (void)k_bit1; (void)k_both; (void)c_idx; (void)c_sign; (void)lut; (void)skewed; (void)flip;
 
   // MMA row r of a tile holds token r ^ ((r >> 1) & 1): neighbouring token rows sit in different halves of the
   // shared-memory banks, and with this order the four token rows one value load touches fall into both halves.
@@ -723,16 +718,15 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
         lds_words<Cfg::kIdxWords>(keys + tok_hi * Cfg::kKeyBytes, iw_hi[u]);
       }
       if constexpr (BITS == 4) {
-        // one code word = 8 coordinates of a token = one k-step: its low half-word selects four centroid bytes (and,
-        // unmasked, four sign bytes: bit 3 of a selector nibble asks for the top bit of the byte 0x02, i.e. 0), its high
-        // half-word the next four
+        // one code word = 8 coordinates of a token = one k-step: its low half-word selects four centroid bytes, its high
+        // half-word the next four; the sign bits of its low and of its high nibbles are a plane each (one logic operation
+        // per four coordinates instead of a permute and half a shift: 64 rows of 32 K tokens 609 -> 592 us)
         int i1[A][4], i1l[A][4], i2[A][4];
 #pragma unroll
         for (int u = 0; u < A; ++u) {
           i1[u][0] = i1[u][1] = i1[u][2] = i1[u][3] = 0;
           i1l[u][0] = i1l[u][1] = i1l[u][2] = i1l[u][3] = 0;
-          i2[u][0] = i2[u][2] = s2_start[0];
-          i2[u][1] = i2[u][3] = s2_start[1];
+          i2[u][0] = i2[u][1] = i2[u][2] = i2[u][3] = 0;
         }
 #pragma unroll
         for (int s = 0; s < Cfg::kSteps8; ++s) {
@@ -756,9 +750,8 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             const uint32_t xl = iw_lo[u][s], xh = iw_hi[u][s];
-            const uint32_t a[4] = {prmt_ptx(kTwo, kTwo, xl), prmt_ptx(kTwo, kTwo, xh),
-                                   prmt_ptx(kTwo, kTwo, xl >> 16), prmt_ptx(kTwo, kTwo, xh >> 16)};
-            mma_s8(i2[u % A], a, qc[u].z, qc[u].w);
+            const uint32_t a[4] = {(xl << 4) & kTop, (xh << 4) & kTop, xl & kTop, xh & kTop};
+            mma_u8s8(i2[u % A], a, qc[u].z, qc[u].w);
           }
         }
 #pragma unroll
@@ -767,7 +760,7 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
           for (int r = 0; r < 4; ++r) {
             // 254 * coarse + fine stays below 2^31 (|coarse| <= 127 * 127 * D); beta1 carries the 1 / 254
             s1[u][r] = (float)(i1[u][r] * 254 + i1l[u][r]) * beta1[r & 1];
-            s2[u][r] = (float)i2[u][r] * beta2[r & 1];
+            s2[u][r] = fmaf((float)i2[u][r], beta2[r & 1], c_sign[r & 1]);
           }
       } else {
         // fields: bit 1 of a 2-bit field (the sign, or the index's upper bit) at the top of its byte, bit 0 next to it
