@@ -95,3 +95,36 @@ def test_even_share_never_exceeds_the_fused_merge_limit(capacity):
     assert max(partials for *_head, partials in pieces) <= FUSED_MAX_CHUNKS
     unclamped, _ = segments(lengths, 1, 592, capacity, 4)
     assert max(partials for *_head, partials in unclamped) > FUSED_MAX_CHUNKS  # the case the clamp is for
+
+
+def pieces_of(lengths: list[int], streams_per_row: int, units: int, capacity: int, min_tiles: int):
+    """(row, first tile, last tile, slot, pieces) of every stream's pieces, or None when there are too many streams."""
+    tiles_row = [(n + TILE - 1) // TILE for n in lengths]
+    total, longest = sum(tiles_row) * streams_per_row, max(tiles_row)
+    streams = sum(1 for n in tiles_row if n) * streams_per_row
+    if total == 0 or streams >= units:
+        return None
+    spare = units - streams
+    limit = max((total + spare - 1) // spare, min_tiles, (longest + capacity - 1) // capacity)
+    out = []
+    for row, n in enumerate(tiles_row):
+        pieces = (n + limit - 1) // limit
+        out += [(row, n * i // pieces, n * (i + 1) // pieces, i, pieces) for i in range(pieces)] * streams_per_row
+    return out, limit
+
+
+@pytest.mark.parametrize("seed", range(40))
+def test_pieces_cover_every_tile_once_and_fit_the_grid(seed):
+    rng = random.Random(100 + seed)
+    lengths = [rng.choice([0, 1, 16, 17, rng.randint(1, 5000)]) for _ in range(rng.choice([1, 3, 16, 70]))]
+    streams_per_row, units, capacity = rng.choice([1, 2, 8]), rng.choice([296, 444, 592]), rng.choice([2, 8, 65])
+    made = pieces_of(lengths, streams_per_row, units, capacity, 8)
+    if made is None:
+        return
+    pieces, limit = made
+    assert len(pieces) <= units
+    covered = [0] * len(lengths)
+    for row, first, last, slot, count in pieces:
+        assert 0 < last - first <= limit and 0 <= slot < count <= capacity
+        covered[row] += last - first
+    assert covered == [(n + TILE - 1) // TILE * streams_per_row for n in lengths]
