@@ -1142,7 +1142,8 @@ static bool tq_use_balanced(const TqDecodeParams& p, int batch) {
   }();
   const int64_t units = (int64_t)p.kv_heads * ((p.groups + 7) / 8);
   const int packed_slots = min(p.chunk_capacity, kFusedMaxChunks) - p.num_window_chunks;
-  if (disabled || p.given_chunks || p.fused.counters == nullptr || !balanced_schedule_fits(batch, units, p.max_len, packed_slots)) return false;
+  if (disabled || p.given_chunks || p.fused.counters == nullptr) return false;
+  if (!balanced_schedule_fits(batch, units, p.max_len, packed_slots)) return false;
   // The plan's longest chunks mean that there are enough of them for a few waves, which the block scheduler hands out as SMs
   // get free (64 rows of 32 K tokens: 609 us, even shares 617; 128 ragged rows of 0.5-16 K: 226 and 234).  With less work
   // the chunks shrink, down to 64 tokens, and every CTA's fixed cost and the number of partials grow (16 rows of 0.4-4 K

@@ -33,7 +33,7 @@ struct TqDecodeParams {
   float scaling;
   anna_tq_layout layout;
   FusedCombine fused;
-  void* query_frags;  // scratch for the rotated fp16 query fragments (tensor-core path), or nullptr
+  void* query_frags;  // query operand images of the tensor-memory path, or nullptr, which keeps the CUDA-core path
 };
 
 // Tensor-memory split pass (tq_decode_umma.cu): 16-bit cache dtypes, head_dim 128, 3- / 4-bit codes, 16-token pages,
