@@ -135,14 +135,15 @@ class _DeviceLengths:
     ``rows`` is a small ring of int64 ``[B]`` tensors; ``rows[pos]`` mirrors the host list ``host``.  An append reads
     ``rows[pos]`` as the lengths before the call and lets the kernel write the lengths after it into the next row of
     the ring, so a steady decode loop uploads no metadata at all.  Tensors handed out from the ring stay valid until
-    the ring wraps (``DEPTH - 1`` further appends to the same layer)."""
+    the ring wraps (``DEPTH - 1`` further appends to the same layer).  The zeros that the first append of new rows reads
+    are a row behind the ring, which no append writes: whoever keeps them has them for good."""
 
     DEPTH = 4
     __slots__ = ("rows", "pos", "host", "slots_dev", "slots_host", "device")
 
     def __init__(self, batch: int, device: torch.device) -> None:
-        self.rows = list(torch.zeros((self.DEPTH, batch), dtype=torch.int64, device=device).unbind(0))
-        self.pos = 0
+        self.rows = list(torch.zeros((self.DEPTH + 1, batch), dtype=torch.int64, device=device).unbind(0))
+        self.pos = self.DEPTH
         self.host: list[int] | None = [0] * batch
         self.slots_dev: torch.Tensor | None = None
         self.slots_host: list[int] | None = None

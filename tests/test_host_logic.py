@@ -431,3 +431,17 @@ def test_block_table_array_follows_the_list():
     row._table_np_valid = 0
     row.block_table.extend([4, 4, 4])
     assert row.table_array().tolist() == [4, 4, 4]
+
+
+def test_lengths_before_the_first_append_are_never_written_again():
+    """The lengths before an append are handed to the caller; those of the first append outlive the ring's wrap."""
+    lengths = cache_module._DeviceLengths(3, torch.device("cpu"))
+    first, after = lengths.before_append([0, 0, 0])
+    host = [4, 4, 4]
+    for _ in range(3 * lengths.DEPTH):
+        after.copy_(torch.tensor(host))                          # what the append kernel does
+        lengths.after_append(host)
+        past, after = lengths.before_append(host)
+        assert past.tolist() == host and past.data_ptr() != after.data_ptr()
+        host = [n + 1 for n in host]
+    assert first.tolist() == [0, 0, 0]
