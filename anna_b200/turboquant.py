@@ -555,8 +555,9 @@ class TurboQuantKVRow:
 
     @staticmethod
     def release_all(rows) -> None:
-        """``release`` of several rows: the pages of rows of one pool go back in one pass, in the same order."""
-        rows = [row for row in rows if row.pool is not None and row.slot >= 0]
+        """``release`` of several rows: the pages of rows of one pool go back in one pass, in the same order.  A row that
+        appears twice (two queries over one context) is released once."""
+        rows = list({id(row): row for row in rows if row.pool is not None and row.slot >= 0}.values())
         pools = {id(row.pool): row.pool for row in rows}
         for pool in pools.values():
             pages: list[int] = []

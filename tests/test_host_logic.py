@@ -445,3 +445,33 @@ def test_lengths_before_the_first_append_are_never_written_again():
         assert past.tolist() == host and past.data_ptr() != after.data_ptr()
         host = [n + 1 for n in host]
     assert first.tolist() == [0, 0, 0]
+
+
+def test_a_row_in_two_places_of_a_batch_is_released_once(launches):
+    """stack() takes the same rows twice (two queries over one context); release() of such a batch gives every page and
+    ring slot back exactly once, in the order in which the rows are released one by one."""
+    config = _config(block=4)
+    pools, orders = [], []
+    for one_by_one in (False, True):
+        allocator = Qwen3PageAllocator(config)
+        caches = [Qwen3DynamicCache(config, allocator=allocator, kv_cache_quantization="turboquant",
+                                    kv_cache_quant_bits=4, kv_cache_residual_len=2) for _ in range(2)]
+        for cache in caches:
+            kv = torch.zeros(1, 2, 11, 64)
+            cache.update(kv, kv, 0, require_dense_cache=False)
+        a, b = caches
+        stacked = Qwen3DynamicCache.stack([a, b, a], config, clone_turboquant_rows=False)
+        query = torch.zeros(3, 8, 1, 64)
+        stacked.turboquant_single_token_decode_attention(0, query, scaling=0.1, num_key_value_groups=4)
+        if one_by_one:
+            for row in stacked.turboquant_rows[0]:
+                row.release()
+        else:
+            stacked.release()
+        pool = allocator.turboquant_layers[0]
+        assert sorted(pool.free_slots) == list(range(pool.slot_capacity()))
+        assert sorted(pool.free_pages) == list(range(pool.capacity())) and pool.used_pages() == 0
+        pools.append(pool)
+        orders.append((list(pool.free_slots), list(pool.free_pages)))
+    assert orders[0] == orders[1]
+    assert pools[0].allocate_slot() == pools[1].allocate_slot() >= 0
