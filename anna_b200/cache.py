@@ -171,21 +171,45 @@ class _DeviceLengths:
         return self.slots_dev
 
 
+def _capturing(device: torch.device) -> bool:
+    with on_device(device):
+        return torch.cuda.is_current_stream_capturing()
+
+
 class _QuantizedStep:
     """What one decode step of a TurboQuant layer needs and the next one can go on from: the rows with their device block
     table, lengths and ring slots, and how many tokens every row still takes without a new page.
 
     It holds while the layer has the same row objects and nothing about any row of the pool has changed since
-    (``TurboQuantLayerPool.version``); otherwise the step is derived from the rows again."""
+    (``TurboQuantLayerPool.version``); otherwise the step is derived from the rows again.  Lengths and slots that were
+    uploaded for this step alone are ordered on the stream ``uploaded_on`` (0 = the legacy default stream; None = the
+    step has none of its own) and are read on that stream only: a decode on another one uploads its own, as does the
+    first one.  A graph capture is the exception (see ``readable``)."""
 
-    __slots__ = ("pool", "version", "rows", "table", "lengths", "lengths_dev", "slots", "slots_dev", "headroom", "longest")
+    __slots__ = ("pool", "version", "rows", "table", "lengths", "lengths_dev", "slots", "slots_dev", "headroom", "longest",
+                 "uploaded_on")
 
     def __init__(self, pool: TurboQuantLayerPool, rows: list, table: torch.Tensor | None, lengths: list[int],
-                 lengths_dev: torch.Tensor, slots: list[int], slots_dev: torch.Tensor, headroom: int) -> None:
+                 lengths_dev: torch.Tensor, slots: list[int], slots_dev: torch.Tensor, headroom: int,
+                 uploaded_on: int | None = None) -> None:
         self.pool, self.version, self.rows = pool, pool.version, list(rows)
         self.table, self.lengths, self.lengths_dev = table, lengths, lengths_dev
         self.slots, self.slots_dev = slots, slots_dev
         self.headroom, self.longest = headroom, max(lengths)
+        self.uploaded_on = uploaded_on
+
+    def readable(self, device: torch.device, captured: list) -> bool:
+        """Whether the current stream may read the step's lengths and slots.  Work under capture runs when the graph is
+        replayed, behind an upload that was made before the capture, so it may read them whichever stream that was on; an
+        upload under capture would copy from a staging buffer that holds other numbers by then.  The graph has only their
+        addresses: they go on the list ``captured``, which the cache keeps."""
+        if self.uploaded_on is None:
+            return True
+        stream = stream_ptr(device) or 0
+        if stream != 0 and _capturing(device):  # the legacy default stream cannot be captured
+            captured.append((self.lengths_dev, self.slots_dev))
+            return True
+        return stream == self.uploaded_on
 
     def holds(self, pool: TurboQuantLayerPool, rows: list, device: torch.device) -> bool:
         return (self.pool is pool and self.version == pool.version and self.slots_dev.device == device
@@ -228,6 +252,7 @@ class Qwen3DynamicCache:
         self._page_headroom: list[int | None] = [None] * layers
         self._table_view: list[torch.Tensor | None] = [None] * layers
         self._tq_step: list[_QuantizedStep | None] = [None] * layers
+        self._captured: list[tuple[torch.Tensor, torch.Tensor]] = []  # step tensors that graphs may read (see readable)
         self.seen_tokens = 0
         self.rope_deltas: torch.Tensor | None = None
         self.reserved_seq_capacity = 0
@@ -758,7 +783,7 @@ class Qwen3DynamicCache:
         pool = self._tq_pool(layer_idx)
         step = self._tq_step[layer_idx]
         if (step is not None and query_states.shape[1] == pool.kv_heads * num_key_value_groups
-                and step.holds(pool, rows, query_states.device)):
+                and step.holds(pool, rows, query_states.device) and step.readable(query_states.device, self._captured)):
             return launch_tq_decode(pool, query_states, step.table, step.slots, step.lengths, scaling, gate,
                                     slots_dev=step.slots_dev, lengths_dev=step.lengths_dev, output=output,
                                     peer_outputs=peer_outputs)
@@ -778,13 +803,17 @@ class Qwen3DynamicCache:
         if state is not None and state.device == device:
             lengths_dev = state.current(lengths)
             slots_dev = state.slots(slots)
+        uploaded_on = None
         if device.type == "cuda" and (lengths_dev is None or slots_dev is None):
             meta = MetadataUploader.for_device(device).upload([lengths, slots])
             lengths_dev = meta[0] if lengths_dev is None else lengths_dev
             slots_dev = meta[1] if slots_dev is None else slots_dev
-        if lengths_dev is not None and None not in rows:
+            uploaded_on = stream_ptr(device) or 0
+        # an upload under capture fills its tensors when the graph is replayed: nobody else may read them
+        if lengths_dev is not None and None not in rows and not (uploaded_on and _capturing(device)):
             # no headroom: the next append derives its step from the rows
-            self._tq_step[layer_idx] = _QuantizedStep(pool, rows, table_dev, lengths, lengths_dev, slots, slots_dev, -1)
+            self._tq_step[layer_idx] = _QuantizedStep(pool, rows, table_dev, lengths, lengths_dev, slots, slots_dev, -1,
+                                                      uploaded_on)
         return launch_tq_decode(pool, query_states, table_dev, slots, lengths, scaling, gate, slots_dev=slots_dev,
                                 lengths_dev=lengths_dev, output=output, peer_outputs=peer_outputs)
 

@@ -5,7 +5,9 @@ Kernel launches are replaced by recorders, so these tests check what would be se
 from __future__ import annotations
 
 import json
+from contextlib import nullcontext
 from pathlib import Path
+from types import SimpleNamespace
 
 import numpy as np
 import pytest
@@ -475,3 +477,55 @@ def test_a_row_in_two_places_of_a_batch_is_released_once(launches):
         orders.append((list(pool.free_slots), list(pool.free_pages)))
     assert orders[0] == orders[1]
     assert pools[0].allocate_slot() == pools[1].allocate_slot() >= 0
+
+
+def test_uploaded_lengths_are_read_on_their_own_stream_only(launches, monkeypatch):
+    """A decode keeps the lengths and slots it uploaded for the next one on the same stream.  Another stream is not ordered
+    behind that upload and gets its own; one made under a graph capture is filled on replay and is not kept; a capture
+    reads what was uploaded before it, and the cache keeps that alive."""
+    config, device = _config(block=4), torch.device("cuda", 0)
+    single = Qwen3DynamicCache(config, batch_size=1, kv_cache_quantization="turboquant", kv_cache_quant_bits=4,
+                               kv_cache_residual_len=8)
+    kv = torch.zeros(1, 2, 5, 64)
+    single.update(kv, kv, 0, require_dense_cache=False)              # inside the window: no block table
+    cache = Qwen3DynamicCache.stack([single], config, clone_turboquant_rows=False)
+    uploads, current = [], SimpleNamespace(stream=None, capturing=False)
+
+    class Uploader:
+        @classmethod
+        def for_device(cls, device):
+            return cls()
+
+        def upload(self, rows):
+            uploads.append(current.stream)
+            return [SimpleNamespace(device=device, values=list(row)) for row in rows]
+
+    read = []
+    monkeypatch.setattr(cache_module, "MetadataUploader", Uploader)
+    monkeypatch.setattr(cache_module, "stream_ptr", lambda device: current.stream)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: current.capturing)
+    monkeypatch.setattr(cache_module, "on_device", lambda device: nullcontext())
+    monkeypatch.setattr(cache_module, "launch_tq_decode",
+                        lambda *args, lengths_dev, slots_dev, **_: read.append((lengths_dev, slots_dev)))
+    query = SimpleNamespace(ndim=4, shape=(1, 8, 1, 64), device=device)
+
+    def decode(stream, capturing=False):
+        current.stream, current.capturing = stream, capturing
+        cache.turboquant_single_token_decode_attention(0, query, scaling=0.1, num_key_value_groups=4)
+        assert read[-1][0].values == [5] and read[-1][1].values == [single.turboquant_rows[0][0].slot]
+
+    decode(None)
+    decode(None)
+    assert uploads == [None] and read[0][0] is read[1][0]
+    decode(7)
+    decode(7)
+    decode(None)
+    assert uploads == [None, 7, None]
+    kept = read[-1]
+    decode(9, capturing=True)                                        # reads what is there ...
+    assert uploads == [None, 7, None] and read[-1] == kept
+    single.turboquant_rows[0][0]._length = 5                         # (the step is stale: counts as a change of the row)
+    decode(9, capturing=True)
+    decode(9)                                                        # ... and leaves nothing behind that replay fills
+    assert uploads == [None, 7, None, 9, 9] and read[-1][0] is not read[-2][0]
+    assert kept in cache._captured
