@@ -136,6 +136,17 @@ __device__ __forceinline__ float fast_exp2(float x) {
 #endif
 constexpr float kLazyRescale = 8.0f;  // log2 units: probabilities stay below 2^8, well inside fp16
 
+// Ring stage that is still free once the copies of `stages` - 1 steps have been started from stage `first` on.
+constexpr __host__ __device__ int ring_free_stage(int first, int stages) { return (first + stages - 1) % stages; }
+constexpr bool ring_free_stage_is_free(int stages) {
+  for (int first = 0; first < stages; ++first)
+    for (int i = 0; i < stages - 1; ++i)
+      if ((first + i) % stages == ring_free_stage(first, stages)) return false;
+  return true;
+}
+static_assert(ring_free_stage_is_free(2) && ring_free_stage_is_free(3) && ring_free_stage_is_free(4),
+              "the rotated queries may not lie where copies are in flight");
+
 template <typename T, int D, int BITS>
 struct TqMmaCfg {
   static constexpr int kSteps = D / 16;
@@ -636,7 +647,8 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
   // folded into the factors
   uint8_t* query = smem_raw + Cfg::kQueryOffset;
   const uint32_t lut[2] = {qc.lut[0], qc.lut[1]};
-  prepare_query_fragments<T, D, BITS>(p, smem_raw, query, (ring.stage + 1) % Cfg::kStages, b, hq0, g_count, qc);
+  prepare_query_fragments<T, D, BITS>(p, smem_raw, query, ring_free_stage(ring.stage, Cfg::kStages), b, hq0, g_count,
+                                      qc);
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // the loop's first copy lands where the rotations were
   __syncthreads();
   const uint4* q_frag = reinterpret_cast<const uint4*>(query) + lane;                     // [s][lane]
