@@ -334,7 +334,7 @@ class Qwen3DynamicCache:
 
     def _tables_of(self, layer_idx: int) -> list[list[int]]:
         if self.uses_turboquant_for_layer(layer_idx):
-            return [[] if row is None else row.block_table for row in self.turboquant_rows[layer_idx]]
+            return [[] if row is None else row._blocks for row in self.turboquant_rows[layer_idx]]
         return self.page_tables[layer_idx]
 
     def _sync_page_table_layer_buffer(self, layer_idx: int, *, batch_size: int,
@@ -681,6 +681,9 @@ class Qwen3DynamicCache:
                 row._attach(pool)
                 row._blocks = pages[batch_idx * blocks:(batch_idx + 1) * blocks]
                 rows[batch_idx] = row
+        # Without shared pages a row is looked at only when its pages run out: most of a large batch has room in its last
+        # one (one token to each of 128 ragged rows: 235 us of host time with a call for every row, 160 without).
+        shared = pool.has_shared_pages
         for batch_idx in range(batch_size):
             row = rows[batch_idx]
             if row is None:
@@ -689,16 +692,20 @@ class Qwen3DynamicCache:
                 rows[batch_idx] = row
             if use_prefix_share:
                 shared_blocks = self._reserve_shared_packed_blocks(row, pool, layer_idx, row.length + append_length)
-            else:
-                row._reserve_blocks(row.length + append_length)
+            elif shared or row._tokens + append_length - row.residual_len > len(row._blocks) * pool.block_size:
+                row._reserve_blocks(row._tokens + append_length)
             if row._privatized_block is not None:  # copy on write replaced a page id: upload that entry again
                 self._resync_row_from(layer_idx, batch_idx, row._privatized_block)
                 row._privatized_block = None
         slots = [row.slot for row in rows]
         lengths = self.layer_lengths[layer_idx]
+        room = None  # tokens that every row takes without a new page
         for batch_idx, row in enumerate(rows):
-            row._tokens += append_length
-            lengths[batch_idx] = row._tokens
+            tokens = row._tokens + append_length
+            lengths[batch_idx] = row._tokens = tokens
+            free = len(row._blocks) * pool.block_size + row.residual_len - tokens
+            if room is None or free < room:
+                room = free
         pool.version += 1
         if device.type == "cuda":
             state = self._device_lengths_of(layer_idx, batch_size, device)
@@ -724,9 +731,8 @@ class Qwen3DynamicCache:
                 self._register_packed_blocks(rows[0], pool, layer_idx)
             if state is not None:
                 # with pages that have several owners the next append has to look for blocks to copy first
-                room = -1
-                if not use_prefix_share and not pool.has_shared_pages:
-                    room = min(len(row._blocks) * pool.block_size + row.residual_len - row._tokens for row in rows)
+                if use_prefix_share or pool.has_shared_pages:
+                    room = -1
                 self._tq_step[layer_idx] = _QuantizedStep(pool, rows, table_dev, list(lengths), new_lengths, slots,
                                                           slots_dev, room)
         self.seen_tokens = max(self.seen_tokens, max(lengths, default=0))

@@ -529,3 +529,38 @@ def test_uploaded_lengths_are_read_on_their_own_stream_only(launches, monkeypatc
     decode(9)                                                        # ... and leaves nothing behind that replay fills
     assert uploads == [None, 7, None, 9, 9] and read[-1][0] is not read[-2][0]
     assert kept in cache._captured
+
+
+def test_an_append_looks_for_pages_of_the_rows_that_run_out_only(launches, monkeypatch):
+    """One token to each row of a ragged batch: a row whose last page has room costs no search for pages; with shared
+    pages in the pool every row is looked at (copy on write)."""
+    config = _config(block=4)
+    allocator = Qwen3PageAllocator(config)
+    singles = []
+    for tokens in range(9, 17):
+        cache = Qwen3DynamicCache(config, allocator=allocator, kv_cache_quantization="turboquant", kv_cache_quant_bits=4,
+                                  kv_cache_residual_len=3)
+        kv = torch.zeros(1, 2, tokens, 64)
+        cache.update(kv, kv, 0, require_dense_cache=False)
+        singles.append(cache)
+    cache = Qwen3DynamicCache.stack(singles, config, clone_turboquant_rows=False)
+    searched = []
+    reserve = TurboQuantKVRow._reserve_blocks
+
+    def counted(row, new_length):
+        searched.append(new_length)
+        reserve(row, new_length)
+
+    monkeypatch.setattr(TurboQuantKVRow, "_reserve_blocks", counted)
+    one = torch.zeros(8, 2, 1, 64)
+    for step in range(1, 9):
+        searched.clear()
+        cache.update(one, one, 0, require_dense_cache=False)
+        lengths = [tokens + step for tokens in range(9, 17)]
+        assert searched == [n for n in lengths if (n - 3) % 4 == 1]  # a new block begins with the token that was quantized
+        assert [len(row.block_table) for row in cache.turboquant_rows[0]] == [(n - 3 + 3) // 4 for n in lengths]
+    clone = cache.clone()
+    searched.clear()
+    cache.update(one, one, 0, require_dense_cache=False)
+    assert len(searched) == 8
+    clone.release()
