@@ -69,7 +69,7 @@ dense_decode_balanced_mma_kernel(const DenseDecodeParams p, const int batch) {
                                    partials, (int64_t)b * streams_per_row + stream);
         __syncthreads();  // the next segment reuses the pipeline and merge buffers
       },
-      0, kBalancedMinTiles, kDenseSegmentTiles);
+      0, kBalancedMinTiles, kDenseSegmentTiles, 0);
 }
 
 template <typename T, int D>
@@ -98,7 +98,7 @@ bool dense_balanced_mma_applicable(const DenseDecodeParams& p, int batch) {
     return flag != nullptr && flag[0] != '\0' && flag[0] != '0';
   }();
   if (disabled || p.fused.counters == nullptr) return false;
-  return balanced_schedule_fits(batch, (int64_t)p.kv_heads * ((p.groups + 7) / 8), p.max_len, p.chunk_capacity);
+  return balanced_schedule_fits(batch, (int64_t)p.kv_heads * ((p.groups + 7) / 8), p.max_len, p.chunk_capacity, 0);
 }
 
 int launch_dense_balanced_mma(const DenseDecodeParams& p, int batch, int head_dim, int dtype, cudaStream_t stream) {

@@ -54,6 +54,16 @@ int anna_kv_device_faults(int* count);
  */
 int anna_kv_selftest_wait_expiry(int* expired, anna_stream_t stream);
 
+/* Self-test, on the host: the schedule by which the persistent decode kernels share the tiles of a ragged batch, walked by
+ * the kernels' own arithmetic.  lengths int64 [B] (tokens per row, of which the newest `tail` have no tile); every row has
+ * streams_per_row streams; units = CTAs; capacity = split-K slots of a stream; min_tiles, segment_tiles, stream_tiles: see
+ * csrc/balanced_schedule.cuh.  segments int32 [max_segments, 7] receives (unit, row, stream, first tile, end tile, slot,
+ * partials) of every segment; *num_segments = how many there are.  No counterpart in the reference.
+ */
+int anna_kv_selftest_even_shares(const int64_t* lengths, int batch, int streams_per_row, int units, int capacity, int tail,
+                                 int min_tiles, int segment_tiles, int stream_tiles, int32_t* segments, int max_segments,
+                                 int* num_segments);
+
 /*
  * Self-test of the tensor-memory matrix multiply (tcgen05) in the two operand arrangements of the packed decode:
  *   d1 float [128][16] = a1 . b1^T   a1 uint8 [128][128], b1 uint8 [16][128]: e4m3 bytes, K contiguous

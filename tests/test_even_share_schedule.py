@@ -1,4 +1,5 @@
-"""CPU: the arithmetic of the even-share schedule of the persistent decode kernels, restated in Python.
+"""CPU: the arithmetic of the even-share schedule of the persistent decode kernels, restated in Python and walked by the
+library's own code.
 
 The device code (anna_b200/csrc/balanced_schedule.cuh) lets every work unit derive its tile range, the slot of each
 partial it writes and the number of partials each stream will receive from three numbers (tiles per row, units,
@@ -7,9 +8,12 @@ covered exactly once, slots of a stream are 0 .. partials-1 without gaps or repe
 than the scratch holds."""
 from __future__ import annotations
 
+import ctypes
 import random
 
 import pytest
+
+from anna_b200 import _lib
 
 TILE = 16
 
@@ -97,34 +101,67 @@ def test_even_share_never_exceeds_the_fused_merge_limit(capacity):
     assert max(partials for *_head, partials in unclamped) > FUSED_MAX_CHUNKS  # the case the clamp is for
 
 
-def pieces_of(lengths: list[int], streams_per_row: int, units: int, capacity: int, min_tiles: int):
-    """(row, first tile, last tile, slot, pieces) of every stream's pieces, or None when there are too many streams."""
-    tiles_row = [(n + TILE - 1) // TILE for n in lengths]
-    total, longest = sum(tiles_row) * streams_per_row, max(tiles_row)
-    streams = sum(1 for n in tiles_row if n) * streams_per_row
-    if total == 0 or streams >= units:
-        return None
-    spare = units - streams
-    limit = max((total + spare - 1) // spare, min_tiles, (longest + capacity - 1) // capacity)
-    out = []
-    for row, n in enumerate(tiles_row):
-        pieces = (n + limit - 1) // limit
-        out += [(row, n * i // pieces, n * (i + 1) // pieces, i, pieces) for i in range(pieces)] * streams_per_row
-    return out, limit
+def walked(lengths: list[int], streams_per_row: int, units: int, capacity: int, *, tail: int = 0, min_tiles: int = 8,
+           segment_tiles: int = 0, stream_tiles: int = 0) -> list[tuple[int, ...]]:
+    """(unit, row, stream, first tile, end tile, slot, partials) of every segment, by the kernels' own arithmetic."""
+    rows, count = (ctypes.c_int64 * len(lengths))(*lengths), ctypes.c_int()
+    room = sum((n + TILE - 1) // TILE for n in lengths) * streams_per_row + 1
+    out = (ctypes.c_int32 * (7 * room))()
+    _lib.check(_lib.lib().anna_kv_selftest_even_shares(rows, len(lengths), streams_per_row, units, capacity, tail, min_tiles,
+                                                       segment_tiles, stream_tiles, out, room, ctypes.byref(count)), "walk")
+    assert count.value <= room
+    return [tuple(out[7 * i:7 * i + 7]) for i in range(count.value)]
 
 
-@pytest.mark.parametrize("seed", range(40))
-def test_pieces_cover_every_tile_once_and_fit_the_grid(seed):
+def random_batch(seed: int):
     rng = random.Random(100 + seed)
     lengths = [rng.choice([0, 1, 16, 17, rng.randint(1, 5000)]) for _ in range(rng.choice([1, 3, 16, 70]))]
-    streams_per_row, units, capacity = rng.choice([1, 2, 8]), rng.choice([296, 444, 592]), rng.choice([2, 8, 65])
-    made = pieces_of(lengths, streams_per_row, units, capacity, 8)
-    if made is None:
-        return
-    pieces, limit = made
-    assert len(pieces) <= units
-    covered = [0] * len(lengths)
-    for row, first, last, slot, count in pieces:
-        assert 0 < last - first <= limit and 0 <= slot < count <= capacity
-        covered[row] += last - first
-    assert covered == [(n + TILE - 1) // TILE * streams_per_row for n in lengths]
+    return lengths, rng.choice([1, 2, 8]), rng.choice([296, 444, 592]), rng.choice([2, 8, 65])
+
+
+@pytest.mark.parametrize("seed", range(12))
+def test_the_restatement_is_what_the_kernels_walk(seed):
+    lengths, streams_per_row, units, capacity = random_batch(seed)
+    restated, _ = segments(lengths, streams_per_row, units, capacity, 8)
+    assert walked(lengths, streams_per_row, units, capacity) == [
+        (unit, row, stream, tile, tile + seg, slot, partials) for unit, row, stream, tile, seg, slot, partials in restated]
+
+
+@pytest.mark.parametrize("segment_tiles,stream_tiles,tail", [(0, 0, 0), (12, 0, 0), (20, 20, 0), (20, 20, 33)])
+@pytest.mark.parametrize("seed", range(40))
+def test_segments_cover_every_tile_once_and_number_the_partials(seed, segment_tiles, stream_tiles, tail):
+    """Shares that cross streams (with and without the first segment's cost on the line) and pieces of single streams."""
+    lengths, streams_per_row, units, capacity = random_batch(seed)
+    made = walked(lengths, streams_per_row, units, capacity, tail=tail, segment_tiles=segment_tiles,
+                  stream_tiles=stream_tiles)
+    streams: dict[tuple[int, int], list[tuple[int, ...]]] = {}
+    for unit, row, stream, first, end, slot, partials in made:
+        assert 0 <= unit < units and first < end
+        streams.setdefault((row, stream), []).append((first, end, slot, partials))
+    tiles = [max(0, n - tail + TILE - 1) // TILE for n in lengths]
+    assert set(streams) == {(row, s) for row, n in enumerate(tiles) if n for s in range(streams_per_row)}
+    for (row, _), parts in streams.items():
+        assert len(parts) <= capacity
+        assert [p[0] for p in parts] == [0] + [p[1] for p in parts[:-1]] and parts[-1][1] == tiles[row]
+        assert [p[2:] for p in parts] == [(slot, len(parts)) for slot in range(len(parts))]
+
+
+@pytest.mark.parametrize("batch,low,high,streams_per_row,units", [(96, 129, 500, 8, 592), (64, 129, 1000, 8, 592),
+                                                                  (64, 312, 2500, 8, 592), (300, 129, 1000, 2, 444)])
+def test_short_streams_do_not_pile_up_in_one_unit(batch, low, high, streams_per_row, units):
+    """A segment costs about 20 tiles beside its own.  No unit gets more than its share of tiles and segments together,
+    plus one segment that begins inside a stream; counting tiles alone, some unit got several times that."""
+    tail, cost, capacity = 128, 20, 2
+    lengths = [low + (high - low) * i // (batch - 1) for i in range(batch)]
+    tiles = [(n - tail + TILE - 1) // TILE for n in lengths]
+    line = streams_per_row * sum(n + cost for n in tiles)
+    share = max((line + units - 1) // units, 8, (max(tiles) + capacity - 2) // (capacity - 1))
+
+    def worst(stream_tiles: int, segment_tiles: int) -> int:
+        spent = [0] * units
+        for unit, _, _, first, end, _, _ in walked(lengths, streams_per_row, units, capacity, tail=tail,
+                                                   segment_tiles=segment_tiles, stream_tiles=stream_tiles):
+            spent[unit] += end - first + cost
+        return max(spent)
+
+    assert worst(cost, cost) <= share + cost < worst(0, 0) / 1.5
