@@ -1148,8 +1148,8 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
   wait_for_prior_grids();
 }
 
-// Which schedule the packed prefix takes.
-static bool tq_use_balanced(const TqDecodeParams& p, int batch) {
+// Which schedule the packed prefix takes; `ctas` = CTAs of the even-share kernel that are resident at once.
+static bool tq_use_balanced(const TqDecodeParams& p, int batch, int head_dim, int ctas) {
   static const bool disabled = [] {
     const char* flag = std::getenv("ANNA_B200_DISABLE_BALANCED");
     return flag != nullptr && flag[0] != '\0' && flag[0] != '0';
@@ -1162,7 +1162,16 @@ static bool tq_use_balanced(const TqDecodeParams& p, int batch) {
   // get free (64 rows of 32 K tokens: 609 us, even shares 617; 128 ragged rows of 0.5-16 K: 226 and 234).  With less work
   // the chunks shrink, down to 64 tokens, and every CTA's fixed cost and the number of partials grow (16 rows of 0.4-4 K
   // tokens, head_dim 256: 69 us, even shares 36; 64 rows of 4-32 K with two KV heads: 196 and 175).
-  return p.chunk_tokens < kTqLongestChunk;
+  if (p.chunk_tokens >= kTqLongestChunk) return false;
+  // A small call, whose chunks are resident at once with room to spare, gains nothing from shares and pays for the scan of
+  // the lengths (one row of 260-2500 tokens, 8 heads, 3 bits: 16.4-18.5 us in shares, 12.3-14.5 in chunks; 4 rows of 500,
+  // 32/8 heads, 4 bits: 16.5 and 12.4), unless it waits for the last CTA's merge, which takes the partials of a head group
+  // in rounds of 128 x 4 dims: even shares have half as many partials (one row of 6000 tokens, 16/2 heads of 256, 2 bits:
+  // 92 partials in four rounds 46 us, shares 34).
+  const int64_t chunks = p.num_chunks - p.num_window_chunks;
+  const int rounds = (min(8, p.groups) * (head_dim / 4) + kMmaThreads - 1) / kMmaThreads;
+  const bool small = batch * units * chunks * 5 <= (int64_t)ctas * 4 && chunks * rounds <= (rounds == 1 ? 40 : 24);
+  return !small;
 }
 
 template <typename T, int D, int BITS, bool kPair>
@@ -1201,18 +1210,18 @@ static int launch_tq_mma(const TqDecodeParams& p, int batch, cudaStream_t stream
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attr;
   config.numAttrs = 1;
-  if (tq_use_balanced(p, batch)) {
-    static int resident[64] = {};  // per device: CTAs of this kernel that fit the whole GPU at once
-    auto balanced = tq_decode_balanced_mma_kernel<T, D, BITS, kPair>;
-    int ctas = (device >= 0 && device < 64) ? resident[device] : 0;
-    if (ctas == 0) {
-      ANNA_CUDA_CHECK(cudaFuncSetAttribute(balanced, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
-      int sms = 0, per_sm = 0;
-      ANNA_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-      ANNA_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, balanced, kMmaThreads, Cfg::kSmemBytes));
-      ctas = sms * (per_sm > 0 ? per_sm : 1);
-      if (device >= 0 && device < 64) resident[device] = ctas;
-    }
+  static int resident[64] = {};  // per device: CTAs of the even-share kernel that fit the whole GPU at once
+  auto balanced = tq_decode_balanced_mma_kernel<T, D, BITS, kPair>;
+  int ctas = (device >= 0 && device < 64) ? resident[device] : 0;
+  if (ctas == 0) {
+    ANNA_CUDA_CHECK(cudaFuncSetAttribute(balanced, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
+    int sms = 0, per_sm = 0;
+    ANNA_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    ANNA_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, balanced, kMmaThreads, Cfg::kSmemBytes));
+    ctas = sms * (per_sm > 0 ? per_sm : 1);
+    if (device >= 0 && device < 64) resident[device] = ctas;
+  }
+  if (tq_use_balanced(p, batch, D, ctas)) {
     config.gridDim = dim3((unsigned)ctas);
     ANNA_CUDA_CHECK(cudaLaunchKernelEx(&config, balanced, p, batch));
     return check_launch("tq_decode_balanced_mma_kernel");
