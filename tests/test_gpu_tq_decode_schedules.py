@@ -10,8 +10,7 @@ import dataclasses
 import pytest
 import torch
 
-from anna_b200 import KVCacheConfig, Qwen3DynamicCache, Qwen3PageAllocator
-from anna_b200.turboquant import launch_tq_decode
+from anna_b200 import KVCacheConfig, Qwen3DynamicCache, Qwen3PageAllocator, _lib
 from tests.helpers import TQ_ATOL
 
 pytestmark = pytest.mark.gpu
@@ -44,9 +43,17 @@ def dense_attention(cache, query, lengths, scaling, gate=None):
     return out if gate is None else out * torch.sigmoid(gate.double())
 
 
+# 2-norm of the difference over that of the result: the keys and values of the 64-bit attention are the dense view's, rounded
+# to the cache dtype (2^-9 of bf16), like the output and, inside, the probabilities and values (2^-11): up to 3.2e-3 together.
+REL = {torch.bfloat16: 1e-2, torch.float16: 1e-2}
+
+
 def assert_close(out, want, dtype):
     tol = TQ_ATOL[dtype]  # what the quantized decode is allowed against the reference everywhere in these tests
     torch.testing.assert_close(out.double(), want, atol=tol, rtol=tol)
+    # an average over a long context is far below that: a lost part of it shows in the relative error, row by row
+    error = (out.double() - want).flatten(1).norm(dim=1) / want.flatten(1).norm(dim=1)
+    assert float(error.max()) < REL[dtype], f"relative error of the rows up to {float(error.max()):.2e}"
 
 
 @pytest.mark.parametrize("bits", [2, 3, 4])
@@ -64,9 +71,10 @@ def test_edges_of_tiles_pairs_and_groups(bits, dim, kv_heads, group, page):
         assert_close(out, dense_attention(cache, query, lengths, scaling, g), dtype)
 
 
-@pytest.mark.parametrize("batch,length", [(1, 40000), (300, 70), (1100, 50)])
+@pytest.mark.parametrize("batch,length", [(1, 40000), (2, 9000), (300, 70), (300, 700), (1100, 50)])
 def test_long_rows_and_large_batches(batch, length):
-    """One row over the whole chip; a tile or two per row; more rows than the even-share schedule takes."""
+    """One row and two over the whole chip; a tile or two per row, which is a small call's chunks, and more, which are shares;
+    more rows than the even-share schedule takes."""
     device, dtype = torch.device("cuda"), torch.bfloat16
     config = KVCacheConfig(num_hidden_layers=1, cache_block_size=16)
     gen = torch.Generator(device=device).manual_seed(3)
@@ -78,6 +86,41 @@ def test_long_rows_and_large_batches(batch, length):
     for _ in range(2):  # the merge counters are back at zero after a call
         out = cache.turboquant_single_token_decode_attention(0, query, scaling=0.1, num_key_value_groups=4)
         assert_close(out, dense_attention(cache, query, [length] * batch, 0.1), dtype)
+
+
+class Arguments:
+    """The library with two arguments of the packed decode replaced: the chunk length and the merge counters."""
+
+    def __init__(self, library, chunk_tokens: int, counters: bool) -> None:
+        self._library, self._chunk_tokens, self._counters = library, chunk_tokens, counters
+
+    def __getattr__(self, name):
+        return getattr(self._library, name)
+
+    def anna_tq_paged_decode(self, *args):
+        args = list(args)
+        assert args[20] >= 2 + -(-2111 // max(self._chunk_tokens, 64))  # the scratch was planned for 64-token chunks
+        args[21] = self._chunk_tokens
+        args[22] = args[22] if self._counters else None
+        return self._library.anna_tq_paged_decode(*args)
+
+
+@pytest.mark.parametrize("counters", [True, False])
+@pytest.mark.parametrize("bits", [2, 3, 4])
+@pytest.mark.parametrize("dim,group", [(128, 3), (128, 8), (128, 12), (256, 3), (256, 8), (256, 12)])
+def test_chunks_of_a_given_length(monkeypatch, bits, dim, group, counters):
+    """The chunk length is the caller's: fixed chunks, whatever the batch, with the merge in the kernel or behind it."""
+    device, dtype, kv_heads = torch.device("cuda"), torch.bfloat16, 2
+    lengths = [1, WINDOW, WINDOW + 1, WINDOW + 127, WINDOW + 128, WINDOW + 145, 700, 2111]
+    cache, gen = ragged_cache(device, lengths, kv_heads=kv_heads, dim=dim, bits=bits, page=16, dtype=dtype)
+    query = torch.randn((len(lengths), kv_heads * group, 1, dim), generator=gen, device=device).to(dtype)
+    want = dense_attention(cache, query, lengths, dim ** -0.5)
+    library = _lib.lib()
+    for chunk_tokens in (128, 1024):
+        monkeypatch.setattr(_lib, "lib", lambda: Arguments(library, chunk_tokens, counters))
+        for _ in range(2):  # the merge counters are back at zero after a call
+            out = cache.turboquant_single_token_decode_attention(0, query, scaling=dim ** -0.5, num_key_value_groups=group)
+            assert_close(out, want, dtype)
 
 
 @pytest.mark.parametrize("group", [4, 8])
