@@ -7,7 +7,7 @@
 // through shared memory before one partial (max, denom, D values) per query head is written out.
 #pragma once
 
-#include "common.cuh"
+#include "fused_combine.cuh"
 
 namespace anna {
 
@@ -212,6 +212,21 @@ __device__ __forceinline__ void cta_merge_store(const TeamState<T, D, G>& st, fl
 // Host-side dispatch helpers -------------------------------------------------------------------------------------
 
 inline int padded_group(int g) { return g <= 1 ? 1 : (g <= 2 ? 2 : (g <= 4 ? 4 : 8)); }
+
+// Whether the last CTA of a (row, head group) of a CUDA-core split pass merges the partials, which saves the second launch
+// (two fp32 rows of 576 tokens: 21.6 -> 18.5 us).  That CTA takes them 128 x 4 values at a time, the merge kernel 128 of each
+// head in a CTA of its own: with 8 heads of 128 dims or more the one CTA has twice the rounds, one behind the other, and the
+// second launch is cheaper (one row of 16000 tokens, 8 heads of 128: 63.3 us merged here, 53.3 with it; of 256: 108.7 and
+// 89.7; 4 heads of 256: 61.6 and 77.9; 8 heads of 64: 33.9 and 39.0).  At head_dim 64 the chunks of several heads are so
+// short that with a few waves of them the arrivals cost more than one launch (16 rows of 4000 tokens, 32/4 heads: 111 and
+// 104 us; of 600 tokens, 16/4 heads: 16.4 and 18.5).
+inline bool merges_in_split(const int32_t* counters, int num_chunks, int batch, int kv_heads, int groups, int head_dim) {
+  if (counters == nullptr || num_chunks > kFusedMaxChunks) return false;
+  const int heads = padded_group(groups);
+  if (head_dim >= 128) return heads < 8;
+  const int64_t streams = (int64_t)batch * kv_heads;
+  return heads <= 2 || streams < 64 || streams * num_chunks <= 148 * 8;
+}
 
 #define ANNA_DISPATCH_DIM(dim, D, ...)                                                       \
   [&]() -> int {                                                                             \

@@ -4,7 +4,10 @@
 
 namespace anna {
 
-template <typename T, int D, int G>
+// kMerge: the CTA that finishes a (row, head group) last merges its partials.  A kernel of its own: with the merge compiled
+// in, the loop's registers and with them the CTAs per SM come out differently (16 rows of 16000 tokens, fp32, 16/4 heads of
+// 64: 178 us without, 187 with it compiled in and not used).
+template <typename T, int D, int G, bool kMerge>
 __global__ void __launch_bounds__(kDecodeThreads)
 dense_decode_split_kernel(const DenseDecodeParams p) {
   using Cfg = DecodeCfg<T, D, G>;
@@ -20,7 +23,7 @@ dense_decode_split_kernel(const DenseDecodeParams p) {
   len = max((int64_t)0, min(len, p.max_len));
   const int64_t t0 = (int64_t)chunk * p.chunk_tokens;
   if (t0 >= len) {
-    if (p.fused.counters != nullptr && chunk == 0)  // nobody else will write the output of an empty row
+    if (kMerge && chunk == 0)  // nobody else will write the output of an empty row
       fused_write_zero_row<T, D, kDecodeThreads>(p.fused, b, kvh * p.groups + g0, g_count);
     return;
   }
@@ -83,7 +86,7 @@ dense_decode_split_kernel(const DenseDecodeParams p) {
   const int64_t part = ((int64_t)b * p.q_heads + hq0) * p.chunk_capacity + chunk;
   cta_merge_store<T, D, G>(st, smem, warp, sub, dl, g_count, p.stats + part * 2, p.values + part * D,
                            (int64_t)p.chunk_capacity * 2, (int64_t)p.chunk_capacity * D);
-  if (p.fused.counters != nullptr) {
+  if constexpr (kMerge) {
     const int64_t head0 = ((int64_t)b * p.q_heads + hq0) * p.chunk_capacity;
     const int chunks = (int)((len + p.chunk_tokens - 1) / p.chunk_tokens);
     fused_combine_tail<T, D, kDecodeThreads>(p.fused, b, hq0, g_count, chunks, p.chunk_capacity, p.stats + head0 * 2,
@@ -91,15 +94,15 @@ dense_decode_split_kernel(const DenseDecodeParams p) {
   }
 }
 
-template <typename T, int D, int G>
-static int launch_dense_split(const DenseDecodeParams& p, int batch, cudaStream_t stream) {
+template <typename T, int D, int G, bool kMerge>
+static int launch_dense_split_kernel(const DenseDecodeParams& p, int batch, cudaStream_t stream) {
   using Cfg = DecodeCfg<T, D, G>;
   const size_t smem_merge = sizeof(float) * (size_t)Cfg::kTeams * G * (D + 2);
   const size_t smem_q = sizeof(float) * (size_t)G * D;
-  const size_t smem_tail = p.fused.counters != nullptr ? sizeof(float) * (size_t)G * kFusedMaxChunks : 0;
+  const size_t smem_tail = kMerge ? sizeof(float) * (size_t)G * kFusedMaxChunks : 0;
   size_t smem = smem_merge > smem_q ? smem_merge : smem_q;
   if (smem < smem_tail) smem = smem_tail;
-  auto kernel = dense_decode_split_kernel<T, D, G>;
+  auto kernel = dense_decode_split_kernel<T, D, G, kMerge>;
   if (smem > 48 * 1024) {
     ANNA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   }
@@ -107,6 +110,13 @@ static int launch_dense_split(const DenseDecodeParams& p, int batch, cudaStream_
   dim3 grid((unsigned)p.num_chunks, (unsigned)(p.kv_heads * group_tiles), (unsigned)batch);
   kernel<<<grid, kDecodeThreads, smem, stream>>>(p);
   return check_launch("dense_decode_split_kernel");
+}
+
+template <typename T, int D, int G>
+static int launch_dense_split(const DenseDecodeParams& p, int batch, cudaStream_t stream) {
+  if constexpr (D < 128 || G < 8)  // the others are never merged here (merges_in_split)
+    if (p.fused.counters != nullptr) return launch_dense_split_kernel<T, D, G, true>(p, batch, stream);
+  return launch_dense_split_kernel<T, D, G, false>(p, batch, stream);
 }
 
 static int run_dense_decode(DenseDecodeParams p, const void* gate, int64_t gate_stride_b, int64_t gate_stride_h,
@@ -139,7 +149,7 @@ static int run_dense_decode(DenseDecodeParams p, const void* gate, int64_t gate_
     }
     rc = launch_dense_split_mma(p, batch, head_dim, dtype, stream);
   } else {
-    const bool merged = split_counters != nullptr && num_chunks <= kFusedMaxChunks;
+    const bool merged = merges_in_split(split_counters, num_chunks, batch, p.kv_heads, p.groups, head_dim);
     if (merged) p.fused = FusedCombine{split_counters, out, out_stride_b, out_stride_h, gate, gate_stride_b, gate_stride_h};
     const int gpad = padded_group(p.groups);
     rc = ANNA_DISPATCH_DTYPE(dtype, T, [&]() -> int {

@@ -30,7 +30,9 @@ __device__ __forceinline__ uint32_t load_packed_bits(const uint8_t* __restrict__
 
 constexpr int kTqUnroll = 2;
 
-template <typename T, int D, int G, int BITS>
+// kMerge: the CTA that finishes a (row, head group) last merges its partials (merges_in_split); a kernel of its own, as for
+// dense_decode_split_kernel.
+template <typename T, int D, int G, int BITS, bool kMerge>
 __global__ void __launch_bounds__(kDecodeThreads) tq_decode_split_kernel(const TqDecodeParams p) {
   using Cfg = DecodeCfg<T, D, G>;
   constexpr int E = D / 32;
@@ -50,7 +52,7 @@ __global__ void __launch_bounds__(kDecodeThreads) tq_decode_split_kernel(const T
   int64_t len = p.lengths[b];
   len = max((int64_t)0, min(len, p.max_len));
   if (len == 0) {
-    if (p.fused.counters != nullptr && chunk == 0)  // nobody else will write the output of an empty row
+    if (kMerge && chunk == 0)  // nobody else will write the output of an empty row
       fused_write_zero_row<T, D, kDecodeThreads>(p.fused, b, kvh * p.groups + g0, g_count);
     return;
   }
@@ -263,7 +265,7 @@ __global__ void __launch_bounds__(kDecodeThreads) tq_decode_split_kernel(const T
   const int64_t part = ((int64_t)b * p.q_heads + hq0) * p.chunk_capacity + out_slot;
   cta_merge_store<T, D, G>(st, smem, warp, sub, dl, g_count, p.stats + part * 2, p.values + part * D,
                            (int64_t)p.chunk_capacity * 2, (int64_t)p.chunk_capacity * D);
-  if (p.fused.counters != nullptr) {
+  if constexpr (kMerge) {
     const int64_t head0 = ((int64_t)b * p.q_heads + hq0) * p.chunk_capacity;
     const int chunks = active_window + (int)((Lq + p.chunk_tokens - 1) / p.chunk_tokens);
     fused_combine_tail<T, D, kDecodeThreads>(p.fused, b, hq0, g_count, chunks, p.chunk_capacity, p.stats + head0 * 2,
@@ -271,15 +273,15 @@ __global__ void __launch_bounds__(kDecodeThreads) tq_decode_split_kernel(const T
   }
 }
 
-template <typename T, int D, int G, int BITS>
-static int launch_tq_split(const TqDecodeParams& p, int batch, cudaStream_t stream) {
+template <typename T, int D, int G, int BITS, bool kMerge>
+static int launch_tq_split_kernel(const TqDecodeParams& p, int batch, cudaStream_t stream) {
   using Cfg = DecodeCfg<T, D, G>;
   const size_t smem_merge = sizeof(float) * (size_t)Cfg::kTeams * G * (D + 2);
   const size_t smem_q = sizeof(float) * (size_t)3 * G * D;
-  const size_t smem_tail = p.fused.counters != nullptr ? sizeof(float) * (size_t)G * kFusedMaxChunks : 0;
+  const size_t smem_tail = kMerge ? sizeof(float) * (size_t)G * kFusedMaxChunks : 0;
   size_t smem = smem_merge > smem_q ? smem_merge : smem_q;
   if (smem < smem_tail) smem = smem_tail;
-  auto kernel = tq_decode_split_kernel<T, D, G, BITS>;
+  auto kernel = tq_decode_split_kernel<T, D, G, BITS, kMerge>;
   if (smem > 48 * 1024) {
     ANNA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   }
@@ -287,6 +289,13 @@ static int launch_tq_split(const TqDecodeParams& p, int batch, cudaStream_t stre
   dim3 grid((unsigned)p.num_chunks, (unsigned)(p.kv_heads * group_tiles), (unsigned)batch);
   kernel<<<grid, kDecodeThreads, smem, stream>>>(p);
   return check_launch("tq_decode_split_kernel");
+}
+
+template <typename T, int D, int G, int BITS>
+static int launch_tq_split(const TqDecodeParams& p, int batch, cudaStream_t stream) {
+  if constexpr (D < 128 || G < 8)  // the others are never merged here (merges_in_split)
+    if (p.fused.counters != nullptr) return launch_tq_split_kernel<T, D, G, BITS, true>(p, batch, stream);
+  return launch_tq_split_kernel<T, D, G, BITS, false>(p, batch, stream);
 }
 
 }  // namespace anna
@@ -381,9 +390,7 @@ static int tq_paged_decode_impl(const void* q, int64_t q_stride_b, int64_t q_str
   }
   if (num_peers > 0)
     return set_error(ANNA_ERR_UNSUPPORTED, "peer outputs need the tensor-core decode path (16-bit cache, head_dim 128/256)");
-  // the last CTA of a (row, head group) merges here, too, which saves the second launch whenever there are counters (two
-  // fp32 rows of 576 tokens: 21.6 -> 18.5 us)
-  const bool merged = split_counters != nullptr && num_chunks <= kFusedMaxChunks;
+  const bool merged = merges_in_split(split_counters, num_chunks, batch, p.kv_heads, p.groups, head_dim);
   if (merged) p.fused = FusedCombine{split_counters, out, out_stride_b, out_stride_h, gate, gate_stride_b, gate_stride_h};
   const int gpad = padded_group(p.groups);
   rc = ANNA_DISPATCH_DTYPE(dtype, T, [&]() -> int {

@@ -45,7 +45,8 @@ def dense_attention(cache, query, lengths, scaling, gate=None):
 
 # 2-norm of the difference over that of the result: the keys and values of the 64-bit attention are the dense view's, rounded
 # to the cache dtype (2^-9 of bf16), like the output and, inside, the probabilities and values (2^-11): up to 3.2e-3 together.
-REL = {torch.bfloat16: 1e-2, torch.float16: 1e-2}
+# In fp32 it is sums in another order: up to 8e-7.
+REL = {torch.bfloat16: 1e-2, torch.float16: 1e-2, torch.float32: 5e-6}
 
 
 def assert_close(out, want, dtype):
@@ -121,6 +122,19 @@ def test_chunks_of_a_given_length(monkeypatch, bits, dim, group, counters):
         for _ in range(2):  # the merge counters are back at zero after a call
             out = cache.turboquant_single_token_decode_attention(0, query, scaling=dim ** -0.5, num_key_value_groups=group)
             assert_close(out, want, dtype)
+
+
+@pytest.mark.parametrize("dim", [64, 128, 256])
+@pytest.mark.parametrize("group", [1, 4, 5, 8])
+def test_fp32_merges_in_one_or_two_kernels(dim, group):
+    """Many 64-token chunks per head: up to 4 heads, or 64 dims, the split kernel merges them, else a second one does."""
+    device, dtype = torch.device("cuda"), torch.float32
+    lengths = [WINDOW, 65 + WINDOW, 3001]
+    cache, gen = ragged_cache(device, lengths, kv_heads=2, dim=dim, bits=4, page=16, dtype=dtype)
+    query = torch.randn((3, 2 * group, 1, dim), generator=gen, device=device)
+    for _ in range(2):
+        out = cache.turboquant_single_token_decode_attention(0, query, scaling=dim ** -0.5, num_key_value_groups=group)
+        assert_close(out, dense_attention(cache, query, lengths, dim ** -0.5), dtype)
 
 
 @pytest.mark.parametrize("group", [4, 8])
