@@ -42,7 +42,10 @@ dense_decode_split_mma_kernel(const DenseDecodeParams p) {
                              (int64_t)b * gridDim.y + blockIdx.y);
 }
 
-// What a segment costs beyond its tiles (first copies, merge: about 3 us), in tiles.
+// What a segment costs beyond its tiles (first copies, merge: about 3 us), in tiles.  Over 450 shapes (1 to 200 rows of 1 to
+// 12000 tokens, head_dim 64 to 256, 1 to 8 query heads per KV head) the mean time was 2 % longer with 6 and 1.3 % shorter with
+// 24, which takes ragged batches of short rows into pieces (48 rows of 37-600 tokens, 32/8 heads: 39 and 18.5 us) and loses
+// on uniform ones (32 rows of 600: 18.5 and 19.7 us).
 constexpr int kDenseSegmentTiles = 12;
 
 // ---------------------------------------------------------------------------------------------------------------------

@@ -732,7 +732,7 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
       if constexpr (BITS == 4) {
         // one code word = 8 coordinates of a token = one k-step: its low half-word selects four centroid bytes, its high
         // half-word the next four; the sign bits of its low and of its high nibbles are a plane each (one logic operation
-        // per four coordinates instead of a permute and half a shift: 64 rows of 32 K tokens 609 -> 592 us)
+        // per four coordinates instead of a permute and half a shift: 64 rows of 32 K tokens 612 -> 596 us)
         int i1[A][4], i1l[A][4], i2[A][4];
 #pragma unroll
         for (int u = 0; u < A; ++u) {
@@ -1159,9 +1159,10 @@ static bool tq_use_balanced(const TqDecodeParams& p, int batch, int head_dim, in
   if (disabled || p.given_chunks || p.fused.counters == nullptr) return false;
   if (!balanced_schedule_fits(batch, units, p.max_len, packed_slots, kTqSegmentTiles)) return false;
   // The plan's longest chunks mean that there are enough of them for a few waves, which the block scheduler hands out as SMs
-  // get free (64 rows of 32 K tokens: 609 us, even shares 617; 128 ragged rows of 0.5-16 K: 226 and 234).  With less work
-  // the chunks shrink, down to 64 tokens, and every CTA's fixed cost and the number of partials grow (16 rows of 0.4-4 K
-  // tokens, head_dim 256: 69 us, even shares 36; 64 rows of 4-32 K with two KV heads: 196 and 175).
+  // get free (64 rows of 32 K tokens, 32/8 heads: 594 us, even shares 613; 600 rows of 0.75-6 K, 48/4 heads: 697 and 742;
+  // but 128 rows of 0.5-16 K, 16/4 heads, for which shares became better when the line began to count segments: 226 and 214).
+  // With less work the chunks shrink, down to 64 tokens, and every CTA's fixed cost and the number of partials grow (16 rows
+  // of 0.4-4 K tokens, 16/2 heads of 256: 70 us, even shares 36; 64 rows of 4-32 K: 196 and 169).
   if (p.chunk_tokens >= kTqLongestChunk) return false;
   // A small call, whose chunks are resident at once with room to spare, gains nothing from shares and pays for the scan of
   // the lengths (one row of 260-2500 tokens, 8 heads, 3 bits: 16.4-18.5 us in shares, 12.3-14.5 in chunks; 4 rows of 500,

@@ -106,9 +106,9 @@ int anna_kv_selftest_umma_ts(const void* a, const void* b, float* d, int* status
  *
  * split_counters (optional, may be NULL): int32 [2, B, Hkv * ceil(G / 8)] that is all-zero on entry (arrival counters,
  * then tile cursors).  When given (and the plan has at most 512 chunks) the split kernel merges the
- * partials inside the split kernel: whoever finishes a (row, kv-head group) last does the merge and puts the counters
- * back to zero, so the buffer can be reused by the next call on the same stream without clearing.  Without it a second
- * small kernel does the merge.
+ * partials: whoever finishes a (row, kv-head group) last does the merge and puts the counters back to zero, so the
+ * buffer can be reused by the next call on the same stream without clearing.  Without it, and on the CUDA-core path
+ * where that is faster, a second small kernel does the merge.
  */
 int anna_decode_plan(int batch, int kv_heads, int64_t max_len, int* chunk_tokens, int* num_chunks);
 
