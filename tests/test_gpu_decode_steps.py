@@ -72,3 +72,32 @@ def test_clone_row_append_and_restack_between_steps():
     for _ in range(PAGE + 2):
         s.append(stacked, 1)
         s.check(stacked)
+
+
+def test_graph_of_a_decode_outlives_the_step_it_was_captured_from():
+    """A re-stacked batch has no lengths on the device yet; a capture reads those that an earlier decode uploaded, on
+    whichever stream, and they stay alive when the cache's step moves on."""
+    s = Steps(3)
+    s.append(s.cache, 70)
+    stacked = Qwen3DynamicCache.stack(s.cache.split_batch(clone_turboquant_rows=False), s.config, clone_turboquant_rows=False)
+    query = torch.randn((3, 4 * HEADS, 1, DIM), generator=s.gen, device=s.device).to(s.dtype)
+
+    def decode():
+        return stacked.turboquant_single_token_decode_attention(0, query, scaling=0.1, num_key_value_groups=4)
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        decode()                                 # this stream's scratch exists before the capture
+    torch.cuda.synchronize()
+    want = decode()                              # the step is the default stream's now
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        captured = decode()
+    stacked.turboquant_rows[0][0]._length = 70   # counts as a change: the next decode uploads anew and the old step goes
+    again = decode()
+    junk = [torch.zeros(64, dtype=torch.int64, device=s.device) for _ in range(64)]  # would take freed memory
+    captured.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(captured, want) and torch.equal(again, want) and len(junk) == 64
