@@ -95,6 +95,23 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
 }
 
 
+_LAUNCH = None
+
+
+def launch():
+    """The call module (csrc/launch_module.cpp), loaded once; raises loudly when it is not there."""
+    global _LAUNCH
+    if _LAUNCH is None:
+        lib()
+        try:
+            from . import _launch
+        except ImportError as exc:
+            raise RuntimeError(f"{PKG_DIR / '_launch.so'} cannot be loaded: {exc}. Run `python -m anna_b200.build`. There is "
+                               "no CPU fallback for this path.") from exc
+        _LAUNCH = _launch
+    return _LAUNCH
+
+
 def library_path() -> Path:
     return LIB_PATH
 

@@ -13,7 +13,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib
-from .fused_ops import dtype_code, on_device, ptr, run_gqa_decode_fused, stream_ptr
+from .fused_ops import dtype_code, launch_module, on_device, ptr, run_gqa_decode_fused, stream_ptr
 
 _FAST_DIMS = (64, 128, 256)
 
@@ -57,6 +57,10 @@ def grouped_query_attention(query_states: torch.Tensor, key_states: torch.Tensor
 
     ``key_lengths`` (int64 ``[B]`` on the device) and ``causal`` may be given instead of the masks; a query that sees
     no key gives zeros (the reference gives NaN there)."""
+    if causal_mask is None and visible_mask is None and key_padding_mask is None and not check_masks:
+        out = launch_module().prefill(query_states, key_states, value_states, key_lengths, scaling, bool(causal))
+        if out is not None:
+            return out
     if query_states.dim() != 4 or key_states.dim() != 4 or value_states.dim() != 4:
         raise ValueError("grouped_query_attention expects [batch, heads, tokens, head_dim] tensors")
     if not query_states.is_cuda:

@@ -1,7 +1,9 @@
-"""Build recipe for libanna_b200_kv.so (hand-written CUDA for sm_100a, no torch headers involved).
+"""Build recipe for libanna_b200_kv.so (hand-written CUDA for sm_100a, no torch headers involved) and for the Python call
+module on top of it.
 
 ``python -m anna_b200.build`` compiles every ``csrc/*.cu`` with nvcc (cross-compiles without a GPU) and links
-them into ``anna_b200/libanna_b200_kv.so`` next to this file, so the library travels with the source tree.
+them into ``anna_b200/libanna_b200_kv.so`` next to this file, so the library travels with the source tree; then
+``csrc/launch_module.cpp`` with the host compiler against the installed torch into ``anna_b200/_launch.so``.
 """
 from __future__ import annotations
 
@@ -16,6 +18,8 @@ PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 BUILD_DIR = PKG_DIR / "_build"
 LIB_PATH = PKG_DIR / "libanna_b200_kv.so"
+MODULE_SOURCE = CSRC / "launch_module.cpp"
+MODULE_PATH = PKG_DIR / "_launch.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -37,6 +41,31 @@ def _stale(target: Path, sources: list[Path]) -> bool:
         return True
     stamp = target.stat().st_mtime
     return any(src.stat().st_mtime > stamp for src in sources)
+
+
+def build_module(force: bool = False, verbose: bool = False) -> Path:
+    """The call module; needs the library, whose C entry points it links."""
+    header = PKG_DIR.parent / "include" / "anna_b200_kv.h"
+    if not force and not _stale(MODULE_PATH, [MODULE_SOURCE, header]):
+        return MODULE_PATH
+    import sysconfig
+
+    import torch
+
+    torch_dir = Path(torch.__file__).resolve().parent
+    cuda_include = Path(_nvcc()).resolve().parent.parent / "include"
+    includes = [header.parent, torch_dir / "include", torch_dir / "include" / "torch" / "csrc" / "api" / "include", cuda_include,
+                sysconfig.get_paths()["include"]]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{path}" for path in includes],
+           str(MODULE_SOURCE), "-o", str(MODULE_PATH), f"-L{torch_dir / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10",
+           "-lc10_cuda", f"-L{PKG_DIR}", f"-l:{LIB_PATH.name}", "-Wl,-rpath,$ORIGIN"]
+    done = subprocess.run(cmd, capture_output=True, text=True)
+    if done.returncode != 0:
+        raise RuntimeError(f"{MODULE_SOURCE.name} failed:\n{done.stderr}")
+    if verbose:
+        sys.stderr.write(done.stderr)
+    return MODULE_PATH
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -69,6 +98,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         done = subprocess.run(cmd, capture_output=True, text=True)
         if done.returncode != 0:
             raise RuntimeError(f"link failed:\n{done.stderr}")
+    build_module(force, verbose)
     return LIB_PATH
 
 

@@ -1,0 +1,376 @@
+// Python entry points of the calls a decode loop makes every step, on the C ABI of libanna_b200_kv.so.
+//
+// A ctypes call converts some forty arguments one by one, and every address, size and stride among them costs a Python
+// call of its own: two thirds of the 18 us of host time of a decode call, whose GPU work for a few short rows takes no
+// longer.  The functions here take the tensors themselves.  They serve the ordinary call only: where an argument is not
+// what they expect they return None before anything has happened, and the caller takes the general path, which converts
+// or rejects it.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/Functions.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Device.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <map>
+#include <tuple>
+
+#include "anna_b200_kv.h"
+
+namespace {
+
+const at::Tensor* tensor(PyObject* obj) {
+  return THPVariable_Check(obj) ? &THPVariable_Unpack(obj) : nullptr;
+}
+// a tensor or None; *ok turns false for anything else
+const at::Tensor* optional_tensor(PyObject* obj, bool* ok) {
+  if (obj == Py_None) return nullptr;
+  const at::Tensor* t = tensor(obj);
+  if (t == nullptr) *ok = false;
+  return t;
+}
+void* address(const at::Tensor* t) { return t == nullptr ? nullptr : t->data_ptr(); }
+const float* floats(const at::Tensor* t) { return static_cast<const float*>(address(t)); }
+
+bool dtype_code(at::ScalarType type, int* code) {
+  switch (type) {
+    case at::kFloat: *code = ANNA_DTYPE_F32; return true;
+    case at::kHalf: *code = ANNA_DTYPE_F16; return true;
+    case at::kBFloat16: *code = ANNA_DTYPE_BF16; return true;
+    default: return false;
+  }
+}
+bool plain(const at::Tensor& t, c10::Device device, int64_t dims) {
+  return t.device() == device && t.layout() == at::kStrided && t.dim() == dims;
+}
+bool on(const at::Tensor* t, c10::Device device) { return t == nullptr || t->device() == device; }
+
+// Split-K scratch of a problem, as split_scratch and query_scratch of fused_ops.py hand it out; dropped by
+// forget_scratch(), which they call whenever a buffer behind it is replaced.  Guarded by the interpreter lock; never
+// destroyed, so that no CUDA memory is freed after the runtime is gone.
+struct Scratch {
+  at::Tensor stats, values, counters, frags;
+  int capacity = 0;
+};
+using ScratchKey = std::tuple<int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t>;
+std::map<ScratchKey, Scratch>& scratch_table() {
+  static auto* table = new std::map<ScratchKey, Scratch>();
+  return *table;
+}
+constexpr size_t kMaxScratch = 256;
+PyObject* scratch_source = nullptr;  // (device, batch, heads, dim, kv_heads, max_len, (max_blocks, block, window) | None)
+
+// false with a Python error set when the scratch cannot be had.  The query's device must be current.
+bool scratch_of(const at::Tensor& query, int64_t stream, int64_t kv_heads, int64_t max_len, int64_t max_blocks, int64_t block,
+                int64_t window, Scratch* out) {
+  const ScratchKey key(query.device().index(), stream, query.size(0), query.size(1), query.size(3), kv_heads, max_len, block,
+                       window);
+  auto& table = scratch_table();
+  const auto found = table.find(key);
+  if (found != table.end()) {
+    *out = found->second;
+    return true;
+  }
+  if (scratch_source == nullptr) {
+    PyErr_SetString(PyExc_RuntimeError, "anna_b200: no scratch source");
+    return false;
+  }
+  PyObject* device = THPDevice_New(query.device());
+  PyObject* got = window > 0
+                      ? PyObject_CallFunction(scratch_source, "NLLLLL(LLL)", device, (long long)query.size(0),
+                                              (long long)query.size(1), (long long)query.size(3), (long long)kv_heads,
+                                              (long long)max_len, (long long)max_blocks, (long long)block, (long long)window)
+                      : PyObject_CallFunction(scratch_source, "NLLLLLO", device, (long long)query.size(0),
+                                              (long long)query.size(1), (long long)query.size(3), (long long)kv_heads,
+                                              (long long)max_len, Py_None);
+  if (got == nullptr) return false;
+  Scratch s;
+  bool ok = PyTuple_Check(got) && PyTuple_GET_SIZE(got) == 5;
+  if (ok) {
+    const at::Tensor* parts[4] = {tensor(PyTuple_GET_ITEM(got, 0)), tensor(PyTuple_GET_ITEM(got, 1)),
+                                  tensor(PyTuple_GET_ITEM(got, 3)), optional_tensor(PyTuple_GET_ITEM(got, 4), &ok)};
+    s.capacity = (int)PyLong_AsLong(PyTuple_GET_ITEM(got, 2));
+    ok = ok && parts[0] != nullptr && parts[1] != nullptr && parts[2] != nullptr;
+    if (ok) {
+      s.stats = *parts[0];
+      s.values = *parts[1];
+      s.counters = *parts[2];
+      if (parts[3] != nullptr) s.frags = *parts[3];
+    }
+  }
+  Py_DECREF(got);
+  if (!ok) {
+    if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "anna_b200: bad scratch");
+    return false;
+  }
+  if (table.size() >= kMaxScratch) table.clear();
+  table[key] = s;
+  *out = std::move(s);
+  return true;
+}
+
+PyObject* failed(const char* what, int status) {
+  return PyErr_Format(PyExc_RuntimeError, "%s failed (status %d): %s", what, status, anna_kv_last_error());
+}
+
+bool int_args(PyObject* const* args, int count, int64_t* out) {
+  for (int i = 0; i < count; ++i) {
+    out[i] = PyLong_AsLongLong(args[i]);
+    if (out[i] == -1 && PyErr_Occurred()) return false;
+  }
+  return true;
+}
+
+// set_scratch_source(callable)
+PyObject* set_scratch_source(PyObject*, PyObject* callable) {
+  Py_INCREF(callable);
+  Py_XSETREF(scratch_source, callable);
+  Py_RETURN_NONE;
+}
+
+PyObject* forget_scratch(PyObject*, PyObject*) {
+  scratch_table().clear();
+  Py_RETURN_NONE;
+}
+
+// tq_decode(query, gate | None, packed_pages | None, table | None, window, slots, lengths, signs1, signs2, centroids, scaling,
+//           kv_heads, block_size, residual_len, bits, value_group, num_pages) -> output | None
+PyObject* tq_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 17) return PyErr_Format(PyExc_TypeError, "tq_decode takes 17 arguments");
+  const at::Tensor* query = tensor(args[0]);
+  bool ok = true;
+  const at::Tensor* gate = optional_tensor(args[1], &ok);
+  const at::Tensor* pages = optional_tensor(args[2], &ok);
+  const at::Tensor* table = optional_tensor(args[3], &ok);
+  const at::Tensor* fixed[6];
+  for (int i = 0; i < 6; ++i) {
+    fixed[i] = tensor(args[4 + i]);
+    ok = ok && fixed[i] != nullptr;
+  }
+  int code = 0;
+  int64_t n[6];  // kv_heads, block_size, residual_len, bits, value_group, num_pages
+  const double scaling = PyFloat_AsDouble(args[10]);
+  if (scaling == -1.0 && PyErr_Occurred()) return nullptr;
+  if (!int_args(args + 11, 6, n)) return nullptr;
+  if (!ok || query == nullptr || !query->is_cuda() || !plain(*query, query->device(), 4) || query->size(2) != 1 ||
+      query->stride(3) != 1 || query->size(0) == 0 || n[0] <= 0 || query->size(1) % n[0] != 0 ||
+      !dtype_code(query->scalar_type(), &code))
+    Py_RETURN_NONE;
+  const c10::Device device = query->device();
+  if (gate != nullptr && (!plain(*gate, device, 4) || gate->stride(3) != 1 || gate->scalar_type() != query->scalar_type() ||
+                          gate->sizes() != query->sizes()))
+    Py_RETURN_NONE;
+  if (fixed[0]->scalar_type() != query->scalar_type() || fixed[0]->dim() != 5 || fixed[0]->size(2) != n[0] ||
+      fixed[0]->size(4) != query->size(3))
+    Py_RETURN_NONE;
+  for (const at::Tensor* t : fixed)
+    if (!on(t, device)) Py_RETURN_NONE;
+  if (!on(pages, device) || !on(table, device)) Py_RETURN_NONE;
+  const c10::cuda::CUDAGuard guard(device);
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
+  const int64_t max_blocks = table == nullptr ? 0 : table->size(1);
+  Scratch s;
+  if (!scratch_of(*query, reinterpret_cast<int64_t>(stream), n[0], max_blocks * n[1] + n[2], max_blocks, n[1], n[2], &s))
+    return nullptr;
+  at::Tensor out = at::empty(query->sizes(), query->options());
+  const int64_t q_sb = query->stride(0), q_sh = query->stride(1), g_sb = gate ? gate->stride(0) : 0,
+                g_sh = gate ? gate->stride(1) : 0;
+  const int batch = (int)query->size(0), heads = (int)query->size(1), dim = (int)query->size(3);
+  int status;
+  {
+    pybind11::gil_scoped_release unlocked;
+    status = anna_tq_paged_decode(
+        query->data_ptr(), q_sb, q_sh, static_cast<const uint8_t*>(address(pages)), static_cast<const int32_t*>(address(table)),
+        table == nullptr ? 0 : table->stride(0), address(fixed[0]), static_cast<const int64_t*>(address(fixed[1])),
+        static_cast<const int64_t*>(address(fixed[2])), floats(fixed[3]), floats(fixed[4]), floats(fixed[5]), address(gate),
+        g_sb, g_sh, out.data_ptr(), out.stride(0), out.stride(1), static_cast<float*>(s.stats.data_ptr()),
+        static_cast<float*>(s.values.data_ptr()), s.capacity, 0, static_cast<int32_t*>(s.counters.data_ptr()),
+        s.frags.defined() ? s.frags.data_ptr() : nullptr, s.frags.defined() ? (size_t)s.frags.numel() : 0, batch, heads,
+        (int)n[0], dim, (int)n[1], (int)n[2], (int)n[3], (int)n[4], n[5], max_blocks, (float)scaling, code, stream);
+  }
+  if (status != 0) return failed("anna_tq_paged_decode", status);
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+// tq_append(keys, values, packed_pages | None, table | None, window, slots, past, new_lengths | None, signs1, signs2, centroids,
+//           boundaries, status | None, block_size, residual_len, bits, value_group, num_pages) -> True | None
+PyObject* tq_append(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 18) return PyErr_Format(PyExc_TypeError, "tq_append takes 18 arguments");
+  const at::Tensor *keys = tensor(args[0]), *values = tensor(args[1]);
+  bool ok = keys != nullptr && values != nullptr;
+  const at::Tensor* pages = optional_tensor(args[2], &ok);
+  const at::Tensor* table = optional_tensor(args[3], &ok);
+  const at::Tensor* window = tensor(args[4]);
+  const at::Tensor* slots = tensor(args[5]);
+  const at::Tensor* past = tensor(args[6]);
+  const at::Tensor* fresh = optional_tensor(args[7], &ok);
+  const at::Tensor* fixed[4];
+  for (int i = 0; i < 4; ++i) {
+    fixed[i] = tensor(args[8 + i]);
+    ok = ok && fixed[i] != nullptr;
+  }
+  const at::Tensor* word = optional_tensor(args[12], &ok);
+  int64_t n[5];  // block_size, residual_len, bits, value_group, num_pages
+  if (!int_args(args + 13, 5, n)) return nullptr;
+  int code = 0;
+  if (!ok || window == nullptr || slots == nullptr || past == nullptr || !keys->is_cuda() || !plain(*keys, keys->device(), 4) ||
+      !plain(*values, keys->device(), 4) || keys->stride(3) != 1 || keys->sizes() != values->sizes() ||
+      keys->strides() != values->strides() || keys->scalar_type() != values->scalar_type() || keys->numel() == 0 ||
+      window->dim() != 5 || window->scalar_type() != keys->scalar_type() || window->size(2) != keys->size(1) ||
+      window->size(4) != keys->size(3) || !dtype_code(keys->scalar_type(), &code))
+    Py_RETURN_NONE;
+  const c10::Device device = keys->device();
+  for (const at::Tensor* t : {pages, table, window, slots, past, fresh, fixed[0], fixed[1], fixed[2], fixed[3], word})
+    if (!on(t, device)) Py_RETURN_NONE;
+  const c10::cuda::CUDAGuard guard(device);
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
+  int status;
+  {
+    pybind11::gil_scoped_release unlocked;
+    status = anna_tq_append(
+        keys->data_ptr(), values->data_ptr(), keys->stride(0), keys->stride(1), keys->stride(2),
+        static_cast<uint8_t*>(address(pages)), static_cast<const int32_t*>(address(table)),
+        table == nullptr ? 0 : table->stride(0), nullptr, 0, address(window), static_cast<const int64_t*>(address(slots)),
+        static_cast<const int64_t*>(address(past)), static_cast<int64_t*>(address(fresh)), floats(fixed[0]), floats(fixed[1]),
+        floats(fixed[2]), floats(fixed[3]), (int)keys->size(0), (int)keys->size(1), (int)keys->size(2), (int)keys->size(3),
+        (int)n[0], (int)n[1], (int)n[2], (int)n[3], n[4], table == nullptr ? 0 : table->size(1), code,
+        static_cast<int32_t*>(address(word)), stream);
+  }
+  if (status != 0) return failed("anna_tq_append", status);
+  Py_RETURN_TRUE;
+  END_HANDLE_TH_ERRORS
+}
+
+// paged_decode(query, key_pages, value_pages, page_table, visible_lengths, scaling, gate | None) -> output | None
+PyObject* paged_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 7) return PyErr_Format(PyExc_TypeError, "paged_decode takes 7 arguments");
+  const at::Tensor* t[5];
+  for (int i = 0; i < 5; ++i)
+    if ((t[i] = tensor(args[i])) == nullptr) Py_RETURN_NONE;
+  const at::Tensor &query = *t[0], &keys = *t[1], &values = *t[2], &table = *t[3], &lengths = *t[4];
+  bool ok = true;
+  const at::Tensor* gate = optional_tensor(args[6], &ok);
+  const double scaling = PyFloat_AsDouble(args[5]);
+  if (scaling == -1.0 && PyErr_Occurred()) return nullptr;
+  int code = 0;
+  if (!ok || !query.is_cuda() || !plain(query, query.device(), 4) || query.size(2) != 1 || query.stride(3) != 1 ||
+      !dtype_code(query.scalar_type(), &code))
+    Py_RETURN_NONE;
+  const c10::Device device = query.device();
+  if (!plain(keys, device, 4) || !plain(values, device, 4) || !plain(table, device, 2) || !plain(lengths, device, 1) ||
+      keys.sizes() != values.sizes() || !keys.is_contiguous() || !values.is_contiguous() ||
+      keys.scalar_type() != query.scalar_type() || values.scalar_type() != query.scalar_type() ||
+      table.scalar_type() != at::kInt || lengths.scalar_type() != at::kLong || table.stride(1) != 1 || lengths.stride(0) != 1)
+    Py_RETURN_NONE;
+  const int64_t batch = query.size(0), heads = query.size(1), dim = query.size(3), kv_heads = keys.size(1),
+                block = keys.size(2), max_blocks = table.size(1);
+  if (keys.numel() == 0 || batch == 0 || heads == 0 || heads % kv_heads != 0 || dim != keys.size(3) || table.size(0) != batch ||
+      lengths.size(0) != batch || max_blocks == 0)
+    Py_RETURN_NONE;
+  int64_t g_sb = 0, g_sh = 0;
+  if (gate != nullptr) {
+    if (gate->device() != device || gate->layout() != at::kStrided || gate->scalar_type() != query.scalar_type() ||
+        gate->dim() < 3 || gate->size(0) != batch)
+      Py_RETURN_NONE;
+    if (gate->dim() == 4 && gate->sizes() == query.sizes() && gate->stride(3) == 1) {
+      g_sb = gate->stride(0);
+      g_sh = gate->stride(1);
+    } else if (gate->dim() == 3 && gate->size(1) == 1 && gate->size(2) == heads * dim && gate->stride(2) == 1) {
+      g_sb = gate->stride(0);
+      g_sh = dim;
+    } else {
+      Py_RETURN_NONE;
+    }
+  }
+  const c10::cuda::CUDAGuard guard(device);
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
+  Scratch s;
+  if (!scratch_of(query, reinterpret_cast<int64_t>(stream), kv_heads, max_blocks * block, 0, block, 0, &s)) return nullptr;
+  at::Tensor out = at::empty(query.sizes(), query.options());
+  int status;
+  {
+    pybind11::gil_scoped_release unlocked;
+    status = anna_paged_gqa_decode(
+        query.data_ptr(), query.stride(0), query.stride(1), keys.data_ptr(), values.data_ptr(),
+        static_cast<const int32_t*>(table.data_ptr()), table.stride(0), static_cast<const int64_t*>(lengths.data_ptr()),
+        address(gate), g_sb, g_sh, out.data_ptr(), heads * dim, dim, static_cast<float*>(s.stats.data_ptr()),
+        static_cast<float*>(s.values.data_ptr()), s.capacity, 0, static_cast<int32_t*>(s.counters.data_ptr()), (int)batch,
+        (int)heads, (int)kv_heads, (int)dim, (int)block, keys.size(0), max_blocks, (float)scaling, code, stream);
+  }
+  if (status != 0) return failed("paged_gqa_decode_fused", status);
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+// prefill(query, keys, values, key_lengths | None, scaling, causal) -> output | None
+PyObject* prefill(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 6) return PyErr_Format(PyExc_TypeError, "prefill takes 6 arguments");
+  const at::Tensor* t[3];
+  for (int i = 0; i < 3; ++i)
+    if ((t[i] = tensor(args[i])) == nullptr) Py_RETURN_NONE;
+  const at::Tensor &query = *t[0], &keys = *t[1], &values = *t[2];
+  bool ok = true;
+  const at::Tensor* lengths = optional_tensor(args[3], &ok);
+  const double scaling = PyFloat_AsDouble(args[4]);
+  if (scaling == -1.0 && PyErr_Occurred()) return nullptr;
+  const int causal = PyObject_IsTrue(args[5]);
+  if (causal < 0) return nullptr;
+  int code = 0;
+  if (!ok || !query.is_cuda() || !plain(query, query.device(), 4) || !dtype_code(query.scalar_type(), &code) ||
+      code == ANNA_DTYPE_F32)
+    Py_RETURN_NONE;
+  const c10::Device device = query.device();
+  const int64_t batch = query.size(0), heads = query.size(1), tokens = query.size(2), dim = query.size(3);
+  if (!plain(keys, device, 4) || !plain(values, device, 4) || keys.sizes() != values.sizes() ||
+      keys.strides() != values.strides() || keys.scalar_type() != query.scalar_type() ||
+      values.scalar_type() != query.scalar_type() || keys.numel() == 0 || query.numel() == 0 || keys.size(0) != batch ||
+      keys.size(3) != dim || heads % keys.size(1) != 0 || (dim != 64 && dim != 128 && dim != 256))
+    Py_RETURN_NONE;
+  if (lengths != nullptr && (!plain(*lengths, device, 1) || lengths->scalar_type() != at::kLong || lengths->size(0) != batch ||
+                             lengths->stride(0) != 1))
+    Py_RETURN_NONE;
+  for (const at::Tensor* x : t) {  // what 16-byte copies need
+    if (x->stride(3) != 1 || reinterpret_cast<uintptr_t>(x->data_ptr()) % 16 != 0) Py_RETURN_NONE;
+    for (int i = 0; i < 3; ++i)
+      if (x->stride(i) % 8 != 0) Py_RETURN_NONE;
+  }
+  const c10::cuda::CUDAGuard guard(device);
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
+  at::Tensor out = at::empty(query.sizes(), query.options());
+  int status;
+  {
+    pybind11::gil_scoped_release unlocked;
+    status = anna_gqa_prefill(query.data_ptr(), query.stride(0), query.stride(1), query.stride(2), keys.data_ptr(),
+                              values.data_ptr(), keys.stride(0), keys.stride(1), keys.stride(2),
+                              static_cast<const int64_t*>(address(lengths)), out.data_ptr(), out.stride(0), out.stride(1),
+                              out.stride(2), (int)batch, (int)heads, (int)keys.size(1), (int)tokens, keys.size(2), (int)dim,
+                              (float)scaling, causal, code, stream);
+  }
+  if (status != 0) return failed("anna_gqa_prefill", status);
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef methods[] = {
+    {"set_scratch_source", set_scratch_source, METH_O, nullptr},
+    {"forget_scratch", forget_scratch, METH_NOARGS, nullptr},
+    {"tq_decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(tq_decode)), METH_FASTCALL, nullptr},
+    {"tq_append", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(tq_append)), METH_FASTCALL, nullptr},
+    {"paged_decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(paged_decode)), METH_FASTCALL, nullptr},
+    {"prefill", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(prefill)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_launch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__launch() { return PyModule_Create(&module); }

@@ -245,7 +245,7 @@ class _Scratch:
         if buf is None or buf.numel() < floats:
             buf = torch.empty(max(floats, 1 << 16), dtype=torch.float32, device=device)
             self._buffers[key] = buf
-            _SPLIT_CACHE.clear()  # cached views point into the old buffer
+            _forget_scratch()  # cached views point into the old buffer
         return buf
 
     def bytes(self, device: torch.device, count: int) -> torch.Tensor:
@@ -254,6 +254,7 @@ class _Scratch:
         if buf is None or buf.numel() < count:
             buf = torch.empty(max(count, 1 << 20), dtype=torch.uint8, device=device)
             self._byte_buffers[key] = buf
+            _forget_scratch()
         return buf
 
     def counters(self, device: torch.device, count: int) -> torch.Tensor:
@@ -262,12 +263,37 @@ class _Scratch:
         if buf is None or buf.numel() < count:
             buf = torch.zeros(max(count, 4096), dtype=torch.int32, device=device)
             self._counters[key] = buf
-            _SPLIT_CACHE.clear()
+            _forget_scratch()
         return buf
 
 
 _SPLIT_CACHE: dict[tuple, tuple] = {}  # split_scratch results by problem shape, device and stream
 _SCRATCH = _Scratch()
+_LAUNCH = None
+
+
+def _forget_scratch() -> None:
+    """A scratch buffer was replaced: nobody may hand out views of the old one any more."""
+    _SPLIT_CACHE.clear()
+    if _LAUNCH is not None:
+        _LAUNCH.forget_scratch()
+
+
+def _scratch_source(device, batch, heads, head_dim, kv_heads, max_len, turboquant):
+    """What the call module keeps per problem: split_scratch and, for the packed decode, query_scratch."""
+    frags = None if turboquant is None else query_scratch(device, batch, heads, kv_heads, head_dim)
+    stats, values, capacity, counters = split_scratch(device, batch, heads, head_dim, kv_heads, max_len,
+                                                      turboquant=turboquant)
+    return stats, values, capacity, counters, frags
+
+
+def launch_module():
+    global _LAUNCH
+    if _LAUNCH is None:
+        module = _lib.launch()
+        module.set_scratch_source(_scratch_source)
+        _LAUNCH = module
+    return _LAUNCH
 
 
 def query_scratch(device: torch.device, batch: int, heads: int, kv_heads: int, head_dim: int) -> torch.Tensor:
@@ -495,6 +521,10 @@ def _op_gqa_decode_splitkv_turboquant_fused_out(query, quantized_key, value_data
 
 def _op_paged_gqa_decode_fused(query, key_pages, value_pages, page_table, visible_lengths, scaling, gate=None):
     name = "paged_gqa_decode_fused"
+    out = (_LAUNCH or launch_module()).paged_decode(query, key_pages, value_pages, page_table, visible_lengths, scaling, gate)
+    if out is not None:
+        return out
+    # not the ordinary call: arguments to be checked, or copied into the layout that the kernels read
     query = _check_query(name, query)
     page_shape, table_shape, length_shape = tuple(key_pages.shape), tuple(page_table.shape), tuple(visible_lengths.shape)
     if len(page_shape) != 4 or value_pages.dim() != 4:

@@ -13,7 +13,8 @@ from array import array
 import torch
 
 from . import _lib
-from .fused_ops import MetadataUploader, dtype_code, on_device, ptr, query_scratch, split_scratch, stream_ptr
+from .fused_ops import (MetadataUploader, dtype_code, launch_module, on_device, ptr, query_scratch, split_scratch,
+                        stream_ptr)
 from .pools import TurboQuantLayerPool, resolve_value_group_size
 from .tq_tables import key_tables
 
@@ -53,6 +54,13 @@ def launch_tq_append(pool: TurboQuantLayerPool, key_states: torch.Tensor, value_
     caller already holds there; ``new_lengths_dev`` (optional) receives ``past + T`` from the kernel;
     ``shared_blocks`` (optional, int32 ``[B, words]`` bit mask on the device) marks blocks whose pages already hold
     their tokens' codes (mapped from a sequence with the same prompt prefix)."""
+    if past_dev is not None and slots_dev is not None and shared_blocks is None and key_states.shape[3] == pool.head_dim:
+        tables = pool.tables
+        if launch_module().tq_append(key_states, value_states, pool.packed_pages, table_dev, pool.window, slots_dev, past_dev,
+                                     new_lengths_dev, tables.signs1, tables.signs2, tables.centroids, tables.boundaries,
+                                     pool.status, pool.block_size, pool.residual_len, pool.bits, pool.value_group,
+                                     pool.capacity()):
+            return
     _require_cuda(key_states, "TurboQuant append")
     key_states = key_states if key_states.stride(3) == 1 else key_states.contiguous()
     if value_states.stride() != key_states.stride():
@@ -87,6 +95,13 @@ def launch_tq_decode(pool: TurboQuantLayerPool, query_states: torch.Tensor, tabl
     that the caller already holds there.  ``output`` (optional, ``[B, Hq, 1, D]``, last dimension contiguous) receives
     the result instead of a new tensor; ``peer_outputs`` are device addresses, in other GPUs' memory, of tensors with
     the strides of ``output`` that receive the same rows (KV-head-sharded decode, see ``sharding.PeerHeadGather``)."""
+    if slots_dev is not None and lengths_dev is not None and output is None and not peer_outputs:
+        tables = pool.tables
+        out = launch_module().tq_decode(query_states, gate, pool.packed_pages, table_dev, pool.window, slots_dev, lengths_dev,
+                                        tables.signs1, tables.signs2, tables.centroids, scaling, pool.kv_heads, pool.block_size,
+                                        pool.residual_len, pool.bits, pool.value_group, pool.capacity())
+        if out is not None:
+            return out
     _require_cuda(query_states, "TurboQuant decode")
     query = query_states if query_states.stride(3) == 1 else query_states.contiguous()
     if gate is not None and gate.stride(3) != 1:
