@@ -648,10 +648,10 @@ class Qwen3DynamicCache:
         self._packed_blocks_registered[layer_idx] = max(self._packed_blocks_registered[layer_idx], done)
 
     def _update_turboquant_layer(self, key_states, value_states, layer_idx: int, *, require_dense_cache: bool):
-        batch_size, kv_heads, append_length, head_dim = (int(v) for v in key_states.shape)
+        batch_size, kv_heads, append_length, head_dim = key_states.shape
         self._ensure_batch_size(batch_size)
         device = key_states.device
-        pool = self._tq_pool(layer_idx)
+        pool = self.allocator.turboquant_layers[layer_idx]
         step = self._tq_step[layer_idx]
         if step is not None and 0 < append_length <= step.headroom:
             past_lengths = self._append_quantized_step(step, pool, key_states, value_states, layer_idx)

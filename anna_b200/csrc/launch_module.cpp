@@ -1,4 +1,5 @@
-// Python entry points of the calls a decode loop makes every step, on the C ABI of libanna_b200_kv.so.
+// Python entry points of the calls a decode loop makes every step, on the C ABI of libanna_b200_kv.so, and the loops over
+// page ids behind the allocators (pools.py).
 //
 // A ctypes call converts some forty arguments one by one, and every address, size and stride among them costs a Python
 // call of its own: two thirds of the 18 us of host time of a decode call, whose GPU work for a few short rows takes no
@@ -360,7 +361,109 @@ PyObject* prefill(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
+// ---- page book: free pages are a list of ints, last in first out; owners are int32 counts by page id --------------------
+
+struct Ints {  // a writable int32 buffer
+  Py_buffer view{};
+  bool held = false;
+  explicit Ints(PyObject* obj) { held = PyObject_GetBuffer(obj, &view, PyBUF_WRITABLE | PyBUF_ND) == 0; }
+  ~Ints() {
+    if (held) PyBuffer_Release(&view);
+  }
+  int32_t* data() const { return static_cast<int32_t*>(view.buf); }
+  Py_ssize_t size() const { return view.len / (Py_ssize_t)sizeof(int32_t); }
+  Ints(const Ints&) = delete;
+  Ints& operator=(const Ints&) = delete;
+};
+
+// take_pages(free, counts, count) -> the last `count` ids of `free`, last one first; they leave `free` with one owner each
+PyObject* take_pages(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  if (nargs != 3 || !PyList_Check(args[0])) return PyErr_Format(PyExc_TypeError, "take_pages(list, counts, count)");
+  PyObject* free_list = args[0];
+  const Py_ssize_t have = PyList_GET_SIZE(free_list), count = PyLong_AsSsize_t(args[2]);
+  if (count < 0 || count > have) {
+    if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "take_pages: more pages than are free");
+    return nullptr;
+  }
+  Ints counts(args[1]);
+  if (!counts.held) return nullptr;
+  for (Py_ssize_t i = 0; i < count; ++i) {
+    const Py_ssize_t id = PyLong_AsSsize_t(PyList_GET_ITEM(free_list, have - 1 - i));
+    if (id == -1 && PyErr_Occurred()) return nullptr;
+    if (id < 0 || id >= counts.size())
+      return PyErr_Format(PyExc_RuntimeError, "Invariant violated: free list page %zd does not exist.", id);
+    if (counts.data()[id] != 0)
+      return PyErr_Format(PyExc_RuntimeError, "Invariant violated: free list page %zd has non-zero refcount.", id);
+  }
+  PyObject* out = PyList_New(count);
+  if (out == nullptr) return nullptr;
+  for (Py_ssize_t i = 0; i < count; ++i) {
+    PyObject* id = PyList_GET_ITEM(free_list, have - 1 - i);
+    counts.data()[PyLong_AsSsize_t(id)] = 1;
+    Py_INCREF(id);
+    PyList_SET_ITEM(out, i, id);
+  }
+  if (PyList_SetSlice(free_list, have - count, have, nullptr) != 0) {
+    Py_DECREF(out);
+    return nullptr;
+  }
+  return out;
+}
+
+// release_pages(ids, counts) -> (ids that lost their last owner, in order; pages that are no longer shared): every id loses
+// one owner, ids without one are passed over
+PyObject* release_pages(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  if (nargs != 2 || !PyList_Check(args[0])) return PyErr_Format(PyExc_TypeError, "release_pages(list, counts)");
+  Ints counts(args[1]);
+  if (!counts.held) return nullptr;
+  const Py_ssize_t n = PyList_GET_SIZE(args[0]);
+  for (Py_ssize_t i = 0; i < n; ++i)
+    if (PyLong_AsSsize_t(PyList_GET_ITEM(args[0], i)) == -1 && PyErr_Occurred()) return nullptr;
+  PyObject* freed = PyList_New(n);
+  if (freed == nullptr) return nullptr;
+  Py_ssize_t last = 0, unshared = 0;
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    PyObject* id = PyList_GET_ITEM(args[0], i);
+    const Py_ssize_t page = PyLong_AsSsize_t(id);
+    if (page < 0 || page >= counts.size() || counts.data()[page] <= 0) continue;
+    const int32_t left = --counts.data()[page];
+    if (left == 1) ++unshared;
+    if (left > 0) continue;
+    Py_INCREF(id);
+    PyList_SET_ITEM(freed, last++, id);
+  }
+  if (last < n) {  // the rest of the new list is empty slots
+    PyObject* part = PyList_GetSlice(freed, 0, last);
+    Py_DECREF(freed);
+    freed = part;
+    if (freed == nullptr) return nullptr;
+  }
+  return Py_BuildValue("Nn", freed, unshared);
+}
+
+// copy_pages(ids, first, last, target): ids[first:last] to the same places of an int32 buffer
+PyObject* copy_pages(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  if (nargs != 4 || !PyList_Check(args[0])) return PyErr_Format(PyExc_TypeError, "copy_pages(list, first, last, target)");
+  const Py_ssize_t first = PyLong_AsSsize_t(args[1]), last = PyLong_AsSsize_t(args[2]);
+  if (PyErr_Occurred()) return nullptr;
+  Ints target(args[3]);
+  if (!target.held) return nullptr;
+  if (first < 0 || last < first || last > PyList_GET_SIZE(args[0]) || last > target.size()) {
+    PyErr_SetString(PyExc_ValueError, "copy_pages: out of range");
+    return nullptr;
+  }
+  for (Py_ssize_t i = first; i < last; ++i) {
+    const long id = PyLong_AsLong(PyList_GET_ITEM(args[0], i));
+    if (id == -1 && PyErr_Occurred()) return nullptr;
+    target.data()[i] = (int32_t)id;
+  }
+  Py_RETURN_NONE;
+}
+
 PyMethodDef methods[] = {
+    {"take_pages", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(take_pages)), METH_FASTCALL, nullptr},
+    {"release_pages", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(release_pages)), METH_FASTCALL, nullptr},
+    {"copy_pages", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(copy_pages)), METH_FASTCALL, nullptr},
     {"set_scratch_source", set_scratch_source, METH_O, nullptr},
     {"forget_scratch", forget_scratch, METH_NOARGS, nullptr},
     {"tq_decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(tq_decode)), METH_FASTCALL, nullptr},

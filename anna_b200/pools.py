@@ -5,8 +5,8 @@ The bookkeeping (LIFO free list, growth by ``max(n, capacity or 16)``, reversed 
 """
 from __future__ import annotations
 
+from array import array
 from collections.abc import Callable
-from itertools import repeat
 
 import torch
 
@@ -24,27 +24,35 @@ def resolve_value_group_size(head_dim: int) -> int:
 
 
 class _PageBook:
+    """Free pages (a list, last in first out) and the number of owners of every page.  The loops over page ids run in the
+    call module: with a dict of owners, taking and giving back the 960 pages of eight 2048-token prompts was 90 us."""
+
     def __init__(self, on_page_freed: Callable[[int], None] | None = None,
                  listening: Callable[[], bool] | None = None) -> None:
         self.free_pages: list[int] = []
-        self.refcount: dict[int, int] = {}
+        self._counts = array("i")    # owners by page id
         self._on_page_freed = on_page_freed
         self._listening = listening  # optional: False while the callback has nothing to do (an empty registry)
         self._shared = 0  # pages with more than one owner
 
+    @property
+    def refcount(self) -> dict[int, int]:
+        """Owners of every page that has one."""
+        return {page_id: rc for page_id, rc in enumerate(self._counts) if rc}
+
+    def owners(self, page_id: int) -> int:
+        return self._counts[page_id] if 0 <= page_id < len(self._counts) else 0
+
+    def _cover(self, pages: int) -> None:
+        if pages > len(self._counts):
+            self._counts.frombytes(bytes(self._counts.itemsize * (pages - len(self._counts))))
+
     def take(self, num_pages: int, capacity: int) -> tuple[list[int], int, list[int]]:
         """Pop up to num_pages from the free list; returns (page ids, new capacity, ids created by growth)."""
         count = min(max(int(num_pages), 0), len(self.free_pages))
-        out: list[int] = []
-        if count > 0:
-            # the last `count` entries of the free list, most recently freed first (the same order as repeated pop())
-            out = self.free_pages[-count:]
-            out.reverse()
-            del self.free_pages[-count:]
-            if not self.refcount.keys().isdisjoint(out):
-                stale = self.refcount.keys() & out
-                raise RuntimeError(f"Invariant violated: free list page {min(stale)} has non-zero refcount.")
-            self.refcount.update(dict.fromkeys(out, 1))
+        self._cover(capacity)
+        # the last `count` entries of the free list, most recently freed first (the same order as repeated pop())
+        out: list[int] = _lib.launch().take_pages(self.free_pages, self._counts, count) if count > 0 else []
         missing = num_pages - len(out)
         new_capacity = capacity
         fresh: list[int] = []
@@ -54,7 +62,8 @@ class _PageBook:
             new_ids = list(range(capacity, new_capacity))
             fresh = new_ids[:missing]
             self.free_pages.extend(reversed(new_ids[missing:]))
-            self.refcount.update(dict.fromkeys(fresh, 1))
+            self._cover(new_capacity)
+            self._counts[capacity:capacity + missing] = array("i", [1]) * missing
             out.extend(fresh)
         return out, new_capacity, fresh
 
@@ -69,59 +78,27 @@ class _PageBook:
         return new_capacity
 
     def retain(self, page_id: int) -> None:
-        rc = self.refcount.get(page_id, 0)
-        self.refcount[page_id] = rc + 1
-        if rc == 1:
+        self._cover(page_id + 1)
+        self._counts[page_id] += 1
+        if self._counts[page_id] == 2:
             self._shared += 1
 
     def release(self, page_id: int) -> None:
-        rc = self.refcount.get(page_id, 0)
-        if rc <= 0:
-            return
-        if rc == 1:
-            self.refcount.pop(page_id, None)
-            self.free_pages.append(page_id)
-            if self._on_page_freed is not None:
-                self._on_page_freed(page_id)
-        else:
-            self.refcount[page_id] = rc - 1
-            if rc == 2:
-                self._shared -= 1
+        self.release_many([page_id])
 
-    def release_many(self, page_ids, *, notify: bool = True) -> None:
-        """release() for every id of `page_ids`, in the given order, in one pass.  `notify=False` skips the per-page
-        callback (for callers that know nobody listens, e.g. an empty prefix registry)."""
-        refcount = self.refcount
-        ids = page_ids if isinstance(page_ids, list) else list(page_ids)
-        counts: list[int] = []
-        if self._shared == 0:
-            # normally every id is held exactly once: one pass at C speed takes all of them out
-            counts = list(map(refcount.pop, ids, repeat(0)))
-        if counts and counts.count(1) == len(ids):
-            freed = ids
-        else:
-            for page_id, rc in zip(ids, counts):  # a free or repeated id among them: put back, then one by one
-                if rc:
-                    refcount[page_id] = rc
-            freed = []
-            for page_id in ids:
-                rc = refcount.get(page_id, 0)
-                if rc == 1:
-                    del refcount[page_id]
-                    freed.append(page_id)
-                elif rc > 1:
-                    refcount[page_id] = rc - 1
-                    if rc == 2:
-                        self._shared -= 1
+    def release_many(self, page_ids) -> None:
+        """Every id of `page_ids` loses one owner, in the given order; an id without one is passed over."""
+        freed, unshared = _lib.launch().release_pages(page_ids if isinstance(page_ids, list) else list(page_ids), self._counts)
+        self._shared -= unshared
         if freed:
             self.free_pages.extend(freed)
-            if notify and self._on_page_freed is not None and (self._listening is None or self._listening()):
+            if self._on_page_freed is not None and (self._listening is None or self._listening()):
                 for page_id in freed:
                     self._on_page_freed(page_id)
 
     def clear(self) -> None:
         self.free_pages.clear()
-        self.refcount.clear()
+        self._counts = array("i")
         self._shared = 0
 
 
@@ -179,7 +156,7 @@ class Qwen3PagedLayerAllocator:
 
     def page_owners(self, page_id: int) -> int:
         """How many block tables map this page (0 for a free page)."""
-        return self._book.refcount.get(page_id, 0)
+        return self._book.owners(page_id)
 
     def release_page(self, page_id: int) -> None:
         self._book.release(page_id)
@@ -302,11 +279,11 @@ class TurboQuantLayerPool:
 
     def page_owners(self, page_id: int) -> int:
         """How many rows map this packed page (0 for a free page)."""
-        return self._book.refcount.get(page_id, 0)
+        return self._book.owners(page_id)
 
     def retain_page(self, page_id: int) -> None:
         """One more owner of a packed page (a sequence that maps it for a shared prompt prefix, or a clone)."""
-        if page_id < 0 or page_id >= self.capacity() or self._book.refcount.get(page_id, 0) <= 0:
+        if page_id < 0 or page_id >= self.capacity() or self._book.owners(page_id) <= 0:
             raise ValueError(f"retain_page: page {page_id} is not a live packed page (capacity {self.capacity()}).")
         self.version += 1
         self._book.retain(page_id)

@@ -8,8 +8,6 @@ whole batch of rows is appended or decoded by one launch.
 """
 from __future__ import annotations
 
-from array import array
-
 import torch
 
 from . import _lib
@@ -460,7 +458,7 @@ class TurboQuantKVRow:
                 grown[:valid] = arr[:valid]
             arr = self._table_np = grown
         if valid < n:
-            arr[valid:n] = array("i", self._blocks[valid:n])
+            _lib.launch().copy_pages(self._blocks, valid, n, arr)
         self._table_np_valid = n
         return arr[:n]
 
@@ -578,9 +576,9 @@ class TurboQuantKVRow:
             pages: list[int] = []
             for row in rows:
                 if row.pool is pool:
-                    pages += row._blocks[::-1]
-            pages.reverse()
-            pool.release_pages(pages)  # which gives back the last one first
+                    pages += row._blocks[::-1]  # the last one of a row goes back first
+            pool.version += 1
+            pool._book.release_many(pages)
         for row in rows:
             row.pool.release_slot(row.slot)
             row._blocks = []
