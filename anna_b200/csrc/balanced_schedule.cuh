@@ -174,54 +174,108 @@ __host__ __device__ __forceinline__ BalancedSegment balanced_segment(const Balan
   return seg;
 }
 
+// The line of a batch of at most 32 rows, worked out by every warp for itself, a row per lane: no barriers and no shared
+// memory between the load of the lengths and the first tile.
+struct WarpLine {
+  int len;          // of this lane's row, without its tail
+  int tiles;        // of each of the row's streams
+  int first, next;  // positions of the row's streams: [first, next)
+
+  __device__ __forceinline__ void load(const int64_t* visible_lengths, int64_t max_len, int batch, int tail) {
+    const int b = threadIdx.x & 31;
+    int64_t n = 0;
+    if (b < batch) n = max((int64_t)0, min(visible_lengths ? visible_lengths[b] : max_len, max_len) - tail);
+    len = (int)n;
+    tiles = (len + kBalancedTileTokens - 1) / kBalancedTileTokens;
+  }
+  // returns all positions
+  __device__ __forceinline__ int scan(int streams_per_row, int stream_tiles, int piece_tiles) {
+    const int lane = threadIdx.x & 31;
+    const int n = balanced_line_length(tiles, stream_tiles, piece_tiles) * streams_per_row;
+    next = n;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, next, d);
+      if (lane >= d) next += v;
+    }
+    first = next - n;
+    return __shfl_sync(0xffffffffu, next, 31);
+  }
+};
+
 // Calls zero_row(b) for this CTA's share of the rows without any visible key, then
 // segment(b, stream, t0, t1, slot, partials_of_stream) for each piece of this CTA's tile range, in order.
 // THREADS = blockDim.x (a multiple of 32, at most 1024 / 8 rows per thread); all threads of the CTA must call it and
 // `segment` may synchronise the CTA.  `tail`: the newest tokens of every row that the line leaves out; the rest: see
-// balanced_cut.
-template <int THREADS, typename ZeroFn, typename SegmentFn>
+// balanced_cut.  kWarpLine: batches of at most 32 rows are lined up in registers (WarpLine), which a kernel has to have room
+// for: un-quantized decode of 4 rows of 60-900 tokens 12.3 -> 10.8 us, but one
+// packed row of 4000 tokens 18.6 -> 20.2, where the row's state went to local memory and back around every segment.
+template <int THREADS, bool kWarpLine, typename ZeroFn, typename SegmentFn>
 __device__ __forceinline__ void balanced_for_each_segment(const int64_t* visible_lengths, int64_t max_len, int batch,
                                                           int streams_per_row, int chunk_capacity, ZeroFn&& zero_row,
                                                           SegmentFn&& segment, int tail, int min_tiles, int segment_tiles,
                                                           int stream_tiles) {
   __shared__ int s_prefix[kBalancedMaxRows + 1];
-  auto row_len = [&](int b) -> int {
-    int64_t len = visible_lengths ? visible_lengths[b] : max_len;
-    return (int)max((int64_t)0, min(len, max_len) - tail);
-  };
+  const bool small = kWarpLine && batch <= 32;
+  WarpLine line{};
   int tiles_of_rows[kBalancedRowsPerThread<THREADS>];
-  balanced_load_tiles<THREADS>(visible_lengths, max_len, batch, tail, tiles_of_rows);
-  int streams = 0;
-  const int max_tiles = balanced_scan<THREADS>(tiles_of_rows, batch, streams_per_row, s_prefix, stream_tiles, 0, &streams);
-  int total = s_prefix[batch];
-  // rows without a visible key have no tile: their zero outputs are dealt round-robin
-  for (int b = blockIdx.x; b < batch; b += gridDim.x)
-    if (s_prefix[b + 1] == s_prefix[b]) zero_row(b);
+  if (small) line.load(visible_lengths, max_len, batch, tail);
+  else balanced_load_tiles<THREADS>(visible_lengths, max_len, batch, tail, tiles_of_rows);
+  int streams = 0, max_tiles, total;
+  if (small) {
+    total = line.scan(streams_per_row, stream_tiles, 0);
+    max_tiles = __reduce_max_sync(0xffffffffu, line.tiles);
+    const unsigned filled = __ballot_sync(0xffffffffu, line.tiles > 0);
+    streams = __popc(filled) * streams_per_row;
+    for (int b = blockIdx.x; b < batch; b += gridDim.x)
+      if (!((filled >> b) & 1u)) zero_row(b);
+  } else {
+    max_tiles = balanced_scan<THREADS>(tiles_of_rows, batch, streams_per_row, s_prefix, stream_tiles, 0, &streams);
+    total = s_prefix[batch];
+    // rows without a visible key have no tile: their zero outputs are dealt round-robin
+    for (int b = blockIdx.x; b < batch; b += gridDim.x)
+      if (s_prefix[b + 1] == s_prefix[b]) zero_row(b);
+  }
   if (total == 0) return;
 
   const BalancedCut cut = balanced_cut(total, streams, max_tiles, (int)gridDim.x, chunk_capacity, min_tiles, segment_tiles,
                                        stream_tiles);
-  if (cut.piece_tiles > 0) {
-    __syncthreads();  // s_prefix is written again: pieces instead of tiles
-    balanced_scan<THREADS>(tiles_of_rows, batch, streams_per_row, s_prefix, 0, cut.piece_tiles, &streams);
-    total = s_prefix[batch];
+  if (cut.piece_tiles > 0) {  // the line of pieces instead of tiles
+    if (small) {
+      total = line.scan(streams_per_row, 0, cut.piece_tiles);
+    } else {
+      __syncthreads();  // s_prefix is written again
+      balanced_scan<THREADS>(tiles_of_rows, batch, streams_per_row, s_prefix, 0, cut.piece_tiles, &streams);
+      total = s_prefix[batch];
+    }
   }
   int pos = (int)min((int64_t)blockIdx.x * cut.share, (int64_t)total);
   const int end = (int)min((int64_t)pos + cut.share, (int64_t)total);
   if (pos >= end) return;
 
-  // row that holds position `pos`: the last b with s_prefix[b] <= pos (rows without tiles are skipped by construction)
-  int lo = 0, hi = batch;  // invariant: s_prefix[lo] <= pos < s_prefix[hi]
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (s_prefix[mid] <= pos) lo = mid; else hi = mid;
+  int b = 0;
+  if (!small) {  // row that holds position `pos`: the last b with s_prefix[b] <= pos (rows without tiles are skipped)
+    int lo = 0, hi = batch;  // invariant: s_prefix[lo] <= pos < s_prefix[hi]
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (s_prefix[mid] <= pos) lo = mid; else hi = mid;
+    }
+    b = lo;
   }
-  int b = lo;
   while (pos < end) {
-    while (s_prefix[b + 1] <= pos) ++b;
-    const int len = row_len(b);
+    int len, row_first;
+    if (small) {
+      b = __popc(__ballot_sync(0xffffffffu, line.next <= pos));  // rows that end at or before it (never all: pos < total)
+      len = __shfl_sync(0xffffffffu, line.len, b);
+      row_first = __shfl_sync(0xffffffffu, line.first, b);
+    } else {
+      while (s_prefix[b + 1] <= pos) ++b;
+      const int64_t n = visible_lengths ? visible_lengths[b] : max_len;
+      len = (int)max((int64_t)0, min(n, max_len) - tail);
+      row_first = s_prefix[b];
+    }
     const int tiles = (len + kBalancedTileTokens - 1) / kBalancedTileTokens;
-    const BalancedSegment seg = balanced_segment(cut, (int)blockIdx.x, pos, end, s_prefix[b], tiles, stream_tiles);
+    const BalancedSegment seg = balanced_segment(cut, (int)blockIdx.x, pos, end, row_first, tiles, stream_tiles);
     if (seg.last > seg.first)
       segment(b, seg.stream, seg.first * kBalancedTileTokens, min(len, seg.last * kBalancedTileTokens), seg.slot,
               seg.partials);

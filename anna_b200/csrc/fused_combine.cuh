@@ -33,17 +33,18 @@ __device__ __forceinline__ void fused_combine_tail(const FusedCombine& fc, int b
                                                    const float* values, float* smem_weights /* [8][kFusedMaxChunks] */,
                                                    int64_t counter_index, int arrivals = 0) {
   __shared__ int s_is_last;
-  __syncthreads();  // all partial stores of this CTA are ordered before the fence below
+  __syncthreads();  // all partial stores of this CTA are ordered before the arrival below
   if (threadIdx.x == 0) {
-    __threadfence();
+    // releases this CTA's partial and acquires those of the CTAs counted before; the barriers on both sides extend that to
+    // the other threads (4 un-quantized rows of 60-900 tokens: 10.8 us with a full fence on either side, 10.3 so)
     int32_t* counter = fc.counters + counter_index;
-    const int prev = atomicAdd(counter, 1);
+    int prev;
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;\n" : "=r"(prev) : "l"(counter) : "memory");
     s_is_last = (prev == (arrivals > 0 ? arrivals : active_chunks) - 1) ? 1 : 0;
     if (s_is_last) *counter = 0;
   }
   __syncthreads();
   if (!s_is_last) return;
-  __threadfence();
 
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -68,32 +69,75 @@ __device__ __forceinline__ void fused_combine_tail(const FusedCombine& fc, int b
     for (int c = lane; c < active_chunks; c += 32) smem_weights[g * kFusedMaxChunks + c] *= inv;
   }
   __syncthreads();
-  // four dims per thread and load: a thread of a 128-thread CTA has a quarter of the serial rounds of loads
-  const bool aligned = (reinterpret_cast<uintptr_t>(values) & 15u) == 0;
-  for (int item = threadIdx.x; aligned && item < g_count * (D / 4); item += THREADS) {
-    const int g = item / (D / 4);
-    const int d = 4 * (item % (D / 4));
-    const float* vals = values + (int64_t)g * chunk_capacity * D + d;
-    const float* w = smem_weights + g * kFusedMaxChunks;
-    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 4
-    for (int c = 0; c < active_chunks; ++c) {
-      const float4 v = __ldcg(reinterpret_cast<const float4*>(vals + (int64_t)c * D));
-      acc[0] = fmaf(v.x, w[c], acc[0]);
-      acc[1] = fmaf(v.y, w[c], acc[1]);
-      acc[2] = fmaf(v.z, w[c], acc[2]);
-      acc[3] = fmaf(v.w, w[c], acc[3]);
-    }
+  auto store = [&](int g, int d, const float4& o) {
+    const float acc[4] = {o.x, o.y, o.z, o.w};
     const T* gate = fc.gate == nullptr ? nullptr
                                        : reinterpret_cast<const T*>(fc.gate) + (int64_t)b * fc.gate_stride_b +
                                              (int64_t)(hq0 + g) * fc.gate_stride_h + d;
     const int64_t offset = (int64_t)b * fc.out_stride_b + (int64_t)(hq0 + g) * fc.out_stride_h + d;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      if (gate) acc[i] *= sigmoidf_fast(ElemTraits<T>::to_float(gate[i]));
-      const T result = ElemTraits<T>::from_float(acc[i]);
+      const T result = ElemTraits<T>::from_float(gate ? acc[i] * sigmoidf_fast(ElemTraits<T>::to_float(gate[i])) : acc[i]);
       reinterpret_cast<T*>(fc.out)[offset + i] = result;
       for (int peer = 0; peer < fc.num_peers; ++peer) reinterpret_cast<T*>(fc.peers[peer])[offset + i] = result;
+    }
+  };
+  // Four dims per thread and load.  What this part takes is the latency of its loads: a head group with more columns of four
+  // dims than the CTA has threads reads all of a thread's columns side by side, kInFlight loads at a time, instead of one
+  // column after the other (16 rows of 0.4-4 K packed tokens, 16/2 heads of 256: 37.1 -> 34.9 us; 64 rows of 4-32 K 170 ->
+  // 168.4).  With 16 loads in flight the even-share kernels lost more to spilled registers than the merge gained, and with one
+  // column per thread eight at a time are no faster than a plain loop (one packed row of 4000 tokens: 20.6 us and 18.5).
+  const bool aligned = (reinterpret_cast<uintptr_t>(values) & 15u) == 0;
+  constexpr int kCols = D / 4;
+  constexpr int kRounds = (8 * kCols + THREADS - 1) / THREADS;
+  constexpr int kInFlight = 8;
+  constexpr int kAtOnce = kInFlight / kRounds;  // partials
+  const int items = g_count * kCols;
+  auto add = [](float4& acc, const float4& v, float w) {
+    acc.x = fmaf(v.x, w, acc.x);
+    acc.y = fmaf(v.y, w, acc.y);
+    acc.z = fmaf(v.z, w, acc.z);
+    acc.w = fmaf(v.w, w, acc.w);
+  };
+  if (aligned && items > THREADS) {
+    float4 acc[kRounds];
+    const float* vals[kRounds];
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const int item = min((int)threadIdx.x + r * THREADS, items - 1);  // past the end: the last column again, not stored
+      acc[r] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      vals[r] = values + (int64_t)(item / kCols) * chunk_capacity * D + 4 * (item % kCols);
+    }
+    for (int c0 = 0; c0 < active_chunks; c0 += kAtOnce) {
+      float4 v[kAtOnce][kRounds];
+#pragma unroll
+      for (int k = 0; k < kAtOnce; ++k)
+#pragma unroll
+        for (int r = 0; r < kRounds; ++r)
+          v[k][r] = __ldcg(reinterpret_cast<const float4*>(vals[r] + (int64_t)min(c0 + k, active_chunks - 1) * D));
+#pragma unroll
+      for (int r = 0; r < kRounds; ++r) {
+        const float* w = smem_weights + min(((int)threadIdx.x + r * THREADS) / kCols, g_count - 1) * kFusedMaxChunks;
+#pragma unroll
+        for (int k = 0; k < kAtOnce; ++k)
+          if (c0 + k < active_chunks) add(acc[r], v[k][r], w[c0 + k]);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const int item = (int)threadIdx.x + r * THREADS;
+      if (item < items) store(item / kCols, 4 * (item % kCols), acc[r]);
+    }
+  } else if (aligned) {
+    if ((int)threadIdx.x < items) {
+      const int g = (int)threadIdx.x / kCols, d = 4 * ((int)threadIdx.x % kCols);
+      const float* vals = values + (int64_t)g * chunk_capacity * D + d;
+      const float* w = smem_weights + g * kFusedMaxChunks;
+      float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+      for (int c = 0; c < active_chunks; ++c)
+        add(acc, __ldcg(reinterpret_cast<const float4*>(vals + (int64_t)c * D)), w[c]);
+      store(g, d, acc);
     }
   }
   for (int item = threadIdx.x; !aligned && item < g_count * D; item += THREADS) {

@@ -57,7 +57,7 @@ dense_decode_balanced_mma_kernel(const DenseDecodeParams p, const int batch) {
   const int group_tiles = (p.groups + 7) / 8;
   const int streams_per_row = p.kv_heads * group_tiles;
   // the fused merge stages at most kFusedMaxChunks weights per head, however large the caller's scratch is
-  balanced_for_each_segment<kMmaThreads>(
+  balanced_for_each_segment<kMmaThreads, true>(
       p.visible_lengths, p.max_len, batch, streams_per_row, min(p.chunk_capacity, kFusedMaxChunks),
       [&](int b) {
         for (int stream = 0; stream < streams_per_row; ++stream) {

@@ -1136,7 +1136,7 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
   init_packed_barriers<T, D, BITS>(smem_raw);
   PackedRing ring{0, 0u, false};
   const TqQueryConsts qc = load_query_consts<D, BITS>(p);
-  balanced_for_each_segment<kMmaThreads>(
+  balanced_for_each_segment<kMmaThreads, false>(
       p.lengths, p.max_len, batch, units, min(p.chunk_capacity, kFusedMaxChunks) - p.num_window_chunks,
       [](int) {},  // rows without packed tokens belong to the window kernel
       [&](int b, int unit, int t0, int t1, int slot, int partials) {
