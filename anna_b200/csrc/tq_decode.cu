@@ -28,7 +28,19 @@ __device__ __forceinline__ uint32_t load_packed_bits(const uint8_t* __restrict__
   }
 }
 
-constexpr int kTqUnroll = 2;
+// Codes and metadata of one token as a lane loads them: everything of a round of tokens is on its way before the first of
+// it is used.
+template <typename T, int CH>
+struct TqTokenRaw {
+  float norm, rnorm;
+  uint32_t idx[CH], sign[CH], val[CH];
+  T scale[CH], zero[CH];
+};
+
+// Tokens a team scores together.  The kernel is a chain of loads (page id, then codes and metadata), so what counts for a
+// short context is how few rounds a chunk takes; wide groups and head slices have no registers for more than two.
+template <typename Cfg, int G>
+constexpr int kTqUnroll = G * Cfg::kDpl <= 16 ? 4 : 2;
 
 // kMerge: the CTA that finishes a (row, head group) last merges its partials (merges_in_split); a kernel of its own, as for
 // dense_decode_split_kernel.
@@ -84,25 +96,59 @@ __global__ void __launch_bounds__(kDecodeThreads) tq_decode_split_kernel(const T
 
   if (threadIdx.x < (1 << M)) sm_cent[threadIdx.x] = p.centroids[threadIdx.x];
 
+  // page ids of the packed tokens are looked up one round ahead, the first ones before the queries are rotated
+  constexpr int U = kTqUnroll<Cfg, G>;
+  constexpr int kStep = kDecodeWarps * Cfg::kTpw * U;
+  const int64_t q_end = min(t1, Lq);
+  const int32_t* table_row = p.block_table + (int64_t)b * p.table_stride;
+  int32_t pid[U];
+  auto block_of = [&](int64_t t) { return p.block_shift >= 0 ? t >> p.block_shift : t / p.block_size; };
+  auto look_up = [&](int64_t base) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t t = base + u * Cfg::kTpw + sub;
+      pid[u] = t < q_end ? table_row[block_of(t)] : -1;
+    }
+  };
+  const int64_t first = t0 + warp * (Cfg::kTpw * U);
+  look_up(first);
+
   // ---- rotate the group's queries: q_smem[0] = q, [1] = fwht(s1*q), [2] = fwht(s2*[1]) ---------------------------
+  // Queries and signs are all loaded before the first store to shared memory: loads that wait for the stores in front of them
+  // (which might alias them) made eight round trips to the L2 cache of this.
   float* q_smem = smem;  // [3][G][D]
   {
-    const T* q_ptr = reinterpret_cast<const T*>(p.q) + (int64_t)b * p.q_stride_b;
-    for (int g = warp; g < G; g += kDecodeWarps) {
+    constexpr int kHeads = (G + kDecodeWarps - 1) / kDecodeWarps;
+    const T* q_ptr = reinterpret_cast<const T*>(p.q) + (int64_t)b * p.q_stride_b + (int64_t)hq0 * p.q_stride_h + lane * E;
+    float s1[E], s2[E];
+    T raw[kHeads][E];
+#pragma unroll
+    for (int j = 0; j < E; ++j) {
+      s1[j] = __ldg(p.signs1 + lane * E + j);
+      s2[j] = __ldg(p.signs2 + lane * E + j);
+    }
+#pragma unroll
+    for (int i = 0; i < kHeads; ++i) {
+      const int g = warp + i * kDecodeWarps;
+#pragma unroll
+      for (int j = 0; j < E; ++j) raw[i][j] = g < g_count ? q_ptr[(int64_t)g * p.q_stride_h + j] : T(0.0f);
+    }
+#pragma unroll
+    for (int i = 0; i < kHeads; ++i) {
+      const int g = warp + i * kDecodeWarps;
+      if (g >= G) break;
       float w[E];
 #pragma unroll
       for (int j = 0; j < E; ++j) {
-        const int d = lane * E + j;
-        w[j] = g < g_count ? ElemTraits<T>::to_float(q_ptr[(int64_t)(hq0 + g) * p.q_stride_h + d]) : 0.0f;
-        q_smem[(0 * G + g) * D + d] = w[j];
-        if (p.signs1[d] < 0.0f) w[j] = -w[j];
+        w[j] = ElemTraits<T>::to_float(raw[i][j]);
+        q_smem[(0 * G + g) * D + lane * E + j] = w[j];
+        if (s1[j] < 0.0f) w[j] = -w[j];
       }
       warp_fwht<E>(w, lane);
 #pragma unroll
       for (int j = 0; j < E; ++j) {
-        const int d = lane * E + j;
-        q_smem[(1 * G + g) * D + d] = w[j];
-        if (p.signs2[d] < 0.0f) w[j] = -w[j];
+        q_smem[(1 * G + g) * D + lane * E + j] = w[j];
+        if (s2[j] < 0.0f) w[j] = -w[j];
       }
       warp_fwht<E>(w, lane);
 #pragma unroll
@@ -115,7 +161,6 @@ __global__ void __launch_bounds__(kDecodeThreads) tq_decode_split_kernel(const T
   st.reset();
 
   // ---- packed prefix ---------------------------------------------------------------------------------------------
-  const int64_t q_end = min(t1, Lq);
   if (t0 < q_end) {
     const float inv_dim = 1.0f / (float)D;
     const float kappa = 1.2533141373155001f * rsqrtf((float)D);  // sqrt(pi/2) / sqrt(D)
@@ -127,33 +172,19 @@ __global__ void __launch_bounds__(kDecodeThreads) tq_decode_split_kernel(const T
       for (int i = 0; i < Cfg::kDpl; ++i)
         q2[g][i] = q_smem[(2 * G + g) * D + lane_dim<Cfg>(dl, i)] * (p.scaling * inv_dim * kappa);
 
-    const int32_t* table_row = p.block_table + (int64_t)b * p.table_stride;
-    constexpr int kStep = kDecodeWarps * Cfg::kTpw * kTqUnroll;
-    for (int64_t base = t0 + warp * (Cfg::kTpw * kTqUnroll); base < q_end; base += kStep) {
-      float s[kTqUnroll][G];
-      float vhat[kTqUnroll][Cfg::kDpl];
-      bool valid[kTqUnroll];
+    for (int64_t base = first; base < q_end; base += kStep) {
+      bool valid[U];
+      TqTokenRaw<T, Cfg::kCh> raw[U];
 #pragma unroll
-      for (int u = 0; u < kTqUnroll; ++u) {
-        const int64_t t = base + u * Cfg::kTpw + sub;
-        valid[u] = false;
-        const uint8_t* chunk_ptr = nullptr;
-        int tok = 0;
-        if (t < q_end) {
-          const int32_t pid = table_row[t / p.block_size];
-          if (pid >= 0 && pid < p.num_pages) {
-            valid[u] = true;
-            tok = (int)(t % p.block_size);
-            chunk_ptr = p.pages + ((int64_t)pid * p.kv_heads + kvh) * p.layout.chunk_bytes;
-          }
-        }
-#pragma unroll
-        for (int g = 0; g < G; ++g) s[u][g] = 0.0f;
-#pragma unroll
-        for (int i = 0; i < Cfg::kDpl; ++i) vhat[u][i] = 0.0f;
+      for (int u = 0; u < U; ++u) {
+        valid[u] = pid[u] >= 0 && pid[u] < p.num_pages;
+        raw[u] = TqTokenRaw<T, Cfg::kCh>{};
         if (!valid[u]) continue;
-        const float norm = __ldg(reinterpret_cast<const float*>(chunk_ptr + p.layout.off_knorm) + tok);
-        const float rnorm = __ldg(reinterpret_cast<const float*>(chunk_ptr + p.layout.off_krnorm) + tok);
+        const int64_t t = base + u * Cfg::kTpw + sub;
+        const int tok = (int)(t - block_of(t) * p.block_size);
+        const uint8_t* chunk_ptr = p.pages + ((int64_t)pid[u] * p.kv_heads + kvh) * p.layout.chunk_bytes;
+        raw[u].norm = __ldg(reinterpret_cast<const float*>(chunk_ptr + p.layout.off_knorm) + tok);
+        raw[u].rnorm = __ldg(reinterpret_cast<const float*>(chunk_ptr + p.layout.off_krnorm) + tok);
         const uint8_t* krow = chunk_ptr + p.layout.off_kcodes + tok * p.layout.key_bytes;
         const uint8_t* vrow = chunk_ptr + p.layout.off_vdata + tok * p.layout.value_bytes;
         const T* scales = reinterpret_cast<const T*>(chunk_ptr + p.layout.off_vscale) + tok * p.layout.groups;
@@ -161,25 +192,37 @@ __global__ void __launch_bounds__(kDecodeThreads) tq_decode_split_kernel(const T
 #pragma unroll
         for (int c = 0; c < Cfg::kCh; ++c) {
           const int d0 = (c * Cfg::kLpt + dl) * kVec;
-          uint32_t idx_bits, sign_bits;  // per coordinate: M index bits, 1 sign bit
           if constexpr (BITS == 3) {
-            idx_bits = load_packed_bits<kVec, 2>(krow, d0);
-            sign_bits = load_packed_bits<kVec, 1>(krow + D / 4, d0);
+            raw[u].idx[c] = load_packed_bits<kVec, 2>(krow, d0);
+            raw[u].sign[c] = load_packed_bits<kVec, 1>(krow + D / 4, d0);
           } else {
-            idx_bits = load_packed_bits<kVec, BITS>(krow, d0);
-            sign_bits = 0;
+            raw[u].idx[c] = load_packed_bits<kVec, BITS>(krow, d0);
           }
+          raw[u].val[c] = load_packed_bits<kVec, VS>(vrow, d0);
+          const int grp = d0 / p.value_group;
+          raw[u].scale[c] = scales[grp];
+          raw[u].zero[c] = zeros[grp];
+        }
+      }
+      look_up(base + kStep);
+      float s[U][G];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+#pragma unroll
+        for (int g = 0; g < G; ++g) s[u][g] = 0.0f;
+#pragma unroll
+        for (int c = 0; c < Cfg::kCh; ++c) {
           float a[G], bsum[G];
 #pragma unroll
           for (int g = 0; g < G; ++g) { a[g] = 0.0f; bsum[g] = 0.0f; }
 #pragma unroll
           for (int i = 0; i < kVec; ++i) {
-            uint32_t code, sbit;
+            uint32_t code, sbit;  // M index bits, 1 sign bit
             if constexpr (BITS == 3) {
-              code = (idx_bits >> (2 * i)) & 3u;
-              sbit = (sign_bits >> i) & 1u;
+              code = (raw[u].idx[c] >> (2 * i)) & 3u;
+              sbit = (raw[u].sign[c] >> i) & 1u;
             } else {
-              const uint32_t field = (idx_bits >> (BITS * i)) & ((1u << BITS) - 1u);
+              const uint32_t field = (raw[u].idx[c] >> (BITS * i)) & ((1u << BITS) - 1u);
               code = field & ((1u << M) - 1u);
               sbit = field >> M;
             }
@@ -192,53 +235,53 @@ __global__ void __launch_bounds__(kDecodeThreads) tq_decode_split_kernel(const T
             }
           }
 #pragma unroll
-          for (int g = 0; g < G; ++g) s[u][g] += norm * fmaf(rnorm, bsum[g], a[g]);
-
-          const uint32_t vbits = load_packed_bits<kVec, VS>(vrow, d0);
-          const int grp = d0 / p.value_group;
-          const float sc = ElemTraits<T>::to_float(scales[grp]);
-          const float zp = ElemTraits<T>::to_float(zeros[grp]);
-#pragma unroll
-          for (int i = 0; i < kVec; ++i) {
-            const float code = (float)((vbits >> (VS * i)) & ((1u << VS) - 1u));
-            vhat[u][c * kVec + i] = fmaf(code, sc, zp);
-          }
+          for (int g = 0; g < G; ++g) s[u][g] += raw[u].norm * fmaf(raw[u].rnorm, bsum[g], a[g]);
         }
       }
 #pragma unroll
       for (int d = Cfg::kLpt / 2; d >= 1; d >>= 1) {
 #pragma unroll
-        for (int u = 0; u < kTqUnroll; ++u)
+        for (int u = 0; u < U; ++u)
 #pragma unroll
           for (int g = 0; g < G; ++g) s[u][g] += __shfl_xor_sync(0xffffffffu, s[u][g], d);
       }
+      float rescale[G];
 #pragma unroll
       for (int g = 0; g < G; ++g) {
         float m_new = st.m[g];
 #pragma unroll
-        for (int u = 0; u < kTqUnroll; ++u) {
+        for (int u = 0; u < U; ++u) {
           if (!valid[u]) s[u][g] = -INFINITY;
           m_new = fmaxf(m_new, s[u][g]);
         }
         const float m_safe = (m_new == -INFINITY) ? 0.0f : m_new;
-        const float rescale = __expf(st.m[g] - m_safe);
-        float lsum = st.l[g] * rescale;
-        float pr[kTqUnroll];
+        rescale[g] = __expf(st.m[g] - m_safe);
+        float lsum = st.l[g] * rescale[g];
 #pragma unroll
-        for (int u = 0; u < kTqUnroll; ++u) {
-          pr[u] = __expf(s[u][g] - m_safe);
-          lsum += pr[u];
+        for (int u = 0; u < U; ++u) {
+          s[u][g] = __expf(s[u][g] - m_safe);
+          lsum += s[u][g];
         }
         st.l[g] = lsum;
         st.m[g] = m_new;
-#pragma unroll
-        for (int i = 0; i < Cfg::kDpl; ++i) {
-          float acc = st.acc[g][i] * rescale;
-#pragma unroll
-          for (int u = 0; u < kTqUnroll; ++u) acc = fmaf(pr[u], vhat[u][i], acc);
-          st.acc[g][i] = acc;
-        }
       }
+#pragma unroll
+      for (int c = 0; c < Cfg::kCh; ++c)
+#pragma unroll
+        for (int i = 0; i < kVec; ++i) {
+          float v[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            v[u] = fmaf((float)((raw[u].val[c] >> (VS * i)) & ((1u << VS) - 1u)), ElemTraits<T>::to_float(raw[u].scale[c]),
+                        ElemTraits<T>::to_float(raw[u].zero[c]));
+#pragma unroll
+          for (int g = 0; g < G; ++g) {
+            float acc = st.acc[g][c * kVec + i] * rescale[g];
+#pragma unroll
+            for (int u = 0; u < U; ++u) acc = fmaf(s[u][g], v[u], acc);
+            st.acc[g][c * kVec + i] = acc;
+          }
+        }
     }
   }
 
