@@ -11,13 +11,14 @@ constexpr int kMmaWarps = 4;
 constexpr int kMmaThreads = kMmaWarps * 32;
 constexpr int kTileTokens = 16;
 
-template <int D>
+// STAGES: tiles per warp in the copy ring
+template <int D, int STAGES = 2>
 struct MmaCfg {
   static constexpr int kSteps = D / 16;                 // k-steps of Q.K and m-tiles of P.V
   static constexpr int kChunksPerRow = D / 8;           // 16-byte chunks per token row
   static constexpr int kRowBytes = D * 2;
   static constexpr int kTileBytes = kTileTokens * kRowBytes;
-  static constexpr int kStages = 2;
+  static constexpr int kStages = STAGES;
   static constexpr int kCopiesPerLane = kTileTokens * kChunksPerRow / 32;
   static constexpr int kRowsPerCopy = 32 / kChunksPerRow > 0 ? 32 / kChunksPerRow : 1;
   static constexpr int kWarpSmem = kStages * 2 * kTileBytes;
@@ -78,11 +79,11 @@ __device__ __forceinline__ void merge_parts_and_store(float* sm_m, const float* 
 // arrivals on counters[counter_index].
 // Token t lives at element offset: paged -> page_table / block_size; ring_len > 0 -> (t % ring_len) * D; else
 // t * kv_stride_t, all relative to the (row, kv head) base the caller put into p.key / p.value.
-template <typename T, int D>
+template <typename T, int D, int STAGES = 2>
 __device__ __forceinline__ void dense_split_mma_body(const DenseDecodeParams& p, uint8_t* smem_raw, int b, int kvh,
                                                      int g0, int g_count, int t0, int t1, int slot,
                                                      int active_chunks, int64_t counter_index) {
-  using Cfg = MmaCfg<D>;
+  using Cfg = MmaCfg<D, STAGES>;
   const int num_tiles = (t1 - t0 + kTileTokens - 1) / kTileTokens;
 
   const int warp = threadIdx.x >> 5;

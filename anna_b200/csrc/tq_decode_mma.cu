@@ -478,34 +478,35 @@ __device__ __forceinline__ void prepare_query_fragments(const TqDecodeParams& p,
   }
 }
 
-// Split pass over the un-quantized window ring of every row: the dense tensor-core body with ring addressing.
-// Grid (num_window_chunks, kv_heads * group tiles, batch).  Also writes the zero output of empty rows.
-template <typename T, int D>
-__global__ void __launch_bounds__(kMmaThreads, MmaCfg<D>::kMinBlocks) tq_window_split_mma_kernel(const TqDecodeParams p) {
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  // The packed-chunk kernel that follows in the stream reads nothing this kernel writes before the arrival counters
-  // say so, and each of its CTAs waits for this grid to complete before it counts itself in or exits, so it may start
-  // as soon as every CTA here has been scheduled.
-  asm volatile("griddepcontrol.launch_dependents;\n" ::);
-  const int slot = blockIdx.x;
+// Lengths of one row: keys, quantized ones among them, and the chunks of the fixed-chunk division that hold any.
+struct RowChunks {
+  int len, quantized, window, packed;
+};
+__device__ __forceinline__ RowChunks row_chunks(const TqDecodeParams& p, int b) {
+  RowChunks r;
+  r.len = (int)max((int64_t)0, min(p.lengths[b], p.max_len));
+  r.quantized = r.len > p.residual_len ? r.len - p.residual_len : 0;
+  r.window = (r.len - r.quantized + p.chunk_tokens - 1) / p.chunk_tokens;
+  r.packed = (r.quantized + p.chunk_tokens - 1) / p.chunk_tokens;
+  return r;
+}
+
+// Chunk `slot` of the un-quantized window ring of a row: the dense tensor-core body with ring addressing.  Also writes the
+// zero output of empty rows.  `arrives`: the chunk counts on the merge counter, as one of all active chunks.
+template <typename T, int D, int STAGES>
+__device__ __forceinline__ void tq_window_chunk(const TqDecodeParams& p, uint8_t* smem_raw, const RowChunks& row, int b,
+                                                int unit, int units, int slot, bool arrives) {
   const int group_tiles = (p.groups + 7) / 8;
-  const int kvh = blockIdx.y / group_tiles;
-  const int g0 = (blockIdx.y % group_tiles) * 8;
+  const int kvh = unit / group_tiles;
+  const int g0 = (unit % group_tiles) * 8;
   const int g_count = min(8, p.groups - g0);
-  const int b = blockIdx.z;
-  const int hq0 = kvh * p.groups + g0;
-  int64_t len64 = p.lengths[b];
-  len64 = max((int64_t)0, min(len64, p.max_len));
-  const int len = (int)len64;
-  const int R = p.residual_len;
-  const int Lq = len > R ? len - R : 0;
-  const int active_window = (len - Lq + p.chunk_tokens - 1) / p.chunk_tokens;
-  const int active_chunks = active_window + (Lq + p.chunk_tokens - 1) / p.chunk_tokens;
-  if (len == 0) {
-    if (p.fused.counters != nullptr && slot == 0) fused_write_zero_row<T, D, kMmaThreads>(p.fused, b, hq0, g_count);
+  if (row.len == 0) {
+    if (p.fused.counters != nullptr && slot == 0)
+      fused_write_zero_row<T, D, kMmaThreads>(p.fused, b, kvh * p.groups + g0, g_count);
     return;
   }
-  if (slot >= active_window) return;
+  if (slot >= row.window) return;
+  const int R = p.residual_len;
   DenseDecodeParams dp{};
   dp.q = p.q; dp.q_stride_b = p.q_stride_b; dp.q_stride_h = p.q_stride_h;
   const int64_t ring_elems = (int64_t)R * D;
@@ -521,11 +522,25 @@ __global__ void __launch_bounds__(kMmaThreads, MmaCfg<D>::kMinBlocks) tq_window_
   dp.chunk_tokens = p.chunk_tokens; dp.num_chunks = p.num_chunks; dp.chunk_capacity = p.chunk_capacity;
   dp.scaling = p.scaling;
   dp.fused = p.fused;
-  if (!p.window_arrives && Lq > 0) dp.fused.counters = nullptr;  // the packed CTAs wait for this grid before they count
-  const int t0 = Lq + slot * p.chunk_tokens;
-  const int t1 = min(len, t0 + p.chunk_tokens);
-  dense_split_mma_body<T, D>(dp, smem_raw, b, kvh, g0, g_count, t0, t1, slot, active_chunks,
-                             (int64_t)b * gridDim.y + blockIdx.y);
+  if (!arrives) dp.fused.counters = nullptr;
+  const int t0 = row.quantized + slot * p.chunk_tokens;
+  const int t1 = min(row.len, t0 + p.chunk_tokens);
+  dense_split_mma_body<T, D, STAGES>(dp, smem_raw, b, kvh, g0, g_count, t0, t1, slot, row.window + row.packed,
+                                     (int64_t)b * units + unit);
+}
+
+// Window chunks of every row, grid (num_window_chunks, kv_heads * group tiles, batch).
+template <typename T, int D>
+__global__ void __launch_bounds__(kMmaThreads, MmaCfg<D>::kMinBlocks) tq_window_split_mma_kernel(const TqDecodeParams p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  // The packed-chunk kernel that follows in the stream reads nothing this kernel writes before the arrival counters
+  // say so, and each of its CTAs waits for this grid to complete before it counts itself in or exits, so it may start
+  // as soon as every CTA here has been scheduled.
+  asm volatile("griddepcontrol.launch_dependents;\n" ::);
+  const RowChunks row = row_chunks(p, blockIdx.z);
+  // the packed CTAs wait for this grid before they count
+  tq_window_chunk<T, D, 2>(p, smem_raw, row, blockIdx.z, blockIdx.y, gridDim.y, blockIdx.x,
+                           p.window_arrives || row.quantized == 0);
 }
 
 // Copy ring of one warp of a packed-prefix CTA; it runs on from one segment to the next.
@@ -1101,15 +1116,9 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
     tq_decode_split_mma_kernel(const TqDecodeParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int b = blockIdx.z;
-  int64_t len64 = p.lengths[b];
-  len64 = max((int64_t)0, min(len64, p.max_len));
-  const int len = (int)len64;
-  const int R = p.residual_len;
-  const int Lq = len > R ? len - R : 0;
-  const int active_window = (len - Lq + p.chunk_tokens - 1) / p.chunk_tokens;
-  const int active_packed = (Lq + p.chunk_tokens - 1) / p.chunk_tokens;
+  const RowChunks row = row_chunks(p, b);
   const int chunk = (int)blockIdx.x - p.num_window_chunks;  // window chunks run in tq_window_split_mma_kernel
-  if (chunk < 0 || chunk >= active_packed) {
+  if (chunk < 0 || chunk >= row.packed) {
     wait_for_prior_grids();
     return;
   }
@@ -1118,8 +1127,44 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
   PackedRing ring{0, 0u, false};
   const TqQueryConsts qc = load_query_consts<D, BITS>(p);
   // active slots stay contiguous: [window | packed]
-  tq_packed_segment<T, D, BITS, kPair>(p, smem_raw, qc, ring, b, (int)blockIdx.y, (int)gridDim.y, t0, min(Lq, t0 + p.chunk_tokens),
-                                active_window + chunk, active_window + active_packed, active_packed);
+  tq_packed_segment<T, D, BITS, kPair>(p, smem_raw, qc, ring, b, (int)blockIdx.y, (int)gridDim.y, t0,
+                                       min(row.quantized, t0 + p.chunk_tokens), row.window + chunk, row.window + row.packed,
+                                       row.packed);
+}
+
+// Small calls: window chunks and packed chunks in one launch, grid (window chunks + packed chunks, units, batch), all of it
+// resident at once; every chunk counts on the merge counter.  The second launch of the other kernels costs the host about
+// as much as the rest of such a call.  With few CTAs there are registers and shared memory to spare, but a window CTA has to
+// live with what a packed one has: its ring holds one tile per warp.
+template <typename T, int D, int BITS>
+struct TqSmallCfg {
+  static constexpr int kMinBlocks = D >= 256 ? 2 : 3;
+  static constexpr int kWindowSmem = MmaCfg<D, 1>::kSmemBytes;
+  static constexpr int kPackedSmem = TqMmaCfg<T, D, BITS>::kSmemBytes;
+  static constexpr int kSmemBytes = kWindowSmem > kPackedSmem ? kWindowSmem : kPackedSmem;
+  // the merge stages its weights in the window CTAs' shared memory, too
+  static_assert(kWindowSmem >= 8 * kFusedMaxChunks * 4, "no room for the weights of the merge");
+};
+
+template <typename T, int D, int BITS, bool kPair>
+__global__ void __launch_bounds__(kMmaThreads, TqSmallCfg<T, D, BITS>::kMinBlocks)
+    tq_decode_small_mma_kernel(const TqDecodeParams p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const int b = blockIdx.z;
+  const RowChunks row = row_chunks(p, b);
+  if ((int)blockIdx.x < p.num_window_chunks) {
+    tq_window_chunk<T, D, 1>(p, smem_raw, row, b, blockIdx.y, gridDim.y, blockIdx.x, true);
+    return;
+  }
+  const int chunk = (int)blockIdx.x - p.num_window_chunks;
+  if (chunk >= row.packed) return;
+  const int t0 = chunk * p.chunk_tokens;
+  init_packed_barriers<T, D, BITS>(smem_raw);
+  PackedRing ring{0, 0u, false};
+  const TqQueryConsts qc = load_query_consts<D, BITS>(p);
+  const int active = row.window + row.packed;
+  tq_packed_segment<T, D, BITS, kPair>(p, smem_raw, qc, ring, b, (int)blockIdx.y, (int)gridDim.y, t0,
+                                       min(row.quantized, t0 + p.chunk_tokens), row.window + chunk, active, active);
 }
 
 // What a segment costs beyond its tiles (query preparation, first copy, merge: about 6 us), in tiles.  Over 512 shapes (1 to
@@ -1148,15 +1193,30 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
   wait_for_prior_grids();
 }
 
-// Which schedule the packed prefix takes; `ctas` = CTAs of the even-share kernel that are resident at once.
-static bool tq_use_balanced(const TqDecodeParams& p, int batch, int head_dim, int ctas) {
+static bool tq_fixed_chunks_only() {
   static const bool disabled = [] {
     const char* flag = std::getenv("ANNA_B200_DISABLE_BALANCED");
     return flag != nullptr && flag[0] != '\0' && flag[0] != '0';
   }();
+  return disabled;
+}
+
+// A small call, whose chunks are resident at once, gains nothing from even shares and pays for the scan of the lengths (one
+// row of 260-2500 tokens, 8 heads, 3 bits: 16.4-18.5 us in shares, 12.3-14.5 in chunks; 4 rows of 500, 32/8 heads, 4 bits: 16.5
+// and 12.4), unless it waits for the last CTA's merge: even shares have half as many partials (one row of 6000 tokens, 16/2
+// heads of 256, 2 bits: 92 partials in four rounds 46 us, shares 34).  `resident` = CTAs that fit the GPU at once.
+static bool tq_small(const TqDecodeParams& p, int batch, int head_dim, int64_t ctas, int resident) {
+  const int64_t chunks = p.num_chunks - p.num_window_chunks;
+  const int rounds = (min(8, p.groups) * (head_dim / 4) + kMmaThreads - 1) / kMmaThreads;
+  return ctas <= resident && chunks * rounds <= (rounds == 1 ? 40 : 24);
+}
+
+// Which schedule the packed prefix of a call that is not small takes; `ctas` = CTAs of the even-share kernel that are
+// resident at once.
+static bool tq_use_balanced(const TqDecodeParams& p, int batch, int head_dim, int ctas) {
   const int64_t units = (int64_t)p.kv_heads * ((p.groups + 7) / 8);
   const int packed_slots = min(p.chunk_capacity, kFusedMaxChunks) - p.num_window_chunks;
-  if (disabled || p.given_chunks || p.fused.counters == nullptr) return false;
+  if (tq_fixed_chunks_only() || p.given_chunks || p.fused.counters == nullptr) return false;
   if (!balanced_schedule_fits(batch, units, p.max_len, packed_slots, kTqSegmentTiles)) return false;
   // The plan's longest chunks mean that there are enough of them for a few waves, which the block scheduler hands out as SMs
   // get free (64 rows of 32 K tokens, 32/8 heads: 594 us, even shares 613; 600 rows of 0.75-6 K, 48/4 heads: 697 and 742;
@@ -1164,15 +1224,22 @@ static bool tq_use_balanced(const TqDecodeParams& p, int batch, int head_dim, in
   // With less work the chunks shrink, down to 64 tokens, and every CTA's fixed cost and the number of partials grow (16 rows
   // of 0.4-4 K tokens, 16/2 heads of 256: 70 us, even shares 36; 64 rows of 4-32 K: 196 and 169).
   if (p.chunk_tokens >= kTqLongestChunk) return false;
-  // A small call, whose chunks are resident at once with room to spare, gains nothing from shares and pays for the scan of
-  // the lengths (one row of 260-2500 tokens, 8 heads, 3 bits: 16.4-18.5 us in shares, 12.3-14.5 in chunks; 4 rows of 500,
-  // 32/8 heads, 4 bits: 16.5 and 12.4), unless it waits for the last CTA's merge, which takes the partials of a head group
-  // in rounds of 128 x 4 dims: even shares have half as many partials (one row of 6000 tokens, 16/2 heads of 256, 2 bits:
-  // 92 partials in four rounds 46 us, shares 34).
-  const int64_t chunks = p.num_chunks - p.num_window_chunks;
-  const int rounds = (min(8, p.groups) * (head_dim / 4) + kMmaThreads - 1) / kMmaThreads;
-  const bool small = batch * units * chunks * 5 <= (int64_t)ctas * 4 && chunks * rounds <= (rounds == 1 ? 40 : 24);
-  return !small;
+  return !tq_small(p, batch, head_dim, batch * units * (p.num_chunks - p.num_window_chunks) * 5, ctas * 4);
+}
+
+// CTAs of a kernel that fit the whole GPU at once, worked out at its first launch on a device, which also lets it have `smem`
+// bytes of shared memory.
+template <typename Kernel>
+static int resident_ctas(Kernel kernel, int smem, int (&known)[64], int device, int* ctas) {
+  *ctas = (device >= 0 && device < 64) ? known[device] : 0;
+  if (*ctas != 0) return ANNA_OK;
+  ANNA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  int sms = 0, per_sm = 0;
+  ANNA_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  ANNA_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kMmaThreads, smem));
+  *ctas = sms * (per_sm > 0 ? per_sm : 1);
+  if (device >= 0 && device < 64) known[device] = *ctas;
+  return ANNA_OK;
 }
 
 template <typename T, int D, int BITS, bool kPair>
@@ -1196,9 +1263,23 @@ static int launch_tq_mma(const TqDecodeParams& p, int batch, cudaStream_t stream
        p.layout.chunk_bytes < Cfg::kTileDataBytes))
     return set_error(ANNA_ERR_INVALID, "packed page layout does not match the decode kernel's tile layout");
   const int group_tiles = (p.groups + 7) / 8;
+  if (!tq_fixed_chunks_only() && !p.given_chunks && p.fused.counters != nullptr && batch <= 65535) {
+    using Small = TqSmallCfg<T, D, BITS>;
+    static int small_resident[64] = {};
+    auto small = tq_decode_small_mma_kernel<T, D, BITS, kPair>;
+    int ctas = 0;
+    const int rc = resident_ctas(small, Small::kSmemBytes, small_resident, device, &ctas);
+    if (rc != ANNA_OK) return rc;
+    const int64_t units = (int64_t)p.kv_heads * group_tiles;
+    if (tq_small(p, batch, D, batch * units * p.num_chunks, ctas)) {
+      const dim3 grid((unsigned)p.num_chunks, (unsigned)units, (unsigned)batch);
+      small<<<grid, kMmaThreads, Small::kSmemBytes, stream>>>(p);
+      return check_launch("tq_decode_small_mma_kernel");
+    }
+  }
   dim3 window_grid((unsigned)p.num_window_chunks, (unsigned)(p.kv_heads * group_tiles), (unsigned)batch);
   tq_window_split_mma_kernel<T, D><<<window_grid, kMmaThreads, MmaCfg<D>::kSmemBytes, stream>>>(p);
-  const int rc = check_launch("tq_window_split_mma_kernel");
+  int rc = check_launch("tq_window_split_mma_kernel");
   if (rc != ANNA_OK) return rc;
   if (p.num_chunks <= p.num_window_chunks) return rc;
   // programmatic dependent launch: the packed chunks run beside the (small) window launch instead of after it
@@ -1211,17 +1292,11 @@ static int launch_tq_mma(const TqDecodeParams& p, int batch, cudaStream_t stream
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attr;
   config.numAttrs = 1;
-  static int resident[64] = {};  // per device: CTAs of the even-share kernel that fit the whole GPU at once
+  static int balanced_resident[64] = {};
   auto balanced = tq_decode_balanced_mma_kernel<T, D, BITS, kPair>;
-  int ctas = (device >= 0 && device < 64) ? resident[device] : 0;
-  if (ctas == 0) {
-    ANNA_CUDA_CHECK(cudaFuncSetAttribute(balanced, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
-    int sms = 0, per_sm = 0;
-    ANNA_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    ANNA_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, balanced, kMmaThreads, Cfg::kSmemBytes));
-    ctas = sms * (per_sm > 0 ? per_sm : 1);
-    if (device >= 0 && device < 64) resident[device] = ctas;
-  }
+  int ctas = 0;
+  rc = resident_ctas(balanced, Cfg::kSmemBytes, balanced_resident, device, &ctas);
+  if (rc != ANNA_OK) return rc;
   if (tq_use_balanced(p, batch, D, ctas)) {
     config.gridDim = dim3((unsigned)ctas);
     ANNA_CUDA_CHECK(cudaLaunchKernelEx(&config, balanced, p, batch));
