@@ -1219,11 +1219,15 @@ static bool tq_use_balanced(const TqDecodeParams& p, int batch, int head_dim, in
   if (tq_fixed_chunks_only() || p.given_chunks || p.fused.counters == nullptr) return false;
   if (!balanced_schedule_fits(batch, units, p.max_len, packed_slots, kTqSegmentTiles)) return false;
   // The plan's longest chunks mean that there are enough of them for a few waves, which the block scheduler hands out as SMs
-  // get free (64 rows of 32 K tokens, 32/8 heads: 594 us, even shares 613; 600 rows of 0.75-6 K, 48/4 heads: 697 and 742;
-  // but 128 rows of 0.5-16 K, 16/4 heads, for which shares became better when the line began to count segments: 226 and 214).
+  // get free.  With six waves or more (counted by the longest row) that is better than even shares (64 rows of 32 K tokens,
+  // 32/8 heads, 6.9 waves: 590 us, shares 611; 600 rows of 0.75-6 K, 48/4 heads, 16 waves: 697 and 742), with fewer the last
+  // one is too empty or too ragged (128 rows of 0.5-16 K, 16/4 heads, 3.5 waves: 227.5 and 217.4; 40 rows of 2-16 K, 32/8
+  // heads: 157 and 136, of 16 K 219 and 205; 64 rows of 8-24 K, 5.2 waves: 323 and 317) -- but not of rows of no more than two
+  // chunks, where even lengths leave nothing to share (128 rows of 8 K, 3.5 waves: 323 and 337; of 1-8 K 226 and 222).
   // With less work the chunks shrink, down to 64 tokens, and every CTA's fixed cost and the number of partials grow (16 rows
   // of 0.4-4 K tokens, 16/2 heads of 256: 70 us, even shares 36; 64 rows of 4-32 K: 196 and 169).
-  if (p.chunk_tokens >= kTqLongestChunk) return false;
+  const int64_t longest = p.num_chunks - p.num_window_chunks;
+  if (p.chunk_tokens >= kTqLongestChunk && (longest <= 2 || batch * units * longest >= (int64_t)6 * ctas)) return false;
   return !tq_small(p, batch, head_dim, batch * units * (p.num_chunks - p.num_window_chunks) * 5, ctas * 4);
 }
 
