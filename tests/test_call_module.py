@@ -1,0 +1,143 @@
+"""The call module (csrc/launch_module.cpp): what it declines, and that the calls it takes give what the general path gives."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from anna_b200 import KVCacheConfig, Qwen3DynamicCache, _lib, attention, fused_ops, turboquant
+
+
+class Declining:
+    """The module with its calls declined, so that the general path runs."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+def general(monkeypatch):
+    monkeypatch.setattr(fused_ops, "_LAUNCH", Declining())
+    for module in (attention, turboquant):
+        monkeypatch.setattr(module, "launch_module", Declining)
+
+
+def test_cpu_tensors_and_other_objects_are_declined():
+    module = _lib.launch()
+    x = torch.zeros(1, 2, 1, 64)
+    pages, table, one = torch.zeros(1, 2, 16, 64), torch.zeros(1, 1, dtype=torch.int32), torch.ones(1, dtype=torch.long)
+    assert module.paged_decode(x, pages, pages, table, one, 1.0, None) is None
+    assert module.paged_decode(x, pages, pages, table, [1], 1.0, None) is None
+    assert module.prefill(x, pages, pages, None, 1.0, True) is None
+    assert module.prefill("q", pages, pages, None, 1.0, True) is None
+    window = torch.zeros(1, 2, 2, 8, 64)
+    assert module.tq_decode(x, None, None, None, window, one, one, x, x, x, 1.0, 2, 16, 8, 4, 32, 0) is None
+    assert module.tq_append(x, x, None, None, window, one, one, None, x, x, x, x, None, 16, 8, 4, 32, 0) is None
+    with pytest.raises(TypeError):
+        module.tq_decode(x)
+    with pytest.raises(TypeError):
+        module.paged_decode(x, pages, pages, table, one, "scale", None)
+
+
+def strided(shape, dtype, device, gen, order):
+    """A tensor of `shape` whose dims lie in memory in `order` (outermost first)."""
+    x = torch.randn([shape[d] for d in order], generator=gen, device=device).to(dtype)
+    return x.permute([order.index(d) for d in range(len(shape))])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("gate", [None, "4d", "4d_strided", "3d", "3d_strided"])
+def test_paged_decode_equals_general_path(cuda_device, dtype, gate):
+    gen = torch.Generator(device=cuda_device).manual_seed(1)
+    batch, heads, kv_heads, dim, page = 3, 8, 2, 128, 16
+    for order in ((0, 1, 2, 3), (1, 0, 2, 3), (2, 0, 1, 3), (0, 1, 3, 2), (3, 0, 1, 2)):
+        query = strided((batch, heads, 1, dim), dtype, cuda_device, gen, order)
+        keys, values = (torch.randn(40, kv_heads, page, dim, generator=gen, device=cuda_device).to(dtype) for _ in range(2))
+        table = torch.randperm(36, generator=gen, device=cuda_device).to(torch.int32).view(3, 12)
+        lengths = torch.tensor([5, 170, 100], device=cuda_device)
+        g = None
+        if gate is not None:
+            g = strided((batch, heads, 1, dim), dtype, cuda_device, gen, order if "strided" in gate else (0, 1, 2, 3))
+            if gate.startswith("3d"):
+                g = strided((batch, 1, heads * dim), dtype, cuda_device, gen, (2, 1, 0) if "strided" in gate else (0, 1, 2))
+        for tab, visible in ((table, lengths), (table.t().contiguous().t(), lengths.repeat_interleave(2)[::2]),
+                             (table[:, :11], lengths)):
+            args = dict(query=query, key_pages=keys, value_pages=values, page_table=tab, visible_lengths=visible,
+                        scaling=0.1, gate=g)
+            out = fused_ops.run_paged_gqa_decode_fused(**args)
+            with pytest.MonkeyPatch.context() as patch:
+                general(patch)
+                assert torch.equal(out, fused_ops.run_paged_gqa_decode_fused(**args))
+            assert out.is_contiguous() and out.shape == query.shape and out.dtype == dtype
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim,query_len,key_len", [(64, 70, 200), (128, 5, 133), (256, 96, 96)])
+def test_prefill_equals_general_path(cuda_device, dim, query_len, key_len):
+    gen = torch.Generator(device=cuda_device).manual_seed(2)
+    for order in ((0, 1, 2, 3), (0, 2, 1, 3), (2, 0, 1, 3), (0, 1, 3, 2)):
+        query = strided((2, 4, query_len, dim), torch.bfloat16, cuda_device, gen, order)
+        keys = strided((2, 2, key_len, dim), torch.bfloat16, cuda_device, gen, order)
+        for values in (strided((2, 2, key_len, dim), torch.bfloat16, cuda_device, gen, order),
+                       strided((2, 2, key_len, dim), torch.bfloat16, cuda_device, gen, (1, 0, 2, 3))):
+            for lengths in (None, torch.tensor([key_len, key_len - 3], device=cuda_device)):
+                for causal in (None, True):
+                    args = dict(scaling=0.1, key_lengths=lengths, causal=causal)
+                    out = attention.grouped_query_attention(query, keys, values, **args)
+                    with pytest.MonkeyPatch.context() as patch:
+                        general(patch)
+                        assert torch.equal(out, attention.grouped_query_attention(query, keys, values, **args))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,dim", [(torch.bfloat16, 128), (torch.float16, 64), (torch.float32, 128)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_cache_steps_equal_general_path(cuda_device, dtype, dim, gated):
+    """Prompt and decode steps over pages that run out, on two streams, with every layout of queries, keys and values."""
+
+    def steps():
+        gen = torch.Generator(device=cuda_device).manual_seed(3)
+        cache = Qwen3DynamicCache(KVCacheConfig(num_hidden_layers=1, cache_block_size=16), batch_size=3,
+                                  kv_cache_quantization="turboquant", kv_cache_quant_bits=3, kv_cache_residual_len=16)
+        outputs = []
+        for i, tokens in enumerate((40, 1, 1, 17, 1, 1, 1, 1)):
+            # (the append rejects token strides that break 16-byte alignment, as those of a transposed single token do)
+            order = ((0, 1, 2, 3), (0, 2, 1, 3), (2, 0, 1, 3), (0, 1, 3, 2) if tokens > 1 else (1, 0, 2, 3))[i % 4]
+            k = strided((3, 2, tokens, dim), dtype, cuda_device, gen, order)
+            v = strided((3, 2, tokens, dim), dtype, cuda_device, gen, order if i % 3 else (0, 1, 2, 3))
+            cache.update(k, v, 0, require_dense_cache=False)
+            q = strided((3, 6, 1, dim), dtype, cuda_device, gen, order)
+            gate = strided((3, 6, 1, dim), dtype, cuda_device, gen, order) if gated else None
+            stream = torch.cuda.Stream(cuda_device) if i == 5 else torch.cuda.current_stream(cuda_device)
+            stream.wait_stream(torch.cuda.current_stream(cuda_device))
+            with torch.cuda.stream(stream):
+                outputs.append(cache.turboquant_single_token_decode_attention(0, q, scaling=0.1, num_key_value_groups=3,
+                                                                              gate=gate))
+            torch.cuda.current_stream(cuda_device).wait_stream(stream)
+        return [*outputs, *cache._gather_layer_cache(0)[:2]]
+
+    ours = steps()
+    with pytest.MonkeyPatch.context() as patch:
+        general(patch)
+        theirs = steps()
+    assert all(torch.equal(a, b) for a, b in zip(ours, theirs, strict=True))
+
+
+@pytest.mark.gpu
+def test_scratch_follows_its_buffers(cuda_device):
+    """A problem that needs larger scratch replaces the buffers; the one before must not go on with the old ones."""
+
+    def call(length):
+        gen = torch.Generator(device=cuda_device).manual_seed(length)
+        blocks = (length + 15) // 16
+        query = torch.randn(1, 8, 1, 128, generator=gen, device=cuda_device, dtype=torch.float16)
+        keys, values = (torch.randn(blocks, 8, 16, 128, generator=gen, device=cuda_device, dtype=torch.float16)
+                        for _ in range(2))
+        table = torch.arange(blocks, dtype=torch.int32, device=cuda_device)[None]
+        return fused_ops.run_paged_gqa_decode_fused(query=query, key_pages=keys, value_pages=values, page_table=table,
+                                                    visible_lengths=torch.tensor([length], device=cuda_device), scaling=0.1)
+
+    before = call(300)
+    scratch = fused_ops._SCRATCH
+    scratch.get(torch.device(cuda_device), 2 * max(buf.numel() for buf in scratch._buffers.values()) + 1)
+    assert not fused_ops._SPLIT_CACHE
+    assert torch.equal(call(300), before)

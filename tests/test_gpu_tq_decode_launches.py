@@ -1,0 +1,45 @@
+"""GPU: packed decode where the choice of its launches turns: one launch for window and packed chunks while all of them are
+resident at once, two beyond that; even shares of long streams of three chunks or more, chunks of shorter ones."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from tests.test_gpu_tq_decode_schedules import WINDOW, assert_close, dense_attention, ragged_cache
+
+pytestmark = pytest.mark.gpu
+
+
+def check(device, lengths, *, heads, kv_heads, dim, bits, page=16, dtype=torch.bfloat16, gated=False):
+    cache, gen = ragged_cache(device, lengths, kv_heads=kv_heads, dim=dim, bits=bits, page=page, dtype=dtype)
+    shape = (len(lengths), heads, 1, dim)
+    query = torch.randn(shape, generator=gen, device=device).to(dtype)
+    gate = torch.randn(shape, generator=gen, device=device).to(dtype) if gated else None
+    out = cache.turboquant_single_token_decode_attention(0, query, scaling=dim ** -0.5, num_key_value_groups=heads // kv_heads,
+                                                         gate=gate)
+    again = cache.turboquant_single_token_decode_attention(0, query, scaling=dim ** -0.5,
+                                                           num_key_value_groups=heads // kv_heads, gate=gate)
+    assert torch.equal(out, again)  # the counters of the merge are zero again
+    assert_close(out, dense_attention(cache, query, lengths, dim ** -0.5, gate), dtype)
+
+
+@pytest.mark.parametrize("bits", [2, 3, 4])
+@pytest.mark.parametrize("dim", [128, 256])
+@pytest.mark.parametrize("group", [1, 4, 8, 11])
+def test_window_and_packed_chunks_in_one_launch(cuda_device, bits, dim, group):
+    for lengths in ([1], [WINDOW], [WINDOW + 1], [WINDOW + 64], [WINDOW + 65, 3, WINDOW, 700], [900, 40, 1, 333, 95]):
+        check(cuda_device, lengths, heads=2 * group, kv_heads=2, dim=dim, bits=bits, page=32 if len(lengths) > 1 else 16,
+              dtype=torch.float16 if group == 4 else torch.bfloat16, gated=group == 8)
+
+
+@pytest.mark.parametrize("rows", [18, 27, 28, 40])
+def test_around_what_is_resident_at_once(cuda_device, rows):
+    """8 KV heads, one window chunk and up to two packed ones: 444 CTAs of the single launch are resident."""
+    check(cuda_device, [WINDOW + 1 + (37 * i) % 128 for i in range(rows)], heads=8, kv_heads=8, dim=128, bits=4)
+
+
+@pytest.mark.parametrize("longest", [8100, 9100])
+def test_long_streams_of_two_and_of_three_chunks(cuda_device, longest):
+    rows = 75 if longest < 8192 else 50
+    check(cuda_device, [longest if i % 7 == 0 else 200 + (911 * i) % longest for i in range(rows)], heads=8, kv_heads=8,
+          dim=128, bits=3)
