@@ -1193,6 +1193,12 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
   wait_for_prior_grids();
 }
 
+// A call that is not small in the plan's chunks may be so in longer ones, up to this many tokens.  128 tokens are one step of a
+// CTA's warps, of which 64 leave half idle; 256 are two, which still costs less than the scan and the second launch of even
+// shares (one row of 4000 tokens, 32/8 heads, 4 bits: 18.5 us in shares, 14.3 so; of 8000 22.5 and 15.4; 4 rows of 1500, 8
+// heads, 3 bits 18.5 and 12.5; 6 rows of 0.3-1.5 K, 8/4 heads of 256 20.0 and 14.4).
+constexpr int kTqSmallChunk = 256;
+
 static bool tq_fixed_chunks_only() {
   static const bool disabled = [] {
     const char* flag = std::getenv("ANNA_B200_DISABLE_BALANCED");
@@ -1275,9 +1281,14 @@ static int launch_tq_mma(const TqDecodeParams& p, int batch, cudaStream_t stream
     const int rc = resident_ctas(small, Small::kSmemBytes, small_resident, device, &ctas);
     if (rc != ANNA_OK) return rc;
     const int64_t units = (int64_t)p.kv_heads * group_tiles;
-    if (tq_small(p, batch, D, batch * units * p.num_chunks, ctas)) {
-      const dim3 grid((unsigned)p.num_chunks, (unsigned)units, (unsigned)batch);
-      small<<<grid, kMmaThreads, Small::kSmemBytes, stream>>>(p);
+    TqDecodeParams sp = p;
+    for (int tokens = p.chunk_tokens; tokens <= max(p.chunk_tokens, kTqSmallChunk); tokens *= 2) {
+      sp.chunk_tokens = tokens;
+      sp.num_window_chunks = (p.residual_len + tokens - 1) / tokens;
+      sp.num_chunks = sp.num_window_chunks + (int)((p.max_len - p.residual_len + tokens - 1) / tokens);
+      if (!tq_small(sp, batch, D, batch * units * sp.num_chunks, ctas)) continue;
+      const dim3 grid((unsigned)sp.num_chunks, (unsigned)units, (unsigned)batch);
+      small<<<grid, kMmaThreads, Small::kSmemBytes, stream>>>(sp);
       return check_launch("tq_decode_small_mma_kernel");
     }
   }
