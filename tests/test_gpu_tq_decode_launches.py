@@ -43,3 +43,11 @@ def test_long_streams_of_two_and_of_three_chunks(cuda_device, longest):
     rows = 75 if longest < 8192 else 50
     check(cuda_device, [longest if i % 7 == 0 else 200 + (911 * i) % longest for i in range(rows)], heads=8, kv_heads=8,
           dim=128, bits=3)
+
+
+@pytest.mark.parametrize("lengths", [[WINDOW + 3520], [WINDOW + 3521], [WINDOW + 128 * 55 + 1], [8100], [1500, 1377, 40, 1501],
+                                     [2500, 200, 1100, 1999, 640, 2048, 311, 900]])
+@pytest.mark.parametrize("dim,bits", [(128, 3), (256, 4)])
+def test_longer_chunks_in_one_launch(cuda_device, lengths, dim, bits):
+    """Chunks of 128 and 256 tokens where 64 give more CTAs than are resident, and lengths beyond those."""
+    check(cuda_device, lengths, heads=16, kv_heads=8, dim=dim, bits=bits, page=32 if dim == 256 else 16)
