@@ -376,6 +376,27 @@ struct Ints {  // a writable int32 buffer
   Ints& operator=(const Ints&) = delete;
 };
 
+// The list itself, or a new one of plain ints where entries are other integers (numpy's); nullptr with an error set for
+// anything that is no integer.  A new reference.
+PyObject* plain_ints(PyObject* list) {
+  const Py_ssize_t n = PyList_GET_SIZE(list);
+  Py_ssize_t plain = 0;
+  while (plain < n && PyLong_Check(PyList_GET_ITEM(list, plain))) ++plain;
+  if (plain == n) {
+    Py_INCREF(list);
+    return list;
+  }
+  PyObject* ints = PyList_GetSlice(list, 0, n);
+  for (Py_ssize_t i = plain; ints != nullptr && i < n; ++i) {
+    PyObject* id = PyNumber_Index(PyList_GET_ITEM(ints, i));
+    if (id == nullptr) Py_CLEAR(ints);
+    else PyList_SetItem(ints, i, id);
+  }
+  return ints;
+}
+// ids that fit no Py_ssize_t are clipped, and so belong to no page either
+Py_ssize_t page_id(PyObject* list, Py_ssize_t i) { return PyNumber_AsSsize_t(PyList_GET_ITEM(list, i), nullptr); }
+
 // take_pages(free, counts, count) -> the last `count` ids of `free`, last one first; they leave `free` with one owner each
 PyObject* take_pages(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (nargs != 3 || !PyList_Check(args[0])) return PyErr_Format(PyExc_TypeError, "take_pages(list, counts, count)");
@@ -385,27 +406,26 @@ PyObject* take_pages(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "take_pages: more pages than are free");
     return nullptr;
   }
-  Ints counts(args[1]);
-  if (!counts.held) return nullptr;
-  for (Py_ssize_t i = 0; i < count; ++i) {
-    const Py_ssize_t id = PyLong_AsSsize_t(PyList_GET_ITEM(free_list, have - 1 - i));
-    if (id == -1 && PyErr_Occurred()) return nullptr;
-    if (id < 0 || id >= counts.size())
-      return PyErr_Format(PyExc_RuntimeError, "Invariant violated: free list page %zd does not exist.", id);
-    if (counts.data()[id] != 0)
-      return PyErr_Format(PyExc_RuntimeError, "Invariant violated: free list page %zd has non-zero refcount.", id);
-  }
-  PyObject* out = PyList_New(count);
+  PyObject* taken = PyList_GetSlice(free_list, have - count, have);
+  PyObject* out = taken == nullptr || PyList_Reverse(taken) != 0 ? nullptr : plain_ints(taken);
+  Py_XDECREF(taken);
   if (out == nullptr) return nullptr;
-  for (Py_ssize_t i = 0; i < count; ++i) {
-    PyObject* id = PyList_GET_ITEM(free_list, have - 1 - i);
-    counts.data()[PyLong_AsSsize_t(id)] = 1;
-    Py_INCREF(id);
-    PyList_SET_ITEM(out, i, id);
-  }
-  if (PyList_SetSlice(free_list, have - count, have, nullptr) != 0) {
-    Py_DECREF(out);
-    return nullptr;
+  {
+    Ints counts(args[1]);
+    Py_ssize_t id = 0;
+    bool ok = counts.held;
+    for (Py_ssize_t i = 0; ok && i < count; ++i) {
+      id = page_id(out, i);
+      ok = id >= 0 && id < counts.size() && counts.data()[id] == 0;
+    }
+    if (!ok && counts.held)
+      PyErr_Format(PyExc_RuntimeError, "Invariant violated: free list page %zd %s.", id,
+                   id >= 0 && id < counts.size() ? "has non-zero refcount" : "does not exist");
+    for (Py_ssize_t i = 0; ok && i < count; ++i) counts.data()[page_id(out, i)] = 1;
+    if (!ok || PyList_SetSlice(free_list, have - count, have, nullptr) != 0) {
+      Py_DECREF(out);
+      return nullptr;
+    }
   }
   return out;
 }
@@ -414,24 +434,27 @@ PyObject* take_pages(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 // one owner, ids without one are passed over
 PyObject* release_pages(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (nargs != 2 || !PyList_Check(args[0])) return PyErr_Format(PyExc_TypeError, "release_pages(list, counts)");
+  PyObject* ids = plain_ints(args[0]);
+  if (ids == nullptr) return nullptr;
   Ints counts(args[1]);
-  if (!counts.held) return nullptr;
-  const Py_ssize_t n = PyList_GET_SIZE(args[0]);
-  for (Py_ssize_t i = 0; i < n; ++i)
-    if (PyLong_AsSsize_t(PyList_GET_ITEM(args[0], i)) == -1 && PyErr_Occurred()) return nullptr;
-  PyObject* freed = PyList_New(n);
-  if (freed == nullptr) return nullptr;
+  const Py_ssize_t n = PyList_GET_SIZE(ids);
+  PyObject* freed = counts.held ? PyList_New(n) : nullptr;
+  if (freed == nullptr) {
+    Py_DECREF(ids);
+    return nullptr;
+  }
   Py_ssize_t last = 0, unshared = 0;
   for (Py_ssize_t i = 0; i < n; ++i) {
-    PyObject* id = PyList_GET_ITEM(args[0], i);
-    const Py_ssize_t page = PyLong_AsSsize_t(id);
+    const Py_ssize_t page = page_id(ids, i);
     if (page < 0 || page >= counts.size() || counts.data()[page] <= 0) continue;
     const int32_t left = --counts.data()[page];
     if (left == 1) ++unshared;
     if (left > 0) continue;
+    PyObject* id = PyList_GET_ITEM(ids, i);
     Py_INCREF(id);
     PyList_SET_ITEM(freed, last++, id);
   }
+  Py_DECREF(ids);
   if (last < n) {  // the rest of the new list is empty slots
     PyObject* part = PyList_GetSlice(freed, 0, last);
     Py_DECREF(freed);

@@ -416,6 +416,26 @@ def test_one_pass_release_equals_page_by_page_release():
             assert a._shared == sum(1 for rc in a.refcount.values() if rc > 1)
 
 
+def test_page_ids_are_any_integers():
+    """numpy integers (a row's own ``table_array()``, an index array) are page ids like plain ones; ids no page can have are
+    passed over; what is no integer is refused before any count changes."""
+    from anna_b200.pools import Qwen3PagedLayerAllocator, TurboQuantLayerPool
+
+    for pool in (Qwen3PagedLayerAllocator(4), TurboQuantLayerPool(4)):
+        book = pool._book
+        pages, _, _ = book.take(8, 0)
+        pool.release_pages(np.array(pages[:3], dtype=np.int32))
+        pool.release_pages([np.int64(pages[3]), 1 << 70, -(1 << 70), -1, 99])
+        book.release(np.int16(pages[4]))
+        assert book.free_pages[-5:] == [2, 1, 0, 3, 4] and all(type(page) is int for page in book.free_pages)
+        assert book.refcount == {5: 1, 6: 1, 7: 1}
+        with pytest.raises(TypeError):
+            pool.release_pages([5, 6.0])
+        assert book.refcount == {5: 1, 6: 1, 7: 1}
+        book.free_pages[-2:] = [np.int32(3), np.int64(4)]
+        assert book.take(2, 16)[0] == [4, 3] and book.owners(np.int64(4)) == 1
+
+
 def test_block_table_array_follows_the_list():
     """TurboQuantKVRow.table_array(): an int32 mirror that converts only what changed since the last call."""
     from anna_b200.turboquant import TurboQuantKVRow
