@@ -31,6 +31,8 @@ class _PageBook:
                  listening: Callable[[], bool] | None = None) -> None:
         self.free_pages: list[int] = []
         self._counts = array("i")    # owners by page id
+        # owners of ids that the pool has no pages for (yet); None while no such id was ever retained, as in ordinary use
+        self._strays: dict[int, int] | None = None
         self._on_page_freed = on_page_freed
         self._listening = listening  # optional: False while the callback has nothing to do (an empty registry)
         self._shared = 0  # pages with more than one owner
@@ -38,21 +40,41 @@ class _PageBook:
     @property
     def refcount(self) -> dict[int, int]:
         """Owners of every page that has one."""
-        return {page_id: rc for page_id, rc in enumerate(self._counts) if rc}
+        return {page_id: rc for page_id, rc in enumerate(self._counts) if rc} | (self._strays or {})
 
     def owners(self, page_id: int) -> int:
-        return self._counts[page_id] if 0 <= page_id < len(self._counts) else 0
+        if 0 <= page_id < len(self._counts):
+            return self._counts[page_id]
+        return self._strays.get(page_id, 0) if self._strays else 0
+
+    def _set_owners(self, page_id: int, owners: int) -> None:
+        if 0 <= page_id < len(self._counts):
+            self._counts[page_id] = owners
+            return
+        if self._strays is None:
+            self._strays = {}
+        if owners:
+            self._strays[page_id] = owners
+        else:
+            self._strays.pop(page_id, None)
 
     def _cover(self, pages: int) -> None:
-        if pages > len(self._counts):
-            self._counts.frombytes(bytes(self._counts.itemsize * (pages - len(self._counts))))
+        known = len(self._counts)
+        if pages > known:
+            self._counts.frombytes(bytes(self._counts.itemsize * (pages - known)))
+            if self._strays:
+                for page_id in [page_id for page_id in self._strays if known <= page_id < pages]:
+                    self._counts[page_id] = self._strays.pop(page_id)
 
     def take(self, num_pages: int, capacity: int) -> tuple[list[int], int, list[int]]:
         """Pop up to num_pages from the free list; returns (page ids, new capacity, ids created by growth)."""
         count = min(max(int(num_pages), 0), len(self.free_pages))
         self._cover(capacity)
         # the last `count` entries of the free list, most recently freed first (the same order as repeated pop())
-        out: list[int] = _lib.launch().take_pages(self.free_pages, self._counts, count) if count > 0 else []
+        out: list[int] = []
+        if count > 0:
+            out = (_lib.launch().take_pages(self.free_pages, self._counts, count) if self._strays is None
+                   else self._take_with_strays(count))
         missing = num_pages - len(out)
         new_capacity = capacity
         fresh: list[int] = []
@@ -78,9 +100,9 @@ class _PageBook:
         return new_capacity
 
     def retain(self, page_id: int) -> None:
-        self._cover(page_id + 1)
-        self._counts[page_id] += 1
-        if self._counts[page_id] == 2:
+        owners = self.owners(page_id) + 1
+        self._set_owners(int(page_id), owners)
+        if owners == 2:
             self._shared += 1
 
     def release(self, page_id: int) -> None:
@@ -88,7 +110,9 @@ class _PageBook:
 
     def release_many(self, page_ids) -> None:
         """Every id of `page_ids` loses one owner, in the given order; an id without one is passed over."""
-        freed, unshared = _lib.launch().release_pages(page_ids if isinstance(page_ids, list) else list(page_ids), self._counts)
+        ids = page_ids if isinstance(page_ids, list) else list(page_ids)
+        freed, unshared = (_lib.launch().release_pages(ids, self._counts) if self._strays is None
+                           else self._release_with_strays(ids))
         self._shared -= unshared
         if freed:
             self.free_pages.extend(freed)
@@ -96,9 +120,32 @@ class _PageBook:
                 for page_id in freed:
                     self._on_page_freed(page_id)
 
+    def _take_with_strays(self, count: int) -> list[int]:
+        out = [int(page_id) for page_id in self.free_pages[:-count - 1:-1]]
+        for page_id in out:
+            if self.owners(page_id) != 0:
+                raise RuntimeError(f"Invariant violated: free list page {page_id} has non-zero refcount.")
+        for page_id in out:
+            self._set_owners(page_id, 1)
+        del self.free_pages[-count:]
+        return out
+
+    def _release_with_strays(self, ids) -> tuple[list[int], int]:
+        freed, unshared = [], 0
+        for page_id in map(int, ids):
+            left = self.owners(page_id) - 1
+            if left < 0:
+                continue
+            self._set_owners(page_id, left)
+            if left == 0:
+                freed.append(page_id)
+            unshared += left == 1
+        return freed, unshared
+
     def clear(self) -> None:
         self.free_pages.clear()
         self._counts = array("i")
+        self._strays = None
         self._shared = 0
 
 

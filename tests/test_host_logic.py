@@ -436,6 +436,32 @@ def test_page_ids_are_any_integers():
         assert book.take(2, 16)[0] == [4, 3] and book.owners(np.int64(4)) == 1
 
 
+def test_owners_of_ids_beyond_the_pool_cost_no_memory():
+    """A pool without pages lets any id be retained (allocator, ops.py:92-245); an id far beyond what it will ever hold is one entry, and
+    ids that the pool grows up to keep their owners."""
+    import tracemalloc
+
+    from anna_b200.pools import Qwen3PagedLayerAllocator
+
+    layer = Qwen3PagedLayerAllocator(4)
+    book = layer._book
+    tracemalloc.start()
+    for page in (1 << 28, 1 << 28, 3, 20):
+        layer.retain_page(page)
+    assert tracemalloc.get_traced_memory()[1] < 1 << 16
+    tracemalloc.stop()
+    assert book.refcount == {1 << 28: 2, 3: 1, 20: 1} and layer.page_owners(1 << 28) == 2 and book._shared == 1
+    layer.release_pages([np.int64(1 << 28), 7])
+    assert book.refcount == {1 << 28: 1, 3: 1, 20: 1} and book.free_pages == [] and book._shared == 0
+    pages, capacity, _ = book.take(5, 0)                                 # fresh pages have one owner, whatever there was
+    assert (pages, capacity) == ([0, 1, 2, 3, 4], 16) and book.refcount == dict.fromkeys([*pages, 20, 1 << 28], 1)
+    book.take(11, 16)
+    with pytest.raises(RuntimeError, match="free list page 20 has non-zero refcount"):
+        book.take(20, book.take(1, 16)[1])
+    layer.release_page(1 << 28)
+    assert book.free_pages[-1] == 1 << 28 and layer.page_owners(1 << 28) == 0
+
+
 def test_block_table_array_follows_the_list():
     """TurboQuantKVRow.table_array(): an int32 mirror that converts only what changed since the last call."""
     from anna_b200.turboquant import TurboQuantKVRow
