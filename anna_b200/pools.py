@@ -23,6 +23,21 @@ def resolve_value_group_size(head_dim: int) -> int:
     return 1
 
 
+_NATIVE = None
+
+
+def native_page_ids():
+    """The call module, whose loops over page ids are C; False where it is not built (page ids need no GPU, and a host without
+    the library can keep un-quantized pages)."""
+    global _NATIVE
+    if _NATIVE is None:
+        try:
+            _NATIVE = _lib.launch()
+        except RuntimeError:
+            _NATIVE = False
+    return _NATIVE
+
+
 class _PageBook:
     """Free pages (a list, last in first out) and the number of owners of every page.  The loops over page ids run in the
     call module: with a dict of owners, taking and giving back the 960 pages of eight 2048-token prompts was 90 us."""
@@ -73,8 +88,8 @@ class _PageBook:
         # the last `count` entries of the free list, most recently freed first (the same order as repeated pop())
         out: list[int] = []
         if count > 0:
-            out = (_lib.launch().take_pages(self.free_pages, self._counts, count) if self._strays is None
-                   else self._take_with_strays(count))
+            native = native_page_ids() if self._strays is None else False
+            out = native.take_pages(self.free_pages, self._counts, count) if native else self._take(count)
         missing = num_pages - len(out)
         new_capacity = capacity
         fresh: list[int] = []
@@ -111,8 +126,8 @@ class _PageBook:
     def release_many(self, page_ids) -> None:
         """Every id of `page_ids` loses one owner, in the given order; an id without one is passed over."""
         ids = page_ids if isinstance(page_ids, list) else list(page_ids)
-        freed, unshared = (_lib.launch().release_pages(ids, self._counts) if self._strays is None
-                           else self._release_with_strays(ids))
+        native = native_page_ids() if self._strays is None else False
+        freed, unshared = native.release_pages(ids, self._counts) if native else self._release(ids)
         self._shared -= unshared
         if freed:
             self.free_pages.extend(freed)
@@ -120,7 +135,7 @@ class _PageBook:
                 for page_id in freed:
                     self._on_page_freed(page_id)
 
-    def _take_with_strays(self, count: int) -> list[int]:
+    def _take(self, count: int) -> list[int]:
         out = [int(page_id) for page_id in self.free_pages[:-count - 1:-1]]
         for page_id in out:
             if self.owners(page_id) != 0:
@@ -130,7 +145,7 @@ class _PageBook:
         del self.free_pages[-count:]
         return out
 
-    def _release_with_strays(self, ids) -> tuple[list[int], int]:
+    def _release(self, ids) -> tuple[list[int], int]:
         freed, unshared = [], 0
         for page_id in map(int, ids):
             left = self.owners(page_id) - 1

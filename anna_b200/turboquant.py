@@ -8,12 +8,14 @@ whole batch of rows is appended or decoded by one launch.
 """
 from __future__ import annotations
 
+from array import array
+
 import torch
 
 from . import _lib
 from .fused_ops import (MetadataUploader, dtype_code, launch_module, on_device, ptr, query_scratch, split_scratch,
                         stream_ptr)
-from .pools import TurboQuantLayerPool, resolve_value_group_size
+from .pools import TurboQuantLayerPool, native_page_ids, resolve_value_group_size
 from .tq_tables import key_tables
 
 # KV-cache TurboQuant bit-widths allowed by Anna runtimes (turboquant.py:52).
@@ -458,7 +460,11 @@ class TurboQuantKVRow:
                 grown[:valid] = arr[:valid]
             arr = self._table_np = grown
         if valid < n:
-            _lib.launch().copy_pages(self._blocks, valid, n, arr)
+            native = native_page_ids()
+            if native:
+                native.copy_pages(self._blocks, valid, n, arr)
+            else:
+                arr[valid:n] = array("i", self._blocks[valid:n])
         self._table_np_valid = n
         return arr[:n]
 

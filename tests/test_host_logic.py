@@ -462,6 +462,34 @@ def test_owners_of_ids_beyond_the_pool_cost_no_memory():
     assert book.free_pages[-1] == 1 << 28 and layer.page_owners(1 << 28) == 0
 
 
+def test_page_ids_without_the_call_module(monkeypatch):
+    """Un-quantized pages on a host where nothing is built: allocation, sharing, release and the table of a row."""
+    from anna_b200 import _lib, pools
+    from anna_b200.turboquant import TurboQuantKVRow
+
+    def missing():
+        raise RuntimeError("not built")
+
+    monkeypatch.setattr(_lib, "launch", missing)
+    monkeypatch.setattr(pools, "_NATIVE", None, raising=False)
+    freed: list[int] = []
+    layer = pools.Qwen3PagedLayerAllocator(4, on_page_freed=freed.append)
+    template = torch.zeros(1, 2, 1, 8)
+    pages = layer.allocate(3, key_template=template, value_template=template)
+    layer.retain_page(1)
+    layer.release_pages(np.array(pages))
+    assert freed == [2, 0] and layer._refcount == {1: 1} and layer._book._shared == 0
+    assert layer.allocate(2, key_template=template, value_template=template) == [0, 2] and layer.capacity() == 16
+    layer.release_page(1)
+    assert layer.free_pages[-1] == 1 and layer._refcount == {0: 1, 2: 1}
+    with pytest.raises(RuntimeError, match="non-zero refcount"):
+        layer.free_pages.append(2)
+        layer.allocate(1, key_template=template, value_template=template)
+    row = TurboQuantKVRow(bits=4, residual_len=8)
+    row.block_table.extend([5, 9, 2])
+    assert row.table_array().tolist() == [5, 9, 2]
+
+
 def test_block_table_array_follows_the_list():
     """TurboQuantKVRow.table_array(): an int32 mirror that converts only what changed since the last call."""
     from anna_b200.turboquant import TurboQuantKVRow
