@@ -464,22 +464,34 @@ PyObject* release_pages(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   return Py_BuildValue("Nn", freed, unshared);
 }
 
-// copy_pages(ids, first, last, target): ids[first:last] to the same places of an int32 buffer
+// copy_pages(ids, first, last, target): ids[first:last] of a list or another sequence to the same places of an int32 buffer
 PyObject* copy_pages(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-  if (nargs != 4 || !PyList_Check(args[0])) return PyErr_Format(PyExc_TypeError, "copy_pages(list, first, last, target)");
+  if (nargs != 4) return PyErr_Format(PyExc_TypeError, "copy_pages(ids, first, last, target)");
   const Py_ssize_t first = PyLong_AsSsize_t(args[1]), last = PyLong_AsSsize_t(args[2]);
   if (PyErr_Occurred()) return nullptr;
+  PyObject* ids = PySequence_Fast(args[0], "copy_pages: page ids must be a sequence");
+  if (ids == nullptr) return nullptr;
   Ints target(args[3]);
-  if (!target.held) return nullptr;
-  if (first < 0 || last < first || last > PyList_GET_SIZE(args[0]) || last > target.size()) {
+  bool ok = target.held;
+  if (ok && (first < 0 || last < first || last > PySequence_Fast_GET_SIZE(ids) || last > target.size())) {
     PyErr_SetString(PyExc_ValueError, "copy_pages: out of range");
-    return nullptr;
+    ok = false;
   }
-  for (Py_ssize_t i = first; i < last; ++i) {
-    const long id = PyLong_AsLong(PyList_GET_ITEM(args[0], i));
-    if (id == -1 && PyErr_Occurred()) return nullptr;
-    target.data()[i] = (int32_t)id;
+  for (Py_ssize_t i = first; ok && i < last; ++i) {
+    if (i >= PySequence_Fast_GET_SIZE(ids)) {  // an entry's __index__ may have shortened the list
+      PyErr_SetString(PyExc_ValueError, "copy_pages: out of range");
+      ok = false;
+      break;
+    }
+    const long id = PyLong_AsLong(PySequence_Fast_GET_ITEM(ids, i));
+    if (id == -1 && PyErr_Occurred()) ok = false;
+    else if (id != (int32_t)id) {
+      PyErr_SetString(PyExc_OverflowError, "copy_pages: page id does not fit 32 bits");
+      ok = false;
+    } else target.data()[i] = (int32_t)id;
   }
+  Py_DECREF(ids);
+  if (!ok) return nullptr;
   Py_RETURN_NONE;
 }
 

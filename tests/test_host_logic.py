@@ -507,6 +507,14 @@ def test_block_table_array_follows_the_list():
     row._table_np_valid = 0
     row.block_table.extend([4, 4, 4])
     assert row.table_array().tolist() == [4, 4, 4]
+    row._table_np_valid = 0
+    for table in ((7, 8), np.array([7, 8]), [np.int64(7), np.int16(8)]):  # set by a caller
+        row.block_table, row._table_np_valid = table, 0
+        assert row.table_array().tolist() == [7, 8]
+    for page in (1 << 31, -(1 << 31) - 1, 1 << 70):
+        row.block_table, row._table_np_valid = [page], 0
+        with pytest.raises(OverflowError):
+            row.table_array()
 
 
 def test_lengths_before_the_first_append_are_never_written_again():
