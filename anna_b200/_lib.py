@@ -103,11 +103,15 @@ def launch():
     global _LAUNCH
     if _LAUNCH is None:
         lib()
+        from .build import module_stamp
         try:
             from . import _launch
         except ImportError as exc:
             raise RuntimeError(f"{PKG_DIR / '_launch.so'} cannot be loaded: {exc}. Run `python -m anna_b200.build`. There is "
                                "no CPU fallback for this path.") from exc
+        if _launch.built_for != module_stamp():  # it would read tensors by another layout than theirs
+            raise RuntimeError(f"{_launch.__file__} was built for {_launch.built_for}, this is {module_stamp()}. Run "
+                               "`python -m anna_b200.build`.")
         _LAUNCH = _launch
     return _LAUNCH
 

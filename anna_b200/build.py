@@ -20,6 +20,7 @@ BUILD_DIR = PKG_DIR / "_build"
 LIB_PATH = PKG_DIR / "libanna_b200_kv.so"
 MODULE_SOURCE = CSRC / "launch_module.cpp"
 MODULE_PATH = PKG_DIR / "_launch.so"
+MODULE_STAMP = BUILD_DIR / "launch_module.stamp"  # what MODULE_PATH was built for
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -43,10 +44,20 @@ def _stale(target: Path, sources: list[Path]) -> bool:
     return any(src.stat().st_mtime > stamp for src in sources)
 
 
+def module_stamp() -> str:
+    """What the call module is compiled against besides its sources: it reads tensors and Python objects by the layout of the
+    installed headers.  Compiled into the module as ``built_for``."""
+    import torch
+
+    return f"torch {torch.__version__}, cxx11 abi {int(torch._C._GLIBCXX_USE_CXX11_ABI)}, {sys.implementation.cache_tag}"
+
+
 def build_module(force: bool = False, verbose: bool = False) -> Path:
     """The call module; needs the library, whose C entry points it links."""
     header = PKG_DIR.parent / "include" / "anna_b200_kv.h"
-    if not force and not _stale(MODULE_PATH, [MODULE_SOURCE, header]):
+    stamp = module_stamp()
+    current = MODULE_STAMP.exists() and MODULE_STAMP.read_text() == stamp
+    if not force and current and not _stale(MODULE_PATH, [MODULE_SOURCE, header]):
         return MODULE_PATH
     import sysconfig
 
@@ -57,7 +68,7 @@ def build_module(force: bool = False, verbose: bool = False) -> Path:
     includes = [header.parent, torch_dir / "include", torch_dir / "include" / "torch" / "csrc" / "api" / "include", cuda_include,
                 sysconfig.get_paths()["include"]]
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{path}" for path in includes],
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DANNA_BUILT_FOR="{stamp}"', *[f"-I{path}" for path in includes],
            str(MODULE_SOURCE), "-o", str(MODULE_PATH), f"-L{torch_dir / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10",
            "-lc10_cuda", f"-L{PKG_DIR}", f"-l:{LIB_PATH.name}", "-Wl,-rpath,$ORIGIN"]
     done = subprocess.run(cmd, capture_output=True, text=True)
@@ -65,6 +76,8 @@ def build_module(force: bool = False, verbose: bool = False) -> Path:
         raise RuntimeError(f"{MODULE_SOURCE.name} failed:\n{done.stderr}")
     if verbose:
         sys.stderr.write(done.stderr)
+    BUILD_DIR.mkdir(exist_ok=True)
+    MODULE_STAMP.write_text(stamp)
     return MODULE_PATH
 
 

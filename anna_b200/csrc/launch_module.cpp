@@ -511,4 +511,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_launch", nullptr, -1, methods, nu
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__launch() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__launch() {
+  PyObject* self = PyModule_Create(&module);
+  if (self != nullptr && PyModule_AddStringConstant(self, "built_for", ANNA_BUILT_FOR) != 0) Py_CLEAR(self);
+  return self;
+}

@@ -1,6 +1,9 @@
 """The call module (csrc/launch_module.cpp): what it declines, and that the calls it takes give what the general path gives."""
 from __future__ import annotations
 
+import sys
+from types import SimpleNamespace
+
 import pytest
 import torch
 
@@ -35,6 +38,29 @@ def test_cpu_tensors_and_other_objects_are_declined():
         module.tq_decode(x)
     with pytest.raises(TypeError):
         module.paged_decode(x, pages, pages, table, one, "scale", None)
+
+
+@pytest.mark.parametrize("changed", ["torch", "python"])
+def test_module_of_other_versions_is_rebuilt_and_not_loaded(monkeypatch, changed):
+    """The module reads tensors and objects by the layout of the headers that it was compiled with."""
+    from anna_b200 import build
+
+    compiled = []
+    monkeypatch.setattr(build.subprocess, "run",
+                        lambda cmd, **kw: compiled.append(cmd) or SimpleNamespace(returncode=1, stderr="", stdout=""))
+    _lib.launch()
+    build.build_module()
+    assert not compiled
+    if changed == "torch":
+        monkeypatch.setattr(torch, "__version__", "2.99.0")
+    else:
+        monkeypatch.setattr(sys.implementation, "cache_tag", "cpython-399")
+    with pytest.raises(RuntimeError, match="launch_module.cpp failed"):
+        build.build_module()
+    assert len(compiled) == 1
+    monkeypatch.setattr(_lib, "_LAUNCH", None)
+    with pytest.raises(RuntimeError, match="was built for"):
+        _lib.launch()
 
 
 def strided(shape, dtype, device, gen, order):
