@@ -411,7 +411,7 @@ static int tq_paged_decode_impl(const void* q, int64_t q_stride_b, int64_t q_str
                       (reinterpret_cast<uintptr_t>(query_scratch) & 15u) == 0;
     p.query_frags = fits ? query_scratch : nullptr;
   }
-  if (tq_split_mma_applicable(p, head_dim, dtype)) {
+  if (tq_split_mma_applicable(p, batch, head_dim, dtype)) {
     const bool umma = tq_split_umma_applicable(p, head_dim, bits, dtype);
     p.window_arrives = umma;
     if (split_counters != nullptr && num_chunks <= kFusedMaxChunks) {
@@ -432,7 +432,7 @@ static int tq_paged_decode_impl(const void* q, int64_t q_stride_b, int64_t q_str
                                 dtype, (cudaStream_t)stream);
   }
   if (num_peers > 0)
-    return set_error(ANNA_ERR_UNSUPPORTED, "peer outputs need the tensor-core decode path (16-bit cache, head_dim 128/256)");
+    return set_error(ANNA_ERR_UNSUPPORTED, "peer outputs need the tensor-core decode path (16-bit cache, head_dim 128/256, aligned query)");
   const bool merged = merges_in_split(split_counters, num_chunks, batch, p.kv_heads, p.groups, head_dim);
   if (merged) p.fused = FusedCombine{split_counters, out, out_stride_b, out_stride_h, gate, gate_stride_b, gate_stride_h};
   const int gpad = padded_group(p.groups);

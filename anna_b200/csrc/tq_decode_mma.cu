@@ -1237,6 +1237,33 @@ static bool tq_use_balanced(const TqDecodeParams& p, int batch, int head_dim, in
   return !tq_small(p, batch, head_dim, batch * units * (p.num_chunks - p.num_window_chunks) * 5, ctas * 4);
 }
 
+// The launches of a call, and the chunks it is cut into.
+struct TqLaunches {
+  TqSchedule schedule;
+  int chunk_tokens, num_window_chunks, num_chunks;
+};
+
+// `one_launch_ctas`, `share_ctas` = CTAs of the kernels that are resident at once.
+static TqLaunches tq_choose_launches(const TqDecodeParams& p, int batch, int head_dim, int one_launch_ctas, int share_ctas) {
+  TqLaunches out{TqSchedule::kOneLaunch, p.chunk_tokens, p.num_window_chunks, p.num_chunks};
+  if (!tq_fixed_chunks_only() && !p.given_chunks && p.fused.counters != nullptr && batch <= 65535) {
+    const int64_t units = (int64_t)p.kv_heads * ((p.groups + 7) / 8);
+    TqDecodeParams sp = p;
+    for (int tokens = p.chunk_tokens; tokens <= max(p.chunk_tokens, kTqSmallChunk); tokens *= 2) {
+      sp.chunk_tokens = tokens;
+      sp.num_window_chunks = (p.residual_len + tokens - 1) / tokens;
+      sp.num_chunks = sp.num_window_chunks + (int)((p.max_len - p.residual_len + tokens - 1) / tokens);
+      if (!tq_small(sp, batch, head_dim, batch * units * sp.num_chunks, one_launch_ctas)) continue;
+      out.chunk_tokens = tokens;
+      out.num_window_chunks = sp.num_window_chunks;
+      out.num_chunks = sp.num_chunks;
+      return out;
+    }
+  }
+  out.schedule = tq_use_balanced(p, batch, head_dim, share_ctas) ? TqSchedule::kEvenShares : TqSchedule::kChunks;
+  return out;
+}
+
 // CTAs of a kernel that fit the whole GPU at once, worked out at its first launch on a device, which also lets it have `smem`
 // bytes of shared memory.
 template <typename Kernel>
@@ -1273,28 +1300,27 @@ static int launch_tq_mma(const TqDecodeParams& p, int batch, cudaStream_t stream
        p.layout.chunk_bytes < Cfg::kTileDataBytes))
     return set_error(ANNA_ERR_INVALID, "packed page layout does not match the decode kernel's tile layout");
   const int group_tiles = (p.groups + 7) / 8;
-  if (!tq_fixed_chunks_only() && !p.given_chunks && p.fused.counters != nullptr && batch <= 65535) {
-    using Small = TqSmallCfg<T, D, BITS>;
-    static int small_resident[64] = {};
-    auto small = tq_decode_small_mma_kernel<T, D, BITS, kPair>;
-    int ctas = 0;
-    const int rc = resident_ctas(small, Small::kSmemBytes, small_resident, device, &ctas);
-    if (rc != ANNA_OK) return rc;
-    const int64_t units = (int64_t)p.kv_heads * group_tiles;
+  using Small = TqSmallCfg<T, D, BITS>;
+  auto small = tq_decode_small_mma_kernel<T, D, BITS, kPair>;
+  auto balanced = tq_decode_balanced_mma_kernel<T, D, BITS, kPair>;
+  static int small_resident[64] = {}, balanced_resident[64] = {};
+  int small_ctas = 0, balanced_ctas = 0;
+  int rc = resident_ctas(small, Small::kSmemBytes, small_resident, device, &small_ctas);
+  if (rc == ANNA_OK) rc = resident_ctas(balanced, Cfg::kSmemBytes, balanced_resident, device, &balanced_ctas);
+  if (rc != ANNA_OK) return rc;
+  const TqLaunches launches = tq_choose_launches(p, batch, D, small_ctas, balanced_ctas);
+  if (launches.schedule == TqSchedule::kOneLaunch) {
     TqDecodeParams sp = p;
-    for (int tokens = p.chunk_tokens; tokens <= max(p.chunk_tokens, kTqSmallChunk); tokens *= 2) {
-      sp.chunk_tokens = tokens;
-      sp.num_window_chunks = (p.residual_len + tokens - 1) / tokens;
-      sp.num_chunks = sp.num_window_chunks + (int)((p.max_len - p.residual_len + tokens - 1) / tokens);
-      if (!tq_small(sp, batch, D, batch * units * sp.num_chunks, ctas)) continue;
-      const dim3 grid((unsigned)sp.num_chunks, (unsigned)units, (unsigned)batch);
-      small<<<grid, kMmaThreads, Small::kSmemBytes, stream>>>(sp);
-      return check_launch("tq_decode_small_mma_kernel");
-    }
+    sp.chunk_tokens = launches.chunk_tokens;
+    sp.num_window_chunks = launches.num_window_chunks;
+    sp.num_chunks = launches.num_chunks;
+    const dim3 grid((unsigned)sp.num_chunks, (unsigned)(p.kv_heads * group_tiles), (unsigned)batch);
+    small<<<grid, kMmaThreads, Small::kSmemBytes, stream>>>(sp);
+    return check_launch("tq_decode_small_mma_kernel");
   }
   dim3 window_grid((unsigned)p.num_window_chunks, (unsigned)(p.kv_heads * group_tiles), (unsigned)batch);
   tq_window_split_mma_kernel<T, D><<<window_grid, kMmaThreads, MmaCfg<D>::kSmemBytes, stream>>>(p);
-  int rc = check_launch("tq_window_split_mma_kernel");
+  rc = check_launch("tq_window_split_mma_kernel");
   if (rc != ANNA_OK) return rc;
   if (p.num_chunks <= p.num_window_chunks) return rc;
   // programmatic dependent launch: the packed chunks run beside the (small) window launch instead of after it
@@ -1307,13 +1333,8 @@ static int launch_tq_mma(const TqDecodeParams& p, int batch, cudaStream_t stream
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attr;
   config.numAttrs = 1;
-  static int balanced_resident[64] = {};
-  auto balanced = tq_decode_balanced_mma_kernel<T, D, BITS, kPair>;
-  int ctas = 0;
-  rc = resident_ctas(balanced, Cfg::kSmemBytes, balanced_resident, device, &ctas);
-  if (rc != ANNA_OK) return rc;
-  if (tq_use_balanced(p, batch, D, ctas)) {
-    config.gridDim = dim3((unsigned)ctas);
+  if (launches.schedule == TqSchedule::kEvenShares) {
+    config.gridDim = dim3((unsigned)balanced_ctas);
     ANNA_CUDA_CHECK(cudaLaunchKernelEx(&config, balanced, p, batch));
     return check_launch("tq_decode_balanced_mma_kernel");
   }
@@ -1365,7 +1386,7 @@ __global__ void wait_expiry_selftest_kernel(int32_t* result) {
   if (threadIdx.x == 0) *result = landed ? 0 : 1;
 }
 
-bool tq_split_mma_applicable(const TqDecodeParams& p, int head_dim, int dtype) {
+bool tq_split_mma_applicable(const TqDecodeParams& p, int batch, int head_dim, int dtype) {
   static const bool disabled = [] {
     const char* flag = std::getenv("ANNA_B200_DISABLE_MMA");
     return flag != nullptr && flag[0] != '\0' && flag[0] != '0';
@@ -1375,6 +1396,10 @@ bool tq_split_mma_applicable(const TqDecodeParams& p, int head_dim, int dtype) {
   if (head_dim != 128 && head_dim != 256) return false;
   if (p.value_group != 32 || p.block_size % kTileTokens != 0 || p.chunk_tokens % kTileTokens != 0) return false;
   if (p.max_len >= (int64_t)1 << 31 || p.query_frags == nullptr) return false;
+  // the window chunks read query rows as aligned 32-bit pairs
+  if ((reinterpret_cast<uintptr_t>(p.q) & 3u) != 0 || (batch > 1 && p.q_stride_b % 2 != 0) ||
+      (p.q_heads > 1 && p.q_stride_h % 2 != 0))
+    return false;
   return true;
 }
 
@@ -1429,5 +1454,34 @@ extern "C" int anna_kv_device_faults(int* count) {
   if (rc == ANNA_OK) rc = anna::prefill_umma_faults(&prefill);
   if (rc != ANNA_OK) return rc;
   *count = mma + umma + prefill;
+  return ANNA_OK;
+}
+
+// Host side of a call's way through the packed decode, for tests without a GPU: what the entry point and launch_tq_mma choose.
+extern "C" int anna_kv_selftest_tq_schedule(const void* q, int64_t q_stride_b, int64_t q_stride_h, int batch, int q_heads,
+                                            int kv_heads, int head_dim, int64_t max_blocks, int block_size, int residual_len,
+                                            int value_group, int dtype, int one_launch_ctas, int share_ctas, int* schedule,
+                                            int* chunk_tokens) {
+  using namespace anna;
+  ANNA_REQUIRE(schedule != nullptr && chunk_tokens != nullptr && kv_heads > 0 && q_heads > 0 && q_heads % kv_heads == 0,
+               "anna_kv_selftest_tq_schedule: bad argument");
+  TqDecodeParams p{};
+  const int rc = anna_tq_decode_plan(batch, kv_heads, max_blocks, block_size, residual_len, &p.chunk_tokens, &p.num_chunks);
+  if (rc != ANNA_OK) return rc;
+  int32_t counters = 0;
+  p.q = q; p.q_stride_b = q_stride_b; p.q_stride_h = q_stride_h;
+  p.q_heads = q_heads; p.kv_heads = kv_heads; p.groups = q_heads / kv_heads;
+  p.block_size = block_size; p.residual_len = residual_len; p.value_group = value_group;
+  p.max_blocks = max_blocks; p.max_len = max_blocks * (int64_t)block_size + residual_len;
+  p.chunk_capacity = p.num_chunks;
+  p.num_window_chunks = (residual_len + p.chunk_tokens - 1) / p.chunk_tokens;
+  p.query_frags = &counters;
+  if (p.num_chunks <= kFusedMaxChunks) p.fused.counters = &counters;
+  *chunk_tokens = p.chunk_tokens;
+  *schedule = (int)TqSchedule::kCudaCores;
+  if (!tq_split_mma_applicable(p, batch, head_dim, dtype)) return ANNA_OK;
+  const TqLaunches launches = tq_choose_launches(p, batch, head_dim, one_launch_ctas, share_ctas);
+  *chunk_tokens = launches.chunk_tokens;
+  *schedule = (int)launches.schedule;
   return ANNA_OK;
 }

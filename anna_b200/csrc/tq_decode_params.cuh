@@ -54,8 +54,11 @@ inline size_t tq_query_scratch_bytes(int batch, int q_heads, int kv_heads, int h
   return units * (frag > image ? frag : image);
 }
 
-// Tensor-core split pass (tq_decode_mma.cu): 16-bit cache dtypes, head_dim 128 / 256, value group 32, page size % 16 == 0.
-bool tq_split_mma_applicable(const TqDecodeParams& p, int head_dim, int dtype);
+// Tensor-core split pass (tq_decode_mma.cu): 16-bit cache dtypes, head_dim 128 / 256, value group 32, page size % 16 == 0,
+// query rows on 4-byte boundaries.
+bool tq_split_mma_applicable(const TqDecodeParams& p, int batch, int head_dim, int dtype);
+// Ways of a call: the CUDA-core kernel; window and packed chunks in one launch; a window launch, then even shares or chunks.
+enum class TqSchedule { kCudaCores = 0, kOneLaunch = 1, kEvenShares = 2, kChunks = 3 };
 int launch_tq_split_mma(const TqDecodeParams& p, int batch, int head_dim, int bits, int dtype, cudaStream_t stream);
 
 // bounded copy waits that expired in the tensor-core packed decode on the current device (tq_decode_mma.cu)

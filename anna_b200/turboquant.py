@@ -104,6 +104,9 @@ def launch_tq_decode(pool: TurboQuantLayerPool, query_states: torch.Tensor, tabl
             return out
     _require_cuda(query_states, "TurboQuant decode")
     query = query_states if query_states.stride(3) == 1 else query_states.contiguous()
+    if peer_outputs and (query.data_ptr() % 4 != 0 or query.stride(0) % 2 != 0 or query.stride(1) % 2 != 0):
+        # only the tensor-core kernels store to peers, and they read query rows as aligned 32-bit pairs
+        query = query.clone(memory_format=torch.contiguous_format)
     if gate is not None and gate.stride(3) != 1:
         gate = gate.contiguous()
     device = query.device

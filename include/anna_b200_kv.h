@@ -64,6 +64,15 @@ int anna_kv_selftest_even_shares(const int64_t* lengths, int batch, int streams_
                                  int min_tiles, int segment_tiles, int stream_tiles, int32_t* segments, int max_segments,
                                  int* num_segments);
 
+/* Self-test, on the host: which way anna_tq_paged_decode takes for such a call with scratch of the plan's size, a fused merge and
+ * no peers: *schedule = 0 the CUDA-core kernel, 1 window and packed chunks in one launch, 2 a window launch and even shares,
+ * 3 a window launch and chunks; *chunk_tokens = tokens of a chunk.  q is not read; one_launch_ctas and share_ctas = CTAs of
+ * those kernels that the GPU holds at once.  No counterpart in the reference.
+ */
+int anna_kv_selftest_tq_schedule(const void* q, int64_t q_stride_b, int64_t q_stride_h, int batch, int q_heads, int kv_heads,
+                                 int head_dim, int64_t max_blocks, int block_size, int residual_len, int value_group, int dtype,
+                                 int one_launch_ctas, int share_ctas, int* schedule, int* chunk_tokens);
+
 /*
  * Self-test of the tensor-memory matrix multiply (tcgen05) in the two operand arrangements of the packed decode:
  *   d1 float [128][16] = a1 . b1^T   a1 uint8 [128][128], b1 uint8 [16][128]: e4m3 bytes, K contiguous

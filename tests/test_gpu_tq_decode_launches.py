@@ -51,3 +51,26 @@ def test_long_streams_of_two_and_of_three_chunks(cuda_device, longest):
 def test_longer_chunks_in_one_launch(cuda_device, lengths, dim, bits):
     """Chunks of 128 and 256 tokens where 64 give more CTAs than are resident, and lengths beyond those."""
     check(cuda_device, lengths, heads=16, kv_heads=8, dim=dim, bits=bits, page=32 if dim == 256 else 16)
+
+
+@pytest.mark.parametrize("dim,bits,heads", [(128, 4, 8), (128, 3, 2), (256, 2, 22)])
+@pytest.mark.parametrize("lengths", [[700], [WINDOW + 5, 1, 2300, 90]])
+def test_query_rows_at_odd_elements(cuda_device, dim, bits, heads, lengths):
+    """Views of a wider projection: an odd offset, an odd head stride, an odd row stride; with and without peers."""
+    cache, gen = ragged_cache(cuda_device, lengths, kv_heads=2, dim=dim, bits=bits, page=16, dtype=torch.bfloat16)
+    batch = len(lengths)
+
+    def randn(*shape):
+        return torch.randn(shape, generator=gen, device=cuda_device).to(torch.bfloat16)
+
+    for query in (randn(batch * heads * dim + 1)[1:].view(batch, heads, 1, dim), randn(batch, heads, 1, dim + 1)[..., :dim],
+                  randn(batch, heads * dim + 1)[:, :-1].unflatten(1, (heads, 1, dim)),
+                  randn(batch, heads * dim + 2)[:, 1:-1].unflatten(1, (heads, 1, dim))):
+        assert query.stride(3) == 1 and (query.data_ptr() % 4 or query.stride(0) % 2 or query.stride(1) % 2)
+        args = dict(scaling=dim ** -0.5, num_key_value_groups=heads // 2)
+        out = cache.turboquant_single_token_decode_attention(0, query, **args)
+        assert_close(out, dense_attention(cache, query, lengths, dim ** -0.5), torch.bfloat16)
+        local, peer = torch.empty_like(out), torch.empty_like(out)
+        cache.turboquant_single_token_decode_attention(0, query, **args, output=local, peer_outputs=(peer.data_ptr(),))
+        assert_close(local, dense_attention(cache, query, lengths, dim ** -0.5), torch.bfloat16)
+        assert torch.equal(local, peer)
