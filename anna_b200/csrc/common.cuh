@@ -18,6 +18,14 @@ namespace anna {
 
 int set_error(int code, const char* fmt, ...);  // formats into the thread-local message, returns `code`
 
+// Addresses that kernels read with wide loads are checked where the strides are: a view may start at any element.
+inline bool aligned_to(const void* address, size_t bytes) { return reinterpret_cast<uintptr_t>(address) % bytes == 0; }
+// bytes of the access by which a lane moves its head_dim / 32 elements (lane_load, lane_copy)
+inline size_t lane_access_bytes(int head_dim, int elem_bytes) {
+  const int bytes = head_dim / 32 * elem_bytes;
+  return bytes >= 16 ? 16 : bytes > 0 ? bytes : 1;
+}
+
 #define ANNA_REQUIRE(cond, ...)                                   \
   do {                                                            \
     if (!(cond)) return ::anna::set_error(ANNA_ERR_INVALID, __VA_ARGS__); \

@@ -135,6 +135,8 @@ extern "C" int anna_paged_kv_gather(const void* key_pages, const void* value_pag
                head_dim, vec);
   ANNA_REQUIRE(out_stride_b % vec == 0 && out_stride_h % vec == 0 && out_stride_t % vec == 0,
                "anna_paged_kv_gather: output strides must keep rows 16-byte aligned");
+  ANNA_REQUIRE(aligned_to(key_pages, 16) && aligned_to(value_pages, 16) && aligned_to(key_out, 16) && aligned_to(value_out, 16),
+               "anna_paged_kv_gather: pages and outputs must be 16-byte aligned");
   KvGatherParams p{key_pages, value_pages, page_table, table_stride, lengths, key_out, value_out, out_stride_b,
                    out_stride_h, out_stride_t, batch, kv_heads, head_dim, block_size, num_pages, max_blocks, max_len};
   const int64_t total = (int64_t)batch * kv_heads * max_len * (head_dim / vec);
@@ -162,6 +164,8 @@ extern "C" int anna_paged_kv_write(const void* k_new, const void* v_new, int64_t
                head_dim, vec);
   ANNA_REQUIRE(kn_stride_b % vec == 0 && kn_stride_h % vec == 0 && kn_stride_t % vec == 0,
                "anna_paged_kv_write: source strides must keep rows 16-byte aligned");
+  ANNA_REQUIRE(aligned_to(k_new, 16) && aligned_to(v_new, 16) && aligned_to(key_pages, 16) && aligned_to(value_pages, 16),
+               "anna_paged_kv_write: keys, values and pages must be 16-byte aligned");
   KvWriteParams p{k_new, v_new, kn_stride_b, kn_stride_h, kn_stride_t, key_pages, value_pages, page_table,
                   table_stride, past_lengths, new_lengths, batch, kv_heads, new_tokens, head_dim, block_size, num_pages,
                   max_blocks, status};

@@ -205,6 +205,7 @@ extern "C" int anna_paged_gqa_decode(const void* q, int64_t q_stride_b, int64_t 
   ANNA_REQUIRE(block_size >= 1 && num_pages >= 1 && max_blocks >= 1 && table_stride >= max_blocks,
                "anna_paged_gqa_decode: bad paging geometry (block_size=%d pages=%lld max_blocks=%lld stride=%lld)",
                block_size, (long long)num_pages, (long long)max_blocks, (long long)table_stride);
+  ANNA_REQUIRE(aligned_to(key_pages, 16) && aligned_to(value_pages, 16), "anna_paged_gqa_decode: pages must be 16-byte aligned");
   DenseDecodeParams p{};
   p.q = q; p.q_stride_b = q_stride_b; p.q_stride_h = q_stride_h;
   p.key = key_pages; p.value = value_pages;
@@ -237,6 +238,7 @@ extern "C" int anna_gqa_decode(const void* q, int64_t q_stride_b, int64_t q_stri
   const int vec = dtype == ANNA_DTYPE_F32 ? 4 : 8;
   ANNA_REQUIRE(kv_stride_b % vec == 0 && kv_stride_h % vec == 0 && kv_stride_t % vec == 0,
                "anna_gqa_decode: K/V strides must keep rows 16-byte aligned");
+  ANNA_REQUIRE(aligned_to(key, 16) && aligned_to(value, 16), "anna_gqa_decode: keys and values must be 16-byte aligned");
   DenseDecodeParams p{};
   p.q = q; p.q_stride_b = q_stride_b; p.q_stride_h = q_stride_h;
   p.key = key; p.value = value;

@@ -311,6 +311,9 @@ extern "C" int anna_tq_append(const void* k_new, const void* v_new, int64_t kn_s
   const int vec = dtype == ANNA_DTYPE_F32 ? 4 : 8;
   ANNA_REQUIRE(kn_stride_b % vec == 0 && kn_stride_h % vec == 0 && kn_stride_t % vec == 0,
                "anna_tq_append: source strides must keep rows 16-byte aligned");
+  const size_t access = lane_access_bytes(head_dim, dtype_bytes_of(dtype));
+  ANNA_REQUIRE(aligned_to(k_new, access) && aligned_to(v_new, access) && aligned_to(window, access),
+               "anna_tq_append: keys, values and window must be aligned to %d bytes", (int)access);
   TqAppendParams p{};
   p.k_new = k_new; p.v_new = v_new;
   p.stride_b = kn_stride_b; p.stride_h = kn_stride_h; p.stride_t = kn_stride_t;

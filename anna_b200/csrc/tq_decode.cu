@@ -368,6 +368,7 @@ static int tq_paged_decode_impl(const void* q, int64_t q_stride_b, int64_t q_str
   ANNA_REQUIRE(batch > 0 && q_heads > 0 && kv_heads > 0 && q_heads % kv_heads == 0,
                "anna_tq_paged_decode: query heads (%d) must be a positive multiple of kv heads (%d)", q_heads, kv_heads);
   ANNA_REQUIRE(residual_len >= 1 && block_size >= 1 && max_blocks >= 0, "anna_tq_paged_decode: bad geometry");
+  ANNA_REQUIRE(aligned_to(window, 16), "anna_tq_paged_decode: the window must be 16-byte aligned");
   const int vec = dtype == ANNA_DTYPE_F32 ? 4 : 8;
   ANNA_REQUIRE(value_group % vec == 0, "anna_tq_paged_decode: value group %d must be a multiple of %d", value_group, vec);
   TqDecodeParams p{};

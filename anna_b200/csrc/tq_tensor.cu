@@ -163,6 +163,8 @@ extern "C" int anna_tq_tensor_quantize(const void* x, int64_t stride_h, int64_t 
   int rc = check_tensor_args("anna_tq_tensor_quantize", heads, tokens, head_dim, bits, dtype, stride_h, stride_t, capacity,
                              offset);
   if (rc != ANNA_OK) return rc;
+  const size_t access = lane_access_bytes(head_dim, dtype_bytes_of(dtype));
+  ANNA_REQUIRE(aligned_to(x, access), "anna_tq_tensor_quantize: the tensor must be aligned to %d bytes", (int)access);
   TqTensorParams p{};
   p.x = x; p.stride_h = stride_h; p.stride_t = stride_t; p.idx = idx; p.norms = norms; p.capacity = capacity;
   p.offset = offset; p.heads = heads; p.tokens = tokens; p.signs1 = signs1; p.boundaries = boundaries;

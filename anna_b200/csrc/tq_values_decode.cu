@@ -193,6 +193,9 @@ extern "C" int anna_gqa_decode_turboquant_values(
   ANNA_REQUIRE(qk_stride_b % vec == 0 && qk_stride_h % vec == 0 && qk_stride_t % vec == 0 && r_stride_b % vec == 0 &&
                    r_stride_h % vec == 0 && r_stride_t % vec == 0,
                "anna_gqa_decode_turboquant_values: key strides must keep rows 16-byte aligned");
+  ANNA_REQUIRE(aligned_to(quantized_key, 16) &&
+                   (residual_len == 0 || (aligned_to(residual_key, 16) && aligned_to(residual_value, 16))),
+               "anna_gqa_decode_turboquant_values: keys and residual must be 16-byte aligned");
   TqValuesParams p{};
   p.q = q; p.q_stride_b = q_stride_b; p.q_stride_h = q_stride_h;
   p.quantized_key = quantized_key; p.qk_stride_b = qk_stride_b; p.qk_stride_h = qk_stride_h; p.qk_stride_t = qk_stride_t;

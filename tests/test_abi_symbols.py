@@ -107,3 +107,39 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "LIB_PATH", tmp_path / "libanna_b200_kv.so")
     with pytest.raises(RuntimeError, match="no CPU fallback"):
         _lib.lib()
+
+
+def test_misaligned_rows_are_refused(library):
+    """A view may start at any element; the kernels read keys, values, pages and windows with wide loads.  Nothing is
+    launched: the addresses are made up and every call is refused before it touches them."""
+    ok, f32, bf16 = 0x10000, _lib.DTYPE_F32, _lib.DTYPE_BF16
+
+    def refused(status):
+        return status == 1 and "aligned" in _lib.last_error()
+
+    def append(dim, dtype, k=ok, v=ok, window=ok):
+        return library.anna_tq_append(k, v, 2 * dim, dim, dim, ok, ok, 8, None, 0, window, ok, ok, None, ok, ok, ok, ok, 1, 2, 1,
+                                      dim, 16, 16, 4, 32, 8, 8, dtype, None, None)
+
+    for dim, dtype, access in ((64, bf16, 4), (64, f32, 8), (128, bf16, 8), (128, f32, 16), (256, bf16, 16)):
+        for name in ("k", "v", "window"):
+            assert refused(append(dim, dtype, **{name: ok + access // 2}))
+    for at in range(4):
+        args = [ok] * 4
+        args[at] += 8
+        k, v, kp, vp = args
+        assert refused(library.anna_paged_kv_write(k, v, 256, 128, 128, kp, vp, ok, 4, ok, None, 1, 2, 1, 128, 16, 8, 4, bf16,
+                                                   None, None))
+        assert refused(library.anna_paged_kv_gather(kp, vp, ok, 4, ok, k, v, 256, 128, 128, 1, 2, 128, 16, 8, 4, 64, bf16, None))
+        if at < 2:
+            assert refused(library.anna_gqa_decode(ok, 256, 128, k, v, 4096, 2048, 128, ok, None, 0, 0, ok, 256, 128, ok, ok, 8, 0,
+                                                   ok, 1, 2, 2, 16, 128, 0.1, bf16, None))
+            assert refused(library.anna_paged_gqa_decode(ok, 256, 128, k, v, ok, 4, ok, None, 0, 0, ok, 256, 128, ok, ok, 8, 0, ok,
+                                                         1, 2, 2, 128, 16, 8, 4, 0.1, bf16, None))
+        if at < 3:
+            assert refused(library.anna_gqa_decode_turboquant_values(
+                ok, 256, 128, k, 4096, 2048, 128, ok, 1024, 512, 64, ok, ok, 64, 32, 4, v, kp, 4096, 2048, 128, None, 0, 0, ok, 256,
+                128, ok, ok, 8, 16, 1, 2, 2, 16, 16, 128, 4, 32, 0.1, bf16, None))
+    assert refused(library.anna_tq_paged_decode(ok, 256, 128, ok, ok, 4, ok + 8, ok, ok, ok, ok, ok, None, 0, 0, ok, 256, 128, ok, ok,
+                                                64, 0, ok, ok, 1 << 20, 1, 2, 2, 128, 16, 16, 4, 32, 8, 4, 0.1, bf16, None))
+    assert refused(library.anna_tq_tensor_quantize(ok + 4, 128, 128, ok, ok, 8, 0, 1, 1, 128, 4, ok, ok, bf16, None))
