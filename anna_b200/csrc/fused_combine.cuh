@@ -1,10 +1,12 @@
 // Split-K merge done by the last CTA that finishes a (row, kv-head group): no second launch, no waiting.
 //
-// Every CTA of the split pass publishes its partial, fences, and bumps a per-(row, group) counter.  The CTA that
+// Every CTA of the split pass publishes its partial and bumps a per-(row, group) counter (an acquire-release).  The CTA that
 // observes the final count owns the merge: it re-reads the partials (L2 resident), applies the optional sigmoid(gate)
 // epilogue and stores the output row.  Nobody spins: a CTA either is last or leaves.  The counter is reset by the
 // merging CTA, so the caller's buffer stays all-zero between launches.
 #pragma once
+
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -26,8 +28,10 @@ constexpr int kFusedMaxChunks = 512;  // weights of one head are staged in share
 
 // Called by all threads of the CTA after they wrote their partial.  `active_chunks` = partials that contribute to this
 // (row, group); `arrivals` of them (0 = all; the others are known to be complete before any arrival) are counted in
-// counters[counter_index]; stats / values point at chunk 0 of query head hq0.  Natural-log stats.  THREADS = blockDim.x.
-template <typename T, int D, int THREADS>
+// counters[counter_index]; stats / values point at chunk 0 of query head hq0.  Natural-log stats.  THREADS = blockDim.x,
+// HEADS = most query heads of a group, MERGE: how the values are read, see below.
+enum class MergeLoads { kOneColumn, kAllColumns, kAllOrTwoColumns };
+template <typename T, int D, int THREADS, int HEADS = 8, MergeLoads MERGE = MergeLoads::kAllOrTwoColumns>
 __device__ __forceinline__ void fused_combine_tail(const FusedCombine& fc, int b, int hq0, int g_count,
                                                    int active_chunks, int chunk_capacity, const float* stats,
                                                    const float* values, float* smem_weights /* [8][kFusedMaxChunks] */,
@@ -89,9 +93,8 @@ __device__ __forceinline__ void fused_combine_tail(const FusedCombine& fc, int b
   // column per thread eight at a time are no faster than a plain loop (one packed row of 4000 tokens: 20.6 us and 18.5).
   const bool aligned = (reinterpret_cast<uintptr_t>(values) & 15u) == 0;
   constexpr int kCols = D / 4;
-  constexpr int kRounds = (8 * kCols + THREADS - 1) / THREADS;
+  constexpr int kRounds = (HEADS * kCols + THREADS - 1) / THREADS;
   constexpr int kInFlight = 8;
-  constexpr int kAtOnce = kInFlight / kRounds;  // partials
   const int items = g_count * kCols;
   auto add = [](float4& acc, const float4& v, float w) {
     acc.x = fmaf(v.x, w, acc.x);
@@ -99,24 +102,26 @@ __device__ __forceinline__ void fused_combine_tail(const FusedCombine& fc, int b
     acc.z = fmaf(v.z, w, acc.z);
     acc.w = fmaf(v.w, w, acc.w);
   };
-  if (aligned && items > THREADS) {
-    float4 acc[kRounds];
-    const float* vals[kRounds];
+  auto side_by_side = [&](auto columns) {
+    constexpr int kColumns = decltype(columns)::value;  // of a thread
+    constexpr int kAtOnce = kInFlight / kColumns;       // partials
+    float4 acc[kColumns];
+    const float* vals[kColumns];
 #pragma unroll
-    for (int r = 0; r < kRounds; ++r) {
+    for (int r = 0; r < kColumns; ++r) {
       const int item = min((int)threadIdx.x + r * THREADS, items - 1);  // past the end: the last column again, not stored
       acc[r] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       vals[r] = values + (int64_t)(item / kCols) * chunk_capacity * D + 4 * (item % kCols);
     }
     for (int c0 = 0; c0 < active_chunks; c0 += kAtOnce) {
-      float4 v[kAtOnce][kRounds];
+      float4 v[kAtOnce][kColumns];
 #pragma unroll
       for (int k = 0; k < kAtOnce; ++k)
 #pragma unroll
-        for (int r = 0; r < kRounds; ++r)
+        for (int r = 0; r < kColumns; ++r)
           v[k][r] = __ldcg(reinterpret_cast<const float4*>(vals[r] + (int64_t)min(c0 + k, active_chunks - 1) * D));
 #pragma unroll
-      for (int r = 0; r < kRounds; ++r) {
+      for (int r = 0; r < kColumns; ++r) {
         const float* w = smem_weights + min(((int)threadIdx.x + r * THREADS) / kCols, g_count - 1) * kFusedMaxChunks;
 #pragma unroll
         for (int k = 0; k < kAtOnce; ++k)
@@ -124,13 +129,22 @@ __device__ __forceinline__ void fused_combine_tail(const FusedCombine& fc, int b
       }
     }
 #pragma unroll
-    for (int r = 0; r < kRounds; ++r) {
+    for (int r = 0; r < kColumns; ++r) {
       const int item = (int)threadIdx.x + r * THREADS;
       if (item < items) store(item / kCols, 4 * (item % kCols), acc[r]);
     }
+  };
+  // No more columns than the group has: with four of them for two (four heads of 256) every second load is in vain (one packed
+  // row of 20000 tokens, 8/2 heads: 42.4 us, 31.0 so, 38.6 one column after the other; 4 un-quantized rows of 3-6 K 14.6, 12.9
+  // and 15.9).  Kernels that know HEADS have one form of the loop, which costs fewer registers than two.
+  constexpr bool kTwo = kRounds > 2 && MERGE == MergeLoads::kAllOrTwoColumns;
+  if (MERGE != MergeLoads::kOneColumn && kRounds > 1 && aligned && items > (kTwo ? 2 : 1) * THREADS) {
+    side_by_side(std::integral_constant<int, kRounds>{});
+  } else if (kTwo && aligned && items > THREADS) {
+    side_by_side(std::integral_constant<int, 2>{});
   } else if (aligned) {
-    if ((int)threadIdx.x < items) {
-      const int g = (int)threadIdx.x / kCols, d = 4 * ((int)threadIdx.x % kCols);
+    for (int item = threadIdx.x; item < items; item += THREADS) {
+      const int g = item / kCols, d = 4 * (item % kCols);
       const float* vals = values + (int64_t)g * chunk_capacity * D + d;
       const float* w = smem_weights + g * kFusedMaxChunks;
       float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);

@@ -493,7 +493,7 @@ __device__ __forceinline__ RowChunks row_chunks(const TqDecodeParams& p, int b) 
 
 // Chunk `slot` of the un-quantized window ring of a row: the dense tensor-core body with ring addressing.  Also writes the
 // zero output of empty rows.  `arrives`: the chunk counts on the merge counter, as one of all active chunks.
-template <typename T, int D, int STAGES>
+template <typename T, int D, int STAGES, int HEADS>
 __device__ __forceinline__ void tq_window_chunk(const TqDecodeParams& p, uint8_t* smem_raw, const RowChunks& row, int b,
                                                 int unit, int units, int slot, bool arrives) {
   const int group_tiles = (p.groups + 7) / 8;
@@ -525,7 +525,7 @@ __device__ __forceinline__ void tq_window_chunk(const TqDecodeParams& p, uint8_t
   if (!arrives) dp.fused.counters = nullptr;
   const int t0 = row.quantized + slot * p.chunk_tokens;
   const int t1 = min(row.len, t0 + p.chunk_tokens);
-  dense_split_mma_body<T, D, STAGES>(dp, smem_raw, b, kvh, g0, g_count, t0, t1, slot, row.window + row.packed,
+  dense_split_mma_body<T, D, STAGES, HEADS, MergeLoads::kAllColumns>(dp, smem_raw, b, kvh, g0, g_count, t0, t1, slot, row.window + row.packed,
                                      (int64_t)b * units + unit);
 }
 
@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(kMmaThreads, MmaCfg<D>::kMinBlocks) tq_window_
   asm volatile("griddepcontrol.launch_dependents;\n" ::);
   const RowChunks row = row_chunks(p, blockIdx.z);
   // the packed CTAs wait for this grid before they count
-  tq_window_chunk<T, D, 2>(p, smem_raw, row, blockIdx.z, blockIdx.y, gridDim.y, blockIdx.x,
+  tq_window_chunk<T, D, 2, 8>(p, smem_raw, row, blockIdx.z, blockIdx.y, gridDim.y, blockIdx.x,
                            p.window_arrives || row.quantized == 0);
 }
 
@@ -550,6 +550,11 @@ struct PackedRing {
   bool dead;       // a bounded wait expired: this warp consumes nothing any more
 };
 
+// Query heads that the merge provides for.  (At head_dim 128 four heads have one column per thread, and the loop for two, which
+// they never reach, stays: without it the 4-bit even-share kernel took 1.6 to 3.4 % longer.)
+template <int D, bool kPair>
+constexpr int kMergeHeads = kPair && D == 256 ? 4 : 8;
+
 // One packed segment: tokens [t0, t1) of the quantized prefix of (row b, unit = kv head and group of 8 query heads).  The
 // partial goes to split-K slot `out_slot` and counts as one of `arrivals`; the CTA that counts last merges `slots` partials.
 // All threads of the CTA call it; it ends with the CTA synchronised against reuse of the ring.
@@ -559,7 +564,7 @@ struct PackedRing {
 // arithmetic, the softmax and the registers behind it are spent once per two tiles instead of once per tile with half of
 // the columns empty; columns j and j + 4 are two partials of head j, merged with those of the other warps.  64 rows of
 // 32 K tokens, 4 bits: 636 -> 614 us; 128 rows of 0.5-16 K, 3 bits: 247 -> 239 us.
-template <typename T, int D, int BITS, bool kPair>
+template <typename T, int D, int BITS, bool kPair, MergeLoads MERGE = MergeLoads::kAllColumns>
 __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8_t* smem_raw,
                                                   const TqQueryConsts& qc, PackedRing& ring, int b, int unit,
                                                   int units, int t0, int t1, int out_slot, int slots, int arrivals) {
@@ -1090,9 +1095,9 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
   if (p.fused.counters != nullptr) {
     const int64_t head0 = ((int64_t)b * p.q_heads + hq0) * p.chunk_capacity;
     __syncthreads();
-    fused_combine_tail<T, D, kMmaThreads>(p.fused, b, hq0, g_count, slots, p.chunk_capacity, p.stats + head0 * 2,
-                                          p.values + head0 * D, reinterpret_cast<float*>(smem_raw),
-                                          (int64_t)b * units + unit, arrivals);
+    fused_combine_tail<T, D, kMmaThreads, kMergeHeads<D, kPair>, MERGE>(
+        p.fused, b, hq0, g_count, slots, p.chunk_capacity, p.stats + head0 * 2, p.values + head0 * D,
+        reinterpret_cast<float*>(smem_raw), (int64_t)b * units + unit, arrivals);
   }
   // the merge buffers lie where the next segment's copies land: order those writes before the copy engine's
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -1153,7 +1158,7 @@ __global__ void __launch_bounds__(kMmaThreads, TqSmallCfg<T, D, BITS>::kMinBlock
   const int b = blockIdx.z;
   const RowChunks row = row_chunks(p, b);
   if ((int)blockIdx.x < p.num_window_chunks) {
-    tq_window_chunk<T, D, 1>(p, smem_raw, row, b, blockIdx.y, gridDim.y, blockIdx.x, true);
+    tq_window_chunk<T, D, 1, kMergeHeads<D, kPair>>(p, smem_raw, row, b, blockIdx.y, gridDim.y, blockIdx.x, true);
     return;
   }
   const int chunk = (int)blockIdx.x - p.num_window_chunks;
@@ -1177,6 +1182,9 @@ template <typename T, int D, int BITS, bool kPair>
 __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
     tq_decode_balanced_mma_kernel(const TqDecodeParams p, const int batch) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
+  // This instance has no registers for the loads of two columns and issues them one after the other (two rows of 12000 tokens,
+  // 16/2 heads: 44.7 us, one column after the other 32.4; one of 20000, 64/8 heads: 45.7 and 36.2).
+  constexpr MergeLoads kMerge = D == 128 && BITS == 3 && !kPair ? MergeLoads::kOneColumn : MergeLoads::kAllColumns;
   const int units = p.kv_heads * ((p.groups + 7) / 8);
   init_packed_barriers<T, D, BITS>(smem_raw);
   PackedRing ring{0, 0u, false};
@@ -1186,8 +1194,8 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
       [](int) {},  // rows without packed tokens belong to the window kernel
       [&](int b, int unit, int t0, int t1, int slot, int partials) {
         const int active_window = (p.residual_len + p.chunk_tokens - 1) / p.chunk_tokens;  // the window of this row is full
-        tq_packed_segment<T, D, BITS, kPair>(p, smem_raw, qc, ring, b, unit, units, t0, t1, active_window + slot,
-                                      active_window + partials, partials);
+        tq_packed_segment<T, D, BITS, kPair, kMerge>(p, smem_raw, qc, ring, b, unit, units, t0, t1, active_window + slot,
+                                                     active_window + partials, partials);
       },
       p.residual_len, kMmaWarps * TqMmaCfg<T, D, BITS>::kTilesPerStep, kTqSegmentTiles, kTqSegmentTiles);
   wait_for_prior_grids();

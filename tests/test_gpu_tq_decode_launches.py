@@ -74,3 +74,10 @@ def test_query_rows_at_odd_elements(cuda_device, dim, bits, heads, lengths):
         cache.turboquant_single_token_decode_attention(0, query, **args, output=local, peer_outputs=(peer.data_ptr(),))
         assert_close(local, dense_attention(cache, query, lengths, dim ** -0.5), torch.bfloat16)
         assert torch.equal(local, peer)
+
+
+@pytest.mark.parametrize("dim,heads,bits", [(128, 16, 3), (128, 10, 2), (256, 8, 3), (256, 6, 4), (256, 10, 2), (256, 16, 4)])
+def test_merges_of_groups_that_fill_the_threads_or_not(cuda_device, dim, heads, bits):
+    """The last CTA's threads have one, two or four columns of four dims of the group, read side by side where an instance has
+    the registers; 2 KV heads, so that one long row leaves many partials to merge."""
+    check(cuda_device, [12000, 11000], heads=heads, kv_heads=2, dim=dim, bits=bits)
