@@ -16,6 +16,12 @@ int set_error(int code, const char* fmt, ...) {
   return code;
 }
 
+std::mutex& launch_lock(cudaStream_t stream) {
+  static std::mutex locks[64];  // streams that share one lose nothing but a moment
+  const uintptr_t handle = reinterpret_cast<uintptr_t>(stream);
+  return locks[(handle >> 4 ^ handle >> 10 ^ handle >> 16) % 64];
+}
+
 struct CombineParams {
   const float* stats;
   const float* values;

@@ -8,6 +8,7 @@
 
 #include <cstdarg>
 #include <cstdio>
+#include <mutex>
 
 #include "../../include/anna_b200_kv.h"
 
@@ -17,6 +18,10 @@ namespace anna {
 // host-side status plumbing
 
 int set_error(int code, const char* fmt, ...);  // formats into the thread-local message, returns `code`
+
+// Held while the launches of one call go out that hand partials to one another in scratch.  Callers keep that scratch per stream,
+// and host threads may share a stream (all of them do by default): the launches of two calls must not mix.
+std::mutex& launch_lock(cudaStream_t stream);
 
 // Addresses that kernels read with wide loads are checked where the strides are: a view may start at any element.
 inline bool aligned_to(const void* address, size_t bytes) { return reinterpret_cast<uintptr_t>(address) % bytes == 0; }

@@ -133,6 +133,7 @@ static int run_dense_decode(DenseDecodeParams p, const void* gate, int64_t gate_
   p.chunk_tokens = chunk_tokens;
   p.num_chunks = num_chunks;
   p.chunk_capacity = chunk_capacity;
+  const std::lock_guard<std::mutex> together(launch_lock(stream));
   if (dense_split_mma_applicable(p, head_dim, dtype)) {
     if (split_counters != nullptr && num_chunks <= kFusedMaxChunks) {
       p.fused = FusedCombine{split_counters, out, out_stride_b, out_stride_h, gate, gate_stride_b, gate_stride_h};

@@ -412,6 +412,7 @@ static int tq_paged_decode_impl(const void* q, int64_t q_stride_b, int64_t q_str
                       (reinterpret_cast<uintptr_t>(query_scratch) & 15u) == 0;
     p.query_frags = fits ? query_scratch : nullptr;
   }
+  const std::lock_guard<std::mutex> together(launch_lock((cudaStream_t)stream));
   if (tq_split_mma_applicable(p, batch, head_dim, dtype)) {
     const bool umma = tq_split_umma_applicable(p, head_dim, bits, dtype);
     p.window_arrives = umma;

@@ -218,6 +218,7 @@ extern "C" int anna_gqa_decode_turboquant_values(
   p.stats = ws.stats; p.values = ws.values;
   p.chunk_tokens = ct; p.num_chunks = chunks; p.chunk_capacity = chunk_capacity;
   const int gpad = padded_group(p.groups);
+  const std::lock_guard<std::mutex> together(launch_lock((cudaStream_t)stream));
   rc = ANNA_DISPATCH_DTYPE(dtype, T, [&]() -> int {
     return ANNA_DISPATCH_DIM(head_dim, D, [&]() -> int {
       return ANNA_DISPATCH_GROUP(gpad, G, [&]() -> int {

@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import sys
+import threading
 from types import SimpleNamespace
 
 import pytest
@@ -167,3 +168,45 @@ def test_scratch_follows_its_buffers(cuda_device):
     scratch.get(torch.device(cuda_device), 2 * max(buf.numel() for buf in scratch._buffers.values()) + 1)
     assert not fused_ops._SPLIT_CACHE
     assert torch.equal(call(300), before)
+
+
+@pytest.mark.gpu
+def test_two_threads_on_one_stream(cuda_device):
+    """The module gives up the interpreter lock while it launches.  Calls of two threads on one stream share its scratch: the
+    launches of a call that hand it partials must not mix with the other's."""
+    problems = []
+    for seed, dtype in ((5, torch.bfloat16), (6, torch.bfloat16)):
+        gen = torch.Generator(device=cuda_device).manual_seed(seed)
+        cache = Qwen3DynamicCache(KVCacheConfig(num_hidden_layers=1, cache_block_size=16), batch_size=24,
+                                  kv_cache_quantization="turboquant", kv_cache_quant_bits=4, kv_cache_residual_len=128)
+        k, v = (torch.randn(24, 8, 700, 128, generator=gen, device=cuda_device).to(dtype) for _ in range(2))
+        cache.update(k, v, 0, require_dense_cache=False)
+        q = torch.randn(24, 32, 1, 128, generator=gen, device=cuda_device).to(dtype)
+
+        def call(cache=cache, q=q):
+            return cache.turboquant_single_token_decode_attention(0, q, scaling=0.1, num_key_value_groups=4)
+
+        problems.append((call, call()))
+    torch.cuda.synchronize(cuda_device)
+    wrong = [torch.zeros((), dtype=torch.int64, device=cuda_device) for _ in problems]
+    start = threading.Barrier(len(problems))
+    errors = []
+
+    def work(i):
+        try:
+            call, want = problems[i]
+            start.wait()
+            for _ in range(60):
+                outputs = [call() for _ in range(20)]
+                for out in outputs:
+                    wrong[i].add_((out != want).any())
+        except Exception as exc:  # a thread's exception is the test's
+            errors.append(exc)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(problems))]
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    assert not errors, errors
+    assert [int(count) for count in wrong] == [0, 0]
