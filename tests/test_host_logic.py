@@ -386,34 +386,78 @@ def test_turboquant_clone_shares_packed_pages_until_the_partial_block_is_written
     assert pool.used_pages() == 4 and all(pool.page_owners(pid) == 1 for t in tables for pid in t)
 
 
-def test_one_pass_release_equals_page_by_page_release():
-    """release_many (both its all-private fast path and its general path) leaves the free list, the owner counts and
-    the callbacks exactly as releasing the pages one by one does (ops.py:214-233 semantics: unknown ids are ignored,
-    a shared page only loses an owner)."""
+class PageModel:
+    """The page book restated page by page (allocator, ops.py:92-245): a page is taken from the end of the free list, the pool
+    grows by max(what is missing, capacity or 16), and a page goes back when its last owner lets go of it."""
+
+    def __init__(self):
+        self.free, self.owners, self.capacity, self.freed = [], {}, 0, []
+
+    def take(self, count):
+        out = []
+        while count > len(out) and self.free:
+            page = self.free.pop()
+            assert page not in self.owners
+            out.append(page)
+        missing = count - len(out)
+        if missing > 0:
+            first, self.capacity = self.capacity, self.capacity + max(missing, self.capacity or 16)
+            out += range(first, first + missing)
+            self.free += range(self.capacity - 1, first + missing - 1, -1)
+        for page in out:
+            self.owners[page] = 1
+        return out
+
+    def retain(self, page):
+        self.owners[page] = self.owners.get(page, 0) + 1
+
+    def release(self, page):
+        if page not in self.owners:
+            return
+        self.owners[page] -= 1
+        if self.owners[page] == 0:
+            del self.owners[page]
+            self.free.append(page)
+            self.freed.append(page)
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_page_book_equals_a_page_by_page_model(monkeypatch, native):
+    """Taking, growth, sharing and release in one pass leave the free list, the owners and the callbacks as the model does:
+    unknown ids are passed over, a shared page only loses an owner, an id may come twice.  In the call module and without it."""
     import random
 
-    from anna_b200.pools import _PageBook
+    from anna_b200 import pools
 
+    if not native:
+        monkeypatch.setattr(pools, "_NATIVE", False)
     rng = random.Random(3)
-    for case in range(40):
-        freed_a: list[int] = []
-        freed_b: list[int] = []
-        a, b = _PageBook(freed_a.append), _PageBook(freed_b.append)
-        for book in (a, b):
-            book.take(64, 0)
-        shared = rng.sample(range(64), rng.choice([0, 0, 3, 10]))
-        for page in shared:
-            a.retain(page)
-            b.retain(page)
-        for _ in range(4):
-            ids = rng.sample(range(80), rng.randint(1, 40))  # ids above 63 were never handed out
-            if rng.random() < 0.3:
-                ids = ids + ids[:2]                           # a page named twice in one call
-            a.release_many(list(ids))
-            for page in ids:
-                b.release(page)
-            assert a.free_pages == b.free_pages and a.refcount == b.refcount and freed_a == freed_b, case
-            assert a._shared == sum(1 for rc in a.refcount.values() if rc > 1)
+    for case in range(60):
+        model, freed, capacity = PageModel(), [], 0
+        book = pools._PageBook(freed.append)
+        for _ in range(12):
+            step = rng.random()
+            if step < 0.4:
+                count = rng.choice([0, 1, 2, 5, 17, 40])
+                pages, capacity, fresh = book.take(count, capacity)
+                assert pages == model.take(count) and fresh == pages[len(pages) - len(fresh):]
+            elif step < 0.6 and model.owners:
+                for page in rng.choices(sorted(model.owners), k=3):
+                    book.retain(page)
+                    model.retain(page)
+            else:
+                ids = [rng.randint(-2, capacity + 5) for _ in range(rng.randint(1, 40))]
+                if rng.random() < 0.3:
+                    ids = ids + ids[:2]
+                if len(ids) == 1:
+                    book.release(ids[0])
+                else:
+                    book.release_many(ids)
+                for page in ids:
+                    model.release(page)
+            assert capacity == model.capacity and book.free_pages == model.free and freed == model.freed, case
+            assert book.refcount == model.owners
+            assert book._shared == sum(1 for owners in model.owners.values() if owners > 1)
 
 
 def test_page_ids_are_any_integers():
