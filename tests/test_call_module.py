@@ -1,4 +1,5 @@
-"""The call module (csrc/launch_module.cpp): what it declines, and that the calls it takes give what the general path gives."""
+"""The call module (csrc/launch_module.cpp): which calls it takes and which it declines, and that those it takes give what the
+general path gives."""
 from __future__ import annotations
 
 import sys
@@ -18,10 +19,57 @@ class Declining:
         return lambda *args: None
 
 
+def install(monkeypatch, module):
+    monkeypatch.setattr(fused_ops, "_LAUNCH", module)
+    for caller in (attention, turboquant):
+        monkeypatch.setattr(caller, "launch_module", lambda: module)
+
+
 def general(monkeypatch):
-    monkeypatch.setattr(fused_ops, "_LAUNCH", Declining())
-    for module in (attention, turboquant):
-        monkeypatch.setattr(module, "launch_module", Declining)
+    install(monkeypatch, Declining())
+
+
+def rows_contiguous(*tensors):
+    return all(t is None or t.stride(-1) == 1 for t in tensors)
+
+
+# what the module takes of the calls in these tests, by the layouts of their arguments
+SERVED = {
+    "paged_decode": lambda query, keys, values, table, lengths, scaling, gate: rows_contiguous(query, table, lengths, gate),
+    "prefill": lambda query, keys, values, lengths, scaling, causal: (
+        rows_contiguous(query, keys, values) and keys.stride() == values.stride()
+        and all(stride % 8 == 0 for t in (query, keys) for stride in t.stride()[:3])),
+    "tq_append": lambda keys, values, *rest: rows_contiguous(keys) and keys.stride() == values.stride(),
+    "tq_decode": lambda query, gate, *rest: rows_contiguous(query, gate),
+}
+
+
+class Watched:
+    """The module; notes of every call whether it was taken, and that this is what SERVED says."""
+
+    def __init__(self):
+        self.module, self.taken = _lib.launch(), {name: [] for name in SERVED}
+
+    def __getattr__(self, name):
+        call = getattr(self.module, name)
+        if name not in SERVED:
+            return call
+
+        def watched(*args):
+            result = call(*args)
+            assert (result is not None) == SERVED[name](*args), name
+            self.taken[name].append(result is not None)
+            return result
+
+        return watched
+
+
+@pytest.fixture
+def watched(monkeypatch):
+    fused_ops.launch_module()
+    module = Watched()
+    install(monkeypatch, module)
+    return module
 
 
 def test_cpu_tensors_and_other_objects_are_declined():
@@ -73,7 +121,7 @@ def strided(shape, dtype, device, gen, order):
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("gate", [None, "4d", "4d_strided", "3d", "3d_strided"])
-def test_paged_decode_equals_general_path(cuda_device, dtype, gate):
+def test_paged_decode_equals_general_path(cuda_device, watched, dtype, gate):
     gen = torch.Generator(device=cuda_device).manual_seed(1)
     batch, heads, kv_heads, dim, page = 3, 8, 2, 128, 16
     for order in ((0, 1, 2, 3), (1, 0, 2, 3), (2, 0, 1, 3), (0, 1, 3, 2), (3, 0, 1, 2)):
@@ -95,11 +143,13 @@ def test_paged_decode_equals_general_path(cuda_device, dtype, gate):
                 general(patch)
                 assert torch.equal(out, fused_ops.run_paged_gqa_decode_fused(**args))
             assert out.is_contiguous() and out.shape == query.shape and out.dtype == dtype
+    taken = watched.taken["paged_decode"]
+    assert len(taken) == 15 and taken.count(True) == (0 if gate == "3d_strided" else 8)
 
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dim,query_len,key_len", [(64, 70, 200), (128, 5, 133), (256, 96, 96)])
-def test_prefill_equals_general_path(cuda_device, dim, query_len, key_len):
+def test_prefill_equals_general_path(cuda_device, watched, dim, query_len, key_len):
     gen = torch.Generator(device=cuda_device).manual_seed(2)
     for order in ((0, 1, 2, 3), (0, 2, 1, 3), (2, 0, 1, 3), (0, 1, 3, 2)):
         query = strided((2, 4, query_len, dim), torch.bfloat16, cuda_device, gen, order)
@@ -113,12 +163,14 @@ def test_prefill_equals_general_path(cuda_device, dim, query_len, key_len):
                     with pytest.MonkeyPatch.context() as patch:
                         general(patch)
                         assert torch.equal(out, attention.grouped_query_attention(query, keys, values, **args))
+    taken = watched.taken["prefill"]
+    assert len(taken) == 32 and taken.count(True) == 12
 
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype,dim", [(torch.bfloat16, 128), (torch.float16, 64), (torch.float32, 128)])
 @pytest.mark.parametrize("gated", [False, True])
-def test_cache_steps_equal_general_path(cuda_device, dtype, dim, gated):
+def test_cache_steps_equal_general_path(cuda_device, watched, dtype, dim, gated):
     """Prompt and decode steps over pages that run out, on two streams, with every layout of queries, keys and values."""
 
     def steps():
@@ -143,6 +195,7 @@ def test_cache_steps_equal_general_path(cuda_device, dtype, dim, gated):
         return [*outputs, *cache._gather_layer_cache(0)[:2]]
 
     ours = steps()
+    assert watched.taken["tq_decode"].count(True) >= 5 and watched.taken["tq_append"].count(True) >= 3
     with pytest.MonkeyPatch.context() as patch:
         general(patch)
         theirs = steps()
@@ -151,23 +204,41 @@ def test_cache_steps_equal_general_path(cuda_device, dtype, dim, gated):
 
 @pytest.mark.gpu
 def test_scratch_follows_its_buffers(cuda_device):
-    """A problem that needs larger scratch replaces the buffers; the one before must not go on with the old ones."""
+    """The module keeps the scratch of a problem and stream until a buffer behind it is replaced by a larger one."""
+    gen = torch.Generator(device=cuda_device).manual_seed(4)
+    query = torch.randn(1, 8, 1, 128, generator=gen, device=cuda_device, dtype=torch.float16)
+    keys, values = (torch.randn(19, 8, 16, 128, generator=gen, device=cuda_device, dtype=torch.float16) for _ in range(2))
+    args = dict(query=query, key_pages=keys, value_pages=values, scaling=0.1,
+                page_table=torch.arange(19, dtype=torch.int32, device=cuda_device)[None],
+                visible_lengths=torch.tensor([300], device=cuda_device))
+    asked = []
 
-    def call(length):
-        gen = torch.Generator(device=cuda_device).manual_seed(length)
-        blocks = (length + 15) // 16
-        query = torch.randn(1, 8, 1, 128, generator=gen, device=cuda_device, dtype=torch.float16)
-        keys, values = (torch.randn(blocks, 8, 16, 128, generator=gen, device=cuda_device, dtype=torch.float16)
-                        for _ in range(2))
-        table = torch.arange(blocks, dtype=torch.int32, device=cuda_device)[None]
-        return fused_ops.run_paged_gqa_decode_fused(query=query, key_pages=keys, value_pages=values, page_table=table,
-                                                    visible_lengths=torch.tensor([length], device=cuda_device), scaling=0.1)
+    def source(*problem):
+        asked.append(problem)
+        return fused_ops._scratch_source(*problem)
 
-    before = call(300)
-    scratch = fused_ops._SCRATCH
-    scratch.get(torch.device(cuda_device), 2 * max(buf.numel() for buf in scratch._buffers.values()) + 1)
-    assert not fused_ops._SPLIT_CACHE
-    assert torch.equal(call(300), before)
+    device, scratch = torch.device(cuda_device), fused_ops._SCRATCH
+    module = fused_ops.launch_module()
+    module.set_scratch_source(source)
+    try:
+        fused_ops._forget_scratch()
+        want = fused_ops.run_paged_gqa_decode_fused(**args)
+        assert len(asked) == 1
+        for replace, buffers in ((scratch.get, scratch._buffers), (scratch.counters, scratch._counters),
+                                 (scratch.bytes, scratch._byte_buffers)):
+            assert torch.equal(fused_ops.run_paged_gqa_decode_fused(**args), want) and len(asked) == 1
+            replace(device, 2 * max((buf.numel() for buf in buffers.values()), default=1 << 20) + 1)
+            assert torch.equal(fused_ops.run_paged_gqa_decode_fused(**args), want) and len(asked) == 2
+            assert asked.pop() == asked[0]
+        stream = torch.cuda.Stream(device)
+        stream.wait_stream(torch.cuda.current_stream(device))
+        with torch.cuda.stream(stream):
+            out = fused_ops.run_paged_gqa_decode_fused(**args)
+        torch.cuda.current_stream(device).wait_stream(stream)
+        assert torch.equal(out, want) and len(asked) == 2  # its own scratch
+    finally:
+        module.set_scratch_source(fused_ops._scratch_source)
+        fused_ops._forget_scratch()
 
 
 @pytest.mark.gpu
