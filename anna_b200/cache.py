@@ -9,7 +9,7 @@ reference's for the same sequence of calls.  What differs is where the bytes liv
   the new tokens of every row (``anna_paged_kv_write``) instead of per-row slice copies (ops.py:748-777);
 * TurboQuant layers keep *packed* pages ``uint8 [P, Hkv, chunk_bytes]`` plus a ring of the newest ``residual_len``
   tokens per sequence; one launch (``anna_tq_append``) does ring update, quantize-on-overflow, bit-packing and page
-  scatter for the whole batch, and one launch pair decodes the whole batch (``anna_tq_paged_decode``) instead of
+  scatter for the whole batch, and one or two launches decode the whole batch (``anna_tq_paged_decode``) instead of
   the per-row Python loops at ops.py:632 and :1057.  The reference never pages quantized rows (ops.py:903-904); the
   rule here is: quantized token ``j`` of a row lives in block ``j // S`` of the row's table, allocated from the
   layer's packed pool when the quantized length first reaches it.
@@ -773,7 +773,7 @@ class Qwen3DynamicCache:
                                                  num_key_value_groups: int, gate: torch.Tensor | None = None,
                                                  output: torch.Tensor | None = None,
                                                  peer_outputs: tuple[int, ...] = ()):
-        """One launch pair for the whole batch (ops.py:1024-1070 loops over rows).  ``output`` / ``peer_outputs``: see
+        """One or two launches for the whole batch (ops.py:1024-1070 loops over rows).  ``output`` / ``peer_outputs``: see
         ``launch_tq_decode`` (not part of the reference's signature; used by the KV-head-sharded layout)."""
         if not self.uses_turboquant_for_layer(layer_idx):
             raise ValueError(f"Layer {layer_idx} does not use TurboQuant-backed KV storage.")
