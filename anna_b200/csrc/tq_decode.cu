@@ -37,15 +37,29 @@ struct TqTokenRaw {
   T scale[CH], zero[CH];
 };
 
+// Single heads of 128 or 256 dims in 16 bits come here for pages that are no multiple of 16.  They have little to do for a token
+// besides finding it: four tokens a round leave too few CTAs, and a second division by the page size instead of a kept remainder
+// is felt (pages of 24, 8/8 heads, 3 bits, us with two tokens loaded one by one / four together, two divisions / so: 64 rows of
+// 900 tokens of 128 dims 95.4 / 106.8 / 92.7, 16 rows of 400 17.1 / 20.5 / 16.1, 64 rows of 2000 of 256 dims 422 / 406 / 364).
+template <typename T, int D, int G>
+constexpr bool kTqSingleHead = sizeof(T) == 2 && D >= 128 && G == 1;
+
 // Tokens a team scores together.  The kernel is a chain of loads (page id, then codes and metadata), so what counts for a
 // short context is how few rounds a chunk takes; wide groups and head slices have no registers for more than two.
-template <typename Cfg, int G>
-constexpr int kTqUnroll = G * Cfg::kDpl <= 16 ? 4 : 2;
+template <typename T, int D, int G>
+constexpr int kTqUnroll = G * DecodeCfg<T, D, G>::kDpl > 16 || kTqSingleHead<T, D, G> ? 2 : 4;
+
+// CTAs per SM that the narrowest instances leave registers for (0: as it comes).  As it comes they hold five, and calls of about
+// 600 to 1200 CTAs take a second wave for the rest (us with two tokens loaded one by one / as it comes / so: 16 rows of 400 tokens,
+// fp32, 16/8 heads of 64 16.7 / 18.6 / 15.6; one row of 8192, bf16, 8/8 heads of 64 20.2 / 21.4 / 19.7).  Batches that fill the
+// GPU lose a little of what four tokens gave them (64 rows of 4000, bf16, 8/8 heads of 64: 196 / 167.3 / 169.4).
+template <typename T, int D, int G>
+constexpr int kTqMinBlocks = kTqSingleHead<T, D, G> && D == 128 ? 7 : DecodeCfg<T, D, G>::kDpl * G <= (D == 64 ? 8 : 4) ? 6 : 0;
 
 // kMerge: the CTA that finishes a (row, head group) last merges its partials (merges_in_split); a kernel of its own, as for
 // dense_decode_split_kernel.
 template <typename T, int D, int G, int BITS, bool kMerge>
-__global__ void __launch_bounds__(kDecodeThreads) tq_decode_split_kernel(const TqDecodeParams p) {
+__global__ void __launch_bounds__(kDecodeThreads, kTqMinBlocks<T, D, G>) tq_decode_split_kernel(const TqDecodeParams p) {
   using Cfg = DecodeCfg<T, D, G>;
   constexpr int E = D / 32;
   constexpr int M = BITS - 1;
@@ -97,17 +111,27 @@ __global__ void __launch_bounds__(kDecodeThreads) tq_decode_split_kernel(const T
   if (threadIdx.x < (1 << M)) sm_cent[threadIdx.x] = p.centroids[threadIdx.x];
 
   // page ids of the packed tokens are looked up one round ahead, the first ones before the queries are rotated
-  constexpr int U = kTqUnroll<Cfg, G>;
+  constexpr int U = kTqUnroll<T, D, G>;
   constexpr int kStep = kDecodeWarps * Cfg::kTpw * U;
   const int64_t q_end = min(t1, Lq);
   const int32_t* table_row = p.block_table + (int64_t)b * p.table_stride;
   int32_t pid[U];
+  int in_page[kTqSingleHead<T, D, G> ? U : 1];
   auto block_of = [&](int64_t t) { return p.block_shift >= 0 ? t >> p.block_shift : t / p.block_size; };
   auto look_up = [&](int64_t base) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int64_t t = base + u * Cfg::kTpw + sub;
-      pid[u] = t < q_end ? table_row[block_of(t)] : -1;
+      if constexpr (kTqSingleHead<T, D, G>) {
+        pid[u] = -1;
+        if (t < q_end) {
+          const int64_t block = block_of(t);
+          in_page[u] = (int)(t - block * p.block_size);
+          pid[u] = table_row[block];
+        }
+      } else {
+        pid[u] = t < q_end ? table_row[block_of(t)] : -1;
+      }
     }
   };
   const int64_t first = t0 + warp * (Cfg::kTpw * U);
@@ -181,7 +205,7 @@ __global__ void __launch_bounds__(kDecodeThreads) tq_decode_split_kernel(const T
         raw[u] = TqTokenRaw<T, Cfg::kCh>{};
         if (!valid[u]) continue;
         const int64_t t = base + u * Cfg::kTpw + sub;
-        const int tok = (int)(t - block_of(t) * p.block_size);
+        const int tok = kTqSingleHead<T, D, G> ? in_page[kTqSingleHead<T, D, G> ? u : 0] : (int)(t - block_of(t) * p.block_size);
         const uint8_t* chunk_ptr = p.pages + ((int64_t)pid[u] * p.kv_heads + kvh) * p.layout.chunk_bytes;
         raw[u].norm = __ldg(reinterpret_cast<const float*>(chunk_ptr + p.layout.off_knorm) + tok);
         raw[u].rnorm = __ldg(reinterpret_cast<const float*>(chunk_ptr + p.layout.off_krnorm) + tok);

@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from tests.test_gpu_tq_decode_schedules import WINDOW, assert_close, dense_attention, ragged_cache
-from tests.test_tq_schedule import CHUNKS, EVEN_SHARES, ONE_LAUNCH, way_of
+from tests.test_tq_schedule import CHUNKS, CUDA_CORES, EVEN_SHARES, ONE_LAUNCH, way_of
 
 pytestmark = pytest.mark.gpu
 
@@ -85,3 +85,12 @@ def test_merges_of_groups_that_fill_the_threads_or_not(cuda_device, dim, heads, 
     """The last CTA's threads have one, two or four columns of four dims of the group, read side by side where an instance has
     the registers; 2 KV heads, so that one long row leaves many partials to merge."""
     check(cuda_device, [12000, 11000], way=EVEN_SHARES, heads=heads, kv_heads=2, dim=dim, bits=bits)
+
+
+@pytest.mark.parametrize("page", [8, 24])
+@pytest.mark.parametrize("dim,bits", [(128, 2), (128, 3), (256, 4)])
+def test_single_heads_on_pages_that_are_no_multiple_of_16(cuda_device, page, dim, bits):
+    """The CUDA-core kernel looks page and place in the page up a round ahead: rounds that end inside a page, at its end and past
+    the last token."""
+    for lengths in ([WINDOW + 1], [WINDOW + page], [WINDOW + 2 * page + 1, 3, WINDOW, 700], [900, 40, 1, 333, 95]):
+        check(cuda_device, lengths, way=CUDA_CORES, heads=4, kv_heads=4, dim=dim, bits=bits, page=page, gated=bits == 3)
