@@ -1203,8 +1203,8 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
 
 // A call that is not small in the plan's chunks may be so in longer ones, up to this many tokens.  128 tokens are one step of a
 // CTA's warps, of which 64 leave half idle; 256 are two, which still costs less than the scan and the second launch of even
-// shares (one row of 4000 tokens, 32/8 heads, 4 bits: 18.5 us in shares, 14.3 so; of 8000 22.5 and 15.4; 4 rows of 1500, 8
-// heads, 3 bits 18.5 and 12.5; 6 rows of 0.3-1.5 K, 8/4 heads of 256 20.0 and 14.4).
+// shares (GPU time, one row of 4000 tokens, 32/8 heads, 4 bits: 17.4 us in shares, 12.0 so; of 8000 20.8 and 13.4; 4 rows of
+// 1500, 8 heads, 3 bits 16.4 and 11.7; 6 rows of 0.3-1.5 K, 8/4 heads of 256 17.5 and 13.0).
 constexpr int kTqSmallChunk = 256;
 
 static bool tq_fixed_chunks_only() {
@@ -1215,10 +1215,13 @@ static bool tq_fixed_chunks_only() {
   return disabled;
 }
 
-// A small call, whose chunks are resident at once, gains nothing from even shares and pays for the scan of the lengths (one
-// row of 260-2500 tokens, 8 heads, 3 bits: 16.4-18.5 us in shares, 12.3-14.5 in chunks; 4 rows of 500, 32/8 heads, 4 bits: 16.5
-// and 12.4), unless it waits for the last CTA's merge: even shares have half as many partials (one row of 6000 tokens, 16/2
-// heads of 256, 2 bits: 92 partials in four rounds 46 us, shares 34).  `resident` = CTAs that fit the GPU at once.
+// A small call, whose chunks are resident at once, gains nothing from even shares and pays for the scan of the lengths (GPU time,
+// one row of 260-2500 tokens, 8 heads, 3 bits: 13.9-16.4 us in shares, 9.9-12.7 in chunks; 4 rows of 500, 32/8 heads, 4 bits: 15.1
+// and 9.9), unless it waits for the last CTA's merge, which even shares give fewer partials (eight heads of 256, two KV heads, one
+// row of 6000 tokens: 92 partials of 64 tokens 31.7 us, shares 27.6; of 3712, 56 partials, 25.4 and 23.5; eight heads of 128, 120
+// partials, 24.0 and 21.9).  The limits are on the safe side: 50 partials of four heads of 128 would still gain (one row of 12928
+// tokens, 32/8 heads: 17.2 and 25.7), and 20 of eight heads of 256 (two of 5248, 32/4 heads: 21.8 and 31.1).
+// `resident` = CTAs that fit the GPU at once.
 static bool tq_small(const TqDecodeParams& p, int batch, int head_dim, int64_t ctas, int resident) {
   const int64_t chunks = p.num_chunks - p.num_window_chunks;
   const int rounds = (min(8, p.groups) * (head_dim / 4) + kMmaThreads - 1) / kMmaThreads;
