@@ -394,8 +394,12 @@ PyObject* plain_ints(PyObject* list) {
   }
   return ints;
 }
-// ids that fit no Py_ssize_t are clipped, and so belong to no page either
-Py_ssize_t page_id(PyObject* list, Py_ssize_t i) { return PyNumber_AsSsize_t(PyList_GET_ITEM(list, i), nullptr); }
+// of a plain int; -1, which is no page either, where it fits no Py_ssize_t
+Py_ssize_t page_id(PyObject* list, Py_ssize_t i) {
+  const Py_ssize_t id = PyLong_AsSsize_t(PyList_GET_ITEM(list, i));
+  if (id == -1) PyErr_Clear();
+  return id;
+}
 
 // take_pages(free, counts, count) -> the last `count` ids of `free`, last one first; they leave `free` with one owner each
 PyObject* take_pages(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
@@ -406,26 +410,31 @@ PyObject* take_pages(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "take_pages: more pages than are free");
     return nullptr;
   }
-  PyObject* taken = PyList_GetSlice(free_list, have - count, have);
-  PyObject* out = taken == nullptr || PyList_Reverse(taken) != 0 ? nullptr : plain_ints(taken);
-  Py_XDECREF(taken);
+  Ints counts(args[1]);
+  PyObject* out = counts.held ? PyList_New(count) : nullptr;
   if (out == nullptr) return nullptr;
-  {
-    Ints counts(args[1]);
-    Py_ssize_t id = 0;
-    bool ok = counts.held;
-    for (Py_ssize_t i = 0; ok && i < count; ++i) {
-      id = page_id(out, i);
-      ok = id >= 0 && id < counts.size() && counts.data()[id] == 0;
+  bool ok = true;
+  for (Py_ssize_t i = 0; ok && i < count; ++i) {
+    PyObject* id = PyList_GET_ITEM(free_list, have - 1 - i);
+    if (PyLong_CheckExact(id)) {
+      Py_INCREF(id);
+    } else {
+      id = PyNumber_Index(id);
+      ok = id != nullptr && PyList_GET_SIZE(free_list) == have;  // (an entry's __index__ may have done anything)
+      if (!ok && !PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "take_pages: the free list has changed");
     }
-    if (!ok && counts.held)
-      PyErr_Format(PyExc_RuntimeError, "Invariant violated: free list page %zd %s.", id,
-                   id >= 0 && id < counts.size() ? "has non-zero refcount" : "does not exist");
-    for (Py_ssize_t i = 0; ok && i < count; ++i) counts.data()[page_id(out, i)] = 1;
-    if (!ok || PyList_SetSlice(free_list, have - count, have, nullptr) != 0) {
-      Py_DECREF(out);
-      return nullptr;
-    }
+    if (id != nullptr) PyList_SET_ITEM(out, i, id);
+    if (!ok) break;
+    const Py_ssize_t page = page_id(out, i);
+    ok = page >= 0 && page < counts.size() && counts.data()[page] == 0;
+    if (!ok)
+      PyErr_Format(PyExc_RuntimeError, "Invariant violated: free list page %zd %s.", page,
+                   page >= 0 && page < counts.size() ? "has non-zero refcount" : "does not exist");
+  }
+  for (Py_ssize_t i = 0; ok && i < count; ++i) counts.data()[page_id(out, i)] = 1;
+  if (!ok || PyList_SetSlice(free_list, have - count, have, nullptr) != 0) {
+    Py_DECREF(out);
+    return nullptr;
   }
   return out;
 }
