@@ -143,7 +143,7 @@ __device__ __forceinline__ void fused_combine_tail(const FusedCombine& fc, int b
   } else if (kTwo && aligned && items > THREADS) {
     side_by_side(std::integral_constant<int, 2>{});
   } else if (aligned) {
-    for (int item = threadIdx.x; item < items; item += THREADS) {
+    auto column = [&](int item) {
       const int g = item / kCols, d = 4 * (item % kCols);
       const float* vals = values + (int64_t)g * chunk_capacity * D + d;
       const float* w = smem_weights + g * kFusedMaxChunks;
@@ -152,6 +152,13 @@ __device__ __forceinline__ void fused_combine_tail(const FusedCombine& fc, int b
       for (int c = 0; c < active_chunks; ++c)
         add(acc, __ldcg(reinterpret_cast<const float4*>(vals + (int64_t)c * D)), w[c]);
       store(g, d, acc);
+    };
+    // a loop also where no thread has a second column: the compiler makes the better code of it at head_dim 256 (16 packed rows of 201
+    // tokens, 4/2 heads: 11.7 us, 12.4 without), and the worse one at 128 (one of 4000, 32/8 heads: 14.1 and 13.6)
+    if constexpr (MERGE == MergeLoads::kOneColumn || D == 256) {
+      for (int item = threadIdx.x; item < items; item += THREADS) column(item);
+    } else {
+      if ((int)threadIdx.x < items) column(threadIdx.x);
     }
   }
   for (int item = threadIdx.x; !aligned && item < g_count * D; item += THREADS) {

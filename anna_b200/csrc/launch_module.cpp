@@ -487,17 +487,18 @@ PyObject* copy_pages(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     ok = false;
   }
   for (Py_ssize_t i = first; ok && i < last; ++i) {
-    if (i >= PySequence_Fast_GET_SIZE(ids)) {  // an entry's __index__ may have shortened the list
-      PyErr_SetString(PyExc_ValueError, "copy_pages: out of range");
-      ok = false;
-      break;
-    }
-    const long id = PyLong_AsLong(PySequence_Fast_GET_ITEM(ids, i));
-    if (id == -1 && PyErr_Occurred()) ok = false;
-    else if (id != (int32_t)id) {
+    PyObject* obj = PySequence_Fast_GET_ITEM(ids, i);
+    const long id = PyLong_AsLong(obj);
+    target.data()[i] = (int32_t)id;
+    if (id == (int32_t)id && id != -1 && PyLong_CheckExact(obj)) continue;
+    ok = !(id == -1 && PyErr_Occurred());
+    if (ok && id != (int32_t)id) {
       PyErr_SetString(PyExc_OverflowError, "copy_pages: page id does not fit 32 bits");
       ok = false;
-    } else target.data()[i] = (int32_t)id;
+    } else if (ok && PySequence_Fast_GET_SIZE(ids) < last) {  // an entry's __index__ may have shortened the list
+      PyErr_SetString(PyExc_ValueError, "copy_pages: out of range");
+      ok = false;
+    }
   }
   Py_DECREF(ids);
   if (!ok) return nullptr;
