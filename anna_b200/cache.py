@@ -26,7 +26,7 @@ import torch
 
 from . import _lib
 from .fused_ops import MetadataUploader, dtype_code, on_device, ptr, stream_ptr
-from .pools import Qwen3PagedLayerAllocator, TurboQuantLayerPool
+from .pools import Qwen3PagedLayerAllocator, TurboQuantLayerPool, native_page_ids
 from .prefix_block_cache import PrefixBlockPool
 from .turboquant import (VALID_KV_CACHE_QUANT_BITS, TurboQuantKVRow, launch_tq_append, launch_tq_decode,
                          launch_tq_gather_dense)
@@ -141,12 +141,19 @@ class _DeviceLengths:
     DEPTH = 4
     __slots__ = ("rows", "pos", "host", "slots_dev", "slots_host", "device")
 
-    def __init__(self, batch: int, device: torch.device) -> None:
-        self.rows = list(torch.zeros((self.DEPTH + 1, batch), dtype=torch.int64, device=device).unbind(0))
-        self.pos = self.DEPTH
-        self.host: list[int] | None = [0] * batch
+    def __init__(self, batch: int, device: torch.device, slots: list[int] | None = None) -> None:
+        """``slots``: of rows that are about to get their first tokens; they go up with the zeros, in one copy."""
         self.slots_dev: torch.Tensor | None = None
         self.slots_host: list[int] | None = None
+        if slots is None:
+            self.rows = list(torch.zeros((self.DEPTH + 1, batch), dtype=torch.int64, device=device).unbind(0))
+        else:
+            self.rows = list(torch.empty((self.DEPTH, batch), dtype=torch.int64, device=device).unbind(0))
+            zeros, self.slots_dev = MetadataUploader.for_device(device).upload([[0] * batch, slots]).unbind(0)
+            self.rows.append(zeros)
+            self.slots_host = list(slots)
+        self.pos = self.DEPTH
+        self.host: list[int] | None = [0] * batch
         self.device = device
 
     def current(self, lengths: list[int]) -> torch.Tensor | None:
@@ -368,10 +375,14 @@ class Qwen3DynamicCache:
             # host mirror of the device table; a full build goes up through the pinned staging ring in one copy
             host = np.full((batch_size, capacity), -1, dtype=np.int32)
             tq_rows = self.turboquant_rows[layer_idx] if self.uses_turboquant_for_layer(layer_idx) else None
+            native = native_page_ids()
             for row_idx, table in enumerate(tables):
                 if table:
                     row = None if tq_rows is None else tq_rows[row_idx]
-                    host[row_idx, : len(table)] = table if row is None else row.table_array()
+                    if row is not None and row._table_np is None and native:  # a new row: no array of its own yet
+                        native.copy_pages(table, 0, len(table), host[row_idx])
+                    else:
+                        host[row_idx, : len(table)] = table if row is None else row.table_array()
             if device.type == "cuda":
                 buffer = MetadataUploader.for_device(device).upload_i32(host.reshape(-1)).view(batch_size, capacity)
             else:  # host-side bookkeeping of a cache that holds no device memory
@@ -528,10 +539,11 @@ class Qwen3DynamicCache:
         self.allocator.release_pages(layer_idx, [shared])
         self._resync_row_from(layer_idx, batch_idx, blk)
 
-    def _device_lengths_of(self, layer_idx: int, batch_size: int, device: torch.device) -> _DeviceLengths:
+    def _device_lengths_of(self, layer_idx: int, batch_size: int, device: torch.device,
+                           slots: list[int] | None = None) -> _DeviceLengths:
         state = self._dev_lengths[layer_idx]
         if state is None or state.device != device or int(state.rows[0].shape[0]) != batch_size:
-            state = self._dev_lengths[layer_idx] = _DeviceLengths(batch_size, device)
+            state = self._dev_lengths[layer_idx] = _DeviceLengths(batch_size, device, slots)
         return state
 
     def _launch_page_write(self, layer: Qwen3PagedLayerAllocator, key_states, value_states, table_dev, past,
@@ -708,7 +720,7 @@ class Qwen3DynamicCache:
                 room = free
         pool.version += 1
         if device.type == "cuda":
-            state = self._device_lengths_of(layer_idx, batch_size, device)
+            state = self._device_lengths_of(layer_idx, batch_size, device, slots)
             past_lengths, new_lengths = state.before_append(past)
             slots_dev = state.slots(slots)
         else:  # bookkeeping only (the launch below refuses CPU tensors)

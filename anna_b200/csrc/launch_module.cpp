@@ -1,5 +1,5 @@
-// Python entry points of the calls a decode loop makes every step, on the C ABI of libanna_b200_kv.so, and the loops over
-// page ids behind the allocators (pools.py).
+// Python entry points of the calls a decode loop makes every step, on the C ABI of libanna_b200_kv.so, the uploads of small arrays
+// (fused_ops.py) and the loops over page ids behind the allocators (pools.py).
 //
 // A ctypes call converts some forty arguments one by one, and every address, size and stride among them costs a Python
 // call of its own: two thirds of the 18 us of host time of a decode call, whose GPU work for a few short rows takes no
@@ -10,6 +10,7 @@
 #include <Python.h>
 
 #include <ATen/Functions.h>
+#include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -17,8 +18,10 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <cstring>
 #include <map>
 #include <tuple>
+#include <vector>
 
 #include "anna_b200_kv.h"
 
@@ -361,6 +364,187 @@ PyObject* prefill(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
+// ---- uploads: small integer arrays go to the GPU through a ring of pinned host buffers, one asynchronous copy each ---------
+
+// The buffers of one device.  They are handed out in turn, under the interpreter lock; a buffer whose last copy is still under way
+// (sixteen uploads back: normally long done) is waited for without the lock, and is out of the ring for other threads meanwhile.
+struct UploadRing {
+  static constexpr int kSlots = 16;
+  int64_t capacity = -1;  // bytes of a buffer
+  at::Tensor buffers[kSlots];
+  cudaEvent_t done[kSlots] = {};
+  bool taken[kSlots] = {};
+  int next = 0;
+};
+std::map<int64_t, UploadRing>& upload_rings() {
+  static auto* rings = new std::map<int64_t, UploadRing>();
+  return *rings;
+}
+
+at::Tensor pinned_bytes(int64_t bytes) { return at::empty({bytes}, at::TensorOptions().dtype(at::kByte).pinned_memory(true)); }
+
+// A tensor of `sizes` with the `bytes` at `data` on the device, ordered on its current stream (the device must be current).
+at::Tensor upload_bytes(c10::DeviceIndex device, const void* data, int64_t bytes, at::IntArrayRef sizes, at::ScalarType type) {
+  UploadRing& ring = upload_rings()[device];
+  int slot = -1;
+  while (slot < 0) {
+    for (int i = 0; i < UploadRing::kSlots && slot < 0; ++i) {
+      const int candidate = (ring.next + i) % UploadRing::kSlots;
+      if (!ring.taken[candidate]) slot = candidate;
+    }
+    if (slot < 0) pybind11::gil_scoped_release others;  // as many threads wait for a buffer each
+  }
+  ring.next = (slot + 1) % UploadRing::kSlots;
+  struct Taken {
+    bool* flag;
+    explicit Taken(bool* f) : flag(f) { *flag = true; }
+    ~Taken() { *flag = false; }
+  } taken(&ring.taken[slot]);
+  if (bytes > ring.capacity) {
+    // all buffers at once, so that an upload under a graph capture, which may not allocate, finds its own
+    ring.capacity = std::max<int64_t>(8192, 2 * bytes);
+    for (int i = 0; i < UploadRing::kSlots; ++i) {
+      if (ring.taken[i] && i != slot) continue;
+      if (ring.done[i] == nullptr) C10_CUDA_CHECK(cudaEventCreateWithFlags(&ring.done[i], cudaEventDisableTiming));
+      C10_CUDA_CHECK(cudaEventSynchronize(ring.done[i]));
+      ring.buffers[i] = pinned_bytes(ring.capacity);
+    }
+  } else {
+    pybind11::gil_scoped_release waiting;
+    C10_CUDA_CHECK(cudaEventSynchronize(ring.done[slot]));
+  }
+  at::Tensor& buffer = ring.buffers[slot];
+  if (buffer.numel() < bytes) buffer = pinned_bytes(ring.capacity);  // it was another thread's when the others grew
+  std::memcpy(buffer.data_ptr(), data, (size_t)bytes);
+  at::Tensor out = at::empty(sizes, at::TensorOptions().dtype(type).device(c10::Device(c10::kCUDA, device)));
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(device).stream();
+  if (bytes > 0) C10_CUDA_CHECK(cudaMemcpyAsync(out.data_ptr(), buffer.data_ptr(), (size_t)bytes, cudaMemcpyHostToDevice, stream));
+  C10_CUDA_CHECK(cudaEventRecord(ring.done[slot], stream));
+  return out;
+}
+
+// upload(device index, rows) -> int64 [len(rows), len(rows[0])] on the device
+PyObject* upload(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 2) return PyErr_Format(PyExc_TypeError, "upload(device, rows)");
+  const long device = PyLong_AsLong(args[0]);
+  if (device == -1 && PyErr_Occurred()) return nullptr;
+  PyObject* rows = PySequence_Fast(args[1], "upload: rows must be a sequence");
+  if (rows == nullptr) return nullptr;
+  std::vector<int64_t> values;
+  const Py_ssize_t n = PySequence_Fast_GET_SIZE(rows);
+  Py_ssize_t width = 0;
+  bool ok = n > 0;
+  if (!ok) PyErr_SetString(PyExc_ValueError, "upload: no rows");
+  for (Py_ssize_t r = 0; ok && r < n; ++r) {
+    PyObject* row = PySequence_Fast(PySequence_Fast_GET_ITEM(rows, r), "upload: a row must be a sequence");
+    ok = row != nullptr;
+    if (!ok) break;
+    const Py_ssize_t count = PySequence_Fast_GET_SIZE(row);
+    if (r == 0) {
+      width = count;
+      values.reserve((size_t)(n * width));
+    }
+    ok = count == width;
+    if (!ok) PyErr_SetString(PyExc_ValueError, "upload: rows of different lengths");
+    for (Py_ssize_t i = 0; ok && i < count; ++i) {
+      if (i >= PySequence_Fast_GET_SIZE(row)) {  // an entry's __index__ may have shortened the list
+        PyErr_SetString(PyExc_ValueError, "upload: rows of different lengths");
+        ok = false;
+        break;
+      }
+      PyObject* entry = PySequence_Fast_GET_ITEM(row, i);
+      int64_t value;
+      if (PyLong_CheckExact(entry)) {
+        value = PyLong_AsLongLong(entry);
+      } else {
+        Py_INCREF(entry);
+        PyObject* id = PyNumber_Index(entry);
+        Py_DECREF(entry);
+        value = id == nullptr ? -1 : PyLong_AsLongLong(id);
+        Py_XDECREF(id);
+      }
+      ok = !(value == -1 && PyErr_Occurred());
+      values.push_back(value);
+    }
+    Py_DECREF(row);
+  }
+  Py_DECREF(rows);
+  if (!ok) return nullptr;
+  const c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+  return THPVariable_Wrap(upload_bytes((c10::DeviceIndex)device, values.data(), (int64_t)values.size() * 8, {(int64_t)n, (int64_t)width}, at::kLong));
+  END_HANDLE_TH_ERRORS
+}
+
+// upload_i32(device index, contiguous int32 buffer) -> int32 [count] on the device
+PyObject* upload_i32(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 2) return PyErr_Format(PyExc_TypeError, "upload_i32(device, buffer)");
+  const long device = PyLong_AsLong(args[0]);
+  if (device == -1 && PyErr_Occurred()) return nullptr;
+  struct View {
+    Py_buffer view{};
+    bool held = false;
+    ~View() {
+      if (held) PyBuffer_Release(&view);
+    }
+  } buffer;
+  buffer.held = PyObject_GetBuffer(args[1], &buffer.view, PyBUF_C_CONTIGUOUS) == 0;
+  if (!buffer.held) return nullptr;
+  if (buffer.view.itemsize != 4) return PyErr_Format(PyExc_TypeError, "upload_i32: 32-bit integers expected");
+  const c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+  return THPVariable_Wrap(upload_bytes((c10::DeviceIndex)device, buffer.view.buf, buffer.view.len, {(int64_t)(buffer.view.len / 4)}, at::kInt));
+  END_HANDLE_TH_ERRORS
+}
+
+// tq_gather_dense(packed_pages | None, table | None, window, slots, lengths, signs1, signs2, centroids, max_len, block_size,
+//                 residual_len, bits, value_group, num_pages) -> (keys, values) | None
+PyObject* tq_gather_dense(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 14) return PyErr_Format(PyExc_TypeError, "tq_gather_dense takes 14 arguments");
+  bool ok = true;
+  const at::Tensor* pages = optional_tensor(args[0], &ok);
+  const at::Tensor* table = optional_tensor(args[1], &ok);
+  const at::Tensor* fixed[6];  // window, slots, lengths, signs1, signs2, centroids
+  for (int i = 0; i < 6; ++i) {
+    fixed[i] = tensor(args[2 + i]);
+    ok = ok && fixed[i] != nullptr;
+  }
+  int64_t n[6];  // max_len, block_size, residual_len, bits, value_group, num_pages
+  if (!int_args(args + 8, 6, n)) return nullptr;
+  int code = 0;
+  if (!ok || !fixed[0]->is_cuda() || !plain(*fixed[0], fixed[0]->device(), 5) || !dtype_code(fixed[0]->scalar_type(), &code) ||
+      fixed[2]->dim() != 1 || fixed[2]->size(0) == 0 || fixed[1]->sizes() != fixed[2]->sizes() || n[0] <= 0)
+    Py_RETURN_NONE;
+  const c10::Device device = fixed[0]->device();
+  for (const at::Tensor* t : fixed)
+    if (!on(t, device)) Py_RETURN_NONE;
+  if (!on(pages, device) || !on(table, device)) Py_RETURN_NONE;
+  const c10::cuda::CUDAGuard guard(device);
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
+  const int64_t batch = fixed[2]->size(0), kv_heads = fixed[0]->size(2), dim = fixed[0]->size(4);
+  at::Tensor keys = at::empty({batch, kv_heads, n[0], dim}, fixed[0]->options());
+  at::Tensor values = at::empty(keys.sizes(), keys.options());
+  int status;
+  {
+    pybind11::gil_scoped_release unlocked;
+    status = anna_tq_gather_dense(
+        static_cast<const uint8_t*>(address(pages)), static_cast<const int32_t*>(address(table)),
+        table == nullptr ? 0 : table->stride(0), address(fixed[0]), static_cast<const int64_t*>(address(fixed[1])),
+        static_cast<const int64_t*>(address(fixed[2])), floats(fixed[3]), floats(fixed[4]), floats(fixed[5]), keys.data_ptr(),
+        values.data_ptr(), keys.stride(0), keys.stride(1), keys.stride(2), (int)batch, (int)kv_heads, (int)dim, (int)n[1],
+        (int)n[2], (int)n[3], (int)n[4], n[5], table == nullptr ? 0 : table->size(1), n[0], code, stream);
+  }
+  if (status != 0) return failed("anna_tq_gather_dense", status);
+  PyObject* pair = PyTuple_New(2);
+  if (pair == nullptr) return nullptr;
+  PyTuple_SET_ITEM(pair, 0, THPVariable_Wrap(std::move(keys)));
+  PyTuple_SET_ITEM(pair, 1, THPVariable_Wrap(std::move(values)));
+  if (PyTuple_GET_ITEM(pair, 0) == nullptr || PyTuple_GET_ITEM(pair, 1) == nullptr) Py_CLEAR(pair);
+  return pair;
+  END_HANDLE_TH_ERRORS
+}
+
 // ---- page book: free pages are a list of ints, last in first out; owners are int32 counts by page id --------------------
 
 struct Ints {  // a writable int32 buffer
@@ -514,6 +698,9 @@ PyMethodDef methods[] = {
     {"tq_decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(tq_decode)), METH_FASTCALL, nullptr},
     {"tq_append", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(tq_append)), METH_FASTCALL, nullptr},
     {"paged_decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(paged_decode)), METH_FASTCALL, nullptr},
+    {"upload", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(upload)), METH_FASTCALL, nullptr},
+    {"upload_i32", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(upload_i32)), METH_FASTCALL, nullptr},
+    {"tq_gather_dense", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(tq_gather_dense)), METH_FASTCALL, nullptr},
     {"prefill", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(prefill)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };

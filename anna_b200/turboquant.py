@@ -188,6 +188,11 @@ def launch_tq_gather_dense(pool: TurboQuantLayerPool, table_dev: torch.Tensor | 
         meta = MetadataUploader.for_device(device).upload([lengths, slots])
         lengths_dev = meta[0] if lengths_dev is None else lengths_dev
         slots_dev = meta[1] if slots_dev is None else slots_dev
+    dense = launch_module().tq_gather_dense(pool.packed_pages, table_dev, pool.window, slots_dev, lengths_dev, tables.signs1,
+                                            tables.signs2, tables.centroids, max_len, pool.block_size, pool.residual_len,
+                                            pool.bits, pool.value_group, pool.capacity())
+    if dense is not None:
+        return dense[0], dense[1], lengths_dev
     keys = torch.empty((batch, pool.kv_heads, max_len, pool.head_dim), dtype=pool.dtype, device=device)
     values = torch.empty_like(keys)
     table_stride = 0 if table_dev is None else table_dev.stride(0)

@@ -6,6 +6,7 @@ import sys
 import threading
 from types import SimpleNamespace
 
+import numpy as np
 import pytest
 import torch
 
@@ -200,6 +201,32 @@ def test_cache_steps_equal_general_path(cuda_device, watched, dtype, dim, gated)
         general(patch)
         theirs = steps()
     assert all(torch.equal(a, b) for a, b in zip(ours, theirs, strict=True))
+
+
+@pytest.mark.gpu
+def test_uploads(cuda_device):
+    """More uploads than the ring has buffers, behind work that keeps the copies waiting; growing ones; other integers."""
+    uploader = fused_ops.MetadataUploader.for_device(torch.device(cuda_device))
+    busy = torch.randn(4096, 4096, device=cuda_device)
+    for _ in range(4):
+        busy = busy @ busy * 1e-3
+    got, want = [], []
+    for i in range(40):
+        rows = [[i * 7 + j for j in range(1 + i * 60)], [-(2 ** 40) - i] * (1 + i * 60)]
+        got.append(uploader.upload(rows))
+        want.append(torch.tensor(rows))
+        words = np.arange(i * 50, i * 50 + 3000, dtype=np.int32)
+        got.append(uploader.upload_i32(words))
+        want.append(torch.from_numpy(words))
+    got += [uploader.upload([[np.int64(3), True]]), uploader.upload([(4,)]), uploader.upload([[]])]
+    want += [torch.tensor([[3, 1]]), torch.tensor([[4]]), torch.empty(1, 0, dtype=torch.int64)]
+    for ours, theirs in zip(got, want, strict=True):
+        assert ours.dtype == theirs.dtype and torch.equal(ours.cpu(), theirs)
+    for rows in ([], [[1, 2], [3]], [[1.5]], [["a"]], 7):
+        with pytest.raises((ValueError, TypeError)):
+            uploader.upload(rows)
+    with pytest.raises(TypeError):
+        uploader.upload_i32(np.zeros(3, dtype=np.int64))
 
 
 @pytest.mark.gpu
