@@ -58,3 +58,30 @@ def test_append_constant_and_zero_vectors(cuda_device):
     keys[:, :, 1] = 1.0
     pair.append(keys, values)
     pair.assert_bit_exact()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("bits", [2, 3, 4])
+@pytest.mark.parametrize("head_dim", [64, 128, 256])
+def test_append_of_chunks_is_bit_exact(cuda_device, dtype, bits, head_dim):
+    """Calls with many tokens hold several of them per warp: chunks that leave warps and the last page partly filled, that read
+    ring slots and rewrite them in the same call, on pages that are no power of two long; then single steps."""
+    pair = TqPair(device=cuda_device, batch=2, kv_heads=3, head_dim=head_dim, bits=bits, residual_len=40, block_size=24,
+                  dtype=dtype)
+    _run_schedule(pair, [333, 1, 171, 1], seed=200 + bits)
+    pair.assert_bit_exact()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_append_of_chunks_with_special_values(cuda_device, dtype):
+    """Zero and constant vectors, groups of equal values, zeros of both signs and ranges below the smallest scale."""
+    pair = TqPair(device=cuda_device, batch=1, kv_heads=4, head_dim=128, bits=4, residual_len=8, block_size=16, dtype=dtype)
+    gen = torch.Generator().manual_seed(5)
+    keys, values = (outlier_kv(gen, (1, 4, 300, 128), dtype) for _ in range(2))
+    keys[:, :, 0] = 0.0
+    values[:, :, 1] = 0.75
+    values[:, :, 2, 32:64] = -0.0
+    values[:, :, 3, ::2] = 0.0
+    values[:, :, 4] *= 1e-7
+    pair.append(keys, values)
+    pair.assert_bit_exact()
