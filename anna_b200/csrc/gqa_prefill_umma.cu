@@ -30,6 +30,7 @@
 #include "umma_utils.cuh"
 
 #include <cstdlib>
+#include <mutex>
 #include <type_traits>
 
 namespace anna {
@@ -129,7 +130,162 @@ __host__ __device__ inline int head_shift_of(int groups) {
   return shift;
 }
 
-template <typename T>
+// ---- keys shared by the CTAs of a cluster --------------------------------------------------------------------------------
+// With few query tiles (one user's chunk, few KV heads) most SMs would have none.  Then the CTAs of a cluster take the same
+// rows and a part of the keys each; every one leaves its unnormalised rows of O with their maxima and sums in its own shared
+// memory, and each merges a part of the rows by reading all of them over distributed shared memory: no workspace, no second
+// launch.  All CTAs of a cluster reach both cluster barriers, whatever became of their waits.
+//
+// A split CTA must have its SM's tensor memory to itself: two CTAs of two clusters that waited for each other's on two SMs
+// would wait for ever, so it asks for more than half of an SM's shared memory.
+constexpr int kMaxSplits = 16;  // the largest cluster
+constexpr uint32_t kSplitMinSmem = 120 * 1024;
+static_assert(2 * kSplitMinSmem > 228 * 1024, "two split CTAs fit one SM");
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_address(uint32_t smem, int rank) {
+  uint32_t addr;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem), "r"(rank));
+  return addr;
+}
+__device__ __forceinline__ float cluster_load(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_load4(uint32_t addr, float* v) {
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(addr) : "memory");
+}
+
+// Partial results of a CTA: rows of D floats, 4 apart in addition so that eight rows written at once (16 bytes each) fall
+// into different banks; then the maxima (log2 units) and the sums, and the weights of the rows that the CTA merges.
+template <int D, int ROWS>
+struct SplitParts {
+  static constexpr int kPitch = D + 4;
+  static constexpr uint32_t kOffMax = ROWS * kPitch * 4, kOffSum = kOffMax + ROWS * 4, kOffWeight = kOffSum + ROWS * 4;
+  static constexpr uint32_t kBytes = kOffWeight + (ROWS + kMaxSplits) * 4;
+  static constexpr uint32_t smem_bytes(uint32_t tiles) {
+    const uint32_t need = kBytes + 1024 > tiles ? kBytes + 1024 : tiles;
+    return need > kSplitMinSmem ? need : kSplitMinSmem;
+  }
+};
+
+// Thread = row: the row of O from tensor memory to shared memory, with its maximum and sum.  Called by whole warps; `any`: the
+// CTA had keys, `wanted`: the row exists.
+template <int D, int ROWS>
+__device__ __forceinline__ void split_store_row(uint8_t* parts, int r, uint32_t t_o, bool any, bool wanted, float m, float l) {
+  using Parts = SplitParts<D, ROWS>;
+  float* dst = reinterpret_cast<float*>(parts) + r * Parts::kPitch;
+  if (any && __any_sync(0xffffffffu, wanted)) {
+#pragma unroll 2
+    for (int c = 0; c < D / 32; ++c) {
+      uint32_t o[32];
+      tmem_ld32(t_o + 32 * c, o);
+      tmem_wait_ld();
+#pragma unroll
+      for (int i = 0; i < 8; ++i) reinterpret_cast<uint4*>(dst + 32 * c)[i] = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+    }
+  }
+  reinterpret_cast<float*>(parts + Parts::kOffMax)[r] = any ? m : -INFINITY;
+  reinterpret_cast<float*>(parts + Parts::kOffSum)[r] = any ? l : 0.0f;
+}
+
+// The weighted parts of a CTA's rows, a thread per four values of a row: kItems rows of a thread's column and kParts parts of them at
+// a time, whose loads are all under way together (remote loads take most of a microsecond).
+template <typename T, int D, int ROWS, int THREADS, int kItems, int kParts>
+__device__ __forceinline__ void split_merge_values(const PrefillParams& p, uint32_t parts, const float* weights, int rows, int rank,
+                                                   int m0, int positions, int hq0, int b) {
+  using Parts = SplitParts<D, ROWS>;
+  constexpr int kPieces = D / 4, kRowStep = THREADS / kPieces;
+  static_assert(THREADS % kPieces == 0, "a thread keeps its column");
+  const int splits = p.splits;
+  const int column = (int)threadIdx.x % kPieces * 4;
+  for (int i0 = (int)threadIdx.x / kPieces; i0 < rows; i0 += kItems * kRowStep) {
+    float acc[kItems][4];
+    bool on[kItems];
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+      const int i = i0 + k * kRowStep;
+      on[k] = i < rows && m0 + ((rank + splits * i) & (positions - 1)) < p.q_len;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[k][e] = 0.0f;
+    }
+    for (int s0 = 0; s0 < splits; s0 += kParts) {
+      float w[kItems][kParts], part[kItems][kParts][4];
+#pragma unroll
+      for (int j = 0; j < kParts; ++j) {
+        const uint32_t from = cluster_address(parts + column * 4, min(s0 + j, splits - 1));
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+          const int i = i0 + k * kRowStep;
+          w[k][j] = on[k] && s0 + j < splits ? weights[i * splits + s0 + j] : 0.0f;
+          if (w[k][j] != 0.0f) cluster_load4(from + (rank + splits * i) * Parts::kPitch * 4, part[k][j]);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kParts; ++j)
+#pragma unroll
+        for (int k = 0; k < kItems; ++k)
+          if (w[k][j] != 0.0f) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[k][e] = fmaf(w[k][j], part[k][j][e], acc[k][e]);
+          }
+    }
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+      if (!on[k]) continue;
+      const int r = rank + splits * (i0 + k * kRowStep);
+      T* out = reinterpret_cast<T*>(p.out) + b * p.out_stride_b + (int64_t)(hq0 + r / positions) * p.out_stride_h +
+               (int64_t)(m0 + (r & (positions - 1))) * p.out_stride_t + column;
+      *reinterpret_cast<uint2*>(out) = make_uint2(pack2<T>(acc[k][0], acc[k][1]), pack2<T>(acc[k][2], acc[k][3]));
+    }
+  }
+}
+
+// Merges rows rank, rank + splits, ... of the cluster's query tile; called by THREADS threads, the first of the CTA.  `parts` and
+// `mine` are the same place, as an address for the others' shared memory and as this CTA's pointer.
+template <typename T, int D, int ROWS, int THREADS>
+__device__ __forceinline__ void split_merge_rows(const PrefillParams& p, uint32_t parts, uint8_t* mine, int rank, int m0, int positions,
+                                                 int hq0, int b) {
+  using Parts = SplitParts<D, ROWS>;
+  const int splits = p.splits;
+  const int rows = (ROWS - rank + splits - 1) / splits;
+  float* weights = reinterpret_cast<float*>(mine + Parts::kOffWeight);
+  // a thread per row: weights of its parts, normalised
+  for (int i = threadIdx.x; i < rows; i += THREADS) {
+    const int r = rank + splits * i;
+    float m[kMaxSplits], l[kMaxSplits], top = -INFINITY, total = 0.0f;
+#pragma unroll
+    for (int s = 0; s < kMaxSplits; ++s) {
+      m[s] = -INFINITY;
+      l[s] = 0.0f;
+      if (s < splits) {
+        m[s] = cluster_load(cluster_address(parts + Parts::kOffMax + 4 * r, s));
+        l[s] = cluster_load(cluster_address(parts + Parts::kOffSum + 4 * r, s));
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < kMaxSplits; ++s) top = fmaxf(top, m[s]);
+#pragma unroll
+    for (int s = 0; s < kMaxSplits; ++s) {
+      // parts without a visible key hold nothing; a part of NaN scores has a NaN sum and no maximum, and counts
+      m[s] = l[s] != 0.0f ? (m[s] == -INFINITY ? 1.0f : up_ex2(m[s] - top)) : 0.0f;
+      total += m[s] * l[s];
+    }
+    const float inv = total > 0.0f ? 1.0f / total : (total == 0.0f ? 0.0f : total);
+#pragma unroll
+    for (int s = 0; s < kMaxSplits; ++s)
+      if (s < splits) weights[i * splits + s] = m[s] == 0.0f ? 0.0f : m[s] * inv;
+  }
+  asm volatile("bar.sync 1, %0;\n" ::"n"(THREADS) : "memory");
+  if (splits <= 3) split_merge_values<T, D, ROWS, THREADS, 8, 2>(p, parts, weights, rows, rank, m0, positions, hq0, b);
+  else split_merge_values<T, D, ROWS, THREADS, 4, 4>(p, parts, weights, rows, rank, m0, positions, hq0, b);
+}
+
+template <typename T, bool kSplit>
 __global__ void __launch_bounds__(kUpThreads, 1)
     gqa_prefill_umma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap map_q,
                             const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v) {
@@ -146,7 +302,9 @@ __global__ void __launch_bounds__(kUpThreads, 1)
   const int heads_here = 1 << head_shift;
   const int positions = kUpCtaRows >> head_shift;
   const int head_sets = p.groups >> head_shift;
-  const int m0 = (int)(gridDim.x - 1 - blockIdx.x) * positions;  // tiles with the most visible keys first
+  const int splits = kSplit ? p.splits : 1;  // the CTAs of a cluster are neighbours along x
+  const int rank = kSplit ? (int)blockIdx.x % splits : 0;
+  const int m0 = (int)((gridDim.x - 1 - blockIdx.x) / splits) * positions;  // tiles with the most visible keys first
   const int kvh = blockIdx.y / head_sets;
   const int hq0 = kvh * p.groups + (blockIdx.y % head_sets) * heads_here;
   const int b = blockIdx.z;
@@ -163,7 +321,9 @@ __global__ void __launch_bounds__(kUpThreads, 1)
   const int last_row = min(m0 + positions, p.q_len) - 1;
   int64_t cta_limit = p.causal ? min(n_keys, past + last_row + 1) : n_keys;
   cta_limit = max(cta_limit, (int64_t)0);
-  const int n_tiles = (int)((cta_limit + kUpKeys - 1) / kUpKeys);
+  const int all_tiles = (int)((cta_limit + kUpKeys - 1) / kUpKeys);
+  const int first_tile = kSplit ? (int)((int64_t)all_tiles * rank / splits) : 0;  // of this CTA's share of the keys
+  const int n_tiles = kSplit ? (int)((int64_t)all_tiles * (rank + 1) / splits) - first_tile : all_tiles;
   // key positions are tensor-map coordinates: they fit 32 bits
   const int n_keys32 = (int)min(n_keys, (int64_t)0x7fffffff);
   int lim = 0;  // keys this thread's row sees
@@ -172,8 +332,8 @@ __global__ void __launch_bounds__(kUpThreads, 1)
   T* out_row = reinterpret_cast<T*>(p.out) + b * p.out_stride_b + (int64_t)hq * p.out_stride_h +
                (int64_t)row * p.out_stride_t;
 
-  if (n_tiles == 0) {  // no row of this CTA sees a key: zeros (uniform over the CTA, nothing was allocated yet)
-    if (softmax && row < p.q_len)
+  if (all_tiles == 0) {  // no row of this CTA sees a key: zeros (uniform over the cluster, nothing was allocated yet)
+    if (rank == 0 && softmax && row < p.q_len)
       for (int c = 0; c < kUpDim / 8; ++c) reinterpret_cast<uint4*>(out_row)[c] = make_uint4(0u, 0u, 0u, 0u);
     return;
   }
@@ -226,7 +386,7 @@ __global__ void __launch_bounds__(kUpThreads, 1)
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kUpSoftmaxRegs));
   }
   if (!softmax) {
-    if (warp == kUpSoftmaxThreads / 32) {
+    if (warp == kUpSoftmaxThreads / 32 && (!kSplit || n_tiles > 0)) {
     // ---- issuing warp: the whole warp walks the loop, one elected lane issues -----------------------------------------
     constexpr uint32_t kFmt = std::is_same<T, __nv_bfloat16>::value ? kUmmaBF16 : kUmmaF16;
     constexpr uint32_t idesc_s = umma_idesc(kFmt, kFmt, false, false, kUpRows, kUpKeys);
@@ -248,16 +408,16 @@ __global__ void __launch_bounds__(kUpThreads, 1)
       if (tile >= n_tiles || !elect_one()) return;
       const uint32_t bar = bar_k0 + kStage * 8, dst = smem + kOffK + kStage * kKvBytes;
       mbar_expect_tx(bar, kKvBytes);
-      tma_load_4d(dst, &map_k, 0, tile * kUpKeys, kvh, b, bar);
-      tma_load_4d(dst + kKvBoxBytes, &map_k, 64, tile * kUpKeys, kvh, b, bar);
+      tma_load_4d(dst, &map_k, 0, (first_tile + tile) * kUpKeys, kvh, b, bar);
+      tma_load_4d(dst + kKvBoxBytes, &map_k, 64, (first_tile + tile) * kUpKeys, kvh, b, bar);
     };
     auto load_v = [&](auto stage_c, int tile) {
       constexpr int kStage = decltype(stage_c)::value;
       if (tile >= n_tiles || !elect_one()) return;
       const uint32_t bar = bar_v0 + kStage * 8, dst = smem + kOffV + kStage * kKvBytes;
       mbar_expect_tx(bar, kKvBytes);
-      tma_load_4d(dst, &map_v, 0, tile * kUpKeys, kvh, b, bar);
-      tma_load_4d(dst + kKvBoxBytes, &map_v, 64, tile * kUpKeys, kvh, b, bar);
+      tma_load_4d(dst, &map_v, 0, (first_tile + tile) * kUpKeys, kvh, b, bar);
+      tma_load_4d(dst + kKvBoxBytes, &map_v, 64, (first_tile + tile) * kUpKeys, kvh, b, bar);
     };
     // S_qt = Q_qt . K(stage)^T into the score columns of query tile qt
     auto issue_scores = [&](auto qt_c, auto stage_c) {
@@ -349,7 +509,7 @@ __global__ void __launch_bounds__(kUpThreads, 1)
     float m_run = -INFINITY, l_run = 0.0f;
     bool ok = true;
     for (int it = 0; it < n_tiles; ++it) {
-      const int key0 = it * kUpKeys;  // first key of the tile
+      const int key0 = (first_tile + it) * kUpKeys;  // first key of the tile
       const int visible = max(0, min(kUpKeys, lim - key0));  // keys of the tile this row sees
       constexpr int kChunk = 32;  // score columns per tensor-memory load
       ok = wait(my_s, it);
@@ -453,8 +613,14 @@ __global__ void __launch_bounds__(kUpThreads, 1)
       if (lane == 0 && key0 + kUpKeys > n_keys32) mbar_arrive(my_p + kBarHalf);
       if (lane == 0) mbar_arrive(my_p);
     }
-    if (ok) ok = wait(my_o, n_tiles - 1);
-    if (ok) {
+    if (ok && (!kSplit || n_tiles > 0)) ok = wait(my_o, n_tiles - 1);
+    if constexpr (kSplit) {
+      // the partial results lie where the operands were: every product of the CTA has to be complete
+      tcgen05_fence_after_sync();
+      asm volatile("bar.sync 1, %0;\n" ::"n"(kUpSoftmaxThreads) : "memory");
+      split_store_row<kUpDim, kUpCtaRows>(smem_raw + (smem - smem_u32(smem_raw)), r_local, t_o, ok && n_tiles > 0, row < p.q_len, m_run,
+                                                l_run);
+    } else if (ok) {
       tcgen05_fence_after_sync();
       const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f;
 #pragma unroll
@@ -482,6 +648,13 @@ __global__ void __launch_bounds__(kUpThreads, 1)
   __syncthreads();
   if (threadIdx.x == 0 && abort_flag != 0) atomicAdd(&g_prefill_umma_faults, 1);
   if (warp == 0) tmem_free(tmem, kTmemCols);
+  if constexpr (kSplit) {
+    cluster_barrier();
+    // by the warps that kept their registers
+    if (softmax)
+      split_merge_rows<T, kUpDim, kUpCtaRows, kUpSoftmaxThreads>(p, smem, smem_raw + (smem - smem_u32(smem_raw)), rank, m0, positions, hq0, b);
+    cluster_barrier();  // the others read this CTA's shared memory
+  }
 }
 
 // ---- head_dim 256 ------------------------------------------------------------------------------------------------------
@@ -510,7 +683,7 @@ struct WideCfg {
   static_assert(kColQ + D / 2 <= kColsPerQTile && QT * kColsPerQTile <= 512, "tensor memory layout");
 };
 
-template <typename T, int D, int QT>
+template <typename T, int D, int QT, bool kSplit>
 __global__ void __launch_bounds__((WideCfg<D, QT>::kThreads), 1)
     gqa_prefill_umma_wide_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap map_q,
                                const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v) {
@@ -529,7 +702,9 @@ __global__ void __launch_bounds__((WideCfg<D, QT>::kThreads), 1)
   const int heads_here = 1 << head_shift;
   const int positions = Cfg::kCtaRows >> head_shift;
   const int head_sets = p.groups >> head_shift;
-  const int m0 = (int)(gridDim.x - 1 - blockIdx.x) * positions;  // tiles with the most visible keys first
+  const int splits = kSplit ? p.splits : 1;  // the CTAs of a cluster are neighbours along x
+  const int rank = kSplit ? (int)blockIdx.x % splits : 0;
+  const int m0 = (int)((gridDim.x - 1 - blockIdx.x) / splits) * positions;  // tiles with the most visible keys first
   const int kvh = blockIdx.y / head_sets;
   const int hq0 = kvh * p.groups + (blockIdx.y % head_sets) * heads_here;
   const int b = blockIdx.z;
@@ -545,15 +720,17 @@ __global__ void __launch_bounds__((WideCfg<D, QT>::kThreads), 1)
   const int last_row = min(m0 + positions, p.q_len) - 1;
   int64_t cta_limit = p.causal ? min(n_keys, past + last_row + 1) : n_keys;
   cta_limit = max(cta_limit, (int64_t)0);
-  const int n_tiles = (int)((cta_limit + kWdKeys - 1) / kWdKeys);
+  const int all_tiles = (int)((cta_limit + kWdKeys - 1) / kWdKeys);
+  const int first_tile = kSplit ? (int)((int64_t)all_tiles * rank / splits) : 0;  // of this CTA's share of the keys
+  const int n_tiles = kSplit ? (int)((int64_t)all_tiles * (rank + 1) / splits) - first_tile : all_tiles;
   const int n_keys32 = (int)min(n_keys, (int64_t)0x7fffffff);
   int lim = 0;  // keys this thread's row sees
   if (row < p.q_len) lim = (int)max((int64_t)0, p.causal ? min((int64_t)n_keys32, past + row + 1) : (int64_t)n_keys32);
   T* out_row = reinterpret_cast<T*>(p.out) + b * p.out_stride_b + (int64_t)hq * p.out_stride_h +
                (int64_t)row * p.out_stride_t;
 
-  if (n_tiles == 0) {  // no row of this CTA sees a key: zeros (uniform over the CTA, nothing was allocated yet)
-    if (warp < kSoftmaxWarps && row < p.q_len)
+  if (all_tiles == 0) {  // no row of this CTA sees a key: zeros (uniform over the cluster, nothing was allocated yet)
+    if (rank == 0 && warp < kSoftmaxWarps && row < p.q_len)
       for (int c = 0; c < kWdDim / 8; ++c) reinterpret_cast<uint4*>(out_row)[c] = make_uint4(0u, 0u, 0u, 0u);
     return;
   }
@@ -611,7 +788,7 @@ __global__ void __launch_bounds__((WideCfg<D, QT>::kThreads), 1)
       mbar_expect_tx(bar, kWdKvBytes);
 #pragma unroll
       for (int i = 0; i < kWdDim / 64; ++i)
-        tma_load_4d(dst + i * kWdKvBoxBytes, keys ? &map_k : &map_v, 64 * i, t * kWdKeys, kvh, b, bar);
+        tma_load_4d(dst + i * kWdKvBoxBytes, keys ? &map_k : &map_v, 64 * i, (first_tile + t) * kWdKeys, kvh, b, bar);
     };
     bool ok = true;
     auto produce = [&](auto stage_c, int t) {
@@ -627,7 +804,7 @@ __global__ void __launch_bounds__((WideCfg<D, QT>::kThreads), 1)
       produce(Zero{}, t);
       if (ok && t + 1 < n_tiles) produce(One{}, t + 1);
     }
-  } else if (warp == kSoftmaxWarps) {
+  } else if (warp == kSoftmaxWarps && (!kSplit || n_tiles > 0)) {
     // ---- products -----------------------------------------------------------------------------------------------------
     constexpr uint32_t kFmt = std::is_same<T, __nv_bfloat16>::value ? kUmmaBF16 : kUmmaF16;
     constexpr uint32_t idesc_s = umma_idesc(kFmt, kFmt, false, false, kWdRows, kWdKeys);
@@ -713,7 +890,7 @@ __global__ void __launch_bounds__((WideCfg<D, QT>::kThreads), 1)
     float m_run = -INFINITY, l_run = 0.0f;
     bool ok = true;
     for (int it = 0; it < n_tiles; ++it) {
-      const int key0 = it * kWdKeys;
+      const int key0 = (first_tile + it) * kWdKeys;
       const int visible = max(0, min(kWdKeys, lim - key0));
       const uint32_t t_s = t_lane + kWdColS + (it & 1) * kWdKeys;
       ok = wait(my_s0 + (it & 1) * 8, it >> 1);
@@ -800,8 +977,13 @@ __global__ void __launch_bounds__((WideCfg<D, QT>::kThreads), 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(my_p0 + (it & 1) * 8);
     }
-    if (ok) ok = wait(my_o0 + ((n_tiles - 1) & 1) * 8, (n_tiles - 1) >> 1);
-    if (ok) {
+    if (ok && (!kSplit || n_tiles > 0)) ok = wait(my_o0 + ((n_tiles - 1) & 1) * 8, (n_tiles - 1) >> 1);
+    if constexpr (kSplit) {
+      tcgen05_fence_after_sync();
+      asm volatile("bar.sync 1, %0;\n" ::"n"(kSoftmaxWarps * 32) : "memory");  // as in the other kernel
+      split_store_row<kWdDim, Cfg::kCtaRows>(smem_raw + (smem - smem_u32(smem_raw)), r_local, t_o, ok && n_tiles > 0, row < p.q_len, m_run,
+                                                l_run);
+    } else if (ok) {
       tcgen05_fence_after_sync();
       const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f;
 #pragma unroll 4
@@ -829,11 +1011,31 @@ __global__ void __launch_bounds__((WideCfg<D, QT>::kThreads), 1)
   __syncthreads();
   if (threadIdx.x == 0 && abort_flag != 0) atomicAdd(&g_prefill_umma_faults, 1);
   if (warp == 0) tmem_free(tmem, kWdTmemCols);
+  if constexpr (kSplit) {
+    cluster_barrier();
+    split_merge_rows<T, kWdDim, Cfg::kCtaRows, Cfg::kThreads>(p, smem, smem_raw + (smem - smem_u32(smem_raw)), rank, m0, positions, hq0, b);
+    cluster_barrier();  // the others read this CTA's shared memory
+  }
 }
 
 }  // namespace
 
-bool prefill_umma_applicable(const PrefillParams& p, int head_dim, int dtype) {
+// What a kernel's CTAs take, in microseconds, fitted to calls of one wave: a key tile, the start and end of a CTA, and for a split
+// one the merge without its values and the values of all rows of a CTA in clusters of up to four (larger ones share the links
+// between SMs with more neighbours: 5.7 us of full rows at head_dim 128 with four, 9 with eight).
+struct PrefillCosts {
+  double tile, fixed, merge, values;
+};
+static PrefillCosts umma_costs(int head_dim) {
+  return head_dim == 256 ? PrefillCosts{0.8, 6.4, 3.0, 6.0}
+                         : (head_dim == 128 ? PrefillCosts{2.1, 5.7, 2.5, 5.5} : PrefillCosts{1.15, 4.65, 3.0, 3.5});
+}
+// the same of gqa_prefill_mma_kernel: 32-key tiles, two CTAs per SM, each with the rows of one query head
+static PrefillCosts mma_costs(int head_dim) {
+  return head_dim == 64 ? PrefillCosts{0.88, 2.3, 0.0, 0.0} : PrefillCosts{1.65, 4.3, 0.0, 0.0};
+}
+
+bool prefill_umma_applicable(const PrefillParams& p, int batch, int q_heads, int head_dim, int dtype) {
   static const bool disabled = [] {
     const char* flag = std::getenv("ANNA_B200_PREFILL_UMMA");
     return flag != nullptr && flag[0] == '0';
@@ -845,11 +1047,21 @@ bool prefill_umma_applicable(const PrefillParams& p, int head_dim, int dtype) {
   if (p.out_stride_b % 8 != 0 || p.out_stride_h % 8 != 0 || p.out_stride_t % 8 != 0) return false;
   if ((reinterpret_cast<uintptr_t>(p.out) & 15u) != 0) return false;
   if (p.key_len <= 0) return false;
-  // The rows of a CTA are query positions x the heads that share a KV head (a power of two, at most 16): chunks that
-  // fill less than half a CTA's rows (and are shorter than 64 positions) leave most of the tile empty, and the mma.sync
-  // kernel serves them.
-  const int cta_rows = head_dim == 256 ? 128 : 256;
-  return p.q_len >= 64 || (int64_t)p.q_len * (1 << head_shift_of(p.groups)) * 2 >= cta_rows;
+  // The rows of a CTA are query positions x the heads that share a KV head (a power of two, at most 16).  Chunks that fill less
+  // than half a CTA's rows (and are shorter than 64 positions) leave most of a tile empty, but over more than a few dozen
+  // keys the mma.sync kernel, which has a CTA read the keys for every head, takes longer all the same (8 positions, 32/8 heads
+  // of 128 over 64 keys 7.5 us and 7.8 here; over 128 10.9 and 7.5; 16 over 4016 213 and 21 split; 64 rows of 5 over 505 284 and 57).
+  const int cta_rows = head_dim == 256 ? 128 : 256, heads_here = 1 << head_shift_of(p.groups);
+  if (p.q_len >= 64 || (int64_t)p.q_len * heads_here * 2 >= cta_rows) return true;
+  int device = 0, sms = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+      sms <= 0)
+    return false;
+  auto microseconds = [&](const PrefillCosts& costs, int64_t ctas, int64_t resident, int64_t keys) {
+    return (double)((ctas + resident - 1) / resident) * (costs.fixed + costs.tile * (double)((p.key_len + keys - 1) / keys));
+  };
+  return microseconds(umma_costs(head_dim), (int64_t)batch * (q_heads / heads_here), sms, head_dim == 128 ? 128 : 64) <
+         microseconds(mma_costs(head_dim), (int64_t)batch * q_heads, 2 * (int64_t)sms, 32);
 }
 
 // Tensor map of a [B, H, L, dim] 16-bit tensor given by element strides, seen as (dim, L, H, B).
@@ -868,9 +1080,94 @@ static bool prefill_tensor_map(CUtensorMap* out, const void* base, int64_t len, 
   return encode_map_16bit(out, base, 4, extents, strides, box);
 }
 
+using SplitResident = int[kMaxSplits + 1];  // CTAs in clusters of a size that the GPU holds at once ([1] 0 = not asked yet)
+
+template <typename Kernel>
+static int split_resident(Kernel kernel, int threads, uint32_t smem, int splits) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3((unsigned)splits);
+  config.blockDim = dim3((unsigned)threads);
+  config.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)splits;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  config.attrs = attr;
+  config.numAttrs = 1;
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) != cudaSuccess) {
+    (void)cudaGetLastError();  // this size is not to be had: never chosen
+    clusters = 0;
+  }
+  return clusters * splits;
+}
+
+// CTAs that share the keys of a query tile: the number that is fastest by these costs and the waves of clusters that the grid
+// makes of it, if that gains something (`filled`: part of a CTA's rows that exist).  Splitting pays for few query tiles over many keys
+// (one user's 123 tokens after 3095, 8/2 heads of 256: 47.5 -> 22.5 us; 4 rows of 24 after 2114, 16/2 heads: 43.3 -> 20); a grid
+// that fills the GPU, or one or two key tiles, stay as they are (119 query tiles of 256 over 3001 keys: 45 us, in pairs 72).
+static int choose_splits(const SplitResident& resident, const PrefillCosts& costs, int64_t base, int64_t tiles, double filled) {
+  int best = 1;
+  double best_cost = 0.0;
+  for (int s = 1; s <= kMaxSplits; ++s) {
+    if ((s > 1 && s > tiles) || resident[s] <= 0) continue;
+    const int64_t waves = (base * s + resident[s] - 1) / resident[s];
+    const double links = s <= 4 ? 1.0 : (s <= 8 ? 1.0 + 0.15 * (s - 4) : 1.8);
+    const double merge = s > 1 ? costs.merge + costs.values * filled * links : 0.0;
+    const double cost = (double)waves * ((double)((tiles + s - 1) / s) * costs.tile + costs.fixed + merge);
+    if (s == 1) best_cost = 0.93 * cost;
+    else if (cost < best_cost) { best_cost = cost; best = s; }
+  }
+  return best;
+}
+
+template <typename Plain, typename Split>
+static int launch_plain_or_split(Plain plain, Split split, const char* name, const PrefillParams& p, const CUtensorMap& map_q,
+                                 const CUtensorMap& map_k, const CUtensorMap& map_v, dim3 grid, int threads, uint32_t plain_smem,
+                                 uint32_t split_smem, int key_tile, const PrefillCosts& costs, int cta_rows, SplitResident (&resident_of)[64],
+                                 cudaStream_t stream) {
+  int device = 0;
+  ANNA_CUDA_CHECK(cudaGetDevice(&device));
+  static std::mutex asking;
+  SplitResident unlisted = {};
+  SplitResident& resident = device >= 0 && device < 64 ? resident_of[device] : unlisted;
+  std::unique_lock<std::mutex> lock(asking);
+  if (resident[1] == 0) {
+    ANNA_CUDA_CHECK(cudaFuncSetAttribute(plain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plain_smem));
+    ANNA_CUDA_CHECK(cudaFuncSetAttribute(split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)split_smem));
+    ANNA_CUDA_CHECK(cudaFuncSetAttribute(split, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    int sms = 0;
+    ANNA_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    for (int s = 2; s <= kMaxSplits; ++s) resident[s] = split_resident(split, threads, split_smem, s);
+    resident[1] = sms;
+  }
+  lock.unlock();
+  const int64_t base = (int64_t)grid.x * grid.y * grid.z;
+  PrefillParams sp = p;
+  const double filled = (double)p.q_len / ((double)grid.x * (cta_rows >> head_shift_of(p.groups)));
+  sp.splits = choose_splits(resident, costs, base, (p.key_len + key_tile - 1) / key_tile, filled);
+  if (sp.splits == 1) {
+    plain<<<grid, threads, plain_smem, stream>>>(sp, map_q, map_k, map_v);
+    return check_launch(name);
+  }
+  grid.x *= (unsigned)sp.splits;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = dim3((unsigned)threads);
+  config.dynamicSmemBytes = split_smem;
+  config.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)sp.splits;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  config.attrs = attr;
+  config.numAttrs = 1;
+  ANNA_CUDA_CHECK(cudaLaunchKernelEx(&config, split, sp, map_q, map_k, map_v));
+  return check_launch(name);
+}
+
 template <typename T>
 static int launch_prefill_umma_t(const PrefillParams& p, int batch, int q_heads, cudaStream_t stream) {
-  auto kernel = gqa_prefill_umma_kernel<T>;
   const int head_shift = head_shift_of(p.groups);
   const int positions = kUpCtaRows >> head_shift;
   CUtensorMap map_q, map_k, map_v;
@@ -880,22 +1177,16 @@ static int launch_prefill_umma_t(const PrefillParams& p, int batch, int q_heads,
       !prefill_tensor_map(&map_k, p.k, p.key_len, kv_heads, batch, p.kv_stride_t, p.kv_stride_h, p.kv_stride_b, kUpKeys, 1) ||
       !prefill_tensor_map(&map_v, p.v, p.key_len, kv_heads, batch, p.kv_stride_t, p.kv_stride_h, p.kv_stride_b, kUpKeys, 1))
     return kPrefillNotServed;  // no encoder in this driver, or a layout it refuses: the mma.sync kernel takes over
-  static bool configured[64] = {};
-  int device = 0;
-  ANNA_CUDA_CHECK(cudaGetDevice(&device));
-  if (device < 0 || device >= 64 || !configured[device]) {
-    ANNA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUpSmem));
-    if (device >= 0 && device < 64) configured[device] = true;
-  }
+  static SplitResident resident[64] = {};
   dim3 grid((unsigned)((p.q_len + positions - 1) / positions), (unsigned)(q_heads >> head_shift), (unsigned)batch);
-  kernel<<<grid, kUpThreads, kUpSmem, stream>>>(p, map_q, map_k, map_v);
-  return check_launch("gqa_prefill_umma_kernel");
+  return launch_plain_or_split(gqa_prefill_umma_kernel<T, false>, gqa_prefill_umma_kernel<T, true>, "gqa_prefill_umma_kernel", p,
+                               map_q, map_k, map_v, grid, kUpThreads, kUpSmem, SplitParts<kUpDim, kUpCtaRows>::smem_bytes(kUpSmem),
+                               kUpKeys, umma_costs(kUpDim), kUpCtaRows, resident, stream);
 }
 
 template <typename T, int D, int QT>
 static int launch_prefill_umma_wide_t(const PrefillParams& p, int batch, int q_heads, cudaStream_t stream) {
   using Cfg = WideCfg<D, QT>;
-  auto kernel = gqa_prefill_umma_wide_kernel<T, D, QT>;
   const int head_shift = head_shift_of(p.groups);
   const int positions = Cfg::kCtaRows >> head_shift;
   CUtensorMap map_q, map_k, map_v;
@@ -907,16 +1198,12 @@ static int launch_prefill_umma_wide_t(const PrefillParams& p, int batch, int q_h
       !prefill_tensor_map(&map_v, p.v, p.key_len, kv_heads, batch, p.kv_stride_t, p.kv_stride_h, p.kv_stride_b, Cfg::kKeys, 1,
                           D))
     return kPrefillNotServed;
-  static bool configured[64] = {};
-  int device = 0;
-  ANNA_CUDA_CHECK(cudaGetDevice(&device));
-  if (device < 0 || device >= 64 || !configured[device]) {
-    ANNA_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem));
-    if (device >= 0 && device < 64) configured[device] = true;
-  }
+  static SplitResident resident[64] = {};
   dim3 grid((unsigned)((p.q_len + positions - 1) / positions), (unsigned)(q_heads >> head_shift), (unsigned)batch);
-  kernel<<<grid, Cfg::kThreads, Cfg::kSmem, stream>>>(p, map_q, map_k, map_v);
-  return check_launch("gqa_prefill_umma_wide_kernel");
+  return launch_plain_or_split(gqa_prefill_umma_wide_kernel<T, D, QT, false>, gqa_prefill_umma_wide_kernel<T, D, QT, true>,
+                               "gqa_prefill_umma_wide_kernel", p, map_q, map_k, map_v, grid, Cfg::kThreads, Cfg::kSmem,
+                               SplitParts<D, Cfg::kCtaRows>::smem_bytes(Cfg::kSmem), Cfg::kKeys,
+                               umma_costs(D), Cfg::kCtaRows, resident, stream);
 }
 
 int launch_prefill_umma(const PrefillParams& p, int batch, int q_heads, int head_dim, int dtype, cudaStream_t stream) {

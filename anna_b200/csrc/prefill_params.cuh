@@ -17,12 +17,13 @@ struct PrefillParams {
   int q_len, groups, causal;
   int64_t key_len;
   float scale_log2;  // scaling * log2(e)
+  int splits;        // tensor-memory kernels: CTAs (of one cluster) that share the keys of a query tile
 };
 
 constexpr int kPrefillNotServed = -1;  // launch_prefill_umma: the caller should use the mma.sync kernel instead
 
-// true when the tensor-memory kernel serves this problem (head_dim 128, 16-bit, not switched off)
-bool prefill_umma_applicable(const PrefillParams& p, int head_dim, int dtype);
+// true when a tensor-memory kernel serves this problem (16-bit, not switched off) and is the faster one
+bool prefill_umma_applicable(const PrefillParams& p, int batch, int q_heads, int head_dim, int dtype);
 int launch_prefill_umma(const PrefillParams& p, int batch, int q_heads, int head_dim, int dtype, cudaStream_t stream);
 int prefill_umma_faults(int* count);
 

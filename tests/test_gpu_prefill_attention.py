@@ -78,6 +78,43 @@ def test_prefill_matches_oracle(cuda_device, dtype, heads, kv_heads, dim, q_len,
     assert torch.equal(again, out)
 
 
+# few query tiles over many keys: the CTAs of a cluster share the keys
+SPLIT = [
+    (torch.bfloat16, 8, 2, 256, 123, (3218,), True),
+    (torch.float16, 16, 2, 128, 24, (2138, 300, 24, 1), True),   # rows with fewer key tiles than CTAs, and queries without keys
+    (torch.bfloat16, 32, 8, 128, 16, (4016,), True),
+    (torch.float16, 8, 8, 64, 40, (3000, 0), True),              # a row without keys
+    (torch.bfloat16, 12, 4, 256, 9, (802,), True),               # three heads per KV head
+    (torch.bfloat16, 6, 2, 128, 200, (1500, 129), False),
+    (torch.float16, 4, 2, 64, 300, (2500, 2437), True),          # several query tiles, the last one partly filled
+]
+
+
+@pytest.mark.parametrize("dtype,heads,kv_heads,dim,q_len,lengths,causal", SPLIT)
+def test_keys_shared_by_a_cluster(cuda_device, dtype, heads, kv_heads, dim, q_len, lengths, causal):
+    """Relative bound: rounding P and the output to 16 bits, 2^-9 (bf16) and 2^-12 (fp16) each, twice that for what they share."""
+    gen = torch.Generator().manual_seed(heads * 100 + q_len)
+    batch, key_len = len(lengths), max(lengths)
+    q = torch.randn(batch, heads, q_len, dim, generator=gen).to(dtype).to(cuda_device)
+    k = torch.randn(batch, kv_heads, key_len, dim, generator=gen).to(dtype).to(cuda_device)
+    v = torch.randn(batch, kv_heads, key_len, dim, generator=gen).to(dtype).to(cuda_device)
+    n = torch.tensor(lengths, dtype=torch.long, device=cuda_device)
+    out = grouped_query_attention(q, k, v, scaling=dim ** -0.5, key_lengths=n, causal=causal)
+    max_abs, rel_l2 = error_stats(to_np(out), _oracle(q, k, v, n, causal))
+    assert max_abs <= ATOL[dtype] and rel_l2 <= 4 * (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12), (max_abs, rel_l2)
+    # a NaN in a query reaches its own row and no other; one in a key reaches every row that sees it
+    q[0, 1, q_len - 1, 3] = float("nan")
+    got = grouped_query_attention(q, k, v, scaling=dim ** -0.5, key_lengths=n, causal=causal)
+    assert bool(got[0, 1, q_len - 1].isnan().all())
+    got[0, 1, q_len - 1] = out[0, 1, q_len - 1]
+    assert torch.equal(got, out)
+    q[0, 1, q_len - 1, 3] = 0.0
+    k[0, 0, lengths[0] // 3, 0] = float("nan")
+    got = grouped_query_attention(q, k, v, scaling=dim ** -0.5, key_lengths=n, causal=causal)
+    seen = got[0, :heads // kv_heads]
+    assert bool(seen.isnan().all()) and bool(got[0, heads // kv_heads:].isfinite().all()) and torch.equal(got[1:], out[1:])
+
+
 @pytest.mark.parametrize("dim,q_len", [(128, 200), (128, 40), (256, 48), (256, 200), (64, 200)])
 def test_keys_behind_a_rows_length_may_hold_anything(cuda_device, dim, q_len):
     """K / V rows past key_lengths[b] are inside the tensors but not part of the row: NaNs there must not reach the
