@@ -79,7 +79,7 @@ __device__ __forceinline__ void merge_parts_and_store(float* sm_m, const float* 
 // arrivals on counters[counter_index].  HEADS = most query heads of a group.
 // Token t lives at element offset: paged -> page_table / block_size; ring_len > 0 -> (t % ring_len) * D; else
 // t * kv_stride_t, all relative to the (row, kv head) base the caller put into p.key / p.value.
-template <typename T, int D, int STAGES = 2, int HEADS = 8, MergeLoads MERGE = MergeLoads::kAllOrTwoColumns>
+template <typename T, int D, int STAGES = 2, int HEADS = 8, MergeLoads MERGE = MergeLoads::kAllOrTwoColumns, bool AHEAD = true>
 __device__ __forceinline__ void dense_split_mma_body(const DenseDecodeParams& p, uint8_t* smem_raw, int b, int kvh,
                                                      int g0, int g_count, int t0, int t1, int slot,
                                                      int active_chunks, int64_t counter_index) {
@@ -324,9 +324,14 @@ __device__ __forceinline__ void dense_split_mma_body(const DenseDecodeParams& p,
   if (p.fused.counters != nullptr) {
     const int64_t head0 = ((int64_t)b * p.q_heads + hq0) * p.chunk_capacity;
     __syncthreads();  // the epilogue buffers above are dead; reuse shared memory for the merge weights
-    fused_combine_tail<T, D, kMmaThreads, HEADS, MERGE>(p.fused, b, hq0, g_count, active_chunks, p.chunk_capacity,
-                                                        p.stats + head0 * 2, p.values + head0 * D,
-                                                        reinterpret_cast<float*>(smem_raw), counter_index);
+    if constexpr (AHEAD)
+      fused_combine_ahead<T, D, kMmaThreads, HEADS, MERGE>(p.fused, b, hq0, g_count, active_chunks, p.chunk_capacity,
+                                                           p.stats + head0 * 2, p.values + head0 * D,
+                                                           reinterpret_cast<float*>(smem_raw), counter_index);
+    else
+      fused_combine_tail<T, D, kMmaThreads, HEADS, MERGE>(p.fused, b, hq0, g_count, active_chunks, p.chunk_capacity,
+                                                          p.stats + head0 * 2, p.values + head0 * D,
+                                                          reinterpret_cast<float*>(smem_raw), counter_index);
   }
 }
 

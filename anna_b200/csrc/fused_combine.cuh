@@ -182,6 +182,214 @@ __device__ __forceinline__ void fused_combine_tail(const FusedCombine& fc, int b
   if (fc.num_peers > 0) __threadfence_system();
 }
 
+// The same with the first values read beside the statistics, and these once.  The merge is a chain of reads from L2 (counter,
+// statistics twice, values a few at a time), so each one taken out of it is 0.6 us of a call that waits for its last CTA (GPU time: 4
+// un-quantized rows of 0.7-5.7 K tokens, 32/4 heads 15.6 -> 13.4 us; 16 packed rows of 0.4-4 K, 16/2 heads of 256 32.1 -> 30.3;
+// 240 calls of 1-60 rows by 4 % in the mean).  Kernels that have no registers to spare for it keep the other one (12 packed rows of
+// 17000, 8/8 heads, 4 bits 74.4 and 75.8 with this one; two fp32 rows of 300-600, 8/2 heads, CUDA cores 13.9 and 15.8).
+template <typename T, int D, int THREADS, int HEADS = 8, MergeLoads MERGE = MergeLoads::kAllOrTwoColumns>
+__device__ __forceinline__ void fused_combine_ahead(const FusedCombine& fc, int b, int hq0, int g_count,
+                                                    int active_chunks, int chunk_capacity, const float* stats,
+                                                   const float* values, float* smem_weights /* [8][kFusedMaxChunks] */,
+                                                   int64_t counter_index, int arrivals = 0) {
+  __shared__ int s_is_last;
+  __syncthreads();  // all partial stores of this CTA are ordered before the arrival below
+  if (threadIdx.x == 0) {
+    // releases this CTA's partial and acquires those of the CTAs counted before; the barriers on both sides extend that to
+    // the other threads (4 un-quantized rows of 60-900 tokens: 10.8 us with a full fence on either side, 10.3 so)
+    int32_t* counter = fc.counters + counter_index;
+    int prev;
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;\n" : "=r"(prev) : "l"(counter) : "memory");
+    s_is_last = (prev == (arrivals > 0 ? arrivals : active_chunks) - 1) ? 1 : 0;
+    if (s_is_last) *counter = 0;
+  }
+  __syncthreads();
+  if (!s_is_last) return;
+
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  constexpr int kWarps = THREADS / 32;
+  auto weigh = [&] {
+    // one warp per head: max, denominator, normalised weights.  Where a lane has at most kHeld partials of a head their statistics are
+    // read once, and those of the warp's next head beside them.
+    constexpr int kHeld = 2;
+    if (active_chunks <= 32 * kHeld && (reinterpret_cast<uintptr_t>(stats) & 7u) == 0) {
+      for (int g0 = warp; g0 < g_count; g0 += 2 * kWarps) {
+        float2 s[2][kHeld];
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int i = 0; i < kHeld; ++i) {
+            const int g = g0 + k * kWarps, c = lane + 32 * i;
+            s[k][i] = g < g_count && c < active_chunks
+                          ? __ldcg(reinterpret_cast<const float2*>(stats + ((int64_t)g * chunk_capacity + c) * 2))
+                          : make_float2(-INFINITY, 0.0f);
+          }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const int g = g0 + k * kWarps;
+          if (g >= g_count) break;
+          float m = s[k][0].x;
+#pragma unroll
+          for (int i = 1; i < kHeld; ++i) m = fmaxf(m, s[k][i].x);
+#pragma unroll
+          for (int d = 16; d >= 1; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+          const float m_ref = m == -INFINITY ? 0.0f : m;
+          float den = 0.0f;
+#pragma unroll
+          for (int i = 0; i < kHeld; ++i) {
+            const float w = __expf(s[k][i].x - m_ref);
+            den += s[k][i].y * w;
+            s[k][i].x = w;
+          }
+#pragma unroll
+          for (int d = 16; d >= 1; d >>= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
+          const float inv = den > 0.0f ? 1.0f / den : 0.0f;
+#pragma unroll
+          for (int i = 0; i < kHeld; ++i)
+            if (lane + 32 * i < active_chunks) smem_weights[g * kFusedMaxChunks + lane + 32 * i] = s[k][i].x * inv;
+        }
+      }
+    } else {
+      for (int g = warp; g < g_count; g += kWarps) {
+        const float* st = stats + (int64_t)g * chunk_capacity * 2;
+        float m = -INFINITY;
+        for (int c = lane; c < active_chunks; c += 32) m = fmaxf(m, __ldcg(st + 2 * c));
+#pragma unroll
+        for (int d = 16; d >= 1; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+        const float m_ref = m == -INFINITY ? 0.0f : m;
+        float den = 0.0f;
+        for (int c = lane; c < active_chunks; c += 32) {
+          const float w = __expf(__ldcg(st + 2 * c) - m_ref);
+          den += __ldcg(st + 2 * c + 1) * w;
+          smem_weights[g * kFusedMaxChunks + c] = w;
+        }
+#pragma unroll
+        for (int d = 16; d >= 1; d >>= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
+        const float inv = den > 0.0f ? 1.0f / den : 0.0f;
+        for (int c = lane; c < active_chunks; c += 32) smem_weights[g * kFusedMaxChunks + c] *= inv;
+      }
+    }
+    __syncthreads();
+  };
+  auto store = [&](int g, int d, const float4& o) {
+    const float acc[4] = {o.x, o.y, o.z, o.w};
+    const T* gate = fc.gate == nullptr ? nullptr
+                                       : reinterpret_cast<const T*>(fc.gate) + (int64_t)b * fc.gate_stride_b +
+                                             (int64_t)(hq0 + g) * fc.gate_stride_h + d;
+    const int64_t offset = (int64_t)b * fc.out_stride_b + (int64_t)(hq0 + g) * fc.out_stride_h + d;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const T result = ElemTraits<T>::from_float(gate ? acc[i] * sigmoidf_fast(ElemTraits<T>::to_float(gate[i])) : acc[i]);
+      reinterpret_cast<T*>(fc.out)[offset + i] = result;
+      for (int peer = 0; peer < fc.num_peers; ++peer) reinterpret_cast<T*>(fc.peers[peer])[offset + i] = result;
+    }
+  };
+  const bool aligned = (reinterpret_cast<uintptr_t>(values) & 15u) == 0;
+  constexpr int kCols = D / 4;
+  constexpr int kRounds = (HEADS * kCols + THREADS - 1) / THREADS;
+  constexpr int kInFlight = 8, kAhead = 4;
+  const int items = g_count * kCols;
+  auto add = [](float4& acc, const float4& v, float w) {
+    acc.x = fmaf(v.x, w, acc.x);
+    acc.y = fmaf(v.y, w, acc.y);
+    acc.z = fmaf(v.z, w, acc.z);
+    acc.w = fmaf(v.w, w, acc.w);
+  };
+  auto side_by_side = [&](auto columns) {
+    constexpr int kColumns = decltype(columns)::value;  // of a thread
+    constexpr int kAtOnce = kInFlight / kColumns;       // partials
+    float4 acc[kColumns];
+    const float* vals[kColumns];
+#pragma unroll
+    for (int r = 0; r < kColumns; ++r) {
+      const int item = min((int)threadIdx.x + r * THREADS, items - 1);  // past the end: the last column again, not stored
+      acc[r] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      vals[r] = values + (int64_t)(item / kCols) * chunk_capacity * D + 4 * (item % kCols);
+    }
+    float4 v[kAtOnce][kColumns];
+    auto load = [&](int c0) {
+#pragma unroll
+      for (int k = 0; k < kAtOnce; ++k)
+#pragma unroll
+        for (int r = 0; r < kColumns; ++r)
+          v[k][r] = __ldcg(reinterpret_cast<const float4*>(vals[r] + (int64_t)min(c0 + k, active_chunks - 1) * D));
+    };
+    load(0);
+    weigh();
+    for (int c0 = 0;;) {
+#pragma unroll
+      for (int r = 0; r < kColumns; ++r) {
+        const float* w = smem_weights + min(((int)threadIdx.x + r * THREADS) / kCols, g_count - 1) * kFusedMaxChunks;
+#pragma unroll
+        for (int k = 0; k < kAtOnce; ++k)
+          if (c0 + k < active_chunks) add(acc[r], v[k][r], w[c0 + k]);
+      }
+      c0 += kAtOnce;
+      if (c0 >= active_chunks) break;
+      load(c0);
+    }
+#pragma unroll
+    for (int r = 0; r < kColumns; ++r) {
+      const int item = (int)threadIdx.x + r * THREADS;
+      if (item < items) store(item / kCols, 4 * (item % kCols), acc[r]);
+    }
+  };
+  constexpr bool kTwo = kRounds > 2 && MERGE == MergeLoads::kAllOrTwoColumns;
+  if (MERGE != MergeLoads::kOneColumn && kRounds > 1 && aligned && items > (kTwo ? 2 : 1) * THREADS) {
+    side_by_side(std::integral_constant<int, kRounds>{});
+  } else if (kTwo && aligned && items > THREADS) {
+    side_by_side(std::integral_constant<int, 2>{});
+  } else if (aligned) {
+    float4 first[kAhead];  // of this thread's first column
+    {
+      const int item = min((int)threadIdx.x, items - 1);
+      const float* vals = values + (int64_t)(item / kCols) * chunk_capacity * D + 4 * (item % kCols);
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k)
+        first[k] = __ldcg(reinterpret_cast<const float4*>(vals + (int64_t)min(k, active_chunks - 1) * D));
+    }
+    weigh();
+    for (int item = threadIdx.x; item < items; item += THREADS) {
+      const int g = item / kCols, d = 4 * (item % kCols);
+      const float* vals = values + (int64_t)g * chunk_capacity * D + d;
+      const float* w = smem_weights + g * kFusedMaxChunks;
+      float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      int c = 0;
+      if (item < THREADS) {
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+          if (k < active_chunks) add(acc, first[k], w[k]);
+        c = kAhead;
+      }
+#pragma unroll 4
+      for (; c < active_chunks; ++c) add(acc, __ldcg(reinterpret_cast<const float4*>(vals + (int64_t)c * D)), w[c]);
+      store(g, d, acc);
+    }
+  } else {
+    weigh();
+  }
+  for (int item = threadIdx.x; !aligned && item < g_count * D; item += THREADS) {
+    const int g = item / D;
+    const int d = item % D;
+    const float* vals = values + (int64_t)g * chunk_capacity * D + d;
+    const float* w = smem_weights + g * kFusedMaxChunks;
+    float acc = 0.0f;
+    for (int c = 0; c < active_chunks; ++c) acc = fmaf(__ldcg(vals + (int64_t)c * D), w[c], acc);
+    if (fc.gate) {
+      const T* gate = reinterpret_cast<const T*>(fc.gate) + (int64_t)b * fc.gate_stride_b +
+                      (int64_t)(hq0 + g) * fc.gate_stride_h;
+      acc *= sigmoidf_fast(ElemTraits<T>::to_float(gate[d]));
+    }
+    const int64_t offset = (int64_t)b * fc.out_stride_b + (int64_t)(hq0 + g) * fc.out_stride_h + d;
+    const T result = ElemTraits<T>::from_float(acc);
+    reinterpret_cast<T*>(fc.out)[offset] = result;
+    for (int peer = 0; peer < fc.num_peers; ++peer) reinterpret_cast<T*>(fc.peers[peer])[offset] = result;
+  }
+  // stores to other GPUs are ordered before whatever this stream signals to them after the kernel
+  if (fc.num_peers > 0) __threadfence_system();
+}
+
 // A row with no visible key has no contributing CTA; the CTA of chunk 0 writes its zeros.
 template <typename T, int D, int THREADS>
 __device__ __forceinline__ void fused_write_zero_row(const FusedCombine& fc, int b, int hq0, int g_count) {

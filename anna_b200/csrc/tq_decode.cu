@@ -335,8 +335,8 @@ __global__ void __launch_bounds__(kDecodeThreads, kTqMinBlocks<T, D, G>) tq_deco
   if constexpr (kMerge) {
     const int64_t head0 = ((int64_t)b * p.q_heads + hq0) * p.chunk_capacity;
     const int chunks = active_window + (int)((Lq + p.chunk_tokens - 1) / p.chunk_tokens);
-    fused_combine_tail<T, D, kDecodeThreads>(p.fused, b, hq0, g_count, chunks, p.chunk_capacity, p.stats + head0 * 2,
-                                             p.values + head0 * D, smem, (int64_t)b * gridDim.y + blockIdx.y);
+    fused_combine_ahead<T, D, kDecodeThreads>(p.fused, b, hq0, g_count, chunks, p.chunk_capacity, p.stats + head0 * 2,
+                                              p.values + head0 * D, smem, (int64_t)b * gridDim.y + blockIdx.y);
   }
 }
 

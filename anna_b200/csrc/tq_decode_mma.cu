@@ -214,22 +214,41 @@ struct TqMmaCfg {
 
 // What the query preparation needs besides the queries: the same for every segment of a CTA.
 struct TqQueryConsts {
+  bool loaded;
   uint32_t flips;    // bit j: coordinate lane * E + j is negated by the first rotation (low byte) / by the second
   uint32_t lut[2];   // 4-bit: the centroids as signed bytes
   float cent_step;   // 4-bit: the value of one step of those bytes
 };
 
+// The constants as they are in memory, so that a kernel can read them beside what else it starts with.
 template <int D, int BITS>
-__device__ __forceinline__ TqQueryConsts load_query_consts(const TqDecodeParams& p) {
+struct TqRawConsts {
+  float s1[D / 32], s2[D / 32], cent[BITS == 4 ? 8 : 1];
+  __device__ __forceinline__ void load(const TqDecodeParams& p) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int j = 0; j < D / 32; ++j) {
+      s1[j] = __ldg(p.signs1 + lane * (D / 32) + j);
+      s2[j] = __ldg(p.signs2 + lane * (D / 32) + j);
+    }
+    if constexpr (BITS == 4) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) cent[e] = __ldg(p.centroids + e);
+    }
+  }
+};
+
+template <int D, int BITS>
+__device__ __forceinline__ TqQueryConsts load_query_consts(const TqRawConsts<D, BITS>& raw) {
   constexpr int E = D / 32;
   constexpr int kEntries = 1 << (BITS - 1);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  TqQueryConsts qc{0u, {0u, 0u}, 0.0f};
+  TqQueryConsts qc{true, 0u, {0u, 0u}, 0.0f};
 #pragma unroll
   for (int j = 0; j < E; ++j) {
-    qc.flips |= (__ldg(p.signs1 + lane * E + j) < 0.0f ? 1u : 0u) << j;
-    qc.flips |= (__ldg(p.signs2 + lane * E + j) < 0.0f ? 1u : 0u) << (8 + j);
+    qc.flips |= (raw.s1[j] < 0.0f ? 1u : 0u) << j;
+    qc.flips |= (raw.s2[j] < 0.0f ? 1u : 0u) << (8 + j);
   }
   if constexpr (BITS == 4) {
     // The byte scale of the centroids is the one, among 256 candidates from 127 down to 63 steps for the largest
@@ -238,7 +257,7 @@ __device__ __forceinline__ TqQueryConsts load_query_consts(const TqDecodeParams&
     float cent[kEntries], cmax = 0.0f;
 #pragma unroll
     for (int e = 0; e < kEntries; ++e) {
-      cent[e] = __ldg(p.centroids + e);
+      cent[e] = raw.cent[e];
       cmax = fmaxf(cmax, fabsf(cent[e]));
     }
     float best_err = INFINITY, best_k = 0.0f;
@@ -278,6 +297,29 @@ __device__ __forceinline__ TqQueryConsts load_query_consts(const TqDecodeParams&
   return qc;
 }
 
+template <typename T>
+__device__ __forceinline__ T elem_of_bits(unsigned short bits);
+template <>
+__device__ __forceinline__ __half elem_of_bits<__half>(unsigned short bits) { return __ushort_as_half(bits); }
+template <>
+__device__ __forceinline__ __nv_bfloat16 elem_of_bits<__nv_bfloat16>(unsigned short bits) { return __ushort_as_bfloat16(bits); }
+
+// This lane's elements (lane * D/32 ...) of the query heads warp and warp + 4, as loaded (rows start on 4-byte boundaries).
+template <typename T, int D>
+struct TqRawQueries {
+  uint32_t w[2][D / 64];
+  __device__ __forceinline__ void load(const TqDecodeParams& p, int b, int hq0, int g_count) {
+    const T* q = reinterpret_cast<const T*>(p.q) + (int64_t)b * p.q_stride_b + (threadIdx.x & 31) * (D / 32);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int g = (int)(threadIdx.x >> 5) + k * kMmaWarps;
+      const uint32_t* row = reinterpret_cast<const uint32_t*>(q + (int64_t)(hq0 + g) * p.q_stride_h);
+#pragma unroll
+      for (int j = 0; j < D / 64; ++j) w[k][j] = g < g_count ? row[j] : 0u;
+    }
+  }
+};
+
 // Rotates the queries of one (row, kv-head group), rounds them to a coarse and a fine byte and leaves them at `query` in
 // shared memory as the B fragments of m16n8k32 in the register order of the score products, with the per-head factors
 // behind them (offsets of TqMmaCfg).  Every CTA does this for itself, once per segment, while its first tiles are on
@@ -286,7 +328,7 @@ __device__ __forceinline__ TqQueryConsts load_query_consts(const TqDecodeParams&
 // 0.5-16 K 253 -> 247 us, 64 rows of 32 K 630 -> 636 us.  The caller synchronises afterwards.
 template <typename T, int D, int BITS>
 __device__ __forceinline__ void prepare_query_fragments(const TqDecodeParams& p, uint8_t* smem_raw, uint8_t* query,
-                                                        int free_stage, int b, int hq0, int g_count,
+                                                        int free_stage, const TqRawQueries<T, D>& raw, int g_count,
                                                         const TqQueryConsts& qc) {
   using Cfg = TqMmaCfg<T, D, BITS>;
   constexpr int E = D / 32;
@@ -318,12 +360,14 @@ __device__ __forceinline__ void prepare_query_fragments(const TqDecodeParams& p,
   const float log2e = 1.4426950408889634f;
   const float f1 = p.scaling * log2e * inv_sqrt_d * inv_sqrt_d;
   const float f2 = p.scaling * log2e * 1.2533141373155001f * inv_sqrt_d * inv_sqrt_d * inv_sqrt_d;
-  const T* q_ptr = reinterpret_cast<const T*>(p.q) + (int64_t)b * p.q_stride_b + (int64_t)hq0 * p.q_stride_h;
-  for (int g = warp; g < g_count; g += kMmaWarps) {
+  for (int k = 0; k < 2; ++k) {
+    const int g = warp + k * kMmaWarps;
+    if (g >= g_count) break;
     float w[E], w1[E];
 #pragma unroll
     for (int j = 0; j < E; ++j) {
-      w[j] = ElemTraits<T>::to_float(q_ptr[(int64_t)g * p.q_stride_h + lane * E + j]);
+      const uint32_t word = k == 0 ? raw.w[0][j / 2] : raw.w[1][j / 2];
+      w[j] = ElemTraits<T>::to_float(elem_of_bits<T>((unsigned short)(j % 2 == 0 ? word : word >> 16)));
       if ((flips >> j) & 1u) w[j] = -w[j];
     }
     warp_fwht<E>(w, lane);
@@ -493,7 +537,7 @@ __device__ __forceinline__ RowChunks row_chunks(const TqDecodeParams& p, int b) 
 
 // Chunk `slot` of the un-quantized window ring of a row: the dense tensor-core body with ring addressing.  Also writes the
 // zero output of empty rows.  `arrives`: the chunk counts on the merge counter, as one of all active chunks.
-template <typename T, int D, int STAGES, int HEADS>
+template <typename T, int D, int STAGES, int HEADS, bool AHEAD>
 __device__ __forceinline__ void tq_window_chunk(const TqDecodeParams& p, uint8_t* smem_raw, const RowChunks& row, int b,
                                                 int unit, int units, int slot, bool arrives) {
   const int group_tiles = (p.groups + 7) / 8;
@@ -525,7 +569,7 @@ __device__ __forceinline__ void tq_window_chunk(const TqDecodeParams& p, uint8_t
   if (!arrives) dp.fused.counters = nullptr;
   const int t0 = row.quantized + slot * p.chunk_tokens;
   const int t1 = min(row.len, t0 + p.chunk_tokens);
-  dense_split_mma_body<T, D, STAGES, HEADS, MergeLoads::kAllColumns>(dp, smem_raw, b, kvh, g0, g_count, t0, t1, slot, row.window + row.packed,
+  dense_split_mma_body<T, D, STAGES, HEADS, MergeLoads::kAllColumns, AHEAD>(dp, smem_raw, b, kvh, g0, g_count, t0, t1, slot, row.window + row.packed,
                                      (int64_t)b * units + unit);
 }
 
@@ -539,7 +583,7 @@ __global__ void __launch_bounds__(kMmaThreads, MmaCfg<D>::kMinBlocks) tq_window_
   asm volatile("griddepcontrol.launch_dependents;\n" ::);
   const RowChunks row = row_chunks(p, blockIdx.z);
   // the packed CTAs wait for this grid before they count
-  tq_window_chunk<T, D, 2, 8>(p, smem_raw, row, blockIdx.z, blockIdx.y, gridDim.y, blockIdx.x,
+  tq_window_chunk<T, D, 2, 8, false>(p, smem_raw, row, blockIdx.z, blockIdx.y, gridDim.y, blockIdx.x,
                            p.window_arrives || row.quantized == 0);
 }
 
@@ -555,6 +599,24 @@ struct PackedRing {
 template <int D, bool kPair>
 constexpr int kMergeHeads = kPair && D == 256 ? 4 : 8;
 
+// EARLY: what a segment starts with (pages, queries, constants) is read side by side, and the constants are worked out while the first
+// copies are on their way.  Kernels of many CTAs per SM, whose latencies others fill, keep the registers instead (64 rows of 32 K,
+// 32/8 heads, in chunks: 583 us, 587 with it; in shares 128 rows of 0.5-16 K, 3 bits, 210.3 -> 207.6, 64 of 4-32 K at head_dim 256,
+// 2 bits, 165.5 -> 162.9).  AHEAD: see fused_combine_ahead.
+constexpr int32_t kPageNotAsked = INT32_MIN;
+
+// Page of the tile that this lane copies in a warp's first step of a segment that starts at token t0, for kernels that know t0 before
+// the row's length: the block table is read beside the length instead of behind it.  Lanes without a tile do not ask.
+template <typename T, int D, int BITS>
+__device__ __forceinline__ int32_t first_page_of(const TqDecodeParams& p, int b, int t0) {
+  constexpr int U = TqMmaCfg<T, D, BITS>::kTilesPerStep;
+  const int lane = threadIdx.x & 31;
+  if (lane >= U) return kPageNotAsked;
+  const uint32_t ts = (uint32_t)(t0 + ((int)(threadIdx.x >> 5) * U + lane) * kTileTokens);
+  const uint32_t blk = p.block_shift >= 0 ? ts >> p.block_shift : ts / (uint32_t)p.block_size;
+  return (int64_t)blk < p.max_blocks ? p.block_table[(int64_t)b * p.table_stride + blk] : kPageNotAsked;
+}
+
 // One packed segment: tokens [t0, t1) of the quantized prefix of (row b, unit = kv head and group of 8 query heads).  The
 // partial goes to split-K slot `out_slot` and counts as one of `arrivals`; the CTA that counts last merges `slots` partials.
 // All threads of the CTA call it; it ends with the CTA synchronised against reuse of the ring.
@@ -564,10 +626,12 @@ constexpr int kMergeHeads = kPair && D == 256 ? 4 : 8;
 // arithmetic, the softmax and the registers behind it are spent once per two tiles instead of once per tile with half of
 // the columns empty; columns j and j + 4 are two partials of head j, merged with those of the other warps.  64 rows of
 // 32 K tokens, 4 bits: 636 -> 614 us; 128 rows of 0.5-16 K, 3 bits: 247 -> 239 us.
-template <typename T, int D, int BITS, bool kPair, MergeLoads MERGE = MergeLoads::kAllColumns>
+template <typename T, int D, int BITS, bool kPair, MergeLoads MERGE = MergeLoads::kAllColumns, bool EARLY = true, bool AHEAD = EARLY>
 __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8_t* smem_raw,
-                                                  const TqQueryConsts& qc, PackedRing& ring, int b, int unit,
-                                                  int units, int t0, int t1, int out_slot, int slots, int arrivals) {
+                                                  TqQueryConsts& qc, PackedRing& ring, int b, int unit,
+                                                  int units, int t0, int t1, int out_slot, int slots, int arrivals,
+                                                  int32_t first_page = kPageNotAsked,
+                                                  TqRawConsts<D, BITS>* consts = nullptr) {
   using Cfg = TqMmaCfg<T, D, BITS>;
   constexpr int U = Cfg::kTilesPerStep;
   constexpr int A = kPair ? 1 : U;  // sets of score accumulators
@@ -607,7 +671,7 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
   // layout of a 16-token page chunk, so with 16-token pages a tile is one linear run; with larger pages it is six runs
   // (codes, norms, residual norms, value codes, scales, zeros).  Lanes 0 .. U-1 look up and copy one tile each; lane 0
   // arms the stage's mbarrier with the bytes of all of them first.  Called by the whole warp.
-  auto issue_step = [&](int step, int stage) {
+  auto issue_step = [&](int step, int stage, int32_t page = kPageNotAsked) {
     int valid = 0;
     const uint8_t* chunk_ptr = nullptr;
     int s0 = 0;
@@ -617,7 +681,7 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
         const int ts = t0 + tile * kTileTokens;
         const uint32_t blk = block_shift >= 0 ? ((uint32_t)ts >> block_shift) : ((uint32_t)ts / block_size);
         s0 = ts - (int)(blk * block_size);  // first slot of the tile inside its page
-        const int32_t pid = table_row[blk];
+        const int32_t pid = page != kPageNotAsked ? page : table_row[blk];
         if (pid >= 0 && pid < p.num_pages) {  // else a hole in the block table: nothing to copy
           valid = min(kTileTokens, t1 - ts);
           chunk_ptr = p.pages + ((int64_t)pid * p.kv_heads + kvh) * p.layout.chunk_bytes;
@@ -649,6 +713,29 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
     }
   };
 
+  // this warp's query rows (heads warp, warp + 4) are on their way, too, before anything waits
+  TqRawQueries<T, D> raw;
+  if constexpr (EARLY) raw.load(p, b, hq0, g_count);
+
+  const int num_steps = (num_tiles + U - 1) / U;
+  const int my_steps = num_steps > warp && !ring.dead ? (num_steps - warp + kMmaWarps - 1) / kMmaWarps : 0;
+#pragma unroll
+  for (int i = 0; i < Cfg::kStages - 1; ++i)
+    if (i < my_steps) issue_step(i, (ring.stage + i) % Cfg::kStages, i == 0 ? first_page : kPageNotAsked);
+  if constexpr (!EARLY) raw.load(p, b, hq0, g_count);
+  if (EARLY && !qc.loaded) {  // the same in all segments; behind the first copies
+    TqRawConsts<D, BITS> mine;
+    if (consts == nullptr) mine.load(p);
+    qc = load_query_consts(consts != nullptr ? *consts : mine);
+  }
+
+  // Q fragments and their factors for this lane's two heads (columns 2tig, 2tig + 1); the softmax scale and log2(e) are
+  // folded into the factors
+  uint8_t* query = smem_raw + Cfg::kQueryOffset;
+  const uint32_t lut[2] = {qc.lut[0], qc.lut[1]};
+  prepare_query_fragments<T, D, BITS>(p, smem_raw, query, ring_free_stage(ring.stage, Cfg::kStages), raw, g_count, qc);
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // the loop's first copy lands where the rotations were
+  __syncthreads();
   float m_run[2] = {-INFINITY, -INFINITY};
   float l_run[2] = {0.0f, 0.0f};
   float o_acc[Cfg::kSteps][4];
@@ -656,21 +743,6 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
   for (int j = 0; j < Cfg::kSteps; ++j)
 #pragma unroll
     for (int r = 0; r < 4; ++r) o_acc[j][r] = 0.0f;
-
-  const int num_steps = (num_tiles + U - 1) / U;
-  const int my_steps = num_steps > warp && !ring.dead ? (num_steps - warp + kMmaWarps - 1) / kMmaWarps : 0;
-#pragma unroll
-  for (int i = 0; i < Cfg::kStages - 1; ++i)
-    if (i < my_steps) issue_step(i, (ring.stage + i) % Cfg::kStages);
-
-  // Q fragments and their factors for this lane's two heads (columns 2tig, 2tig + 1); the softmax scale and log2(e) are
-  // folded into the factors
-  uint8_t* query = smem_raw + Cfg::kQueryOffset;
-  const uint32_t lut[2] = {qc.lut[0], qc.lut[1]};
-  prepare_query_fragments<T, D, BITS>(p, smem_raw, query, ring_free_stage(ring.stage, Cfg::kStages), b, hq0, g_count,
-                                      qc);
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // the loop's first copy lands where the rotations were
-  __syncthreads();
   const uint4* q_frag = reinterpret_cast<const uint4*>(query) + lane;                     // [s][lane]
   const uint2* q_fine = reinterpret_cast<const uint2*>(query + Cfg::kFragBytes) + lane;   // 4-bit
   const uint4* q_frag2 = reinterpret_cast<const uint4*>(query + Cfg::kFragBytes) + lane;  // planes
@@ -1095,9 +1167,14 @@ __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8
   if (p.fused.counters != nullptr) {
     const int64_t head0 = ((int64_t)b * p.q_heads + hq0) * p.chunk_capacity;
     __syncthreads();
-    fused_combine_tail<T, D, kMmaThreads, kMergeHeads<D, kPair>, MERGE>(
-        p.fused, b, hq0, g_count, slots, p.chunk_capacity, p.stats + head0 * 2, p.values + head0 * D,
-        reinterpret_cast<float*>(smem_raw), (int64_t)b * units + unit, arrivals);
+    if constexpr (AHEAD)
+      fused_combine_ahead<T, D, kMmaThreads, kMergeHeads<D, kPair>, MERGE>(
+          p.fused, b, hq0, g_count, slots, p.chunk_capacity, p.stats + head0 * 2, p.values + head0 * D,
+          reinterpret_cast<float*>(smem_raw), (int64_t)b * units + unit, arrivals);
+    else
+      fused_combine_tail<T, D, kMmaThreads, kMergeHeads<D, kPair>, MERGE>(
+          p.fused, b, hq0, g_count, slots, p.chunk_capacity, p.stats + head0 * 2, p.values + head0 * D,
+          reinterpret_cast<float*>(smem_raw), (int64_t)b * units + unit, arrivals);
   }
   // the merge buffers lie where the next segment's copies land: order those writes before the copy engine's
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -1130,11 +1207,13 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
   const int t0 = chunk * p.chunk_tokens;
   init_packed_barriers<T, D, BITS>(smem_raw);
   PackedRing ring{0, 0u, false};
-  const TqQueryConsts qc = load_query_consts<D, BITS>(p);
+  TqRawConsts<D, BITS> consts;
+  consts.load(p);
+  TqQueryConsts qc = load_query_consts(consts);
   // active slots stay contiguous: [window | packed]
-  tq_packed_segment<T, D, BITS, kPair>(p, smem_raw, qc, ring, b, (int)blockIdx.y, (int)gridDim.y, t0,
-                                       min(row.quantized, t0 + p.chunk_tokens), row.window + chunk, row.window + row.packed,
-                                       row.packed);
+  tq_packed_segment<T, D, BITS, kPair, MergeLoads::kAllColumns, false>(
+      p, smem_raw, qc, ring, b, (int)blockIdx.y, (int)gridDim.y, t0, min(row.quantized, t0 + p.chunk_tokens), row.window + chunk,
+      row.window + row.packed, row.packed);
 }
 
 // Small calls: window chunks and packed chunks in one launch, grid (window chunks + packed chunks, units, batch), all of it
@@ -1156,20 +1235,25 @@ __global__ void __launch_bounds__(kMmaThreads, TqSmallCfg<T, D, BITS>::kMinBlock
     tq_decode_small_mma_kernel(const TqDecodeParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int b = blockIdx.z;
+  const int chunk = (int)blockIdx.x - p.num_window_chunks;
+  const int t0 = chunk * p.chunk_tokens;
+  // the page, the constants and the lengths are read side by side
+  const int32_t first_page = chunk >= 0 ? first_page_of<T, D, BITS>(p, b, t0) : kPageNotAsked;
+  TqRawConsts<D, BITS> consts;
+  consts.load(p);
   const RowChunks row = row_chunks(p, b);
-  if ((int)blockIdx.x < p.num_window_chunks) {
-    tq_window_chunk<T, D, 1, kMergeHeads<D, kPair>>(p, smem_raw, row, b, blockIdx.y, gridDim.y, blockIdx.x, true);
+  if (chunk < 0) {
+    tq_window_chunk<T, D, 1, kMergeHeads<D, kPair>, true>(p, smem_raw, row, b, blockIdx.y, gridDim.y, blockIdx.x, true);
     return;
   }
-  const int chunk = (int)blockIdx.x - p.num_window_chunks;
   if (chunk >= row.packed) return;
-  const int t0 = chunk * p.chunk_tokens;
   init_packed_barriers<T, D, BITS>(smem_raw);
   PackedRing ring{0, 0u, false};
-  const TqQueryConsts qc = load_query_consts<D, BITS>(p);
+  TqQueryConsts qc{};
   const int active = row.window + row.packed;
   tq_packed_segment<T, D, BITS, kPair>(p, smem_raw, qc, ring, b, (int)blockIdx.y, (int)gridDim.y, t0,
-                                       min(row.quantized, t0 + p.chunk_tokens), row.window + chunk, active, active);
+                                       min(row.quantized, t0 + p.chunk_tokens), row.window + chunk, active, active, first_page,
+                                       &consts);
 }
 
 // What a segment costs beyond its tiles (query preparation, first copy, merge: about 6 us), in tiles.  Over 512 shapes (1 to
@@ -1185,16 +1269,17 @@ __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
   // This instance has no registers for the loads of two columns and issues them one after the other (two rows of 12000 tokens,
   // 16/2 heads: 44.7 us, one column after the other 32.4; one of 20000, 64/8 heads: 45.7 and 36.2).
   constexpr MergeLoads kMerge = D == 128 && BITS == 3 && !kPair ? MergeLoads::kOneColumn : MergeLoads::kAllColumns;
+  constexpr bool kAhead = !(D == 128 && BITS == 4 && kPair);  // nor this one for the merge's loads ahead
   const int units = p.kv_heads * ((p.groups + 7) / 8);
   init_packed_barriers<T, D, BITS>(smem_raw);
   PackedRing ring{0, 0u, false};
-  const TqQueryConsts qc = load_query_consts<D, BITS>(p);
+  TqQueryConsts qc{};
   balanced_for_each_segment<kMmaThreads, false>(
       p.lengths, p.max_len, batch, units, min(p.chunk_capacity, kFusedMaxChunks) - p.num_window_chunks,
       [](int) {},  // rows without packed tokens belong to the window kernel
       [&](int b, int unit, int t0, int t1, int slot, int partials) {
         const int active_window = (p.residual_len + p.chunk_tokens - 1) / p.chunk_tokens;  // the window of this row is full
-        tq_packed_segment<T, D, BITS, kPair, kMerge>(p, smem_raw, qc, ring, b, unit, units, t0, t1, active_window + slot,
+        tq_packed_segment<T, D, BITS, kPair, kMerge, true, kAhead>(p, smem_raw, qc, ring, b, unit, units, t0, t1, active_window + slot,
                                                      active_window + partials, partials);
       },
       p.residual_len, kMmaWarps * TqMmaCfg<T, D, BITS>::kTilesPerStep, kTqSegmentTiles, kTqSegmentTiles);
