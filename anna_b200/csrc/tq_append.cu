@@ -34,7 +34,7 @@ struct TqAppendParams {
   int32_t* status;
 };
 
-constexpr int kAppendWarps = 8;
+constexpr int kAppendWarps = 8;  // of a CTA; fewer where a call has fewer tokens
 constexpr int kAppendBulkCtasPerSm = 4;  // 128 registers per thread
 
 // Number of boundaries below `s` (= index of the nearest centroid) by bisection over the sorted boundaries: three
@@ -119,10 +119,11 @@ __global__ void __launch_bounds__(kAppendWarps * 32) tq_append_kernel(const TqAp
   const int32_t* table_row = p.block_table + (int64_t)b * p.table_stride;
 
   const int warp = threadIdx.x >> 5;
-  const int u_stride = p.u_chunks * kAppendWarps;
+  const int warps = blockDim.x >> 5;
+  const int u_stride = p.u_chunks * warps;
 
   // ---- window items: plain copies, unless the slot's old occupant is quantized (and rewritten) by a quantize item ----
-  for (int u = (int)blockIdx.x * kAppendWarps + warp; u < nw; u += u_stride) {
+  for (int u = (int)blockIdx.x * warps + warp; u < nw; u += u_stride) {
     const int pw = wstart + u;
     const int k = div_r(pw - L + R);  // smallest k >= 1 with pw - k*R < L
     const int p_old = pw - k * R;
@@ -134,7 +135,7 @@ __global__ void __launch_bounds__(kAppendWarps * 32) tq_append_kernel(const TqAp
 
   // ---- quantize items.  The trip count depends on the CTA alone, so every warp stays converged through the warp
   // exchanges of the body; a warp past the end repeats the last item and stores nothing. ------------------------------
-  for (int base = (int)blockIdx.x * kAppendWarps; base < nq; base += u_stride) {
+  for (int base = (int)blockIdx.x * warps; base < nq; base += u_stride) {
     const bool active = base + warp < nq;
     const int pos = Lq + (active ? base + warp : nq - 1);
     float x[E], v[E];
@@ -632,6 +633,13 @@ extern "C" int anna_tq_append(const void* k_new, const void* v_new, int64_t kn_s
           q.u_chunks = bulk_chunks(heads_total, (new_tokens + kBulkWarps * (32 * kBulkCoords / D) - 1) / (kBulkWarps * (32 * kBulkCoords / D)), ctas);
           bulk<<<dim3((unsigned)q.u_chunks, (unsigned)kv_heads, (unsigned)batch), kBulkWarps * 32, 0, (cudaStream_t)stream>>>(q);
           return check_launch("tq_append_bulk_kernel");
+        }
+        if (new_tokens < kAppendWarps) {
+          // Steps of a few tokens: a warp per token and no idle ones, which took the registers that other CTAs' tokens need (one token
+          // to each of 512 rows, 8 heads: 38.9 us with 8 warps, 13.2 so; four 41.0 and 26.8).
+          q.u_chunks = 1;
+          kernel<<<dim3(1u, (unsigned)kv_heads, (unsigned)batch), new_tokens * 32, 0, (cudaStream_t)stream>>>(q);
+          return check_launch("tq_append_kernel");
         }
         int ctas = 0;
         const int rc = bulk_resident_ctas(kernel, kAppendWarps * 32, resident, device, &ctas);
