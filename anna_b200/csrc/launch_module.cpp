@@ -423,56 +423,42 @@ at::Tensor upload_bytes(c10::DeviceIndex device, const void* data, int64_t bytes
   return out;
 }
 
-// upload(device index, rows) -> int64 [len(rows), len(rows[0])] on the device
+// Rows that are lists or tuples of ints and of one length, one after the other; false for all others.  Nothing here runs code of
+// the objects (an __index__ could shorten the very lists that are being read).
+bool plain_rows(PyObject* rows, std::vector<int64_t>* values, int64_t* count, int64_t* width) {
+  if (!PyList_CheckExact(rows) && !PyTuple_CheckExact(rows)) return false;
+  *count = PySequence_Fast_GET_SIZE(rows);
+  for (Py_ssize_t r = 0; r < *count; ++r) {
+    PyObject* row = PySequence_Fast_GET_ITEM(rows, r);
+    if (!PyList_CheckExact(row) && !PyTuple_CheckExact(row)) return false;
+    const Py_ssize_t entries = PySequence_Fast_GET_SIZE(row);
+    if (r == 0) {
+      *width = entries;
+      values->reserve((size_t)(*count * entries));
+    }
+    if (entries != *width) return false;
+    for (Py_ssize_t i = 0; i < entries; ++i) {
+      PyObject* entry = PySequence_Fast_GET_ITEM(row, i);
+      if (!PyLong_CheckExact(entry)) return false;
+      int overflow = 0;
+      values->push_back(PyLong_AsLongLongAndOverflow(entry, &overflow));
+      if (overflow != 0) return false;
+    }
+  }
+  return *count > 0;
+}
+
+// upload(device index, rows) -> int64 [len(rows), len(rows[0])] on the device | None
 PyObject* upload(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   if (nargs != 2) return PyErr_Format(PyExc_TypeError, "upload(device, rows)");
   const long device = PyLong_AsLong(args[0]);
   if (device == -1 && PyErr_Occurred()) return nullptr;
-  PyObject* rows = PySequence_Fast(args[1], "upload: rows must be a sequence");
-  if (rows == nullptr) return nullptr;
   std::vector<int64_t> values;
-  const Py_ssize_t n = PySequence_Fast_GET_SIZE(rows);
-  Py_ssize_t width = 0;
-  bool ok = n > 0;
-  if (!ok) PyErr_SetString(PyExc_ValueError, "upload: no rows");
-  for (Py_ssize_t r = 0; ok && r < n; ++r) {
-    PyObject* row = PySequence_Fast(PySequence_Fast_GET_ITEM(rows, r), "upload: a row must be a sequence");
-    ok = row != nullptr;
-    if (!ok) break;
-    const Py_ssize_t count = PySequence_Fast_GET_SIZE(row);
-    if (r == 0) {
-      width = count;
-      values.reserve((size_t)(n * width));
-    }
-    ok = count == width;
-    if (!ok) PyErr_SetString(PyExc_ValueError, "upload: rows of different lengths");
-    for (Py_ssize_t i = 0; ok && i < count; ++i) {
-      if (i >= PySequence_Fast_GET_SIZE(row)) {  // an entry's __index__ may have shortened the list
-        PyErr_SetString(PyExc_ValueError, "upload: rows of different lengths");
-        ok = false;
-        break;
-      }
-      PyObject* entry = PySequence_Fast_GET_ITEM(row, i);
-      int64_t value;
-      if (PyLong_CheckExact(entry)) {
-        value = PyLong_AsLongLong(entry);
-      } else {
-        Py_INCREF(entry);
-        PyObject* id = PyNumber_Index(entry);
-        Py_DECREF(entry);
-        value = id == nullptr ? -1 : PyLong_AsLongLong(id);
-        Py_XDECREF(id);
-      }
-      ok = !(value == -1 && PyErr_Occurred());
-      values.push_back(value);
-    }
-    Py_DECREF(row);
-  }
-  Py_DECREF(rows);
-  if (!ok) return nullptr;
+  int64_t count = 0, width = 0;
+  if (!plain_rows(args[1], &values, &count, &width)) Py_RETURN_NONE;
   const c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
-  return THPVariable_Wrap(upload_bytes((c10::DeviceIndex)device, values.data(), (int64_t)values.size() * 8, {(int64_t)n, (int64_t)width}, at::kLong));
+  return THPVariable_Wrap(upload_bytes((c10::DeviceIndex)device, values.data(), (int64_t)values.size() * 8, {count, width}, at::kLong));
   END_HANDLE_TH_ERRORS
 }
 

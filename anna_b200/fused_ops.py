@@ -12,6 +12,7 @@ import ctypes
 import os
 import threading
 
+import numpy as np
 import torch
 
 from . import _lib
@@ -125,7 +126,13 @@ class MetadataUploader:
 
     def upload(self, rows: list[list[int]]) -> torch.Tensor:
         """int64 [len(rows), len(rows[0])] on the device; the copy is ordered on the current stream."""
-        return self._module.upload(self.device.index, rows)
+        out = self._module.upload(self.device.index, rows)
+        if out is None:  # not lists of ints of one length: what numpy makes of them
+            host = np.empty((len(rows), len(rows[0])), dtype=np.int64)
+            for idx, row in enumerate(rows):
+                host[idx] = row
+            out = self._module.upload(self.device.index, host.tolist())
+        return out
 
     def upload_i32(self, values) -> torch.Tensor:
         """int32 copy of a flat numpy int32 array on the device, through the same pinned ring."""

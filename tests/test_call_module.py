@@ -203,6 +203,28 @@ def test_cache_steps_equal_general_path(cuda_device, watched, dtype, dim, gated)
     assert all(torch.equal(a, b) for a, b in zip(ours, theirs, strict=True))
 
 
+def test_uploads_of_other_rows_run_no_code_of_theirs():
+    """The module reads the rows in place, so an entry whose __index__ takes rows or entries away must not run meanwhile."""
+    module, ran = _lib.launch(), []
+
+    class Shortens:
+        def __init__(self, what):
+            self.what = what
+
+        def __index__(self):
+            ran.append(self.what)
+            self.what.clear()
+            return 1
+
+    rows = [[1, 2], [3, 4], [5, 6]]
+    rows[0][1] = Shortens(rows)
+    row = [1, 2, 3]
+    row[0] = Shortens(row)
+    for other in (rows, [row, [4, 5, 6]], [row], [[1, 2], [3]], [], [[]] * 2 + [[1]], [np.arange(3)], iter([[1]]), [[1 << 63]], [[1.0]], 7):
+        assert module.upload(0, other) is None
+    assert not ran and len(rows) == 3 and len(row) == 3
+
+
 @pytest.mark.gpu
 def test_uploads(cuda_device):
     """More uploads than the ring has buffers, behind work that keeps the copies waiting; growing ones; other integers."""
@@ -218,12 +240,15 @@ def test_uploads(cuda_device):
         words = np.arange(i * 50, i * 50 + 3000, dtype=np.int32)
         got.append(uploader.upload_i32(words))
         want.append(torch.from_numpy(words))
-    got += [uploader.upload([[np.int64(3), True]]), uploader.upload([(4,)]), uploader.upload([[]])]
-    want += [torch.tensor([[3, 1]]), torch.tensor([[4]]), torch.empty(1, 0, dtype=torch.int64)]
+    # whatever numpy makes int64 of
+    others = [([[np.int64(3), True]], [[3, 1]]), ([(4,)], [[4]]), (([5, 6], np.array([7, 8])), [[5, 6], [7, 8]]),
+              ([[1.5, -2.5], (3, 4.0)], [[1, -2], [3, 4]]), ([[1, 2], [3]], [[1, 2], [3, 3]]), (np.arange(6).reshape(2, 3), [[0, 1, 2], [3, 4, 5]])]
+    got += [uploader.upload([[]]), *(uploader.upload(rows) for rows, _ in others)]
+    want += [torch.empty(1, 0, dtype=torch.int64), *(torch.tensor(rows) for _, rows in others)]
     for ours, theirs in zip(got, want, strict=True):
         assert ours.dtype == theirs.dtype and torch.equal(ours.cpu(), theirs)
-    for rows in ([], [[1, 2], [3]], [[1.5]], [["a"]], 7):
-        with pytest.raises((ValueError, TypeError)):
+    for rows in ([], [[1], [2, 3]], [["a"]], [[1 << 63]], 7):
+        with pytest.raises((IndexError, ValueError, OverflowError, TypeError)):
             uploader.upload(rows)
     with pytest.raises(TypeError):
         uploader.upload_i32(np.zeros(3, dtype=np.int64))
