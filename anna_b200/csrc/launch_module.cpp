@@ -462,10 +462,10 @@ PyObject* upload(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// upload_i32(device index, contiguous int32 buffer) -> int32 [count] on the device
-PyObject* upload_i32(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+// upload_array(device index, contiguous buffer of int32 or int64) -> its entries, flat, on the device
+PyObject* upload_array(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
-  if (nargs != 2) return PyErr_Format(PyExc_TypeError, "upload_i32(device, buffer)");
+  if (nargs != 2) return PyErr_Format(PyExc_TypeError, "upload_array(device, buffer)");
   const long device = PyLong_AsLong(args[0]);
   if (device == -1 && PyErr_Occurred()) return nullptr;
   struct View {
@@ -475,11 +475,15 @@ PyObject* upload_i32(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
       if (held) PyBuffer_Release(&view);
     }
   } buffer;
-  buffer.held = PyObject_GetBuffer(args[1], &buffer.view, PyBUF_C_CONTIGUOUS) == 0;
+  buffer.held = PyObject_GetBuffer(args[1], &buffer.view, PyBUF_C_CONTIGUOUS | PyBUF_FORMAT) == 0;
   if (!buffer.held) return nullptr;
-  if (buffer.view.itemsize != 4) return PyErr_Format(PyExc_TypeError, "upload_i32: 32-bit integers expected");
+  const char* format = buffer.view.format == nullptr ? "" : buffer.view.format;
+  const bool narrow = std::strcmp(format, "i") == 0;
+  if (!narrow && std::strcmp(format, "l") != 0 && std::strcmp(format, "q") != 0)
+    return PyErr_Format(PyExc_TypeError, "upload_array: int32 or int64 expected, got '%s'", format);
   const c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
-  return THPVariable_Wrap(upload_bytes((c10::DeviceIndex)device, buffer.view.buf, buffer.view.len, {(int64_t)(buffer.view.len / 4)}, at::kInt));
+  return THPVariable_Wrap(upload_bytes((c10::DeviceIndex)device, buffer.view.buf, buffer.view.len,
+                                       {(int64_t)(buffer.view.len / buffer.view.itemsize)}, narrow ? at::kInt : at::kLong));
   END_HANDLE_TH_ERRORS
 }
 
@@ -685,7 +689,7 @@ PyMethodDef methods[] = {
     {"tq_append", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(tq_append)), METH_FASTCALL, nullptr},
     {"paged_decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(paged_decode)), METH_FASTCALL, nullptr},
     {"upload", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(upload)), METH_FASTCALL, nullptr},
-    {"upload_i32", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(upload_i32)), METH_FASTCALL, nullptr},
+    {"upload_array", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(upload_array)), METH_FASTCALL, nullptr},
     {"tq_gather_dense", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(tq_gather_dense)), METH_FASTCALL, nullptr},
     {"prefill", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(prefill)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},

@@ -131,12 +131,12 @@ class MetadataUploader:
             host = np.empty((len(rows), len(rows[0])), dtype=np.int64)
             for idx, row in enumerate(rows):
                 host[idx] = row
-            out = self._module.upload(self.device.index, host.tolist())
+            out = self._module.upload_array(self.device.index, host).view(host.shape)
         return out
 
     def upload_i32(self, values) -> torch.Tensor:
-        """int32 copy of a flat numpy int32 array on the device, through the same pinned ring."""
-        return self._module.upload_i32(self.device.index, values)
+        """int32 copy of a flat numpy array on the device, through the same pinned ring."""
+        return self._module.upload_array(self.device.index, np.ascontiguousarray(values, dtype=np.int32))
 
 
 def _require_cuda(name: str, **tensors: torch.Tensor | None) -> torch.device:

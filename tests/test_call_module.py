@@ -250,8 +250,11 @@ def test_uploads(cuda_device):
     for rows in ([], [[1], [2, 3]], [["a"]], [[1 << 63]], 7):
         with pytest.raises((IndexError, ValueError, OverflowError, TypeError)):
             uploader.upload(rows)
+    for values in (np.arange(5), np.arange(10, dtype=np.int32)[::2], np.array([1.5, -2.5]), np.array([True, False]), np.zeros(0, dtype=np.int64)):
+        ours = uploader.upload_i32(values)
+        assert ours.dtype == torch.int32 and ours.cpu().tolist() == values.astype(np.int32).tolist()
     with pytest.raises(TypeError):
-        uploader.upload_i32(np.zeros(3, dtype=np.int64))
+        _lib.launch().upload_array(0, np.zeros(3, dtype=np.float32))
 
 
 @pytest.mark.gpu
