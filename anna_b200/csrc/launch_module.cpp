@@ -12,6 +12,7 @@
 #include <ATen/Functions.h>
 #include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Device.h>
@@ -20,6 +21,7 @@
 
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <tuple>
 #include <vector>
 
@@ -368,12 +370,16 @@ PyObject* prefill(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 
 // The buffers of one device.  They are handed out in turn, under the interpreter lock; a buffer whose last copy is still under way
 // (sixteen uploads back: normally long done) is waited for without the lock, and is out of the ring for other threads meanwhile.
+// A slot gets its event, and a buffer that is large enough, when its turn comes: a failure in between leaves the others as they are.
 struct UploadRing {
   static constexpr int kSlots = 16;
-  int64_t capacity = -1;  // bytes of a buffer
-  at::Tensor buffers[kSlots];
-  cudaEvent_t done[kSlots] = {};
-  bool taken[kSlots] = {};
+  struct Slot {
+    at::Tensor buffer;
+    cudaEvent_t done = nullptr;
+    bool taken = false;
+  };
+  Slot slots[kSlots];
+  int64_t capacity = 8192;  // bytes of a buffer that is made now
   int next = 0;
 };
 std::map<int64_t, UploadRing>& upload_rings() {
@@ -381,45 +387,98 @@ std::map<int64_t, UploadRing>& upload_rings() {
   return *rings;
 }
 
-at::Tensor pinned_bytes(int64_t bytes) { return at::empty({bytes}, at::TensorOptions().dtype(at::kByte).pinned_memory(true)); }
+// Host copies for uploads that a graph captures: every replay reads its copy again, so the graph owns it.  One whose graph is gone
+// serves a later capture (a graph's last reference may end on a thread of the driver, which may not free it).
+struct CapturedBytes {
+  void* data;
+  size_t size;
+};
+std::mutex captured_free_lock;
+std::vector<CapturedBytes*>& captured_free() {
+  static auto* list = new std::vector<CapturedBytes*>();
+  return *list;
+}
+void captured_give_back(void* bytes) {
+  const std::lock_guard<std::mutex> lock(captured_free_lock);
+  captured_free().push_back(static_cast<CapturedBytes*>(bytes));
+}
+CapturedBytes* captured_take(size_t size) {
+  {
+    const std::lock_guard<std::mutex> lock(captured_free_lock);
+    auto& list = captured_free();
+    for (size_t i = 0; i < list.size(); ++i) {
+      if (list[i]->size < size) continue;
+      CapturedBytes* found = list[i];
+      list.erase(list.begin() + (std::ptrdiff_t)i);
+      return found;
+    }
+  }
+  size_t rounded = 256;
+  while (rounded < size) rounded *= 2;
+  void* data = nullptr;
+  C10_CUDA_CHECK(cudaHostAlloc(&data, rounded, cudaHostAllocPortable));
+  return new CapturedBytes{data, rounded};
+}
+
+// Copies the `bytes` at `data` to `out`, as part of the graph that `stream` captures.
+void upload_captured(void* out, const void* data, size_t bytes, cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  cudaGraph_t graph = nullptr;
+  C10_CUDA_CHECK(cudaStreamGetCaptureInfo(stream, &status, &id, &graph, nullptr, nullptr));
+  TORCH_CHECK(status == cudaStreamCaptureStatusActive, "anna_b200: upload under a graph capture that has failed");
+  CapturedBytes* kept = captured_take(bytes);
+  cudaUserObject_t owner = nullptr;
+  const cudaError_t made = cudaUserObjectCreate(&owner, kept, captured_give_back, 1, cudaUserObjectNoDestructorSync);
+  if (made != cudaSuccess) captured_give_back(kept);
+  C10_CUDA_CHECK(made);
+  const cudaError_t moved = cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove);
+  if (moved != cudaSuccess) (void)cudaUserObjectRelease(owner, 1);  // gives the copy back
+  C10_CUDA_CHECK(moved);
+  std::memcpy(kept->data, data, bytes);
+  C10_CUDA_CHECK(cudaMemcpyAsync(out, kept->data, bytes, cudaMemcpyHostToDevice, stream));
+}
 
 // A tensor of `sizes` with the `bytes` at `data` on the device, ordered on its current stream (the device must be current).
 at::Tensor upload_bytes(c10::DeviceIndex device, const void* data, int64_t bytes, at::IntArrayRef sizes, at::ScalarType type) {
-  UploadRing& ring = upload_rings()[device];
-  int slot = -1;
-  while (slot < 0) {
-    for (int i = 0; i < UploadRing::kSlots && slot < 0; ++i) {
-      const int candidate = (ring.next + i) % UploadRing::kSlots;
-      if (!ring.taken[candidate]) slot = candidate;
-    }
-    if (slot < 0) pybind11::gil_scoped_release others;  // as many threads wait for a buffer each
+  at::Tensor out = at::empty(sizes, at::TensorOptions().dtype(type).device(c10::Device(c10::kCUDA, device)));
+  if (bytes == 0) return out;
+  // waiting for an event and making pinned memory would end any thread's capture otherwise
+  const c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(device).stream();
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
+    upload_captured(out.data_ptr(), data, (size_t)bytes, stream);
+    return out;
   }
-  ring.next = (slot + 1) % UploadRing::kSlots;
+  UploadRing& ring = upload_rings()[device];
+  UploadRing::Slot* slot = nullptr;
+  while (slot == nullptr) {
+    for (int i = 0; i < UploadRing::kSlots && slot == nullptr; ++i) {
+      const int candidate = (ring.next + i) % UploadRing::kSlots;
+      if (ring.slots[candidate].taken) continue;
+      slot = &ring.slots[candidate];
+      ring.next = (candidate + 1) % UploadRing::kSlots;
+    }
+    if (slot == nullptr) pybind11::gil_scoped_release others;  // as many threads wait for a buffer each
+  }
   struct Taken {
     bool* flag;
     explicit Taken(bool* f) : flag(f) { *flag = true; }
     ~Taken() { *flag = false; }
-  } taken(&ring.taken[slot]);
-  if (bytes > ring.capacity) {
-    // all buffers at once, so that an upload under a graph capture, which may not allocate, finds its own
-    ring.capacity = std::max<int64_t>(8192, 2 * bytes);
-    for (int i = 0; i < UploadRing::kSlots; ++i) {
-      if (ring.taken[i] && i != slot) continue;
-      if (ring.done[i] == nullptr) C10_CUDA_CHECK(cudaEventCreateWithFlags(&ring.done[i], cudaEventDisableTiming));
-      C10_CUDA_CHECK(cudaEventSynchronize(ring.done[i]));
-      ring.buffers[i] = pinned_bytes(ring.capacity);
-    }
+  } taken(&slot->taken);
+  if (slot->done == nullptr) {
+    C10_CUDA_CHECK(cudaEventCreateWithFlags(&slot->done, cudaEventDisableTiming));
   } else {
     pybind11::gil_scoped_release waiting;
-    C10_CUDA_CHECK(cudaEventSynchronize(ring.done[slot]));
+    C10_CUDA_CHECK(cudaEventSynchronize(slot->done));
   }
-  at::Tensor& buffer = ring.buffers[slot];
-  if (buffer.numel() < bytes) buffer = pinned_bytes(ring.capacity);  // it was another thread's when the others grew
-  std::memcpy(buffer.data_ptr(), data, (size_t)bytes);
-  at::Tensor out = at::empty(sizes, at::TensorOptions().dtype(type).device(c10::Device(c10::kCUDA, device)));
-  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(device).stream();
-  if (bytes > 0) C10_CUDA_CHECK(cudaMemcpyAsync(out.data_ptr(), buffer.data_ptr(), (size_t)bytes, cudaMemcpyHostToDevice, stream));
-  C10_CUDA_CHECK(cudaEventRecord(ring.done[slot], stream));
+  if (slot->buffer.numel() < bytes) {
+    if (ring.capacity < bytes) ring.capacity = 2 * bytes;
+    slot->buffer = at::empty({ring.capacity}, at::TensorOptions().dtype(at::kByte).pinned_memory(true));
+  }
+  std::memcpy(slot->buffer.data_ptr(), data, (size_t)bytes);
+  C10_CUDA_CHECK(cudaMemcpyAsync(out.data_ptr(), slot->buffer.data_ptr(), (size_t)bytes, cudaMemcpyHostToDevice, stream));
+  C10_CUDA_CHECK(cudaEventRecord(slot->done, stream));
   return out;
 }
 

@@ -336,3 +336,38 @@ def test_two_threads_on_one_stream(cuda_device):
         thread.join()
     assert not errors, errors
     assert [int(count) for count in wrong] == [0, 0]
+
+
+@pytest.mark.gpu
+def test_uploads_under_a_capture(cuda_device):
+    """A captured upload has a host copy of its own, which replays read for as long as the graph lives; the ring goes on
+    without it, in sizes that it had and in larger ones."""
+    uploader = fused_ops.MetadataUploader.for_device(torch.device(cuda_device))
+
+    def capture(first, sizes):
+        rows = [[list(range(first + n, first + 2 * n))] for n in sizes]
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            captured = [uploader.upload(row) for row in rows] + [uploader.upload_i32(np.array(row[0])) for row in rows]
+        return graph, captured, [torch.tensor(row) for row in rows] + [torch.tensor(row[0], dtype=torch.int32) for row in rows]
+
+    def replayed(graph, captured, want):
+        for out in captured:
+            out.fill_(-7)
+        graph.replay()
+        return all(torch.equal(out.cpu(), row) for out, row in zip(captured, want, strict=True))
+
+    uploader.upload([[1]])
+    first = capture(0, [1, 700, 5000, 20000])
+    assert replayed(*first)
+    for i in range(40):                                              # the ring goes round, and grows
+        rows = [[i] * (1 + 900 * i)]
+        assert uploader.upload(rows).cpu().tolist() == rows
+    second = capture(1000, [3, 30000])
+    assert replayed(*second) and replayed(*first)
+    del first
+    torch.cuda.synchronize()
+    third = capture(5000, [1, 700, 5000, 20000])                     # may have the host copies of the first
+    for i in range(20):
+        assert uploader.upload([[i, -i]]).cpu().tolist() == [[i, -i]]
+    assert replayed(*third) and replayed(*second)
