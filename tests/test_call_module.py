@@ -225,6 +225,34 @@ def test_uploads_of_other_rows_run_no_code_of_theirs():
     assert not ran and len(rows) == 3 and len(row) == 3
 
 
+def test_uploads_without_the_module(monkeypatch):
+    """Un-quantized pages are written by the library alone, and their lengths and tables go up without the call module."""
+    def missing():
+        raise RuntimeError("not built")
+
+    monkeypatch.setattr(_lib, "launch", missing)
+    uploader = fused_ops.MetadataUploader(torch.device("cpu"))
+    rows = uploader.upload([[1, 2, 3], [1 << 40, 5, 6]])
+    assert rows.dtype == torch.int64 and rows.tolist() == [[1, 2, 3], [1 << 40, 5, 6]]
+    words = uploader.upload_i32(np.arange(6)[::2])
+    assert words.dtype == torch.int32 and words.tolist() == [0, 2, 4]
+
+
+@pytest.mark.gpu
+def test_pages_are_written_without_the_module(cuda_device, monkeypatch):
+    def missing():
+        raise RuntimeError("not built")
+
+    monkeypatch.setattr(_lib, "launch", missing)
+    monkeypatch.setattr(fused_ops.MetadataUploader, "_instances", {})
+    gen = torch.Generator(device=cuda_device).manual_seed(3)
+    keys, values = (torch.randn(2, 2, 41, 64, generator=gen, device=cuda_device, dtype=torch.bfloat16) for _ in range(2))
+    cache = Qwen3DynamicCache(KVCacheConfig(num_hidden_layers=1, cache_block_size=16), batch_size=2)
+    for at in range(0, 41, 20):
+        dense = cache.update(keys[:, :, at:at + 20], values[:, :, at:at + 20], 0)
+    assert torch.equal(dense[0][:, :, :41], keys) and torch.equal(dense[1][:, :, :41], values)
+
+
 @pytest.mark.gpu
 def test_uploads(cuda_device):
     """More uploads than the ring has buffers, behind work that keeps the copies waiting; growing ones; other integers."""
