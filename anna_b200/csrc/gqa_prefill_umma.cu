@@ -29,6 +29,7 @@
 #include "tma_utils.cuh"
 #include "umma_utils.cuh"
 
+#include <atomic>
 #include <cstdlib>
 #include <mutex>
 #include <type_traits>
@@ -1035,6 +1036,19 @@ static PrefillCosts mma_costs(int head_dim) {
   return head_dim == 64 ? PrefillCosts{0.88, 2.3, 0.0, 0.0} : PrefillCosts{1.65, 4.3, 0.0, 0.0};
 }
 
+// The current device and its SMs, asked for once per device (host time of a call of 5 positions over 20 keys with a query in every call
+// 5.17 us, so 5.04).
+static int sm_count(int* device, int* sms) {
+  static std::atomic<int> known[64];
+  ANNA_CUDA_CHECK(cudaGetDevice(device));
+  const bool listed = *device >= 0 && *device < 64;
+  *sms = listed ? known[*device].load(std::memory_order_relaxed) : 0;
+  if (*sms > 0) return ANNA_OK;
+  ANNA_CUDA_CHECK(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, *device));
+  if (listed) known[*device].store(*sms, std::memory_order_relaxed);
+  return ANNA_OK;
+}
+
 bool prefill_umma_applicable(const PrefillParams& p, int batch, int q_heads, int head_dim, int dtype) {
   static const bool disabled = [] {
     const char* flag = std::getenv("ANNA_B200_PREFILL_UMMA");
@@ -1054,9 +1068,7 @@ bool prefill_umma_applicable(const PrefillParams& p, int batch, int q_heads, int
   const int cta_rows = head_dim == 256 ? 128 : 256, heads_here = 1 << head_shift_of(p.groups);
   if (p.q_len >= 64 || (int64_t)p.q_len * heads_here * 2 >= cta_rows) return true;
   int device = 0, sms = 0;
-  if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-      sms <= 0)
-    return false;
+  if (sm_count(&device, &sms) != ANNA_OK || sms <= 0) return false;
   auto microseconds = [&](const PrefillCosts& costs, int64_t ctas, int64_t resident, int64_t keys) {
     return (double)((ctas + resident - 1) / resident) * (costs.fixed + costs.tile * (double)((p.key_len + keys - 1) / keys));
   };
@@ -1067,7 +1079,7 @@ bool prefill_umma_applicable(const PrefillParams& p, int batch, int q_heads, int
 // Tensor map of a [B, H, L, dim] 16-bit tensor given by element strides, seen as (dim, L, H, B).
 static bool prefill_tensor_map(CUtensorMap* out, const void* base, int64_t len, int heads, int batch, int64_t stride_t,
                                int64_t stride_h, int64_t stride_b, uint32_t box_len, uint32_t box_heads,
-                               int dim = kUpDim) {
+                               int dim) {
   if (len <= 0 || heads <= 0 || batch <= 0) return false;
   const uint64_t extents[4] = {(uint64_t)dim, (uint64_t)len, (uint64_t)heads, (uint64_t)batch};
   uint64_t strides[3] = {(uint64_t)stride_t * 2, (uint64_t)stride_h * 2, (uint64_t)stride_b * 2};
@@ -1080,14 +1092,29 @@ static bool prefill_tensor_map(CUtensorMap* out, const void* base, int64_t len, 
   return encode_map_16bit(out, base, 4, extents, strides, box);
 }
 
-using SplitResident = int[kMaxSplits + 1];  // CTAs in clusters of a size that the GPU holds at once ([1] 0 = not asked yet)
+// What the launches of a pair of kernels need to know of a device.  Each part is worked out by the first call that needs it and
+// published by its flag: later calls take no lock.
+struct SplitResident {
+  std::atomic<bool> plain_ready, split_ready;  // the kernel's attributes are set
+  int ctas[kMaxSplits + 1];                    // CTAs in clusters of a size that the GPU holds at once
+};
 
-template <typename Kernel>
-static int split_resident(Kernel kernel, int threads, uint32_t smem, int splits) {
+// The kernels of a head_dim and type: one CTA per query tile, and clusters that share its keys.
+struct PrefillKernels {
+  const void *plain, *split;
+  const char* name;
+  int threads;
+  uint32_t plain_smem, split_smem;
+  int key_tile, cta_rows;
+  PrefillCosts costs;
+  SplitResident* resident;  // of 64 devices
+};
+
+static int split_resident(const PrefillKernels& kernels, int splits) {
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3((unsigned)splits);
-  config.blockDim = dim3((unsigned)threads);
-  config.dynamicSmemBytes = smem;
+  config.blockDim = dim3((unsigned)kernels.threads);
+  config.dynamicSmemBytes = kernels.split_smem;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)splits;
@@ -1095,7 +1122,7 @@ static int split_resident(Kernel kernel, int threads, uint32_t smem, int splits)
   config.attrs = attr;
   config.numAttrs = 1;
   int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&clusters, kernels.split, &config) != cudaSuccess) {
     (void)cudaGetLastError();  // this size is not to be had: never chosen
     clusters = 0;
   }
@@ -1106,7 +1133,7 @@ static int split_resident(Kernel kernel, int threads, uint32_t smem, int splits)
 // makes of it, if that gains something (`filled`: part of a CTA's rows that exist).  Splitting pays for few query tiles over many keys
 // (one user's 123 tokens after 3095, 8/2 heads of 256: 47.5 -> 22.5 us; 4 rows of 24 after 2114, 16/2 heads: 43.3 -> 20); a grid
 // that fills the GPU, or one or two key tiles, stay as they are (119 query tiles of 256 over 3001 keys: 45 us, in pairs 72).
-static int choose_splits(const SplitResident& resident, const PrefillCosts& costs, int64_t base, int64_t tiles, double filled) {
+static int choose_splits(const int (&resident)[kMaxSplits + 1], const PrefillCosts& costs, int64_t base, int64_t tiles, double filled) {
   int best = 1;
   double best_cost = 0.0;
   for (int s = 1; s <= kMaxSplits; ++s) {
@@ -1121,100 +1148,104 @@ static int choose_splits(const SplitResident& resident, const PrefillCosts& cost
   return best;
 }
 
-template <typename Plain, typename Split>
-static int launch_plain_or_split(Plain plain, Split split, const char* name, const PrefillParams& p, const CUtensorMap& map_q,
-                                 const CUtensorMap& map_k, const CUtensorMap& map_v, dim3 grid, int threads, uint32_t plain_smem,
-                                 uint32_t split_smem, int key_tile, const PrefillCosts& costs, int cta_rows, SplitResident (&resident_of)[64],
-                                 cudaStream_t stream) {
-  int device = 0;
-  ANNA_CUDA_CHECK(cudaGetDevice(&device));
-  static std::mutex asking;
+// The number for a call of `grid` CTAs without sharing; afterwards the chosen kernel's attributes are set on the current device.
+static int splits_for(const PrefillKernels& kernels, const PrefillParams& p, dim3 grid, int* splits) {
+  static std::mutex first_calls;
+  int device = 0, sms = 0;
+  const int rc = sm_count(&device, &sms);
+  if (rc != ANNA_OK) return rc;
   SplitResident unlisted = {};
-  SplitResident& resident = device >= 0 && device < 64 ? resident_of[device] : unlisted;
-  std::unique_lock<std::mutex> lock(asking);
-  if (resident[1] == 0) {
-    ANNA_CUDA_CHECK(cudaFuncSetAttribute(plain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plain_smem));
-    ANNA_CUDA_CHECK(cudaFuncSetAttribute(split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)split_smem));
-    ANNA_CUDA_CHECK(cudaFuncSetAttribute(split, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    int sms = 0;
-    ANNA_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    for (int s = 2; s <= kMaxSplits; ++s) resident[s] = split_resident(split, threads, split_smem, s);
-    resident[1] = sms;
+  SplitResident& known = device >= 0 && device < 64 ? kernels.resident[device] : unlisted;
+  const int64_t base = (int64_t)grid.x * grid.y * grid.z, tiles = (p.key_len + kernels.key_tile - 1) / kernels.key_tile;
+  const double filled = (double)p.q_len / ((double)grid.x * (kernels.cta_rows >> head_shift_of(p.groups)));
+  bool ready = known.split_ready.load(std::memory_order_acquire);
+  if (!ready) {
+    // Where no number would gain anything with every SM taken, as most grids show, the second kernel is not loaded, nor the
+    // driver asked for fifteen cluster sizes.
+    int most[kMaxSplits + 1];
+    for (int s = 1; s <= kMaxSplits; ++s) most[s] = sms;
+    *splits = choose_splits(most, kernels.costs, base, tiles, filled);
+    if (*splits > 1) {
+      const std::lock_guard<std::mutex> lock(first_calls);
+      if (!known.split_ready.load(std::memory_order_relaxed)) {
+        ANNA_CUDA_CHECK(cudaFuncSetAttribute(kernels.split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kernels.split_smem));
+        ANNA_CUDA_CHECK(cudaFuncSetAttribute(kernels.split, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        known.ctas[1] = sms;
+        for (int s = 2; s <= kMaxSplits; ++s) known.ctas[s] = split_resident(kernels, s);
+        known.split_ready.store(true, std::memory_order_release);
+      }
+      ready = true;
+    }
   }
-  lock.unlock();
-  const int64_t base = (int64_t)grid.x * grid.y * grid.z;
+  if (ready) *splits = choose_splits(known.ctas, kernels.costs, base, tiles, filled);
+  if (*splits == 1 && !known.plain_ready.load(std::memory_order_acquire)) {
+    const std::lock_guard<std::mutex> lock(first_calls);
+    ANNA_CUDA_CHECK(cudaFuncSetAttribute(kernels.plain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kernels.plain_smem));
+    known.plain_ready.store(true, std::memory_order_release);
+  }
+  return ANNA_OK;
+}
+
+static int launch_plain_or_split(const PrefillKernels& kernels, const PrefillParams& p, const CUtensorMap& map_q, const CUtensorMap& map_k,
+                                 const CUtensorMap& map_v, dim3 grid, cudaStream_t stream) {
   PrefillParams sp = p;
-  const double filled = (double)p.q_len / ((double)grid.x * (cta_rows >> head_shift_of(p.groups)));
-  sp.splits = choose_splits(resident, costs, base, (p.key_len + key_tile - 1) / key_tile, filled);
-  if (sp.splits == 1) {
-    plain<<<grid, threads, plain_smem, stream>>>(sp, map_q, map_k, map_v);
-    return check_launch(name);
-  }
-  grid.x *= (unsigned)sp.splits;
+  const int rc = splits_for(kernels, p, grid, &sp.splits);
+  if (rc != ANNA_OK) return rc;
+  const void* arguments[] = {&sp, &map_q, &map_k, &map_v};
   cudaLaunchConfig_t config = {};
-  config.gridDim = grid;
-  config.blockDim = dim3((unsigned)threads);
-  config.dynamicSmemBytes = split_smem;
+  config.gridDim = dim3(grid.x * (unsigned)sp.splits, grid.y, grid.z);
+  config.blockDim = dim3((unsigned)kernels.threads);
+  config.dynamicSmemBytes = sp.splits > 1 ? kernels.split_smem : kernels.plain_smem;
   config.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)sp.splits;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   config.attrs = attr;
-  config.numAttrs = 1;
-  ANNA_CUDA_CHECK(cudaLaunchKernelEx(&config, split, sp, map_q, map_k, map_v));
-  return check_launch(name);
+  config.numAttrs = sp.splits > 1 ? 1 : 0;
+  ANNA_CUDA_CHECK(cudaLaunchKernelExC(&config, sp.splits > 1 ? kernels.split : kernels.plain, const_cast<void**>(arguments)));
+  return check_launch(kernels.name);
 }
 
 template <typename T>
-static int launch_prefill_umma_t(const PrefillParams& p, int batch, int q_heads, cudaStream_t stream) {
-  const int head_shift = head_shift_of(p.groups);
-  const int positions = kUpCtaRows >> head_shift;
-  CUtensorMap map_q, map_k, map_v;
-  const int kv_heads = q_heads / p.groups;
-  if (!prefill_tensor_map(&map_q, p.q, p.q_len, q_heads, batch, p.q_stride_t, p.q_stride_h, p.q_stride_b,
-                          (uint32_t)positions, 1u << head_shift) ||
-      !prefill_tensor_map(&map_k, p.k, p.key_len, kv_heads, batch, p.kv_stride_t, p.kv_stride_h, p.kv_stride_b, kUpKeys, 1) ||
-      !prefill_tensor_map(&map_v, p.v, p.key_len, kv_heads, batch, p.kv_stride_t, p.kv_stride_h, p.kv_stride_b, kUpKeys, 1))
-    return kPrefillNotServed;  // no encoder in this driver, or a layout it refuses: the mma.sync kernel takes over
-  static SplitResident resident[64] = {};
-  dim3 grid((unsigned)((p.q_len + positions - 1) / positions), (unsigned)(q_heads >> head_shift), (unsigned)batch);
-  return launch_plain_or_split(gqa_prefill_umma_kernel<T, false>, gqa_prefill_umma_kernel<T, true>, "gqa_prefill_umma_kernel", p,
-                               map_q, map_k, map_v, grid, kUpThreads, kUpSmem, SplitParts<kUpDim, kUpCtaRows>::smem_bytes(kUpSmem),
-                               kUpKeys, umma_costs(kUpDim), kUpCtaRows, resident, stream);
+static PrefillKernels umma_kernels() {
+  static SplitResident resident[64];
+  return {reinterpret_cast<const void*>(gqa_prefill_umma_kernel<T, false>), reinterpret_cast<const void*>(gqa_prefill_umma_kernel<T, true>),
+          "gqa_prefill_umma_kernel", kUpThreads, kUpSmem, SplitParts<kUpDim, kUpCtaRows>::smem_bytes(kUpSmem), kUpKeys, kUpCtaRows,
+          umma_costs(kUpDim), resident};
 }
-
 template <typename T, int D, int QT>
-static int launch_prefill_umma_wide_t(const PrefillParams& p, int batch, int q_heads, cudaStream_t stream) {
+static PrefillKernels umma_wide_kernels() {
   using Cfg = WideCfg<D, QT>;
-  const int head_shift = head_shift_of(p.groups);
-  const int positions = Cfg::kCtaRows >> head_shift;
-  CUtensorMap map_q, map_k, map_v;
-  const int kv_heads = q_heads / p.groups;
-  if (!prefill_tensor_map(&map_q, p.q, p.q_len, q_heads, batch, p.q_stride_t, p.q_stride_h, p.q_stride_b,
-                          (uint32_t)positions, 1u << head_shift, D) ||
-      !prefill_tensor_map(&map_k, p.k, p.key_len, kv_heads, batch, p.kv_stride_t, p.kv_stride_h, p.kv_stride_b, Cfg::kKeys, 1,
-                          D) ||
-      !prefill_tensor_map(&map_v, p.v, p.key_len, kv_heads, batch, p.kv_stride_t, p.kv_stride_h, p.kv_stride_b, Cfg::kKeys, 1,
-                          D))
-    return kPrefillNotServed;
-  static SplitResident resident[64] = {};
-  dim3 grid((unsigned)((p.q_len + positions - 1) / positions), (unsigned)(q_heads >> head_shift), (unsigned)batch);
-  return launch_plain_or_split(gqa_prefill_umma_wide_kernel<T, D, QT, false>, gqa_prefill_umma_wide_kernel<T, D, QT, true>,
-                               "gqa_prefill_umma_wide_kernel", p, map_q, map_k, map_v, grid, Cfg::kThreads, Cfg::kSmem,
-                               SplitParts<D, Cfg::kCtaRows>::smem_bytes(Cfg::kSmem), Cfg::kKeys,
-                               umma_costs(D), Cfg::kCtaRows, resident, stream);
+  static SplitResident resident[64];
+  return {reinterpret_cast<const void*>(gqa_prefill_umma_wide_kernel<T, D, QT, false>),
+          reinterpret_cast<const void*>(gqa_prefill_umma_wide_kernel<T, D, QT, true>), "gqa_prefill_umma_wide_kernel", Cfg::kThreads, Cfg::kSmem,
+          SplitParts<D, Cfg::kCtaRows>::smem_bytes(Cfg::kSmem), Cfg::kKeys, Cfg::kCtaRows, umma_costs(D), resident};
+}
+static PrefillKernels prefill_kernels(int head_dim, int dtype) {
+  const bool bf16 = dtype == ANNA_DTYPE_BF16;
+  if (head_dim == 256) return bf16 ? umma_wide_kernels<__nv_bfloat16, 256, 1>() : umma_wide_kernels<__half, 256, 1>();
+  if (head_dim == 64) return bf16 ? umma_wide_kernels<__nv_bfloat16, 64, 2>() : umma_wide_kernels<__half, 64, 2>();
+  return bf16 ? umma_kernels<__nv_bfloat16>() : umma_kernels<__half>();
+}
+static dim3 prefill_grid(const PrefillKernels& kernels, const PrefillParams& p, int batch, int q_heads) {
+  const int head_shift = head_shift_of(p.groups), positions = kernels.cta_rows >> head_shift;
+  return dim3((unsigned)((p.q_len + positions - 1) / positions), (unsigned)(q_heads >> head_shift), (unsigned)batch);
 }
 
 int launch_prefill_umma(const PrefillParams& p, int batch, int q_heads, int head_dim, int dtype, cudaStream_t stream) {
-  if (head_dim == 256)
-    return dtype == ANNA_DTYPE_BF16 ? launch_prefill_umma_wide_t<__nv_bfloat16, 256, 1>(p, batch, q_heads, stream)
-                                    : launch_prefill_umma_wide_t<__half, 256, 1>(p, batch, q_heads, stream);
-  if (head_dim == 64)
-    return dtype == ANNA_DTYPE_BF16 ? launch_prefill_umma_wide_t<__nv_bfloat16, 64, 2>(p, batch, q_heads, stream)
-                                    : launch_prefill_umma_wide_t<__half, 64, 2>(p, batch, q_heads, stream);
-  return dtype == ANNA_DTYPE_BF16 ? launch_prefill_umma_t<__nv_bfloat16>(p, batch, q_heads, stream)
-                                  : launch_prefill_umma_t<__half>(p, batch, q_heads, stream);
+  const PrefillKernels kernels = prefill_kernels(head_dim, dtype);
+  const int head_shift = head_shift_of(p.groups), kv_heads = q_heads / p.groups;
+  const uint32_t positions = (uint32_t)(kernels.cta_rows >> head_shift), key_tile = (uint32_t)kernels.key_tile;
+  CUtensorMap map_q, map_k, map_v;
+  if (!prefill_tensor_map(&map_q, p.q, p.q_len, q_heads, batch, p.q_stride_t, p.q_stride_h, p.q_stride_b, positions, 1u << head_shift,
+                          head_dim) ||
+      !prefill_tensor_map(&map_k, p.k, p.key_len, kv_heads, batch, p.kv_stride_t, p.kv_stride_h, p.kv_stride_b, key_tile, 1,
+                          head_dim) ||
+      !prefill_tensor_map(&map_v, p.v, p.key_len, kv_heads, batch, p.kv_stride_t, p.kv_stride_h, p.kv_stride_b, key_tile, 1,
+                          head_dim))
+    return kPrefillNotServed;  // no encoder in this driver, or a layout it refuses: the mma.sync kernel takes over
+  return launch_plain_or_split(kernels, p, map_q, map_k, map_v, prefill_grid(kernels, p, batch, q_heads), stream);
 }
 
 int prefill_umma_faults(int* count) {
