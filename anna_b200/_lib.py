@@ -43,6 +43,7 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "anna_kv_selftest_even_shares": (c_i32, [c_ptr] + [c_i32] * 8 + [c_ptr, c_i32, ctypes.POINTER(c_i32)]),
     "anna_kv_selftest_tq_schedule": (c_i32, [c_ptr, c_i64, c_i64] + [c_i32] * 4 + [c_i64] + [c_i32] * 6 +
                                      [ctypes.POINTER(c_i32)] * 2),
+    "anna_kv_selftest_prefill_choice": (c_i32, [c_i32] * 4 + [c_i64, c_i32, c_i32, ctypes.POINTER(c_i32), ctypes.POINTER(c_i32)]),
     "anna_kv_selftest_umma": (c_i32, [c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, ctypes.POINTER(c_i32), c_ptr]),
     "anna_decode_plan": (c_i32, [c_i32, c_i32, c_i64, ctypes.POINTER(c_i32), ctypes.POINTER(c_i32)]),
     "anna_paged_kv_write": (c_i32, [c_ptr, c_ptr, c_i64, c_i64, c_i64, c_ptr, c_ptr, c_ptr, c_i64, c_ptr, c_ptr, c_i32,

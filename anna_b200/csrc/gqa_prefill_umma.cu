@@ -137,8 +137,8 @@ __host__ __device__ inline int head_shift_of(int groups) {
 // memory, and each merges a part of the rows by reading all of them over distributed shared memory: no workspace, no second
 // launch.  All CTAs of a cluster reach both cluster barriers, whatever became of their waits.
 //
-// A split CTA must have its SM's tensor memory to itself: two CTAs of two clusters that waited for each other's on two SMs
-// would wait for ever, so it asks for more than half of an SM's shared memory.
+// Two CTAs do not share an SM's tensor memory, so a split CTA asks for more than half of its shared memory: then the number of
+// clusters that the driver says are resident counts one CTA per SM.
 constexpr int kMaxSplits = 16;  // the largest cluster
 constexpr uint32_t kSplitMinSmem = 120 * 1024;
 static_assert(2 * kSplitMinSmem > 228 * 1024, "two split CTAs fit one SM");
@@ -1049,6 +1049,23 @@ static int sm_count(int* device, int* sms) {
   return ANNA_OK;
 }
 
+static bool fills_half_a_cta(const PrefillParams& p, int head_dim) {
+  return p.q_len >= 64 || ((int64_t)p.q_len << head_shift_of(p.groups)) * 2 >= (head_dim == 256 ? 128 : 256);
+}
+
+// The rows of a CTA are query positions x the heads that share a KV head (a power of two, at most 16).  Chunks that fill less
+// than half a CTA's rows (and are shorter than 64 positions) leave most of a tile empty, but over more than a few dozen
+// keys the mma.sync kernel, which has a CTA read the keys for every head, takes longer all the same (8 positions, 32/8 heads
+// of 128 over 64 keys 7.5 us and 7.8 here; over 128 10.9 and 7.5; 16 over 4016 213 and 21 split; 64 rows of 5 over 505 284 and 57).
+static bool umma_is_faster(const PrefillParams& p, int batch, int q_heads, int head_dim, int sms) {
+  if (fills_half_a_cta(p, head_dim)) return true;
+  auto microseconds = [&](const PrefillCosts& costs, int64_t ctas, int64_t resident, int64_t keys) {
+    return (double)((ctas + resident - 1) / resident) * (costs.fixed + costs.tile * (double)((p.key_len + keys - 1) / keys));
+  };
+  return microseconds(umma_costs(head_dim), (int64_t)batch * (q_heads >> head_shift_of(p.groups)), sms, head_dim == 128 ? 128 : 64) <
+         microseconds(mma_costs(head_dim), (int64_t)batch * q_heads, 2 * (int64_t)sms, 32);
+}
+
 bool prefill_umma_applicable(const PrefillParams& p, int batch, int q_heads, int head_dim, int dtype) {
   static const bool disabled = [] {
     const char* flag = std::getenv("ANNA_B200_PREFILL_UMMA");
@@ -1061,19 +1078,10 @@ bool prefill_umma_applicable(const PrefillParams& p, int batch, int q_heads, int
   if (p.out_stride_b % 8 != 0 || p.out_stride_h % 8 != 0 || p.out_stride_t % 8 != 0) return false;
   if ((reinterpret_cast<uintptr_t>(p.out) & 15u) != 0) return false;
   if (p.key_len <= 0) return false;
-  // The rows of a CTA are query positions x the heads that share a KV head (a power of two, at most 16).  Chunks that fill less
-  // than half a CTA's rows (and are shorter than 64 positions) leave most of a tile empty, but over more than a few dozen
-  // keys the mma.sync kernel, which has a CTA read the keys for every head, takes longer all the same (8 positions, 32/8 heads
-  // of 128 over 64 keys 7.5 us and 7.8 here; over 128 10.9 and 7.5; 16 over 4016 213 and 21 split; 64 rows of 5 over 505 284 and 57).
-  const int cta_rows = head_dim == 256 ? 128 : 256, heads_here = 1 << head_shift_of(p.groups);
-  if (p.q_len >= 64 || (int64_t)p.q_len * heads_here * 2 >= cta_rows) return true;
+  if (fills_half_a_cta(p, head_dim)) return true;
   int device = 0, sms = 0;
   if (sm_count(&device, &sms) != ANNA_OK || sms <= 0) return false;
-  auto microseconds = [&](const PrefillCosts& costs, int64_t ctas, int64_t resident, int64_t keys) {
-    return (double)((ctas + resident - 1) / resident) * (costs.fixed + costs.tile * (double)((p.key_len + keys - 1) / keys));
-  };
-  return microseconds(umma_costs(head_dim), (int64_t)batch * (q_heads / heads_here), sms, head_dim == 128 ? 128 : 64) <
-         microseconds(mma_costs(head_dim), (int64_t)batch * q_heads, 2 * (int64_t)sms, 32);
+  return umma_is_faster(p, batch, q_heads, head_dim, sms);
 }
 
 // Tensor map of a [B, H, L, dim] 16-bit tensor given by element strides, seen as (dim, L, H, B).
@@ -1133,7 +1141,7 @@ static int split_resident(const PrefillKernels& kernels, int splits) {
 // makes of it, if that gains something (`filled`: part of a CTA's rows that exist).  Splitting pays for few query tiles over many keys
 // (one user's 123 tokens after 3095, 8/2 heads of 256: 47.5 -> 22.5 us; 4 rows of 24 after 2114, 16/2 heads: 43.3 -> 20); a grid
 // that fills the GPU, or one or two key tiles, stay as they are (119 query tiles of 256 over 3001 keys: 45 us, in pairs 72).
-static int choose_splits(const int (&resident)[kMaxSplits + 1], const PrefillCosts& costs, int64_t base, int64_t tiles, double filled) {
+static int choose_splits(const int* resident, const PrefillCosts& costs, int64_t base, int64_t tiles, double filled) {
   int best = 1;
   double best_cost = 0.0;
   for (int s = 1; s <= kMaxSplits; ++s) {
@@ -1148,6 +1156,16 @@ static int choose_splits(const int (&resident)[kMaxSplits + 1], const PrefillCos
   return best;
 }
 
+// What choose_splits looks at: CTAs without sharing, key tiles, and the part of the CTAs' rows that exists.
+struct SplitCall {
+  int64_t base, tiles;
+  double filled;
+  SplitCall(const PrefillKernels& kernels, const PrefillParams& p, dim3 grid)
+      : base((int64_t)grid.x * grid.y * grid.z),
+        tiles((p.key_len + kernels.key_tile - 1) / kernels.key_tile),
+        filled((double)p.q_len / ((double)grid.x * (kernels.cta_rows >> head_shift_of(p.groups)))) {}
+};
+
 // The number for a call of `grid` CTAs without sharing; afterwards the chosen kernel's attributes are set on the current device.
 static int splits_for(const PrefillKernels& kernels, const PrefillParams& p, dim3 grid, int* splits) {
   static std::mutex first_calls;
@@ -1156,15 +1174,14 @@ static int splits_for(const PrefillKernels& kernels, const PrefillParams& p, dim
   if (rc != ANNA_OK) return rc;
   SplitResident unlisted = {};
   SplitResident& known = device >= 0 && device < 64 ? kernels.resident[device] : unlisted;
-  const int64_t base = (int64_t)grid.x * grid.y * grid.z, tiles = (p.key_len + kernels.key_tile - 1) / kernels.key_tile;
-  const double filled = (double)p.q_len / ((double)grid.x * (kernels.cta_rows >> head_shift_of(p.groups)));
+  const SplitCall call(kernels, p, grid);
   bool ready = known.split_ready.load(std::memory_order_acquire);
   if (!ready) {
     // Where no number would gain anything with every SM taken, as most grids show, the second kernel is not loaded, nor the
     // driver asked for fifteen cluster sizes.
     int most[kMaxSplits + 1];
     for (int s = 1; s <= kMaxSplits; ++s) most[s] = sms;
-    *splits = choose_splits(most, kernels.costs, base, tiles, filled);
+    *splits = choose_splits(most, kernels.costs, call.base, call.tiles, call.filled);
     if (*splits > 1) {
       const std::lock_guard<std::mutex> lock(first_calls);
       if (!known.split_ready.load(std::memory_order_relaxed)) {
@@ -1177,7 +1194,7 @@ static int splits_for(const PrefillKernels& kernels, const PrefillParams& p, dim
       ready = true;
     }
   }
-  if (ready) *splits = choose_splits(known.ctas, kernels.costs, base, tiles, filled);
+  if (ready) *splits = choose_splits(known.ctas, kernels.costs, call.base, call.tiles, call.filled);
   if (*splits == 1 && !known.plain_ready.load(std::memory_order_acquire)) {
     const std::lock_guard<std::mutex> lock(first_calls);
     ANNA_CUDA_CHECK(cudaFuncSetAttribute(kernels.plain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kernels.plain_smem));
@@ -1256,3 +1273,25 @@ int prefill_umma_faults(int* count) {
 }
 
 }  // namespace anna
+
+// The choice between the kernels, without a launch: tests ask which one a call takes.
+extern "C" int anna_kv_selftest_prefill_choice(int batch, int q_heads, int kv_heads, int q_len, int64_t key_len, int head_dim, int dtype,
+                                               const int* cluster_ctas, int* splits) {
+  using namespace anna;
+  ANNA_REQUIRE(splits != nullptr && batch > 0 && kv_heads > 0 && q_heads > 0 && q_heads % kv_heads == 0 && q_len > 0 && key_len > 0,
+               "anna_kv_selftest_prefill_choice: bad argument");
+  PrefillParams p{};
+  p.q_len = q_len; p.key_len = key_len; p.groups = q_heads / kv_heads;
+  *splits = 0;
+  if (cluster_ctas == nullptr) {
+    if (!prefill_umma_applicable(p, batch, q_heads, head_dim, dtype)) return ANNA_OK;
+    const PrefillKernels kernels = prefill_kernels(head_dim, dtype);
+    return splits_for(kernels, p, prefill_grid(kernels, p, batch, q_heads), splits);
+  }
+  if ((head_dim != 64 && head_dim != 128 && head_dim != 256) || (dtype != ANNA_DTYPE_F16 && dtype != ANNA_DTYPE_BF16)) return ANNA_OK;
+  if (!umma_is_faster(p, batch, q_heads, head_dim, cluster_ctas[1])) return ANNA_OK;
+  const PrefillKernels kernels = prefill_kernels(head_dim, dtype);
+  const SplitCall call(kernels, p, prefill_grid(kernels, p, batch, q_heads));
+  *splits = choose_splits(cluster_ctas, kernels.costs, call.base, call.tiles, call.filled);
+  return ANNA_OK;
+}

@@ -73,6 +73,14 @@ int anna_kv_selftest_tq_schedule(const void* q, int64_t q_stride_b, int64_t q_st
                                  int head_dim, int64_t max_blocks, int block_size, int residual_len, int value_group, int dtype,
                                  int one_launch_ctas, int share_ctas, int* schedule, int* chunk_tokens);
 
+/* Which kernel anna_gqa_prefill takes for such a call on aligned rows: *splits = 0 the mma.sync kernel, 1 the tensor-memory kernel
+ * of the head_dim with one CTA per query tile, n clusters of n CTAs that share the keys of a query tile.  cluster_ctas = SMs at [1]
+ * and CTAs in clusters of n that the GPU holds at once at [n], n = 2 .. 16 (17 ints; then it needs no GPU), or NULL: those of the
+ * current device.  No counterpart in the reference.
+ */
+int anna_kv_selftest_prefill_choice(int batch, int q_heads, int kv_heads, int q_len, int64_t key_len, int head_dim, int dtype,
+                                    const int* cluster_ctas, int* splits);
+
 /*
  * Self-test of the tensor-memory matrix multiply (tcgen05) in the two operand arrangements of the packed decode:
  *   d1 float [128][16] = a1 . b1^T   a1 uint8 [128][128], b1 uint8 [16][128]: e4m3 bytes, K contiguous

@@ -2,6 +2,10 @@
 fixture computed by the reference's own grouped_query_attention (src/anna/model/ops.py:1552-1574)."""
 from __future__ import annotations
 
+import ctypes
+import os
+import subprocess
+import sys
 from pathlib import Path
 
 import numpy as np
@@ -9,9 +13,9 @@ import pytest
 import torch
 
 import oracle
-from anna_b200 import grouped_query_attention
+from anna_b200 import _lib, grouped_query_attention
 from anna_b200 import attention as attention_module
-from tests.helpers import ATOL, error_stats, to_np
+from tests.helpers import ATOL, DTYPE_CODE, error_stats, to_np
 
 pytestmark = pytest.mark.gpu
 GOLDEN = Path(__file__).resolve().parent / "golden"
@@ -26,6 +30,14 @@ def _model_masks(lengths: torch.Tensor, q_len: int, key_len: int, causal: bool):
         q_positions = (lengths - q_len)[:, None] + torch.arange(q_len, device=lengths.device)[None, :]
         causal_mask = positions[:, None, :] > q_positions[:, :, None]
     return causal_mask, visible
+
+
+def _kernel_of(batch, heads, kv_heads, q_len, key_len, dim, dtype) -> int:
+    """0: the mma.sync kernel, 1: the tensor-memory kernel, n: its clusters of n CTAs, which share the keys of a query tile."""
+    splits = ctypes.c_int(-1)
+    _lib.check(_lib.lib().anna_kv_selftest_prefill_choice(batch, heads, kv_heads, q_len, key_len, dim, DTYPE_CODE[dtype], None,
+                                                          ctypes.byref(splits)), "anna_kv_selftest_prefill_choice")
+    return splits.value
 
 
 def _oracle(q, k, v, lengths, causal):
@@ -78,6 +90,32 @@ def test_prefill_matches_oracle(cuda_device, dtype, heads, kv_heads, dim, q_len,
     assert torch.equal(again, out)
 
 
+@pytest.mark.parametrize("dtype,heads,kv_heads,dim,q_len,key_len,lengths,causal", [
+    (torch.bfloat16, 8, 2, 128, 8, 33, (33, 20), True),          # a few positions over a few keys stay with mma.sync
+    (torch.float16, 6, 2, 128, 9, 50, (50, 9, 3), False),
+    (torch.bfloat16, 8, 8, 128, 20, 64, (64, 20, 0), True),
+    (torch.float16, 16, 2, 256, 5, 30, (30, 7), True),
+    (torch.bfloat16, 32, 8, 256, 8, 31, (31, 8, 1), False),
+    (torch.bfloat16, 12, 4, 64, 7, 64, (64, 33, 5), True),
+])
+def test_short_chunks_over_few_keys(cuda_device, dtype, heads, kv_heads, dim, q_len, key_len, lengths, causal):
+    assert _kernel_of(len(lengths), heads, kv_heads, q_len, key_len, dim, dtype) == 0
+    test_prefill_matches_oracle(cuda_device, dtype, heads, kv_heads, dim, q_len, key_len, lengths, causal)
+
+
+def test_the_other_kernel_serves_every_shape(cuda_device):
+    """Where the driver refuses a tensor map, mma.sync takes what the tensor-memory kernels take otherwise: the same cases again in a
+    process of its own in which those are switched off."""
+    if os.environ.get("ANNA_B200_PREFILL_UMMA") == "0":
+        assert _kernel_of(1, 8, 2, 1024, 1024, 128, torch.bfloat16) == 0
+        return
+    done = subprocess.run([sys.executable, "-m", "pytest", "-q", "-x", "-p", "no:cacheprovider", __file__, "-k",
+                           "matches_oracle or reference_fixture or hold_anything or keep_growing or other_kernel"],
+                          env=dict(os.environ, ANNA_B200_PREFILL_UMMA="0"), cwd=Path(__file__).resolve().parent.parent,
+                          capture_output=True, text=True, timeout=600)
+    assert done.returncode == 0, done.stdout[-3000:]
+
+
 # few query tiles over many keys: the CTAs of a cluster share the keys
 SPLIT = [
     (torch.bfloat16, 8, 2, 256, 123, (3218,), True),
@@ -87,6 +125,16 @@ SPLIT = [
     (torch.bfloat16, 12, 4, 256, 9, (802,), True),               # three heads per KV head
     (torch.bfloat16, 6, 2, 128, 200, (1500, 129), False),
     (torch.float16, 4, 2, 64, 300, (2500, 2437), True),          # several query tiles, the last one partly filled
+    # clusters of two to four: the merge has registers for more rows and fewer parts at a time up to three
+    (torch.bfloat16, 9, 3, 64, 279, (792, 700, 280), True),
+    (torch.float16, 9, 3, 64, 48, (324, 324, 300), True),
+    (torch.bfloat16, 9, 3, 128, 278, (936, 278, 500, 900), True),
+    (torch.float16, 2, 2, 128, 6, (265,), False),
+    (torch.bfloat16, 9, 3, 256, 144, (1359, 1000, 144), True),
+    (torch.float16, 12, 4, 256, 15, (572, 15, 300), True),
+    (torch.bfloat16, 1, 1, 64, 141, (475, 475), True),
+    (torch.bfloat16, 4, 4, 128, 5, (507,), True),
+    (torch.float16, 1, 1, 256, 149, (969,), True),
 ]
 
 
@@ -95,6 +143,7 @@ def test_keys_shared_by_a_cluster(cuda_device, dtype, heads, kv_heads, dim, q_le
     """Relative bound: rounding P and the output to 16 bits, 2^-9 (bf16) and 2^-12 (fp16) each, twice that for what they share."""
     gen = torch.Generator().manual_seed(heads * 100 + q_len)
     batch, key_len = len(lengths), max(lengths)
+    assert _kernel_of(batch, heads, kv_heads, q_len, key_len, dim, dtype) > 1
     q = torch.randn(batch, heads, q_len, dim, generator=gen).to(dtype).to(cuda_device)
     k = torch.randn(batch, kv_heads, key_len, dim, generator=gen).to(dtype).to(cuda_device)
     v = torch.randn(batch, kv_heads, key_len, dim, generator=gen).to(dtype).to(cuda_device)
@@ -103,12 +152,12 @@ def test_keys_shared_by_a_cluster(cuda_device, dtype, heads, kv_heads, dim, q_le
     max_abs, rel_l2 = error_stats(to_np(out), _oracle(q, k, v, n, causal))
     assert max_abs <= ATOL[dtype] and rel_l2 <= 4 * (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12), (max_abs, rel_l2)
     # a NaN in a query reaches its own row and no other; one in a key reaches every row that sees it
-    q[0, 1, q_len - 1, 3] = float("nan")
+    q[0, -1, q_len - 1, 3] = float("nan")
     got = grouped_query_attention(q, k, v, scaling=dim ** -0.5, key_lengths=n, causal=causal)
-    assert bool(got[0, 1, q_len - 1].isnan().all())
-    got[0, 1, q_len - 1] = out[0, 1, q_len - 1]
+    assert bool(got[0, -1, q_len - 1].isnan().all())
+    got[0, -1, q_len - 1] = out[0, -1, q_len - 1]
     assert torch.equal(got, out)
-    q[0, 1, q_len - 1, 3] = 0.0
+    q[0, -1, q_len - 1, 3] = 0.0
     k[0, 0, lengths[0] // 3, 0] = float("nan")
     got = grouped_query_attention(q, k, v, scaling=dim ** -0.5, key_lengths=n, causal=causal)
     seen = got[0, :heads // kv_heads]
@@ -163,10 +212,6 @@ def test_scores_that_keep_growing_along_the_keys(cuda_device, dtype, dim):
 def test_tensor_memory_kernel_reported_no_expired_wait(cuda_device):
     """Runs after the cases above in this file: none of the bounded waits of the copy-engine / tensor-memory kernels may
     have run out."""
-    import ctypes
-
-    from anna_b200 import _lib
-
     q = torch.randn(1, 4, 128, 128, device=cuda_device, dtype=torch.bfloat16)
     k = torch.randn(1, 1, 256, 128, device=cuda_device, dtype=torch.bfloat16)
     out = grouped_query_attention(q, k, k, scaling=128 ** -0.5, key_lengths=torch.tensor([256], device=cuda_device),
@@ -221,7 +266,7 @@ def test_chunked_prefill_over_turboquant_cache_matches_oracle(cuda_device):
     """The reference's prefill flow on a quantized cache (ops.py:2008-2025): update(require_dense_cache=True) hands back
     the de-quantized prefix + window + chunk as dense K/V, the chunk's queries attend to it causally.  Rows of different
     lengths, two chunks each; the expectation is the oracle row's materialize() followed by the oracle attention."""
-    from tests.helpers import DTYPE_CODE, TQ_ATOL, TqPair
+    from tests.helpers import TQ_ATOL, TqPair
 
     dtype, heads, kv_heads, dim, bits, residual = torch.bfloat16, 8, 2, 128, 4, 16
     pair = TqPair(device=cuda_device, batch=2, kv_heads=kv_heads, head_dim=dim, bits=bits, residual_len=residual,
