@@ -374,10 +374,16 @@ static int launch_materialize(TqMaterializeParams p, int batch, int kv_heads, in
   if (!tq_make_layout(head_dim, bits, block_size, dtype_bytes_of(dtype), value_group, &p.layout))
     return set_error(ANNA_ERR_INVALID, "TurboQuant materialize: unsupported geometry D=%d bits=%d S=%d group=%d", head_dim,
                      bits, block_size, value_group);
+  const int64_t row_bytes = dtype_bytes_of(dtype);
+  const size_t access = lane_access_bytes(head_dim, (int)row_bytes);
+  auto steps_aligned = [&](int64_t stride, int64_t count) { return count <= 1 || stride * row_bytes % (int64_t)access == 0; };
+  ANNA_REQUIRE(aligned_to(p.key_out, access) && aligned_to(p.value_out, access) && aligned_to(p.window, access) && aligned_to(p.pages, 4) &&
+                   steps_aligned(p.out_stride_b, batch) && steps_aligned(p.out_stride_h, kv_heads) &&
+                   steps_aligned(p.out_stride_t, p.max_quantized_len),
+               "TurboQuant materialize: outputs, their strides and the window must be aligned to %d bytes, pages to 4", (int)access);
   const int64_t per_cta = (int64_t)kMaterializeWarps * kMaterializeTokens;
   dim3 grid((unsigned)((p.max_quantized_len + per_cta - 1) / per_cta), (unsigned)kv_heads, (unsigned)batch);
   // the bulk kernel's lanes move 16 bytes of dense rows, 8 of packed ones, and hold 16 values of one group
-  const int64_t row_bytes = dtype_bytes_of(dtype);
   const bool bulk = value_group >= kBulkCoords && aligned_to(p.key_out, 16) && aligned_to(p.value_out, 16) &&
                     aligned_to(p.window, 16) && aligned_to(p.pages, 8) && p.out_stride_b * row_bytes % 16 == 0 &&
                     p.out_stride_h * row_bytes % 16 == 0 && p.out_stride_t * row_bytes % 16 == 0;
