@@ -601,8 +601,27 @@ constexpr int kMergeHeads = kPair && D == 256 ? 4 : 8;
 
 // EARLY: what a segment starts with (pages, queries, constants) is read side by side, and the constants are worked out while the first
 // copies are on their way.  Kernels of many CTAs per SM, whose latencies others fill, keep the registers instead (64 rows of 32 K,
-// 32/8 heads, in chunks: 583 us, 587 with it; in shares 128 rows of 0.5-16 K, 3 bits, 210.3 -> 207.6, 64 of 4-32 K at head_dim 256,
-// 2 bits, 165.5 -> 162.9).  AHEAD: see fused_combine_ahead.
+// 32/8 heads, in chunks: 583 us, 587 with it).  AHEAD: see fused_combine_ahead.  In the other two launches the longer code and its
+// registers cost some instances more than the order gains, so each has what measured best: GPU times against neither of the two, means
+// over 160-170 shapes per instance (1 to 128 rows of 30 tokens to 32 K, 1 to 12 query heads per KV head).
+template <int D, int BITS, bool kPair>
+struct TqSmallOrder {
+  // AHEAD alone and both.  Head_dim 128, 4 bits: pairs 0.945 and 0.942 (one row of 4000 tokens, 32/8 heads, 11.6 us and 12.1, neither
+  // 12.0), eight heads 0.896 and 0.913; 2 bits: pairs 0.946 and 0.951, eight heads 0.907 and 0.906; 3 bits: 0.945 and 0.927, 0.924 and
+  // 0.926.  Head_dim 256, by bits: pairs 1.007, 1.020, 0.967 and 0.993, 0.995, 0.971 (four heads in 2 and 3 bits 1.004 and 1.014 with
+  // both; neither there was no faster than that over other shapes), eight heads 0.963, 0.973, 0.976 and 0.967, 0.954, 0.980.
+  static constexpr bool kEarly = D == 256 || BITS == 3 || (BITS == 2 && !kPair);
+};
+// Even shares have both (0.94-0.98) but for 4-bit pairs, which are the slower for it in short shares.
+template <int D, int BITS, bool kPair>
+constexpr bool kShareOrders = BITS == 4 && kPair;
+template <int D, int BITS, bool kPair, bool kShort>
+struct TqShareOrder {
+  // head_dim 128: EARLY has no registers for AHEAD
+  static constexpr bool kEarly = !(kShareOrders<D, BITS, kPair> && kShort);
+  static constexpr bool kAhead = !kShareOrders<D, BITS, kPair> || kShort == (D == 128);
+};
+
 constexpr int32_t kPageNotAsked = INT32_MIN;
 
 // Page of the tile that this lane copies in a warp's first step of a segment that starts at token t0, for kernels that know t0 before
@@ -626,7 +645,7 @@ __device__ __forceinline__ int32_t first_page_of(const TqDecodeParams& p, int b,
 // arithmetic, the softmax and the registers behind it are spent once per two tiles instead of once per tile with half of
 // the columns empty; columns j and j + 4 are two partials of head j, merged with those of the other warps.  64 rows of
 // 32 K tokens, 4 bits: 636 -> 614 us; 128 rows of 0.5-16 K, 3 bits: 247 -> 239 us.
-template <typename T, int D, int BITS, bool kPair, MergeLoads MERGE = MergeLoads::kAllColumns, bool EARLY = true, bool AHEAD = EARLY>
+template <typename T, int D, int BITS, bool kPair, MergeLoads MERGE = MergeLoads::kAllColumns, bool EARLY = false, bool AHEAD = EARLY>
 __device__ __forceinline__ void tq_packed_segment(const TqDecodeParams& p, uint8_t* smem_raw,
                                                   TqQueryConsts& qc, PackedRing& ring, int b, int unit,
                                                   int units, int t0, int t1, int out_slot, int slots, int arrivals,
@@ -1233,14 +1252,17 @@ struct TqSmallCfg {
 template <typename T, int D, int BITS, bool kPair>
 __global__ void __launch_bounds__(kMmaThreads, TqSmallCfg<T, D, BITS>::kMinBlocks)
     tq_decode_small_mma_kernel(const TqDecodeParams p) {
+  constexpr bool kEarly = TqSmallOrder<D, BITS, kPair>::kEarly;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int b = blockIdx.z;
   const int chunk = (int)blockIdx.x - p.num_window_chunks;
   const int t0 = chunk * p.chunk_tokens;
-  // the page, the constants and the lengths are read side by side
-  const int32_t first_page = chunk >= 0 ? first_page_of<T, D, BITS>(p, b, t0) : kPageNotAsked;
+  int32_t first_page = kPageNotAsked;
   TqRawConsts<D, BITS> consts;
-  consts.load(p);
+  if constexpr (kEarly) {  // the page, the constants and the lengths are read side by side
+    if (chunk >= 0) first_page = first_page_of<T, D, BITS>(p, b, t0);
+    consts.load(p);
+  }
   const RowChunks row = row_chunks(p, b);
   if (chunk < 0) {
     tq_window_chunk<T, D, 1, kMergeHeads<D, kPair>, true>(p, smem_raw, row, b, blockIdx.y, gridDim.y, blockIdx.x, true);
@@ -1250,10 +1272,14 @@ __global__ void __launch_bounds__(kMmaThreads, TqSmallCfg<T, D, BITS>::kMinBlock
   init_packed_barriers<T, D, BITS>(smem_raw);
   PackedRing ring{0, 0u, false};
   TqQueryConsts qc{};
+  if constexpr (!kEarly) {
+    consts.load(p);
+    qc = load_query_consts(consts);
+  }
   const int active = row.window + row.packed;
-  tq_packed_segment<T, D, BITS, kPair>(p, smem_raw, qc, ring, b, (int)blockIdx.y, (int)gridDim.y, t0,
-                                       min(row.quantized, t0 + p.chunk_tokens), row.window + chunk, active, active, first_page,
-                                       &consts);
+  tq_packed_segment<T, D, BITS, kPair, MergeLoads::kAllColumns, kEarly, true>(
+      p, smem_raw, qc, ring, b, (int)blockIdx.y, (int)gridDim.y, t0, min(row.quantized, t0 + p.chunk_tokens), row.window + chunk, active,
+      active, first_page, &consts);
 }
 
 // What a segment costs beyond its tiles (query preparation, first copy, merge: about 6 us), in tiles.  Over 512 shapes (1 to
@@ -1262,25 +1288,31 @@ __global__ void __launch_bounds__(kMmaThreads, TqSmallCfg<T, D, BITS>::kMinBlock
 constexpr int kTqSegmentTiles = 20;
 
 // Persistent variant: one resident wave, every CTA takes an even share of the packed tiles (balanced_schedule.cuh).
-template <typename T, int D, int BITS, bool kPair>
+template <typename T, int D, int BITS, bool kPair, bool kShort>
 __global__ void __launch_bounds__(kMmaThreads, TqMmaCfg<T, D, BITS>::kMinBlocks)
     tq_decode_balanced_mma_kernel(const TqDecodeParams p, const int batch) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // This instance has no registers for the loads of two columns and issues them one after the other (two rows of 12000 tokens,
   // 16/2 heads: 44.7 us, one column after the other 32.4; one of 20000, 64/8 heads: 45.7 and 36.2).
   constexpr MergeLoads kMerge = D == 128 && BITS == 3 && !kPair ? MergeLoads::kOneColumn : MergeLoads::kAllColumns;
-  constexpr bool kAhead = !(D == 128 && BITS == 4 && kPair);  // nor this one for the merge's loads ahead
+  using Order = TqShareOrder<D, BITS, kPair, kShort>;
   const int units = p.kv_heads * ((p.groups + 7) / 8);
   init_packed_barriers<T, D, BITS>(smem_raw);
   PackedRing ring{0, 0u, false};
   TqQueryConsts qc{};
+  if constexpr (!Order::kEarly) {
+    TqRawConsts<D, BITS> consts;
+    consts.load(p);
+    qc = load_query_consts(consts);
+  }
   balanced_for_each_segment<kMmaThreads, false>(
       p.lengths, p.max_len, batch, units, min(p.chunk_capacity, kFusedMaxChunks) - p.num_window_chunks,
       [](int) {},  // rows without packed tokens belong to the window kernel
       [&](int b, int unit, int t0, int t1, int slot, int partials) {
         const int active_window = (p.residual_len + p.chunk_tokens - 1) / p.chunk_tokens;  // the window of this row is full
-        tq_packed_segment<T, D, BITS, kPair, kMerge, true, kAhead>(p, smem_raw, qc, ring, b, unit, units, t0, t1, active_window + slot,
-                                                     active_window + partials, partials);
+        tq_packed_segment<T, D, BITS, kPair, kMerge, Order::kEarly, Order::kAhead>(p, smem_raw, qc, ring, b, unit, units, t0, t1,
+                                                                                   active_window + slot, active_window + partials,
+                                                                                   partials);
       },
       p.residual_len, kMmaWarps * TqMmaCfg<T, D, BITS>::kTilesPerStep, kTqSegmentTiles, kTqSegmentTiles);
   wait_for_prior_grids();
@@ -1331,6 +1363,17 @@ static bool tq_use_balanced(const TqDecodeParams& p, int batch, int head_dim, in
   const int64_t longest = p.num_chunks - p.num_window_chunks;
   if (p.chunk_tokens >= kTqLongestChunk && (longest <= 2 || batch * units * longest >= (int64_t)6 * ctas)) return false;
   return !tq_small(p, batch, head_dim, batch * units * (p.num_chunks - p.num_window_chunks) * 5, ctas * 4);
+}
+
+// Shares of so few tokens (counted by the longest row) are short.  4-bit pairs, GPU time in the order of short shares and of long ones,
+// against neither: head_dim 128, shares of 64-256 tokens 0.989 and 1.016 (18 rows of 0.5-3 K, 2/2 heads: single calls 18.8 and 19.7
+// us), 256-512 0.992 and 1.001, 512-768 0.995 and 0.993, above 2048 1.004 and 0.968; head_dim 256, of 32-128 tokens 1 and 1.08, 128-384 1
+// and 1.00 (single shapes up to 1.12), 384-768 1 and 0.989, above 2048 1 and 0.980.
+constexpr int64_t kTqShortShare = 512;
+
+static bool tq_short_shares(const TqDecodeParams& p, int batch, int ctas) {
+  const int64_t units = (int64_t)p.kv_heads * ((p.groups + 7) / 8);
+  return batch * units * (p.max_len - p.residual_len) < kTqShortShare * ctas;
 }
 
 // The launches of a call, and the chunks it is cut into.
@@ -1398,7 +1441,7 @@ static int launch_tq_mma(const TqDecodeParams& p, int batch, cudaStream_t stream
   const int group_tiles = (p.groups + 7) / 8;
   using Small = TqSmallCfg<T, D, BITS>;
   auto small = tq_decode_small_mma_kernel<T, D, BITS, kPair>;
-  auto balanced = tq_decode_balanced_mma_kernel<T, D, BITS, kPair>;
+  auto balanced = tq_decode_balanced_mma_kernel<T, D, BITS, kPair, false>;
   static int small_resident[64] = {}, balanced_resident[64] = {};
   int small_ctas = 0, balanced_ctas = 0;
   int rc = resident_ctas(small, Small::kSmemBytes, small_resident, device, &small_ctas);
@@ -1430,6 +1473,18 @@ static int launch_tq_mma(const TqDecodeParams& p, int batch, cudaStream_t stream
   config.attrs = attr;
   config.numAttrs = 1;
   if (launches.schedule == TqSchedule::kEvenShares) {
+    if constexpr (kShareOrders<D, BITS, kPair>) {
+      if (tq_short_shares(p, batch, balanced_ctas)) {
+        auto in_short = tq_decode_balanced_mma_kernel<T, D, BITS, kPair, true>;
+        static int short_resident[64] = {};
+        int short_ctas = 0;
+        rc = resident_ctas(in_short, Cfg::kSmemBytes, short_resident, device, &short_ctas);
+        if (rc != ANNA_OK) return rc;
+        config.gridDim = dim3((unsigned)short_ctas);
+        ANNA_CUDA_CHECK(cudaLaunchKernelEx(&config, in_short, p, batch));
+        return check_launch("tq_decode_balanced_mma_kernel");
+      }
+    }
     config.gridDim = dim3((unsigned)balanced_ctas);
     ANNA_CUDA_CHECK(cudaLaunchKernelEx(&config, balanced, p, batch));
     return check_launch("tq_decode_balanced_mma_kernel");

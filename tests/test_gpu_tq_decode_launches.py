@@ -56,6 +56,15 @@ def test_longer_chunks_in_one_launch(cuda_device, lengths, dim, bits):
           page=32 if dim == 256 else 16)
 
 
+@pytest.mark.parametrize("dim,kv_heads,rows", [(128, 8, 9), (256, 4, 13)])
+@pytest.mark.parametrize("group", [1, 3, 4])
+@pytest.mark.parametrize("longest", [1800, 3000, 6500])
+def test_short_and_long_shares_of_4_bit_pairs(cuda_device, dim, kv_heads, rows, group, longest):
+    """Shares of up to 512 tokens take an instance of their own: 303104 tokens of 592 CTAs at head_dim 128, 227328 of 444 at 256."""
+    check(cuda_device, [longest if i % 4 == 0 else 1 + (977 * i) % longest for i in range(rows)], way=EVEN_SHARES, heads=group * kv_heads,
+          kv_heads=kv_heads, dim=dim, bits=4, dtype=torch.float16 if group == 3 else torch.bfloat16, gated=group == 3)
+
+
 @pytest.mark.parametrize("dim,bits,heads", [(128, 4, 8), (128, 3, 2), (256, 2, 22)])
 @pytest.mark.parametrize("lengths", [[700], [WINDOW + 5, 1, 2300, 90]])
 def test_query_rows_at_odd_elements(cuda_device, dim, bits, heads, lengths):
