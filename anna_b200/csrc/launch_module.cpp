@@ -370,7 +370,7 @@ PyObject* prefill(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 
 // The buffers of one device.  They are handed out in turn, under the interpreter lock; a buffer whose last copy is still under way
 // (sixteen uploads back: normally long done) is waited for without the lock, and is out of the ring for other threads meanwhile.
-// A slot gets its event, and a buffer that is large enough, when its turn comes: a failure in between leaves the others as they are.
+// A slot that has no event or too small a buffer gets it when its turn comes: a failure in between leaves the others as they are.
 struct UploadRing {
   static constexpr int kSlots = 16;
   struct Slot {
@@ -468,13 +468,24 @@ at::Tensor upload_bytes(c10::DeviceIndex device, const void* data, int64_t bytes
   } taken(&slot->taken);
   if (slot->done == nullptr) {
     C10_CUDA_CHECK(cudaEventCreateWithFlags(&slot->done, cudaEventDisableTiming));
-  } else {
+  } else if (cudaEventQuery(slot->done) != cudaSuccess) {
+    (void)cudaGetLastError();
     pybind11::gil_scoped_release waiting;
     C10_CUDA_CHECK(cudaEventSynchronize(slot->done));
   }
   if (slot->buffer.numel() < bytes) {
     if (ring.capacity < bytes) ring.capacity = 2 * bytes;
-    slot->buffer = at::empty({ring.capacity}, at::TensorOptions().dtype(at::kByte).pinned_memory(true));
+    auto grow = [&](UploadRing::Slot& small) {
+      if (small.buffer.numel() < ring.capacity)
+        small.buffer = at::empty({ring.capacity}, at::TensorOptions().dtype(at::kByte).pinned_memory(true));
+    };
+    grow(*slot);
+    // and those whose copies are done, so that the next uploads of this size find theirs
+    for (UploadRing::Slot& other : ring.slots) {
+      if (other.taken) continue;
+      if (other.done == nullptr || cudaEventQuery(other.done) == cudaSuccess) grow(other);
+      else (void)cudaGetLastError();
+    }
   }
   std::memcpy(slot->buffer.data_ptr(), data, (size_t)bytes);
   C10_CUDA_CHECK(cudaMemcpyAsync(out.data_ptr(), slot->buffer.data_ptr(), (size_t)bytes, cudaMemcpyHostToDevice, stream));
@@ -521,10 +532,11 @@ PyObject* upload(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// upload_array(device index, contiguous buffer of int32 or int64) -> its entries, flat, on the device
-PyObject* upload_array(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+// upload_i32(device index, buffer), upload_i64(device index, buffer) -> the buffer's entries, flat, on the device | None unless it is
+// contiguous and of that type
+PyObject* upload_buffer(PyObject* const* args, Py_ssize_t nargs, at::ScalarType type) {
   HANDLE_TH_ERRORS
-  if (nargs != 2) return PyErr_Format(PyExc_TypeError, "upload_array(device, buffer)");
+  if (nargs != 2) return PyErr_Format(PyExc_TypeError, "upload of a buffer: (device, buffer)");
   const long device = PyLong_AsLong(args[0]);
   if (device == -1 && PyErr_Occurred()) return nullptr;
   struct View {
@@ -535,16 +547,20 @@ PyObject* upload_array(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     }
   } buffer;
   buffer.held = PyObject_GetBuffer(args[1], &buffer.view, PyBUF_C_CONTIGUOUS | PyBUF_FORMAT) == 0;
-  if (!buffer.held) return nullptr;
+  if (!buffer.held) {
+    PyErr_Clear();
+    Py_RETURN_NONE;
+  }
   const char* format = buffer.view.format == nullptr ? "" : buffer.view.format;
-  const bool narrow = std::strcmp(format, "i") == 0;
-  if (!narrow && std::strcmp(format, "l") != 0 && std::strcmp(format, "q") != 0)
-    return PyErr_Format(PyExc_TypeError, "upload_array: int32 or int64 expected, got '%s'", format);
+  const bool fits = type == at::kInt ? std::strcmp(format, "i") == 0 : std::strcmp(format, "l") == 0 || std::strcmp(format, "q") == 0;
+  if (!fits) Py_RETURN_NONE;
   const c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
   return THPVariable_Wrap(upload_bytes((c10::DeviceIndex)device, buffer.view.buf, buffer.view.len,
-                                       {(int64_t)(buffer.view.len / buffer.view.itemsize)}, narrow ? at::kInt : at::kLong));
+                                       {(int64_t)(buffer.view.len / buffer.view.itemsize)}, type));
   END_HANDLE_TH_ERRORS
 }
+PyObject* upload_i32(PyObject*, PyObject* const* args, Py_ssize_t nargs) { return upload_buffer(args, nargs, at::kInt); }
+PyObject* upload_i64(PyObject*, PyObject* const* args, Py_ssize_t nargs) { return upload_buffer(args, nargs, at::kLong); }
 
 // tq_gather_dense(packed_pages | None, table | None, window, slots, lengths, signs1, signs2, centroids, max_len, block_size,
 //                 residual_len, bits, value_group, num_pages) -> (keys, values) | None
@@ -748,7 +764,8 @@ PyMethodDef methods[] = {
     {"tq_append", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(tq_append)), METH_FASTCALL, nullptr},
     {"paged_decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(paged_decode)), METH_FASTCALL, nullptr},
     {"upload", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(upload)), METH_FASTCALL, nullptr},
-    {"upload_array", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(upload_array)), METH_FASTCALL, nullptr},
+    {"upload_i64", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(upload_i64)), METH_FASTCALL, nullptr},
+    {"upload_i32", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(upload_i32)), METH_FASTCALL, nullptr},
     {"tq_gather_dense", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(tq_gather_dense)), METH_FASTCALL, nullptr},
     {"prefill", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(prefill)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},

@@ -114,6 +114,7 @@ class MetadataUploader:
 
     def __init__(self, device: torch.device) -> None:
         self.device = device
+        self._index = device.index
         try:
             self._module = _lib.launch()
         except RuntimeError:  # writing un-quantized pages takes the library alone: synchronous copies do for its lengths and tables
@@ -129,22 +130,26 @@ class MetadataUploader:
 
     def upload(self, rows: list[list[int]]) -> torch.Tensor:
         """int64 [len(rows), len(rows[0])] on the device; the copy is ordered on the current stream."""
-        out = None if self._module is None else self._module.upload(self.device.index, rows)
+        module = self._module
+        out = None if module is None else module.upload(self._index, rows)
         if out is None:  # not lists of ints of one length: what numpy makes of them
             host = np.empty((len(rows), len(rows[0])), dtype=np.int64)
             for idx, row in enumerate(rows):
                 host[idx] = row
-            out = self._upload_array(host).view(host.shape)
+            out = self._copy(host) if module is None else module.upload_i64(self._index, host).view(host.shape)
         return out
 
     def upload_i32(self, values) -> torch.Tensor:
         """int32 copy of a flat numpy array on the device, through the same pinned ring."""
-        return self._upload_array(np.ascontiguousarray(values, dtype=np.int32))
+        module = self._module
+        out = None if module is None else module.upload_i32(self._index, values)
+        if out is None:  # another type, strides, or no module
+            host = np.ascontiguousarray(values, dtype=np.int32)
+            out = self._copy(host) if module is None else module.upload_i32(self._index, host)
+        return out
 
-    def _upload_array(self, host: np.ndarray) -> torch.Tensor:
-        if self._module is None:
-            return torch.from_numpy(host).reshape(-1).to(self.device)
-        return self._module.upload_array(self.device.index, host)
+    def _copy(self, host: np.ndarray) -> torch.Tensor:
+        return torch.from_numpy(host).to(self.device)
 
 
 def _require_cuda(name: str, **tensors: torch.Tensor | None) -> torch.device:
