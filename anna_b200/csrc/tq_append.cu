@@ -294,8 +294,8 @@ constexpr __host__ __device__ uint32_t round_residue(int count, int step) {
 //
 // What bounds that kernel is the issue rate, and most of its instructions are spent once per token in all lanes alike (square
 // roots, reciprocals, addresses, page ids, scales) or on exchanges between lanes; here they serve 2 to 8 tokens, 4 of the
-// butterfly levels stay inside a lane instead of 2, and sums, differences and most products go two to an instruction: 247
-// instructions per packed token-head instead of 567 (3 bits, head_dim 128), issued in 55 % of the cycles by 13 warps per SM.
+// butterfly levels stay inside a lane instead of 2, and sums, differences and most products go two to an instruction: 236
+// instructions per packed token-head instead of 584 (3 bits, head_dim 128), issued in 58 % of the cycles by 14 warps per SM.
 // GPU time of a call: 8 x 2048 tokens, 4 heads of 128, 3 bits 55.3 -> 32.8 us; 64 x 2048, 8 heads, 4 bits 726 -> 418; 16 x
 // 1500, 2 heads of 256 63.5 -> 49; one row of 953, 2 heads of 256 12.3 -> 10.3.
 template <typename T, int D, int BITS>
@@ -546,7 +546,7 @@ constexpr int64_t kBulkTokenHeads = 1024;
 constexpr int kBulkTokens = 8;
 
 // Whether tq_append_bulk_kernel takes a call: its lanes move 16 bytes and hold 16 coordinates of one value group.
-static bool append_in_bulk(const TqAppendParams& p, int head_dim) {
+static bool append_in_bulk(const TqAppendParams& p) {
   if (p.value_group < kBulkCoords || !aligned_to(p.k_new, 16) || !aligned_to(p.v_new, 16) || !aligned_to(p.window, 16) ||
       !aligned_to(p.pages, 8))
     return false;
@@ -624,7 +624,7 @@ extern "C" int anna_tq_append(const void* k_new, const void* v_new, int64_t kn_s
         ANNA_CUDA_CHECK(cudaGetDevice(&device));
         const int64_t heads_total = (int64_t)kv_heads * batch;
         TqAppendParams q = p;
-        if (append_in_bulk(p, head_dim)) {
+        if (append_in_bulk(p)) {
           auto bulk = tq_append_bulk_kernel<T, D, BITS>;
           static int bulk_resident[64] = {};
           int ctas = 0;

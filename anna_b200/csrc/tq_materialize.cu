@@ -215,7 +215,7 @@ __device__ __forceinline__ void bulk_fwht_signs(__half2 (&s)[kBulkPairs], int la
 
 // The same tokens and the same results as tq_materialize_kernel, several tokens per warp (tq_bulk.cuh), for value groups of 16
 // or more and 16-byte aligned rows.  The codes of a warp's next tokens are on their way while it works on the current ones.
-// That kernel is bound by its instructions, too: 8 x 2176 tokens, 4 heads of 128, 3 bits 45.1 -> 24.6 us (180 instructions per
+// That kernel is bound by its instructions, too: 8 x 2176 tokens, 4 heads of 128, 3 bits 45.1 -> 24.6 us (169 instructions per
 // token-head); 64 x 2176, 8 heads, 4 bits 485 -> 233; one row of 1081 tokens, 2 heads of 256 22.5 -> 10.2.
 template <typename T, int D, int BITS>
 __global__ void __launch_bounds__(kBulkWarps * 32, kMaterializeBulkCtasPerSm)
