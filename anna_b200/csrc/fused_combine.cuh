@@ -26,6 +26,94 @@ struct FusedCombine {
 
 constexpr int kFusedMaxChunks = 512;  // weights of one head are staged in shared memory
 
+// ---- what both forms of the merge below are made of ----------------------------------------------------------------------
+
+// Counts this CTA's partial; true in all threads of the CTA that is the last of `arrivals`.
+__device__ __forceinline__ bool merge_arrive(const FusedCombine& fc, int64_t counter_index, int arrivals) {
+  __shared__ int s_is_last;
+  __syncthreads();  // all partial stores of this CTA are ordered before the arrival below
+  if (threadIdx.x == 0) {
+    // releases this CTA's partial and acquires those of the CTAs counted before; the barriers on both sides extend that to
+    // the other threads (4 un-quantized rows of 60-900 tokens: 10.8 us with a full fence on either side, 10.3 so)
+    int32_t* counter = fc.counters + counter_index;
+    int prev;
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;\n" : "=r"(prev) : "l"(counter) : "memory");
+    s_is_last = (prev == arrivals - 1) ? 1 : 0;
+    if (s_is_last) *counter = 0;
+  }
+  __syncthreads();
+  return s_is_last != 0;
+}
+
+// A warp works out the weights of one head: max, denominator, normalised weights.
+__device__ __forceinline__ void merge_weigh_head(const float* stats, int chunk_capacity, int active_chunks, float* smem_weights, int g,
+                                                 int lane) {
+  const float* st = stats + (int64_t)g * chunk_capacity * 2;
+  float m = -INFINITY;
+  for (int c = lane; c < active_chunks; c += 32) m = fmaxf(m, __ldcg(st + 2 * c));
+#pragma unroll
+  for (int d = 16; d >= 1; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+  const float m_ref = m == -INFINITY ? 0.0f : m;
+  float den = 0.0f;
+  for (int c = lane; c < active_chunks; c += 32) {
+    const float w = __expf(__ldcg(st + 2 * c) - m_ref);
+    den += __ldcg(st + 2 * c + 1) * w;
+    smem_weights[g * kFusedMaxChunks + c] = w;
+  }
+#pragma unroll
+  for (int d = 16; d >= 1; d >>= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
+  const float inv = den > 0.0f ? 1.0f / den : 0.0f;
+  for (int c = lane; c < active_chunks; c += 32) smem_weights[g * kFusedMaxChunks + c] *= inv;
+}
+
+__device__ __forceinline__ void merge_add(float4& acc, const float4& v, float w) {
+  acc.x = fmaf(v.x, w, acc.x);
+  acc.y = fmaf(v.y, w, acc.y);
+  acc.z = fmaf(v.z, w, acc.z);
+  acc.w = fmaf(v.w, w, acc.w);
+}
+
+// Four dims of a query head, gated, to this GPU's output and the peers'.
+template <typename T>
+__device__ __forceinline__ void merge_store4(const FusedCombine& fc, int b, int hq, int d, const float4& o) {
+  const float acc[4] = {o.x, o.y, o.z, o.w};
+  const T* gate = fc.gate == nullptr ? nullptr
+                                     : reinterpret_cast<const T*>(fc.gate) + (int64_t)b * fc.gate_stride_b +
+                                           (int64_t)hq * fc.gate_stride_h + d;
+  const int64_t offset = (int64_t)b * fc.out_stride_b + (int64_t)hq * fc.out_stride_h + d;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const T result = ElemTraits<T>::from_float(gate ? acc[i] * sigmoidf_fast(ElemTraits<T>::to_float(gate[i])) : acc[i]);
+    reinterpret_cast<T*>(fc.out)[offset + i] = result;
+    for (int peer = 0; peer < fc.num_peers; ++peer) reinterpret_cast<T*>(fc.peers[peer])[offset + i] = result;
+  }
+}
+
+// The whole sum, one dim per thread, where the values are not aligned for four; then the fence behind the peers' stores.
+template <typename T, int D, int THREADS>
+__device__ __forceinline__ void merge_finish(const FusedCombine& fc, int b, int hq0, int g_count, int active_chunks, int chunk_capacity,
+                                             const float* values, const float* smem_weights, bool aligned) {
+  for (int item = threadIdx.x; !aligned && item < g_count * D; item += THREADS) {
+    const int g = item / D;
+    const int d = item % D;
+    const float* vals = values + (int64_t)g * chunk_capacity * D + d;
+    const float* w = smem_weights + g * kFusedMaxChunks;
+    float acc = 0.0f;
+    for (int c = 0; c < active_chunks; ++c) acc = fmaf(__ldcg(vals + (int64_t)c * D), w[c], acc);
+    if (fc.gate) {
+      const T* gate = reinterpret_cast<const T*>(fc.gate) + (int64_t)b * fc.gate_stride_b +
+                      (int64_t)(hq0 + g) * fc.gate_stride_h;
+      acc *= sigmoidf_fast(ElemTraits<T>::to_float(gate[d]));
+    }
+    const int64_t offset = (int64_t)b * fc.out_stride_b + (int64_t)(hq0 + g) * fc.out_stride_h + d;
+    const T result = ElemTraits<T>::from_float(acc);
+    reinterpret_cast<T*>(fc.out)[offset] = result;
+    for (int peer = 0; peer < fc.num_peers; ++peer) reinterpret_cast<T*>(fc.peers[peer])[offset] = result;
+  }
+  // stores to other GPUs are ordered before whatever this stream signals to them after the kernel
+  if (fc.num_peers > 0) __threadfence_system();
+}
+
 // Called by all threads of the CTA after they wrote their partial.  `active_chunks` = partials that contribute to this
 // (row, group); `arrivals` of them (0 = all; the others are known to be complete before any arrival) are counted in
 // counters[counter_index]; stats / values point at chunk 0 of query head hq0.  Natural-log stats.  THREADS = blockDim.x,
@@ -36,56 +124,14 @@ __device__ __forceinline__ void fused_combine_tail(const FusedCombine& fc, int b
                                                    int active_chunks, int chunk_capacity, const float* stats,
                                                    const float* values, float* smem_weights /* [8][kFusedMaxChunks] */,
                                                    int64_t counter_index, int arrivals = 0) {
-  __shared__ int s_is_last;
-  __syncthreads();  // all partial stores of this CTA are ordered before the arrival below
-  if (threadIdx.x == 0) {
-    // releases this CTA's partial and acquires those of the CTAs counted before; the barriers on both sides extend that to
-    // the other threads (4 un-quantized rows of 60-900 tokens: 10.8 us with a full fence on either side, 10.3 so)
-    int32_t* counter = fc.counters + counter_index;
-    int prev;
-    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;\n" : "=r"(prev) : "l"(counter) : "memory");
-    s_is_last = (prev == (arrivals > 0 ? arrivals : active_chunks) - 1) ? 1 : 0;
-    if (s_is_last) *counter = 0;
-  }
-  __syncthreads();
-  if (!s_is_last) return;
+  if (!merge_arrive(fc, counter_index, arrivals > 0 ? arrivals : active_chunks)) return;
 
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   constexpr int kWarps = THREADS / 32;
-  // one warp per head: max, denominator, normalised weights
-  for (int g = warp; g < g_count; g += kWarps) {
-    const float* st = stats + (int64_t)g * chunk_capacity * 2;
-    float m = -INFINITY;
-    for (int c = lane; c < active_chunks; c += 32) m = fmaxf(m, __ldcg(st + 2 * c));
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
-    const float m_ref = m == -INFINITY ? 0.0f : m;
-    float den = 0.0f;
-    for (int c = lane; c < active_chunks; c += 32) {
-      const float w = __expf(__ldcg(st + 2 * c) - m_ref);
-      den += __ldcg(st + 2 * c + 1) * w;
-      smem_weights[g * kFusedMaxChunks + c] = w;
-    }
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
-    const float inv = den > 0.0f ? 1.0f / den : 0.0f;
-    for (int c = lane; c < active_chunks; c += 32) smem_weights[g * kFusedMaxChunks + c] *= inv;
-  }
+  for (int g = warp; g < g_count; g += kWarps) merge_weigh_head(stats, chunk_capacity, active_chunks, smem_weights, g, lane);
   __syncthreads();
-  auto store = [&](int g, int d, const float4& o) {
-    const float acc[4] = {o.x, o.y, o.z, o.w};
-    const T* gate = fc.gate == nullptr ? nullptr
-                                       : reinterpret_cast<const T*>(fc.gate) + (int64_t)b * fc.gate_stride_b +
-                                             (int64_t)(hq0 + g) * fc.gate_stride_h + d;
-    const int64_t offset = (int64_t)b * fc.out_stride_b + (int64_t)(hq0 + g) * fc.out_stride_h + d;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const T result = ElemTraits<T>::from_float(gate ? acc[i] * sigmoidf_fast(ElemTraits<T>::to_float(gate[i])) : acc[i]);
-      reinterpret_cast<T*>(fc.out)[offset + i] = result;
-      for (int peer = 0; peer < fc.num_peers; ++peer) reinterpret_cast<T*>(fc.peers[peer])[offset + i] = result;
-    }
-  };
+  auto store = [&](int g, int d, const float4& o) { merge_store4<T>(fc, b, hq0 + g, d, o); };
   // Four dims per thread and load.  What this part takes is the latency of its loads: a head group with more columns of four
   // dims than the CTA has threads reads all of a thread's columns side by side, kInFlight loads at a time, instead of one
   // column after the other (16 rows of 0.4-4 K packed tokens, 16/2 heads of 256: 37.1 -> 34.9 us; 64 rows of 4-32 K 170 ->
@@ -96,12 +142,6 @@ __device__ __forceinline__ void fused_combine_tail(const FusedCombine& fc, int b
   constexpr int kRounds = (HEADS * kCols + THREADS - 1) / THREADS;
   constexpr int kInFlight = 8;
   const int items = g_count * kCols;
-  auto add = [](float4& acc, const float4& v, float w) {
-    acc.x = fmaf(v.x, w, acc.x);
-    acc.y = fmaf(v.y, w, acc.y);
-    acc.z = fmaf(v.z, w, acc.z);
-    acc.w = fmaf(v.w, w, acc.w);
-  };
   auto side_by_side = [&](auto columns) {
     constexpr int kColumns = decltype(columns)::value;  // of a thread
     constexpr int kAtOnce = kInFlight / kColumns;       // partials
@@ -125,7 +165,7 @@ __device__ __forceinline__ void fused_combine_tail(const FusedCombine& fc, int b
         const float* w = smem_weights + min(((int)threadIdx.x + r * THREADS) / kCols, g_count - 1) * kFusedMaxChunks;
 #pragma unroll
         for (int k = 0; k < kAtOnce; ++k)
-          if (c0 + k < active_chunks) add(acc[r], v[k][r], w[c0 + k]);
+          if (c0 + k < active_chunks) merge_add(acc[r], v[k][r], w[c0 + k]);
       }
     }
 #pragma unroll
@@ -150,7 +190,7 @@ __device__ __forceinline__ void fused_combine_tail(const FusedCombine& fc, int b
       float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll 4
       for (int c = 0; c < active_chunks; ++c)
-        add(acc, __ldcg(reinterpret_cast<const float4*>(vals + (int64_t)c * D)), w[c]);
+        merge_add(acc, __ldcg(reinterpret_cast<const float4*>(vals + (int64_t)c * D)), w[c]);
       store(g, d, acc);
     };
     // a loop also where no thread has a second column: the compiler makes the better code of it at head_dim 256 (16 packed rows of 201
@@ -161,25 +201,7 @@ __device__ __forceinline__ void fused_combine_tail(const FusedCombine& fc, int b
       if ((int)threadIdx.x < items) column(threadIdx.x);
     }
   }
-  for (int item = threadIdx.x; !aligned && item < g_count * D; item += THREADS) {
-    const int g = item / D;
-    const int d = item % D;
-    const float* vals = values + (int64_t)g * chunk_capacity * D + d;
-    const float* w = smem_weights + g * kFusedMaxChunks;
-    float acc = 0.0f;
-    for (int c = 0; c < active_chunks; ++c) acc = fmaf(__ldcg(vals + (int64_t)c * D), w[c], acc);
-    if (fc.gate) {
-      const T* gate = reinterpret_cast<const T*>(fc.gate) + (int64_t)b * fc.gate_stride_b +
-                      (int64_t)(hq0 + g) * fc.gate_stride_h;
-      acc *= sigmoidf_fast(ElemTraits<T>::to_float(gate[d]));
-    }
-    const int64_t offset = (int64_t)b * fc.out_stride_b + (int64_t)(hq0 + g) * fc.out_stride_h + d;
-    const T result = ElemTraits<T>::from_float(acc);
-    reinterpret_cast<T*>(fc.out)[offset] = result;
-    for (int peer = 0; peer < fc.num_peers; ++peer) reinterpret_cast<T*>(fc.peers[peer])[offset] = result;
-  }
-  // stores to other GPUs are ordered before whatever this stream signals to them after the kernel
-  if (fc.num_peers > 0) __threadfence_system();
+  merge_finish<T, D, THREADS>(fc, b, hq0, g_count, active_chunks, chunk_capacity, values, smem_weights, aligned);
 }
 
 // The same with the first values read beside the statistics, and these once.  The merge is a chain of reads from L2 (counter,
@@ -192,19 +214,7 @@ __device__ __forceinline__ void fused_combine_ahead(const FusedCombine& fc, int 
                                                     int active_chunks, int chunk_capacity, const float* stats,
                                                    const float* values, float* smem_weights /* [8][kFusedMaxChunks] */,
                                                    int64_t counter_index, int arrivals = 0) {
-  __shared__ int s_is_last;
-  __syncthreads();  // all partial stores of this CTA are ordered before the arrival below
-  if (threadIdx.x == 0) {
-    // releases this CTA's partial and acquires those of the CTAs counted before; the barriers on both sides extend that to
-    // the other threads (4 un-quantized rows of 60-900 tokens: 10.8 us with a full fence on either side, 10.3 so)
-    int32_t* counter = fc.counters + counter_index;
-    int prev;
-    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;\n" : "=r"(prev) : "l"(counter) : "memory");
-    s_is_last = (prev == (arrivals > 0 ? arrivals : active_chunks) - 1) ? 1 : 0;
-    if (s_is_last) *counter = 0;
-  }
-  __syncthreads();
-  if (!s_is_last) return;
+  if (!merge_arrive(fc, counter_index, arrivals > 0 ? arrivals : active_chunks)) return;
 
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -251,51 +261,16 @@ __device__ __forceinline__ void fused_combine_ahead(const FusedCombine& fc, int 
         }
       }
     } else {
-      for (int g = warp; g < g_count; g += kWarps) {
-        const float* st = stats + (int64_t)g * chunk_capacity * 2;
-        float m = -INFINITY;
-        for (int c = lane; c < active_chunks; c += 32) m = fmaxf(m, __ldcg(st + 2 * c));
-#pragma unroll
-        for (int d = 16; d >= 1; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
-        const float m_ref = m == -INFINITY ? 0.0f : m;
-        float den = 0.0f;
-        for (int c = lane; c < active_chunks; c += 32) {
-          const float w = __expf(__ldcg(st + 2 * c) - m_ref);
-          den += __ldcg(st + 2 * c + 1) * w;
-          smem_weights[g * kFusedMaxChunks + c] = w;
-        }
-#pragma unroll
-        for (int d = 16; d >= 1; d >>= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
-        const float inv = den > 0.0f ? 1.0f / den : 0.0f;
-        for (int c = lane; c < active_chunks; c += 32) smem_weights[g * kFusedMaxChunks + c] *= inv;
-      }
+      for (int g = warp; g < g_count; g += kWarps) merge_weigh_head(stats, chunk_capacity, active_chunks, smem_weights, g, lane);
     }
     __syncthreads();
   };
-  auto store = [&](int g, int d, const float4& o) {
-    const float acc[4] = {o.x, o.y, o.z, o.w};
-    const T* gate = fc.gate == nullptr ? nullptr
-                                       : reinterpret_cast<const T*>(fc.gate) + (int64_t)b * fc.gate_stride_b +
-                                             (int64_t)(hq0 + g) * fc.gate_stride_h + d;
-    const int64_t offset = (int64_t)b * fc.out_stride_b + (int64_t)(hq0 + g) * fc.out_stride_h + d;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const T result = ElemTraits<T>::from_float(gate ? acc[i] * sigmoidf_fast(ElemTraits<T>::to_float(gate[i])) : acc[i]);
-      reinterpret_cast<T*>(fc.out)[offset + i] = result;
-      for (int peer = 0; peer < fc.num_peers; ++peer) reinterpret_cast<T*>(fc.peers[peer])[offset + i] = result;
-    }
-  };
+  auto store = [&](int g, int d, const float4& o) { merge_store4<T>(fc, b, hq0 + g, d, o); };
   const bool aligned = (reinterpret_cast<uintptr_t>(values) & 15u) == 0;
   constexpr int kCols = D / 4;
   constexpr int kRounds = (HEADS * kCols + THREADS - 1) / THREADS;
   constexpr int kInFlight = 8, kAhead = 4;
   const int items = g_count * kCols;
-  auto add = [](float4& acc, const float4& v, float w) {
-    acc.x = fmaf(v.x, w, acc.x);
-    acc.y = fmaf(v.y, w, acc.y);
-    acc.z = fmaf(v.z, w, acc.z);
-    acc.w = fmaf(v.w, w, acc.w);
-  };
   auto side_by_side = [&](auto columns) {
     constexpr int kColumns = decltype(columns)::value;  // of a thread
     constexpr int kAtOnce = kInFlight / kColumns;       // partials
@@ -323,7 +298,7 @@ __device__ __forceinline__ void fused_combine_ahead(const FusedCombine& fc, int 
         const float* w = smem_weights + min(((int)threadIdx.x + r * THREADS) / kCols, g_count - 1) * kFusedMaxChunks;
 #pragma unroll
         for (int k = 0; k < kAtOnce; ++k)
-          if (c0 + k < active_chunks) add(acc[r], v[k][r], w[c0 + k]);
+          if (c0 + k < active_chunks) merge_add(acc[r], v[k][r], w[c0 + k]);
       }
       c0 += kAtOnce;
       if (c0 >= active_chunks) break;
@@ -359,35 +334,17 @@ __device__ __forceinline__ void fused_combine_ahead(const FusedCombine& fc, int 
       if (item < THREADS) {
 #pragma unroll
         for (int k = 0; k < kAhead; ++k)
-          if (k < active_chunks) add(acc, first[k], w[k]);
+          if (k < active_chunks) merge_add(acc, first[k], w[k]);
         c = kAhead;
       }
 #pragma unroll 4
-      for (; c < active_chunks; ++c) add(acc, __ldcg(reinterpret_cast<const float4*>(vals + (int64_t)c * D)), w[c]);
+      for (; c < active_chunks; ++c) merge_add(acc, __ldcg(reinterpret_cast<const float4*>(vals + (int64_t)c * D)), w[c]);
       store(g, d, acc);
     }
   } else {
     weigh();
   }
-  for (int item = threadIdx.x; !aligned && item < g_count * D; item += THREADS) {
-    const int g = item / D;
-    const int d = item % D;
-    const float* vals = values + (int64_t)g * chunk_capacity * D + d;
-    const float* w = smem_weights + g * kFusedMaxChunks;
-    float acc = 0.0f;
-    for (int c = 0; c < active_chunks; ++c) acc = fmaf(__ldcg(vals + (int64_t)c * D), w[c], acc);
-    if (fc.gate) {
-      const T* gate = reinterpret_cast<const T*>(fc.gate) + (int64_t)b * fc.gate_stride_b +
-                      (int64_t)(hq0 + g) * fc.gate_stride_h;
-      acc *= sigmoidf_fast(ElemTraits<T>::to_float(gate[d]));
-    }
-    const int64_t offset = (int64_t)b * fc.out_stride_b + (int64_t)(hq0 + g) * fc.out_stride_h + d;
-    const T result = ElemTraits<T>::from_float(acc);
-    reinterpret_cast<T*>(fc.out)[offset] = result;
-    for (int peer = 0; peer < fc.num_peers; ++peer) reinterpret_cast<T*>(fc.peers[peer])[offset] = result;
-  }
-  // stores to other GPUs are ordered before whatever this stream signals to them after the kernel
-  if (fc.num_peers > 0) __threadfence_system();
+  merge_finish<T, D, THREADS>(fc, b, hq0, g_count, active_chunks, chunk_capacity, values, smem_weights, aligned);
 }
 
 // A row with no visible key has no contributing CTA; the CTA of chunk 0 writes its zeros.
