@@ -606,8 +606,8 @@ constexpr int kMergeHeads = kPair && D == 256 ? 4 : 8;
 // over 160-170 shapes per instance (1 to 128 rows of 30 tokens to 32 K, 1 to 12 query heads per KV head).
 template <int D, int BITS, bool kPair>
 struct TqSmallOrder {
-  // AHEAD alone and both.  Head_dim 128, 4 bits: pairs 0.945 and 0.942 (one row of 4000 tokens, 32/8 heads, 11.6 us and 12.1, neither
-  // 12.0), eight heads 0.896 and 0.913; 2 bits: pairs 0.946 and 0.951, eight heads 0.907 and 0.906; 3 bits: 0.945 and 0.927, 0.924 and
+  // AHEAD alone and both.  Head_dim 128, 4 bits: pairs 0.945 and 0.942 (one row of 4000 tokens, 32/8 heads, 11.5 us and 11.7, neither
+  // 11.8), eight heads 0.896 and 0.913; 2 bits: pairs 0.946 and 0.951, eight heads 0.907 and 0.906; 3 bits: 0.945 and 0.927, 0.924 and
   // 0.926.  Head_dim 256, by bits: pairs 1.007, 1.020, 0.967 and 0.993, 0.995, 0.971 (four heads in 2 and 3 bits 1.004 and 1.014 with
   // both; neither there was no faster than that over other shapes), eight heads 0.963, 0.973, 0.976 and 0.967, 0.954, 0.980.
   static constexpr bool kEarly = D == 256 || BITS == 3 || (BITS == 2 && !kPair);
